@@ -88,7 +88,8 @@ template <int BN, int STAGES, bool A_MN, bool B_MN, int SBN = BN>
 MACO_DEVICE bool gemm_produce_tile(uint8_t* smem, const GemmCtrl& c, const CUtensorMap* tmA,
                                    const CUtensorMap* tmB, int m0, int n0, int k0, int k_blocks,
                                    uint32_t& it, uint64_t budget_ns, long long* prof = nullptr, int k_step = kBK,
-                                   int b_blocked_row0 = -1) {
+                                   int b_blocked_row0 = -1, uint32_t b_ahead = 0) {
+  // b_ahead: the first b_ahead k-blocks have their stage armed and B on its way already (gemm_produce_b_ahead)
   // b_blocked_row0 >= 0: B is stored tile by tile ([N / BN][K / 64][BN][64], see ops.block_weight) and its tensor map
   // is the 2-D view [rows, 64]; k-block kb of this tile is the contiguous BN x 64 block at row b_blocked_row0 + kb * BN.
   // (A K-major [N, K] weight read once from HBM comes in as BN separate 128-byte pieces per box, one per DRAM
@@ -102,10 +103,13 @@ MACO_DEVICE bool gemm_produce_tile(uint8_t* smem, const GemmCtrl& c, const CUten
   int k = k0;
   for (int kb = 0; kb < k_blocks; ++kb, k += k_step) {
     const long long t0 = prof ? clock64() : 0;
-    if (!mbar_wait(&c.empty[s], ph ^ 1, budget_ns, c.abort_word)) { it += kb; return false; }
+    const bool b_done = (uint32_t)kb < b_ahead;
+    if (!b_done) {
+      if (!mbar_wait(&c.empty[s], ph ^ 1, budget_ns, c.abort_word)) { it += kb; return false; }
+      mbar_arrive_expect_tx(&c.full[s], L::kLoadBytes);
+    }
     if (prof) prof[0] += clock64() - t0;
     uint8_t* sb = sa + L::kABytes;
-    mbar_arrive_expect_tx(&c.full[s], L::kLoadBytes);
     if constexpr (!A_MN) {
       tma_load_2d(sa, tmA, &c.full[s], k, m0);
     } else {
@@ -113,7 +117,8 @@ MACO_DEVICE bool gemm_produce_tile(uint8_t* smem, const GemmCtrl& c, const CUten
       for (int j = 0; j < kBM / 64; ++j) tma_load_2d(sa + j * 8192, tmA, &c.full[s], m0 + j * 64, k);
     }
     if constexpr (!B_MN) {
-      if (b_blocked_row0 >= 0) tma_load_2d(sb, tmB, &c.full[s], 0, b_blocked_row0 + kb * BN);
+      if (b_done) {}
+      else if (b_blocked_row0 >= 0) tma_load_2d(sb, tmB, &c.full[s], 0, b_blocked_row0 + kb * BN);
       else tma_load_2d(sb, tmB, &c.full[s], k, n0);
     } else {
 #pragma unroll
@@ -122,6 +127,24 @@ MACO_DEVICE bool gemm_produce_tile(uint8_t* smem, const GemmCtrl& c, const CUten
     if (++s == STAGES) { s = 0; ph ^= 1; sa = smem; } else { sa += L::kStageBytes; }
   }
   it += k_blocks;
+  return true;
+}
+
+// The B half of a tile's first k-blocks (K-major B), ahead of everything the tile waits for: arms each stage for both
+// operands and loads B; gemm_produce_tile then brings in A. At most STAGES k-blocks; `ahead` counts them.
+template <int BN, int STAGES, int SBN = BN>
+MACO_DEVICE bool gemm_produce_b_ahead(uint8_t* smem, const GemmCtrl& c, const CUtensorMap* tmB, int n0, int k0, int k_blocks,
+                                      uint32_t it, uint64_t budget_ns, int b_blocked_row0, uint32_t& ahead) {
+  using L = GemmSmemLayout<BN, STAGES, SBN>;
+  const uint32_t most = k_blocks < STAGES ? (uint32_t)k_blocks : (uint32_t)STAGES;
+  for (ahead = 0; ahead < most; ++ahead) {
+    const uint32_t u = it + ahead, s = u % STAGES, ph = (u / STAGES) & 1;
+    if (!mbar_wait(&c.empty[s], ph ^ 1, budget_ns, c.abort_word)) return false;
+    mbar_arrive_expect_tx(&c.full[s], L::kLoadBytes);
+    uint8_t* sb = smem + s * L::kStageBytes + L::kABytes;
+    if (b_blocked_row0 >= 0) tma_load_2d(sb, tmB, &c.full[s], 0, b_blocked_row0 + (int)ahead * BN);
+    else tma_load_2d(sb, tmB, &c.full[s], k0 + (int)ahead * kBK, n0);
+  }
   return true;
 }
 

@@ -28,6 +28,7 @@
 //    {status, task, event, cta} in the host-mapped status block, raises the launch-wide abort
 //    word, and all CTAs drain and return.
 #include "elementwise.cuh"
+#include "row_tasks.cuh"
 #include "gemm_tcgen05.cuh"
 #include "comm_tasks.cuh"
 #include "attention_decode.cuh"
@@ -42,10 +43,15 @@ namespace {
 constexpr int kMkBN = 256;
 constexpr int kMkStages = 4;
 using MkLayout = GemmSmemLayout<kMkBN, kMkStages>;
-constexpr int kMkExtraSmem = 1024;     // scheduler heads / current-task slots live after the GEMM control block
+constexpr int kMkExtraSmem = 3072;     // scheduler heads / current-task slots, then the three roles' descriptor slots
+constexpr int kStreamOffset = 1024;    // byte offset of the descriptor slots inside that block
+constexpr uint32_t kStreamSlots = 4;   // descriptors per role: the current one, up to kStreamAhead on their way
+constexpr uint32_t kStreamAhead = 3;
 constexpr int kMkScratchSmem = 28672;  // scratch of non-GEMM tasks (the operand ring is NOT free for them:
                                        // the producer warp may already be filling it for the next GEMM task)
 constexpr int kMkSmemBytes = MkLayout::kTotalBytes + kMkExtraSmem + kMkScratchSmem;
+static_assert(kStreamOffset + 3 * kStreamSlots * sizeof(MacoTaskDesc) <= kMkExtraSmem, "descriptor slots");
+static_assert(kMkScratchSmem >= (int)kRowScratch, "staged row tasks must fit the scratch block");
 static_assert(kMkScratchSmem >= kEpiStageBytes, "epilogue staging must fit the scratch block");
 static_assert(kMkScratchSmem >= kAttnScratchBytes && kMkScratchSmem >= kAttnTcScratchBytes, "attention scratch must fit the scratch block");
 static_assert(kMkSmemBytes <= 227 * 1024, "persistent kernel exceeds the shared memory of an SM");
@@ -81,58 +87,43 @@ __device__ void report_failure(const MacoProgram& p, uint32_t status, uint32_t t
   }
 }
 
-// Bounded wait until *flag >= expect (wrap-safe). Leaves early when the launch was aborted.
+// Bounded wait until *flag >= expect (wrap-safe). Leaves early when the launch was aborted. The polls are relaxed (an
+// acquire at gpu scope empties the SM's L1, which the other warps' tasks are using); the value that ends the
+// wait is read once more with acquire semantics.
 __device__ bool mk_wait(const MacoProgram& p, const uint32_t* flag, uint32_t expect, bool sys) {
   uint32_t v = sys ? ld_acquire_sys_u32(flag) : ld_acquire_gpu_u32(flag);
   if ((int32_t)(v - expect) >= 0) return true;
   const uint64_t t0 = globaltimer_ns();
   uint32_t spins = 0;
   while (true) {
-    v = sys ? ld_acquire_sys_u32(flag) : ld_acquire_gpu_u32(flag);
-    if ((int32_t)(v - expect) >= 0) return true;
+    v = sys ? ld_relaxed_sys_u32(flag) : ld_relaxed_gpu_u32(flag);
+    if ((int32_t)(v - expect) >= 0) {
+      if (sys) (void)ld_acquire_sys_u32(flag); else (void)ld_acquire_gpu_u32(flag);
+      return true;
+    }
     if ((++spins & 31u) == 0) {
       if (aborted(p)) return false;
       if (globaltimer_ns() - t0 > p.budget_ns) return false;
     }
-    __nanosleep(32);
+    __nanosleep(20);
   }
 }
 
+// Both conditions of a task. Counters are read with acquire loads (at .sys scope for those other GPUs bump), never
+// with a full fence: a fence at system scope also waits for this GPU's outstanding writes to peers and to the host
+// and takes tens of microseconds while a host -> device copy is in flight. A condition with count 0 always holds (a
+// block that is already in place) and is not read at all.
 __device__ bool wait_deps(const MacoProgram& p, const MacoTaskDesc& d, uint32_t task, volatile uint32_t* cta_abort,
                           uint64_t* wait_ns) {
   const uint64_t t0 = wait_ns ? globaltimer_ns() : 0;
-  {
-    // Common case, every condition already holds. Counters bumped by this GPU only are read together with
-    // relaxed loads and ordered by ONE .gpu fence. Counters bumped by other GPUs are read with an acquire load
-    // at .sys scope instead of a relaxed load plus fence.acq_rel.sys: the full fence at system scope also waits
-    // for this GPU's outstanding writes to peers and to the host, and takes tens of microseconds while a
-    // host -> device copy is in flight (measured: +300 us per step of the tensor-parallel layer).
-    // A condition with count 0 always holds (a block that is already in place) and is not read at all.
-    bool sat = true, any_gpu = false;
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const int e = d.wait_event[j];
-      if (e < 0 || d.wait_count[j] == 0) continue;
-      const bool sys = (d.flags & (j == 0 ? MACO_TF_WAIT0_SYS : MACO_TF_WAIT1_SYS)) != 0;
-      const bool prev = (d.flags & (j == 0 ? MACO_TF_WAIT0_PREV : MACO_TF_WAIT1_PREV)) != 0;
-      const uint32_t need = (p.epoch - (prev ? 1u : 0u)) * d.wait_count[j];
-      const uint32_t v = sys ? ld_acquire_sys_u32(&p.events[e]) : ld_relaxed_gpu_u32(&p.events[e]);
-      any_gpu |= !sys;
-      if ((int32_t)(v - need) < 0) sat = false;
-    }
-    if (sat) {
-      if (any_gpu) fence_acq_rel_gpu();
-      if (wait_ns) *wait_ns += globaltimer_ns() - t0;
-      return true;
-    }
-  }
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int e = d.wait_event[j];
-    if (e < 0 || d.wait_count[j] == 0) continue;
+    const uint32_t count = d.wait_count[j];
+    if (e < 0 || count == 0) continue;
     const bool sys = (d.flags & (j == 0 ? MACO_TF_WAIT0_SYS : MACO_TF_WAIT1_SYS)) != 0;
     const bool prev = (d.flags & (j == 0 ? MACO_TF_WAIT0_PREV : MACO_TF_WAIT1_PREV)) != 0;
-    if (!mk_wait(p, &p.events[e], (p.epoch - (prev ? 1u : 0u)) * d.wait_count[j], sys)) {
+    if (!mk_wait(p, &p.events[e], (p.epoch - (prev ? 1u : 0u)) * count, sys)) {
       report_failure(p, sys ? MACO_STATUS_PEER_TIMEOUT : MACO_STATUS_TIMEOUT, task, (uint32_t)e, cta_abort);
       return false;
     }
@@ -197,56 +188,79 @@ __device__ bool desc_ok(const MacoProgram& p, const MacoTaskDesc& d) {
   return true;
 }
 
-// Next entry of this worker's queue. false = aborted / timed out.
-__device__ bool fetch_task(const MacoProgram& p, uint32_t w, uint32_t i, uint32_t q_base, uint32_t& task,
-                           volatile uint32_t* cta_abort) {
-  if (p.mode == MACO_MODE_STATIC) {
-    const uint32_t n = p.static_count[w];
-    const uint32_t* q = p.static_queue + (size_t)w * p.static_stride;
-    task = i < n ? q[i] : MACO_QUEUE_TERMINATE;
-    if (i + 1 < n) {
-      // the next descriptor is on its way while this task runs (the three roles share the L1 line)
-      const MacoTaskDesc* nd = p.tasks + (q[i + 1] & MACO_QUEUE_INDEX_MASK);
-      asm volatile("prefetch.global.L1 [%0];" :: "l"(nd));
-    }
-    return true;
-  }
-  const uint32_t pos = q_base + i;
-  if (!mk_wait(p, &p.heads[w], pos + 1, false)) {
-    report_failure(p, MACO_STATUS_TIMEOUT, 0xfffffffeu, w, cta_abort);
-    return false;
-  }
-  task = ld_relaxed_gpu_u32(&p.ring[(size_t)w * MACO_WORKER_QUEUE_SIZE + (pos & (MACO_WORKER_QUEUE_SIZE - 1))]);
-  return true;
-}
+// One role's view of its worker's task sequence. Static queues: the worker's descriptors lie next to one another in
+// `tasks`, and the role's leading thread copies them into shared memory three tasks ahead (cp.async), so that a task
+// starts with its descriptor one shared-memory read away instead of two or three dependent L2 round trips. Dynamic mode:
+// the task index comes from the worker's ring and the descriptor is copied on arrival. Only the leading thread calls
+// next(); other threads of the role may read the slot behind a barrier of theirs and until their next one.
+struct TaskStream {
+  MacoTaskDesc* slots;       // [kStreamSlots] in shared memory
+  uint32_t w, begin, n, i;   // worker, first task, tasks (static mode), next position
 
-__device__ __forceinline__ bool is_gemm(uint32_t type) { return type == MACO_TASK_MATMUL || type == MACO_TASK_LINEAR; }
-
-__device__ __forceinline__ MacoTaskDesc load_desc(const MacoProgram& p, uint32_t task) {
-  MacoTaskDesc d;
-  const uint4* src = reinterpret_cast<const uint4*>(p.tasks + task);
-  uint4* dst = reinterpret_cast<uint4*>(&d);
+  __device__ __forceinline__ void prefetch(const MacoProgram& p, uint32_t k) const {
+    if (k < n) {
+      const uint8_t* src = reinterpret_cast<const uint8_t*>(p.tasks + begin + k);
+      const uint32_t dst = smem_u32(slots + (k & (kStreamSlots - 1)));
 #pragma unroll
-  for (int i = 0; i < 8; ++i) dst[i] = src[i];
-  return d;
-}
+      for (int j = 0; j < (int)(sizeof(MacoTaskDesc) / 16); ++j) cp_async16(dst + j * 16, src + j * 16);
+    }
+    cp_async_commit();
+  }
+  __device__ __forceinline__ void start(const MacoProgram& p, MacoTaskDesc* s, uint32_t worker, uint32_t q_base) {
+    slots = s; w = worker; i = 0; begin = 0; n = 0;
+    if (p.mode == MACO_MODE_STATIC) {
+      begin = p.queue_begin[worker];
+      n = p.queue_begin[worker + 1] - begin;
+      for (uint32_t k = 0; k < kStreamAhead; ++k) prefetch(p, k);
+    } else {
+      begin = q_base;
+    }
+  }
+  // The next task and its index; null at the end of the queue, or (failed set) after an abort.
+  __device__ __forceinline__ const MacoTaskDesc* next(const MacoProgram& p, uint32_t& task, bool& failed, volatile uint32_t* cta_abort) {
+    MacoTaskDesc* slot = slots + (i & (kStreamSlots - 1));
+    if (p.mode == MACO_MODE_STATIC) {
+      if (i >= n) return nullptr;
+      cp_async_wait<kStreamAhead - 1>();
+      prefetch(p, i + kStreamAhead);                    // into the slot of task i - 1
+      task = begin + i;
+    } else {
+      const uint32_t pos = begin + i;
+      if (!mk_wait(p, &p.heads[w], pos + 1, false)) {
+        report_failure(p, MACO_STATUS_TIMEOUT, 0xfffffffeu, w, cta_abort);
+        failed = true;
+        return nullptr;
+      }
+      task = ld_relaxed_gpu_u32(&p.ring[(size_t)w * MACO_WORKER_QUEUE_SIZE + (pos & (MACO_WORKER_QUEUE_SIZE - 1))]);
+      if (task == MACO_QUEUE_TERMINATE) return nullptr;
+      const uint4* src = reinterpret_cast<const uint4*>(p.tasks + task);
+#pragma unroll
+      for (int j = 0; j < (int)(sizeof(MacoTaskDesc) / 16); ++j) reinterpret_cast<uint4*>(slot)[j] = src[j];
+    }
+    ++i;
+    return slot;
+  }
+};
 
 // ---- producer warp (lane 0), two-CTA programs ----------------------------------------------------
 // Every GEMM task of such a program is one half (128 rows) of a 256 x BN tile; the two halves sit at the same
 // position of the GEMM sequences of workers 2j and 2j+1 (one cluster). Each CTA waits for ITS half's
 // conditions and loads its rows of A and its half of B; the leader's MMA warp starts when both have landed.
-__device__ void producer_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_base, uint8_t* smem, const GemmCtrl& c) {
+__device__ void producer_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_base, uint8_t* smem, const GemmCtrl& c,
+                                   MacoTaskDesc* desc_slots) {
+  TaskStream ts;
+  ts.start(p, desc_slots, w, q_base);
   uint32_t it = 0;
   bool ok = true;
   const uint32_t rank = cluster_ctarank();
   const CUtensorMap* tmaps = reinterpret_cast<const CUtensorMap*>(p.tmaps);
-  for (uint32_t i = 0; ok; ++i) {
+  while (ok) {
     uint32_t task;
-    if (!fetch_task(p, w, i, q_base, task, c.abort_word)) { ok = false; break; }
-    if (task == MACO_QUEUE_TERMINATE) break;
-    task &= MACO_QUEUE_INDEX_MASK;
-    const MacoTaskDesc& d = p.tasks[task];
-    if (!is_gemm(d.type)) continue;
+    bool failed = false;
+    const MacoTaskDesc* dp = ts.next(p, task, failed, c.abort_word);
+    if (dp == nullptr) { ok = !failed; break; }
+    const MacoTaskDesc& d = *dp;
+    if (!is_gemm_type(d.type)) continue;
     if (p.debug != 0 && !desc_ok(p, d)) { report_failure(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word); ok = false; break; }
     if (!wait_deps(p, d, task, c.abort_word, nullptr)) { ok = false; break; }
     const MacoGemmArgs& g = d.u.gemm;
@@ -276,16 +290,18 @@ __device__ void producer_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_
 
 // ---- MMA warp (lane 0) of the pair's leader ------------------------------------------------------
 __device__ void mma_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_base, uint8_t* smem, const GemmCtrl& c,
-                              uint32_t tmem_base) {
+                              uint32_t tmem_base, MacoTaskDesc* desc_slots) {
+  TaskStream ts;
+  ts.start(p, desc_slots, w, q_base);
   uint32_t it = 0, seq = 0;
   bool ok = true;
-  for (uint32_t i = 0; ok; ++i) {
+  while (ok) {
     uint32_t task;
-    if (!fetch_task(p, w, i, q_base, task, c.abort_word)) break;
-    if (task == MACO_QUEUE_TERMINATE) break;
-    task &= MACO_QUEUE_INDEX_MASK;
-    const MacoTaskDesc& d = p.tasks[task];
-    if (!is_gemm(d.type)) continue;
+    bool failed = false;
+    const MacoTaskDesc* dp = ts.next(p, task, failed, c.abort_word);
+    if (dp == nullptr) break;
+    const MacoTaskDesc& d = *dp;
+    if (!is_gemm_type(d.type)) continue;
     const MacoGemmArgs& g = d.u.gemm;
     const int sel = (g.bn == 128 ? 4 : 0) | (g.a_mn ? 2 : 0) | ((g.b_mn & 1) ? 1 : 0);
     switch (sel) {
@@ -312,27 +328,45 @@ __device__ void mma_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_base,
 __device__ int producer_gemm_task(const MacoProgram& p, const MacoTaskDesc& d, uint32_t task, uint8_t* smem, const GemmCtrl& c,
                                   const CUtensorMap* tmaps, const AttnPipe& apipe, uint32_t ait, uint32_t& it, int& owner) {
   if (p.debug != 0 && !desc_ok(p, d)) { report_failure(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word); return 0; }
-  if (!wait_deps(p, d, task, c.abort_word, nullptr)) return 0;
   const MacoGemmArgs& g = d.u.gemm;
-  // run-time guarded tile: every role reads the same (final) count after the task's conditions hold
-  if ((d.flags & MACO_TF_COUNTED) && ld_relaxed_gpu_u32(g.count_ptr) <= g.count_base) return 1;
-  fence_proxy_async_all();           // operands were written by generic-proxy stores of other CTAs
-  if (owner == 2 && !attn_ring_drained(apipe, ait)) return 0;
-  owner = 1;
   const CUtensorMap* ta = tmaps + g.tmap_a;
   const CUtensorMap* tb = tmaps + g.tmap_b;
   const int sel = (g.bn == 128 ? 4 : 0) | (g.a_mn ? 2 : 0) | ((g.b_mn & 1) ? 1 : 0);
+  if (d.flags & MACO_TF_COUNTED) {
+    if (!wait_deps(p, d, task, c.abort_word, nullptr)) return 0;
+    // run-time guarded tile: every role reads the same (final) count after the task's conditions hold
+    if (ld_relaxed_gpu_u32(g.count_ptr) <= g.count_base) return 1;
+  }
+  if (owner == 2 && !attn_ring_drained(apipe, ait)) return 0;
+  owner = 1;
+  // B of a weight is on its way before the tile's conditions hold: a decode step is a chain of dependent
+  // weight-streaming phases, and this keeps up to a full ring (128 KB per SM) of the next phase's weights in
+  // flight while the last one drains.
+  uint32_t ahead = 0;
+  if ((d.flags & (MACO_TF_B_STATIC | MACO_TF_COUNTED)) == MACO_TF_B_STATIC && (sel & 1) == 0) {
+    const int b_row = (g.b_mn & 2) ? (int)(((uint32_t)g.n0 / 256u * g.count_base + (uint32_t)g.k0 / (uint32_t)kBK) * 256u) : -1;
+    const bool ok_b = g.bn == 256
+        ? gemm_produce_b_ahead<256, kMkStages, kMkBN>(smem, c, tb, g.n0, g.k0, g.k_blocks, it, p.budget_ns, b_row, ahead)
+        : gemm_produce_b_ahead<128, kMkStages, kMkBN>(smem, c, tb, g.n0, g.k0, g.k_blocks, it, p.budget_ns, b_row, ahead);
+    if (!ok_b) {
+      it += ahead;
+      report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
+      return 0;
+    }
+  }
+  if (!(d.flags & MACO_TF_COUNTED) && !wait_deps(p, d, task, c.abort_word, nullptr)) { it += ahead; return 0; }
+  fence_proxy_async_all();           // operands were written by generic-proxy stores of other CTAs
   bool ok;
   // b_mn bit 1: blocked B (256-column tiles only); count_base then holds the weight's total number of k-blocks
   const int b_row0 = (g.b_mn & 2) ? (int)(((uint32_t)g.n0 / 256u * g.count_base + (uint32_t)g.k0 / (uint32_t)kBK) * 256u) : -1;
   switch (sel) {
-    case 0: ok = gemm_produce_tile<256, kMkStages, false, false, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns, nullptr, kBK, b_row0); break;
+    case 0: ok = gemm_produce_tile<256, kMkStages, false, false, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns, nullptr, kBK, b_row0, ahead); break;
     case 1: ok = gemm_produce_tile<256, kMkStages, false, true, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
-    case 2: ok = gemm_produce_tile<256, kMkStages, true, false, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
+    case 2: ok = gemm_produce_tile<256, kMkStages, true, false, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns, nullptr, kBK, -1, ahead); break;
     case 3: ok = gemm_produce_tile<256, kMkStages, true, true, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
-    case 4: ok = gemm_produce_tile<128, kMkStages, false, false, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
+    case 4: ok = gemm_produce_tile<128, kMkStages, false, false, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns, nullptr, kBK, -1, ahead); break;
     case 5: ok = gemm_produce_tile<128, kMkStages, false, true, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
-    case 6: ok = gemm_produce_tile<128, kMkStages, true, false, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
+    case 6: ok = gemm_produce_tile<128, kMkStages, true, false, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns, nullptr, kBK, -1, ahead); break;
     default: ok = gemm_produce_tile<128, kMkStages, true, true, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
   }
   if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
@@ -340,8 +374,10 @@ __device__ int producer_gemm_task(const MacoProgram& p, const MacoTaskDesc& d, u
 }
 
 __device__ void producer_role(const MacoProgram& p, uint32_t w, uint32_t q_base, uint8_t* smem, const GemmCtrl& c,
-                              uint64_t* attn_ring_bars) {
+                              uint64_t* attn_ring_bars, MacoTaskDesc* desc_slots) {
   const uint32_t lane = threadIdx.x & 31;
+  TaskStream ts;
+  if (lane == 0) ts.start(p, desc_slots, w, q_base);
   uint32_t it = 0;                   // stage uses of the GEMM ring (lane 0)
   uint32_t ait = 0;                  // stage uses of the attention ring (same memory); every lane keeps the same count
   int owner = 0;                     // lane 0: which pipeline used the operand memory last: 1 GEMM, 2 attention
@@ -352,15 +388,13 @@ __device__ void producer_role(const MacoProgram& p, uint32_t w, uint32_t q_base,
   for (uint32_t i = 0; ok; ++i) {
     uint32_t task = 0, verdict = 0;  // 0 run, 1 end of queue, 2 failure
     if (lane == 0) {
-      if (!fetch_task(p, w, i, q_base, task, c.abort_word)) verdict = 2;
-      else if (task == MACO_QUEUE_TERMINATE) verdict = 1;
+      bool failed = false;
+      if (ts.next(p, task, failed, c.abort_word) == nullptr) verdict = failed ? 2u : 1u;
     }
     verdict = __shfl_sync(0xffffffffu, verdict, 0);
-    task = __shfl_sync(0xffffffffu, task, 0);
     if (verdict == 2) { ok = false; break; }
     if (verdict == 1) break;
-    task &= MACO_QUEUE_INDEX_MASK;
-    const MacoTaskDesc& d = p.tasks[task];   // read in place (L1/L2 resident): a register copy would cost 32 registers
+    const MacoTaskDesc& d = desc_slots[i & (kStreamSlots - 1)];
     if (d.type == MACO_TASK_ATTENTION && attn_pipelined(d.u.elt)) {
       // K / V rows of the split stream through the operand ring; the general warps consume them
       uint32_t go = 1;               // 1 produce, 0 stop silently (the wait reported), 2 stop and report
@@ -386,7 +420,7 @@ __device__ void producer_role(const MacoProgram& p, uint32_t w, uint32_t q_base,
       }
       continue;
     }
-    if (!is_gemm(d.type)) continue;
+    if (!is_gemm_type(d.type)) continue;
     uint32_t carry_on = 1;
     if (lane == 0) carry_on = (uint32_t)producer_gemm_task(p, d, task, smem, c, tmaps, apipe, ait, it, owner);
     carry_on = __shfl_sync(0xffffffffu, carry_on, 0);
@@ -398,16 +432,18 @@ __device__ void producer_role(const MacoProgram& p, uint32_t w, uint32_t q_base,
 // ---- MMA warp (lane 0) --------------------------------------------------------------------------
 __device__ void mma_role(const MacoProgram& p, uint32_t w, uint32_t q_base, uint8_t* smem, const GemmCtrl& c,
                          uint32_t tmem_base, volatile uint32_t* attn_done, uint64_t* attn_bars, uint64_t* p_ready,
-                         volatile uint32_t* pv_flags, uint8_t* scratch_smem) {
+                         volatile uint32_t* pv_flags, uint8_t* scratch_smem, MacoTaskDesc* desc_slots) {
+  TaskStream ts;
+  ts.start(p, desc_slots, w, q_base);
   uint32_t it = 0, seq = 0, attn_seen = 0;
   uint32_t ait = 0, attn_chunks = 0;   // attention ring uses / chunks so far: the same counts the general warps keep
   bool ok = true;
-  for (uint32_t i = 0; ok; ++i) {
+  while (ok) {
     uint32_t task;
-    if (!fetch_task(p, w, i, q_base, task, c.abort_word)) break;
-    if (task == MACO_QUEUE_TERMINATE) break;
-    task &= MACO_QUEUE_INDEX_MASK;
-    const MacoTaskDesc& d = p.tasks[task];   // read in place (L1/L2 resident): a register copy would cost 32 registers
+    bool failed = false;
+    const MacoTaskDesc* dp = ts.next(p, task, failed, c.abort_word);
+    if (dp == nullptr) break;
+    const MacoTaskDesc& d = *dp;
     if (d.type == MACO_TASK_ATTENTION && attn_pipelined(d.u.elt)) {
       // The attention task issues its own tensor-core products into the low TMEM columns: this warp must
       // not start the next GEMM tile's accumulator there before the general warps have finished the task
@@ -432,7 +468,7 @@ __device__ void mma_role(const MacoProgram& p, uint32_t w, uint32_t q_base, uint
       }
       continue;
     }
-    if (!is_gemm(d.type)) continue;
+    if (!is_gemm_type(d.type)) continue;
     const MacoGemmArgs& g = d.u.gemm;
     if (d.flags & MACO_TF_COUNTED) {
       if (!wait_deps(p, d, task, c.abort_word, nullptr)) break;
@@ -477,57 +513,60 @@ __device__ __noinline__ void run_moe(const MacoProgram& p, uint32_t type, const 
 template <int CG>
 __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, const GemmCtrl& c, uint32_t tmem_base,
                              volatile uint32_t* slots, uint8_t* scratch_smem, uint8_t* ring_smem, uint64_t* bulk_bars,
-                             uint64_t* attn_bars, uint64_t* attn_p_ready) {
+                             uint64_t* attn_bars, uint64_t* attn_p_ready, MacoTaskDesc* desc_slots) {
   const int tid = threadIdx.x - 64;          // 0..127
   // two-CTA programs: the epilogue warps of both CTAs report "accumulator drained" to the leader's barrier
   uint32_t pair_empty_bar = 0;
   if constexpr (CG == 2) pair_empty_bar = mapa_u32(smem_u32(&c.tmem_empty[0]), 0);
   const bool leader = tid == 0;
+  TaskStream ts;
+  if (leader) ts.start(p, desc_slots, w, q_base);
   // Communication workers never get GEMM tasks, so their operand ring is free to stage bulk copies.
   const bool comm_worker = p.num_comm_workers > 0 && w >= p.num_workers - p.num_comm_workers;
   BulkCtx bulk{ring_smem, bulk_bars, kBulkBuffers, kBulkBufBytes, slots + 12};   // phase word: zeroed at kernel start
   uint32_t seq = 0, done = 0, it = 0;      // it: ring stages consumed so far (kept in step with the TMA and MMA warps)
   uint32_t attn_chunks = 0, ait = 0;       // attention chunks done (parity of its MMA barriers), uses of its ring
   uint32_t attn_tasks = 0;                 // pipelined attention tasks done (parity of the "Q staged" barrier)
+  enum : uint32_t { kEnd = 0, kRun = 1, kSkip = 2, kStop = 3 };
   for (uint32_t i = 0;; ++i) {
-    volatile uint32_t* cur = slots + (i & 1u) * 4;     // [0] task, [1] dependencies satisfied, [2] failure
+    volatile uint32_t* cur = slots + (i & 1u) * 4;     // [0] verdict on the task, [2] failure, [3] last arrival
+    uint32_t task = 0;                                 // leader only
+    uint64_t t_start = 0, wait_ns = 0;
     if (leader) {
-      uint32_t task;
-      if (!fetch_task(p, w, i, q_base, task, c.abort_word)) task = MACO_QUEUE_TERMINATE - 1;   // abort marker
-      cur[0] = task;
+      // One thread fetches the task and waits for what it depends on; one barrier hands both to the others. (A GEMM
+      // tile's conditions are the TMA warp's to wait for: here the accumulator's barrier stands for them.)
+      bool failed = false;
+      uint32_t verdict = kEnd;
+      const MacoTaskDesc* dp = ts.next(p, task, failed, c.abort_word);
+      if (failed) {
+        verdict = kStop;
+      } else if (dp != nullptr) {
+        if (p.trace != nullptr) t_start = globaltimer_ns();
+        verdict = kRun;
+        if (p.debug != 0 && !desc_ok(p, *dp)) {
+          report_failure(p, MACO_STATUS_BAD_TASK, task, dp->type, c.abort_word);
+          verdict = kStop;
+        } else if (!is_gemm_type(dp->type) || (dp->flags & MACO_TF_COUNTED)) {
+          if (!wait_deps(p, *dp, task, c.abort_word, p.trace ? &wait_ns : nullptr)) verdict = kStop;
+          else if (is_gemm_type(dp->type) && ld_relaxed_gpu_u32(dp->u.gemm.count_ptr) <= dp->u.gemm.count_base) verdict = kSkip;
+        }
+      }
+      cur[0] = verdict;
       cur[2] = 0;
     }
     general_bar();
-    const uint32_t raw_entry = cur[0];
-    if (raw_entry >= MACO_QUEUE_TERMINATE - 1) {
-      const uint32_t task = raw_entry;
+    const uint32_t verdict = cur[0];
+    if (verdict == kEnd || verdict == kStop) {
       // consume the TERMINATE entry too, so the next launch starts behind it
-      if (leader && task == MACO_QUEUE_TERMINATE && p.mode == MACO_MODE_DYNAMIC) st_release_gpu_u32(&p.tails[w], q_base + i + 1);
+      if (leader && verdict == kEnd && p.mode == MACO_MODE_DYNAMIC) st_release_gpu_u32(&p.tails[w], q_base + i + 1);
       break;
     }
-    // bit 31 of a static queue entry: no GEMM task follows in this worker's queue, the operand ring is idle
-    const uint32_t task = raw_entry & MACO_QUEUE_INDEX_MASK;
-    const bool ring_free = comm_worker || (raw_entry & MACO_QUEUE_RING_FREE) != 0;
-    const MacoTaskDesc& d = p.tasks[task];   // read in place (L1/L2 resident): a register copy would cost 32 registers
-    uint64_t t_start = 0, wait_ns = 0;
-    if (leader && p.trace != nullptr) t_start = globaltimer_ns();
-    if (p.debug != 0 && !desc_ok(p, d)) {            // uniform over the 128 threads (same descriptor)
-      if (leader) report_failure(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word);
-      break;
-    }
-    bool skip_tile = false;
-    if (is_gemm(d.type) && (d.flags & MACO_TF_COUNTED)) {
-      if (leader) {
-        const bool okw = wait_deps(p, d, task, c.abort_word, nullptr);
-        cur[1] = !okw ? 0u : (ld_relaxed_gpu_u32(d.u.gemm.count_ptr) <= d.u.gemm.count_base ? 2u : 1u);
-      }
-      general_bar();
-      if (cur[1] == 0) cur[2] = 1;
-      skip_tile = cur[1] != 1;
-    }
-    if (is_gemm(d.type) && skip_tile) {
-      // nothing to compute: the tile's rows hold no tokens (it still signals below)
-    } else if (is_gemm(d.type)) {
+    const MacoTaskDesc& d = desc_slots[i & (kStreamSlots - 1)];
+    // static queues: no user of the operand ring follows in this worker's queue
+    const bool ring_free = comm_worker || (d.flags & MACO_TF_RING_FREE) != 0;
+    if (verdict == kSkip) {
+      // counted tile without rows: nothing to compute (it still signals below)
+    } else if (is_gemm_type(d.type)) {
       const MacoGemmArgs& g = d.u.gemm;
       const GemmEpilogue& e = p.epis[g.epi];
       void* out_base = e.out;
@@ -573,50 +612,43 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
           }
         }
       }
-    } else {
-      if (leader) cur[1] = wait_deps(p, d, task, c.abort_word, p.trace ? &wait_ns : nullptr) ? 1u : 0u;
-      general_bar();
-      if (cur[1] != 0) {
-        if (d.type >= 200 && d.type < 300) {
-          if (!run_comm(p, d, tid, ring_free ? &bulk : nullptr)) {
-            cur[2] = 1;
-            if (leader) report_failure(p, MACO_STATUS_BAD_TASK, task, d.u.comm.op, c.abort_word);
-          }
-        } else if (d.type == MACO_TASK_ATTENTION && attn_pipelined(d.u.elt)) {
-          if constexpr (CG == 1) {
-            const AttnPipe pipe{ring_smem, attn_bars + 4, attn_bars + 4 + kAttnStages, p.budget_ns, c.abort_word,
-                                nullptr, attn_bars, tmem_base, attn_p_ready, slots + 20, attn_tasks};
-            if (!attn_consume(d.u.elt, tid, scratch_smem, pipe, ait, attn_chunks)) cur[2] = 1;
-            ait += attn_stage_uses(d.u.elt);
-            ++attn_tasks;
-            general_bar();
-            if (leader) slots[13] = slots[13] + 1;                 // lets the MMA warp move past this task
-          } else {
-            // the tensor-core attention task issues one-CTA MMAs; a kernel has one cta_group (the builder
-            // keeps such tasks out of two-CTA programs)
-            cur[2] = 1;
-            if (leader) report_failure(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word);
-          }
-        } else if (d.type == MACO_TASK_ATTENTION || d.type == MACO_TASK_ATTN_MERGE) {
-          run_attn(d.type, d.u.elt, tid, scratch_smem);
-        } else if (d.type == MACO_TASK_TOPK || d.type == MACO_TASK_MOE_COUNTS || d.type == MACO_TASK_MOE_RETURN ||
-                   d.type == MACO_TASK_SPLITK_FIN || d.type == MACO_TASK_MOE_COMBINE) {
-          run_moe(p, d.type, d.u.elt, tid, scratch_smem, ring_free ? &bulk : nullptr);
-        } else if (d.type != MACO_TASK_NOP) {
-          if (!run_elt(d.type, d.u.elt, tid)) {
-            cur[2] = 1;
-            if (leader) report_failure(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word);
-          }
-        }
-      } else if (leader) {
+    } else if (d.type >= 200 && d.type < 300) {
+      if (!run_comm(p, d, tid, ring_free ? &bulk : nullptr)) {
         cur[2] = 1;
+        if (leader) report_failure(p, MACO_STATUS_BAD_TASK, task, d.u.comm.op, c.abort_word);
+      }
+    } else if (d.type == MACO_TASK_ATTENTION && attn_pipelined(d.u.elt)) {
+      if constexpr (CG == 1) {
+        const AttnPipe pipe{ring_smem, attn_bars + 4, attn_bars + 4 + kAttnStages, p.budget_ns, c.abort_word,
+                            nullptr, attn_bars, tmem_base, attn_p_ready, slots + 20, attn_tasks};
+        if (!attn_consume(d.u.elt, tid, scratch_smem, pipe, ait, attn_chunks)) cur[2] = 1;
+        ait += attn_stage_uses(d.u.elt);
+        ++attn_tasks;
+        general_bar();
+        if (leader) slots[13] = slots[13] + 1;                 // lets the MMA warp move past this task
+      } else {
+        // the tensor-core attention task issues one-CTA MMAs; a kernel has one cta_group (the builder
+        // keeps such tasks out of two-CTA programs)
+        cur[2] = 1;
+        if (leader) report_failure(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word);
+      }
+    } else if (d.type == MACO_TASK_ATTENTION || d.type == MACO_TASK_ATTN_MERGE) {
+      run_attn(d.type, d.u.elt, tid, scratch_smem);
+    } else if (d.type == MACO_TASK_TOPK || d.type == MACO_TASK_MOE_COUNTS || d.type == MACO_TASK_MOE_RETURN ||
+               d.type == MACO_TASK_SPLITK_FIN || d.type == MACO_TASK_MOE_COMBINE) {
+      run_moe(p, d.type, d.u.elt, tid, scratch_smem, ring_free ? &bulk : nullptr);
+    } else if (d.type != MACO_TASK_NOP) {
+      if (!elt_run_staged(d.type, d.u.elt, tid, scratch_smem) && !run_elt(d.type, d.u.elt, tid)) {
+        cur[2] = 1;
+        if (leader) report_failure(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word);
       }
     }
     if (leader && *c.abort_word != 0) cur[2] = 1;
     general_bar();                              // every thread's stores are issued, failure word final
     if (cur[2] != 0) break;
     if (leader) {
-      fence_proxy_async_all();                  // later TMA reads of this output by other CTAs
+      // (A consumer that reads this output through TMA orders the two proxies itself, with a proxy fence behind its
+      // acquire; one on this side as well was half a microsecond per task.)
       signal_done(p, d);
       ++done;
       if (p.mode == MACO_MODE_DYNAMIC) st_release_gpu_u32(&p.tails[w], q_base + i + 1);
@@ -745,23 +777,24 @@ __device__ __forceinline__ void persistent_body(const MacoProgram& p) {
     }
     __syncthreads();
     const uint32_t q_base = extra[16];
+    MacoTaskDesc* desc_slots = reinterpret_cast<MacoTaskDesc*>(reinterpret_cast<uint8_t*>(extra) + kStreamOffset);
     if (warp == 0) {
       if constexpr (CG == 2) {
-        if (lane == 0) producer_role_pair(p, w, q_base, smem, c);
+        if (lane == 0) producer_role_pair(p, w, q_base, smem, c, desc_slots);
       } else {
-        producer_role(p, w, q_base, smem, c, attn_bars + 4);          // all 32 lanes (see the role)
+        producer_role(p, w, q_base, smem, c, attn_bars + 4, desc_slots);          // all 32 lanes (see the role)
       }
       __syncwarp();
     } else if (warp == 1) {
       if (lane == 0) {
-        if constexpr (CG == 2) { if (cluster_ctarank() == 0) mma_role_pair(p, w, q_base, smem, c, tmem_base); }
+        if constexpr (CG == 2) { if (cluster_ctarank() == 0) mma_role_pair(p, w, q_base, smem, c, tmem_base, desc_slots + kStreamSlots); }
         else mma_role(p, w, q_base, smem, c, tmem_base, extra + 13, attn_bars, attn_p_ready, extra + 20,
-                      reinterpret_cast<uint8_t*>(extra) + kMkExtraSmem);
+                      reinterpret_cast<uint8_t*>(extra) + kMkExtraSmem, desc_slots + kStreamSlots);
       }
       __syncwarp();
     } else {
       general_role<CG>(p, w, q_base, c, tmem_base, extra, reinterpret_cast<uint8_t*>(extra) + kMkExtraSmem, smem, bulk_bars, attn_bars,
-                       attn_p_ready);
+                       attn_p_ready, desc_slots + 2 * kStreamSlots);
     }
   } else {
     if constexpr (CG == 1) { if (warp == 0) scheduler_role(p, extra); }

@@ -211,7 +211,9 @@ enum MacoTaskFlags {
   MACO_TF_WAIT0_PREV = 16,        /* wait_event[0] refers to the previous launch: (epoch-1) * count */
   MACO_TF_WAIT1_PREV = 32,
   MACO_TF_ANY_WORKER = 64,        /* host-side placement hint only */
-  MACO_TF_COUNTED = 128           /* GEMM tile guarded by a row count known only at run time (MoE) */
+  MACO_TF_COUNTED = 128,          /* GEMM tile guarded by a row count known only at run time (MoE) */
+  MACO_TF_RING_FREE = 256,        /* static queues: no user of the operand ring follows in this worker's queue */
+  MACO_TF_B_STATIC = 512          /* GEMM tile: no task of the program writes B (a weight), so its loads need not wait for the tile's conditions */
 };
 
 /* A dispatch group for the scheduler CTA: a run of consecutive tasks that becomes ready together. */
@@ -223,22 +225,19 @@ struct MacoGroupDesc {
   uint32_t _pad;
 };
 
-#define MACO_QUEUE_TERMINATE 0xffffffffu
-#define MACO_QUEUE_RING_FREE 0x80000000u   /* static queue entry: no GEMM task follows in this queue */
-#define MACO_QUEUE_INDEX_MASK 0x7fffffffu
+#define MACO_QUEUE_TERMINATE 0xffffffffu   /* dynamic mode: ring entry that ends a worker's queue */
 
 enum MacoKernelMode { MACO_MODE_STATIC = 0, MACO_MODE_DYNAMIC = 1 };
 
 /* Everything one launch of the persistent kernel needs; passed by value. */
 struct MacoProgram {
-  const struct MacoTaskDesc* tasks;
+  const struct MacoTaskDesc* tasks; /* static mode: in queue order, so a worker streams its descriptors from consecutive addresses */
   const void* tmaps;              /* CUtensorMap[ ] (128 bytes each, 64-byte aligned) */
   const struct GemmEpilogue* epis;
   uint32_t* events;               /* monotonic counters, never reset; threshold scales with epoch */
   uint32_t* peer_events[MACO_MAX_PEERS];
   uint8_t* peer_heap[MACO_MAX_PEERS];
-  const uint32_t* static_queue;   /* [num_workers][static_stride] task indices */
-  const uint32_t* static_count;   /* [num_workers] */
+  const uint32_t* queue_begin;    /* static mode: worker w runs tasks [queue_begin[w], queue_begin[w + 1]) in order */
   uint32_t* ring;                 /* [num_workers][MACO_WORKER_QUEUE_SIZE] (dynamic mode) */
   uint32_t* heads;                /* [num_workers] published by the scheduler */
   uint32_t* tails;                /* [num_workers] published by the workers */
@@ -250,7 +249,7 @@ struct MacoProgram {
   struct MacoTraceRecord* trace;  /* [num_tasks] or null */
   unsigned long long budget_ns;
   uint32_t num_tasks, num_groups, num_workers, num_comm_workers;
-  uint32_t static_stride, mode, epoch;
+  uint32_t mode, epoch;
   int32_t rank, world;
   uint32_t cta_group;             /* 1: one-CTA GEMM tiles; 2: every GEMM task is half of a two-CTA tile (cluster launch) */
   uint32_t debug;                 /* non-zero: workers re-check every descriptor (events, peers, heap extents) before running it */

@@ -29,6 +29,8 @@ MODE_STATIC, MODE_DYNAMIC = 0, 1
 TF_WAIT0_SYS, TF_WAIT1_SYS, TF_COMM_WORKER, TF_SIGNAL_SYS, TF_WAIT0_PREV, TF_WAIT1_PREV = 1, 2, 4, 8, 16, 32
 TF_ANY_WORKER = 64      # host-side placement hint: spread over compute AND communication workers
 TF_COUNTED = 128        # GEMM tile guarded by a run-time row count
+TF_RING_FREE = 256      # set at build: no user of the operand ring follows in the worker's static queue
+TF_B_STATIC = 512       # GEMM tile whose B no task of the program writes: loaded ahead of the tile's wait conditions
 COMM_PUSH, COMM_REDUCE_LOCAL, COMM_REDUCE_PULL, COMM_ALLREDUCE, COMM_ALLREDUCE_MC, COMM_PULL, COMM_REDUCE_LOCAL_BCAST, COMM_PUSH_MC = range(8)
 MAX_PEERS = 16
 WORKER_QUEUE_SIZE = 1024
@@ -53,12 +55,12 @@ class _ProgramStruct(ctypes.Structure):
     _fields_ = [
         ("tasks", ctypes.c_void_p), ("tmaps", ctypes.c_void_p), ("epis", ctypes.c_void_p), ("events", ctypes.c_void_p),
         ("peer_events", ctypes.c_void_p * MAX_PEERS), ("peer_heap", ctypes.c_void_p * MAX_PEERS),
-        ("static_queue", ctypes.c_void_p), ("static_count", ctypes.c_void_p), ("ring", ctypes.c_void_p),
+        ("queue_begin", ctypes.c_void_p), ("ring", ctypes.c_void_p),
         ("heads", ctypes.c_void_p), ("tails", ctypes.c_void_p), ("groups", ctypes.c_void_p),
         ("abort_word", ctypes.c_void_p), ("counters", ctypes.c_void_p), ("mc_heap", ctypes.c_void_p),
         ("status", ctypes.c_void_p), ("trace", ctypes.c_void_p), ("budget_ns", ctypes.c_ulonglong),
         ("num_tasks", ctypes.c_uint32), ("num_groups", ctypes.c_uint32), ("num_workers", ctypes.c_uint32),
-        ("num_comm_workers", ctypes.c_uint32), ("static_stride", ctypes.c_uint32), ("mode", ctypes.c_uint32),
+        ("num_comm_workers", ctypes.c_uint32), ("mode", ctypes.c_uint32),
         ("epoch", ctypes.c_uint32), ("rank", ctypes.c_int32), ("world", ctypes.c_int32),
         ("cta_group", ctypes.c_uint32), ("debug", ctypes.c_uint32), ("heap_bytes", ctypes.c_uint64),
         ("num_events", ctypes.c_uint32), ("num_tmaps", ctypes.c_uint32), ("num_epis", ctypes.c_uint32), ("_pad", ctypes.c_uint32),
@@ -1049,14 +1051,29 @@ class Program:
         self.heap = b.heap
         n = len(b.tasks)
         self.num_tasks = n
-        tasks = np.zeros(max(n, 1), dtype=TASK_DTYPE)
-        for i, t in enumerate(b.tasks):
-            rec = tasks[i]
-            rec["type"], rec["flags"], rec["node_id"] = t["type"], t["flags"], t["node_id"]
-            rec["wait_event"], rec["wait_count"], rec["signal_event"] = t["wait_event"], t["wait_count"], t["signal_event"]
-            rec["signal_peer"], rec["signal_peer_event"] = t["signal_peer"], t["signal_peer_event"]
-            raw = t["raw"]
-            rec["raw"][: len(raw)] = np.frombuffer(raw, dtype=np.uint8)
+        queues = assign_static_queues(b.tasks, self.num_workers, self.num_comm_workers)
+        from ..config import config as _dbg_cfg
+        if _dbg_cfg.debug and b.heap is None and self.mode == MODE_STATIC:
+            # debug layer: run the queues on the host first; an order that can deadlock is reported here, with the
+            # stuck tasks, instead of as a device-side wait that runs out (single-rank programs: nothing to wait
+            # for on a peer)
+            simulate_static_queues([(b.tasks, queues)])
+        # Static programs upload their descriptors in queue order, worker after worker: a worker streams its own
+        # from consecutive addresses, without an index table in between.
+        order = [i for q in queues for i in q] if self.mode == MODE_STATIC else list(range(n))
+        queue_begin = np.cumsum([0] + [len(q) for q in queues]).astype(np.uint32)
+        head = struct.Struct("<HHI2i2I2iii")
+        pad = bytes(TASK_DTYPE.itemsize - head.size)
+        blob = b"".join([head.pack(t["type"], t["flags"], t["node_id"], *t["wait_event"], *t["wait_count"], *t["signal_event"],
+                                   t["signal_peer"], t["signal_peer_event"]) + t["raw"] + pad[len(t["raw"]):]
+                         for t in map(b.tasks.__getitem__, order)] or [bytes(TASK_DTYPE.itemsize)])
+        tasks = np.frombuffer(bytearray(blob), dtype=TASK_DTYPE)
+        if self.mode == MODE_STATIC:
+            # tasks behind the queue's last ring user (GEMM tiles, pipelined attention): the worker's operand ring
+            # is idle from there on, and communication tasks may stage bulk copies in it
+            for w, q in enumerate(queues):
+                last_gemm = max((k for k, t in enumerate(q) if b.tasks[t]["type"] in (100, 101, 102)), default=-1)
+                tasks["flags"][int(queue_begin[w]) + last_gemm + 1: int(queue_begin[w + 1])] |= TF_RING_FREE
         self._tasks_np = tasks
         self.task_types = tasks["type"].copy()
         dev = self.device
@@ -1085,24 +1102,7 @@ class Program:
             self.d_events = torch.zeros(self.num_events + 64, dtype=torch.int32, device=dev)
         self.d_ctrl = torch.zeros(8, dtype=torch.int32, device=dev)        # [0] abort word, [1] task counter
         W = self.num_workers
-        queues = assign_static_queues(b.tasks, self.num_workers, self.num_comm_workers)
-        from ..config import config as _dbg_cfg
-        if _dbg_cfg.debug and b.heap is None and self.mode == MODE_STATIC:
-            # debug layer: run the queues on the host first; an order that can deadlock is reported here, with the
-            # stuck tasks, instead of as a device-side wait that runs out (single-rank programs: nothing to wait
-            # for on a peer)
-            simulate_static_queues([(b.tasks, queues)])
-        stride = max(1, max(len(q) for q in queues))
-        sq = np.full((W, stride), QUEUE_TERMINATE, dtype=np.uint32)
-        for w, q in enumerate(queues):
-            sq[w, : len(q)] = q
-            # entries behind the queue's last ring user (GEMM tiles, pipelined attention) carry bit 31: the
-            # worker's operand ring is idle from there on, and communication tasks may stage bulk copies in it
-            last_gemm = max((k for k, t in enumerate(q) if b.tasks[t]["type"] in (100, 101, 102)), default=-1)
-            sq[w, last_gemm + 1: len(q)] |= np.uint32(0x80000000)
-        self.static_stride = stride
-        self.d_static_queue = up(sq)
-        self.d_static_count = up(np.array([len(q) for q in queues], dtype=np.uint32))
+        self.d_queue_begin = up(queue_begin)
         if self.mode == MODE_DYNAMIC:
             self.d_ring = torch.zeros(W * WORKER_QUEUE_SIZE, dtype=torch.int32, device=dev)
             self.d_heads = torch.zeros(W, dtype=torch.int32, device=dev)
@@ -1114,7 +1114,7 @@ class Program:
         ps = _ProgramStruct()
         ps.tasks, ps.tmaps, ps.epis = self.d_tasks.data_ptr(), self.d_tmaps.data_ptr(), self.d_epis.data_ptr()
         ps.events = self.d_events.data_ptr()
-        ps.static_queue, ps.static_count = self.d_static_queue.data_ptr(), self.d_static_count.data_ptr()
+        ps.queue_begin = self.d_queue_begin.data_ptr()
         if self.mode == MODE_DYNAMIC:
             ps.ring, ps.heads, ps.tails = self.d_ring.data_ptr(), self.d_heads.data_ptr(), self.d_tails.data_ptr()
         ps.groups = self.d_groups.data_ptr()
@@ -1124,7 +1124,7 @@ class Program:
         ps.trace = self.d_trace.data_ptr() if self.d_trace is not None else None
         ps.budget_ns = int(b.wait_budget_ms * 1e6)
         ps.num_tasks, ps.num_groups, ps.num_workers, ps.num_comm_workers = n, self.num_groups, W, self.num_comm_workers
-        ps.static_stride, ps.mode, ps.epoch = stride, self.mode, 0
+        ps.mode, ps.epoch = self.mode, 0
         ps.rank, ps.world = 0, 1
         ps.cta_group = 2 if b.cta_pair else 1
         from ..config import config as _cfg
