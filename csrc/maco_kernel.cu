@@ -34,6 +34,7 @@
 #include "attention_decode.cuh"
 #include "moe_tasks.cuh"
 #include "splitk_tasks.cuh"
+#include "fewrow_gemm.cuh"
 #include "host_common.h"
 
 using namespace maco;
@@ -50,6 +51,7 @@ constexpr uint32_t kStreamAhead = 3;
 constexpr int kMkScratchSmem = 28672;  // scratch of non-GEMM tasks (the operand ring is NOT free for them:
                                        // the producer warp may already be filling it for the next GEMM task)
 constexpr int kMkSmemBytes = MkLayout::kTotalBytes + kMkExtraSmem + kMkScratchSmem;
+static_assert(kFewWBytes + 64 * kFewK * 2 <= (uint32_t)MkLayout::kStageBytes, "a few-row stage must fit a ring stage");
 static_assert(kStreamOffset + 3 * kStreamSlots * sizeof(MacoTaskDesc) <= kMkExtraSmem, "descriptor slots");
 static_assert(kMkScratchSmem >= (int)kRowScratch, "staged row tasks must fit the scratch block");
 static_assert(kMkScratchSmem >= kEpiStageBytes, "epilogue staging must fit the scratch block");
@@ -171,6 +173,7 @@ __device__ bool desc_ok(const MacoProgram& p, const MacoTaskDesc& d) {
     if (g.tmap_a >= p.num_tmaps || g.tmap_b >= p.num_tmaps || g.epi >= p.num_epis) return false;
     if (g.peer >= p.world || g.peer < -2) return false;
     if (g.peer != -1 && (p.heap_bytes == 0 || g.out_off >= p.heap_bytes)) return false;
+    if (g.b_mn & kFewFlag) return g.k_blocks >= 0 && g.bn >= 16 && g.bn <= 64 && g.bn % 16 == 0 && g.count_base > 0;
     return g.k_blocks >= 0 && (g.bn == 128 || g.bn == 256);
   }
   if (d.type >= 200 && d.type < 300 && d.u.comm.rows != 0) {
@@ -324,6 +327,29 @@ __device__ void mma_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_base,
 // the K / V stream of a decode-attention task is six TMA boxes per 64 KB chunk, and one thread issues a few TMA
 // operations per microsecond only; lanes 0-5 issue the six boxes with ONE warp instruction.
 
+// A few-row GEMM task on lane 0: the weights (operand A here) of up to a whole ring go out before the task waits for its
+// tokens, unless a task of the program writes them.
+__device__ int producer_few_task(const MacoProgram& p, const MacoTaskDesc& d, uint32_t task, uint8_t* smem, const GemmCtrl& c,
+                                 const CUtensorMap* tmW, const CUtensorMap* tmX, uint32_t& it) {
+  const MacoGemmArgs& g = d.u.gemm;
+  const uint64_t pol = l2_evict_first();
+  const uint32_t steps = (uint32_t)g.k_blocks;
+  uint32_t ahead = 0;
+  bool ok = true;
+  if (d.flags & MACO_TF_B_STATIC)
+    for (; ok && ahead < steps && ahead < (uint32_t)kMkStages; ++ahead)
+      ok = few_load_weights<kMkStages, MkLayout::kStageBytes>(smem, c, tmW, g, it + ahead, ahead, pol, p.budget_ns);
+  if (ok && !wait_deps(p, d, task, c.abort_word, nullptr)) { it += ahead; return 0; }
+  fence_proxy_async_all();           // the tokens were written by generic-proxy stores of other CTAs
+  for (uint32_t st = 0; ok && st < steps; ++st) {
+    if (st >= ahead) ok = few_load_weights<kMkStages, MkLayout::kStageBytes>(smem, c, tmW, g, it + st, st, pol, p.budget_ns);
+    if (ok) few_load_tokens<kMkStages, MkLayout::kStageBytes>(smem, c, tmX, g, it + st, st);
+  }
+  it += steps;
+  if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
+  return ok ? 1 : 0;
+}
+
 // One GEMM task on lane 0: 1 = carry on, 0 = stop (failure already reported where it has a reporter).
 __device__ int producer_gemm_task(const MacoProgram& p, const MacoTaskDesc& d, uint32_t task, uint8_t* smem, const GemmCtrl& c,
                                   const CUtensorMap* tmaps, const AttnPipe& apipe, uint32_t ait, uint32_t& it, int& owner) {
@@ -339,6 +365,7 @@ __device__ int producer_gemm_task(const MacoProgram& p, const MacoTaskDesc& d, u
   }
   if (owner == 2 && !attn_ring_drained(apipe, ait)) return 0;
   owner = 1;
+  if (g.b_mn & kFewFlag) return producer_few_task(p, d, task, smem, c, ta, tb, it);
   // B of a weight is on its way before the tile's conditions hold: a decode step is a chain of dependent
   // weight-streaming phases, and this keeps up to a full ring (128 KB per SM) of the next phase's weights in
   // flight while the last one drains.
@@ -474,6 +501,11 @@ __device__ void mma_role(const MacoProgram& p, uint32_t w, uint32_t q_base, uint
       if (!wait_deps(p, d, task, c.abort_word, nullptr)) break;
       if (ld_relaxed_gpu_u32(g.count_ptr) <= g.count_base) continue;
     }
+    if (g.b_mn & kFewFlag) {
+      ok = few_mma_tile<kMkStages, MkLayout::kStageBytes, kMkBN>(smem, c, tmem_base, g, it, seq, p.budget_ns);
+      ++seq;
+      continue;
+    }
     const int sel = (g.bn == 128 ? 4 : 0) | (g.a_mn ? 2 : 0) | ((g.b_mn & 1) ? 1 : 0);
     switch (sel) {
       case 0: ok = gemm_mma_tile<256, kMkStages, false, false, kMkBN>(smem, c, tmem_base, g.idesc, g.k_blocks, it, seq, p.budget_ns); break;
@@ -564,8 +596,15 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
     const MacoTaskDesc& d = desc_slots[i & (kStreamSlots - 1)];
     // static queues: no user of the operand ring follows in this worker's queue
     const bool ring_free = comm_worker || (d.flags & MACO_TF_RING_FREE) != 0;
+    bool signals = true;
     if (verdict == kSkip) {
       // counted tile without rows: nothing to compute (it still signals below)
+    } else if (CG == 1 && is_gemm_type(d.type) && (d.u.gemm.b_mn & kFewFlag)) {
+      const int r = few_epilogue<kMkBN>(c, tmem_base, p.epis[d.u.gemm.epi], d.u.gemm, tid, seq, p.budget_ns, scratch_smem, cur + 3,
+                                        [] { general_bar(); });
+      if (r == 0) cur[2] = 1;
+      signals = r == 2;                                // the tile's event counts finished tiles, not parts
+      ++seq;
     } else if (is_gemm_type(d.type)) {
       const MacoGemmArgs& g = d.u.gemm;
       const GemmEpilogue& e = p.epis[g.epi];
@@ -649,7 +688,7 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
     if (leader) {
       // (A consumer that reads this output through TMA orders the two proxies itself, with a proxy fence behind its
       // acquire; one on this side as well was half a microsecond per task.)
-      signal_done(p, d);
+      if (signals) signal_done(p, d);
       ++done;
       if (p.mode == MACO_MODE_DYNAMIC) st_release_gpu_u32(&p.tails[w], q_base + i + 1);
       if (p.trace != nullptr) {

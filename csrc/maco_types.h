@@ -73,7 +73,11 @@ enum MacoEpilogueMode {
      tile's operand block has a 16-byte record {int32 token, int32 k, float weight, pad} at `aux`[r]; the 16-bit
      output row goes to row token * bias_type + k of the destination (ld_out elements per row), scaled by the weight
      after rounding the product to the output type. Rows at or beyond the task's run-time count are not written. */
-  MACO_EPI_SCATTER_ROWS = 10
+  MACO_EPI_SCATTER_ROWS = 10,
+  /* Few-row GEMM with swapped operands (csrc/fewrow_gemm.cuh): `out` = fp32 workspace [tokens, features] (ld_out), N =
+     tokens, `bias` = uint32 arrival counters (one per finished tile, never reset), `aux` = a MacoEltArgs in device memory:
+     in0 / ld_in the workspace, rows = tokens, in1 = residual rows or MacoQkRopeParams, out / ld_out / dtype, i0 = operator. */
+  MACO_EPI_FEWROW = 11
 };
 
 struct GemmEpilogue {
@@ -117,7 +121,9 @@ struct MacoStatusBlock {          /* lives in host-mapped pinned memory */
 struct MacoGemmArgs {             /* one output tile */
   uint16_t tmap_a, tmap_b;        /* indices into the tensor-map table */
   uint16_t epi;                   /* index into the epilogue table */
-  uint8_t a_mn, b_mn;             /* operand majors (bit 0: MN-major). b_mn bit 1: B is stored tile by tile ([N/256][K/64][256][64]); count_base = its total k-blocks */
+  uint8_t a_mn, b_mn;             /* operand majors (bit 0: MN-major). b_mn bit 1: B is stored tile by tile ([N/256][K/64][256][64]); count_base = its total k-blocks.
+                                     b_mn bit 2: few-row task: tmap_a = weights, tmap_b = tokens, m0 = first feature, k_blocks in steps of 128, bn = padded tokens,
+                                     row_off = index of its arrival counter, count_base = arrivals that complete the tile */
   int32_t m0, n0, k0, k_blocks;
   uint32_t idesc;
   int32_t peer;                   /* -1: store to the epilogue's out; >= 0: into that rank's heap at out_off; -2: into every rank's heap at out_off */

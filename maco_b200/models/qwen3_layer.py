@@ -108,7 +108,7 @@ class Qwen3DecodeLayer:
         if self.fused_rope:
             # QK-norm, RoPE and the K / V cache update happen in the finishing pass of the projection itself: no QKV
             # buffer, no separate tasks, one dependency hop less before attention
-            e_qkv = b.gemm_splitk(self.h1, self.w_qkv, None, epilogue="qk_rope", a_ready=e_h1, w_blocked=self.wb_qkv,
+            e_qkv = b.gemm_splitk(self.h1, self.w_qkv, None, epilogue="qk_rope", a_ready=e_h1, w_blocked=self.wb_qkv, w_static=True,
                                   rope=dict(q_out=self.q_rot, k_cache=self.k_cache, v_cache=self.v_cache, q_norm=self.q_norm,
                                             k_norm=self.k_norm, cos_sin=self.cos_sin, hq=hq, hkv=hkv, pos=self.pos, eps=self.eps))
             ready = [(e_qkv.all_event[0], e_qkv.all_event[1], False, False)]
@@ -119,7 +119,7 @@ class Qwen3DecodeLayer:
     def _rope_tasks(self, b, e_h1):
         B, H, D, hq, hkv, G, S = self.batch, self.hidden, self.D, self.hq, self.hkv, self.G, self.S
         qw = (hq + 2 * hkv) * D
-        e_qkv = b.gemm_splitk(self.h1, self.w_qkv, self.qkv, a_ready=e_h1, w_blocked=self.wb_qkv)
+        e_qkv = b.gemm_splitk(self.h1, self.w_qkv, self.qkv, a_ready=e_h1, w_blocked=self.wb_qkv, w_static=True)
         qkv_done = (e_qkv.all_event[0], e_qkv.all_event[1], False, False)
         # QK-norm + RoPE: q into its own buffer, k straight into the cache row of the new token, v copied
         # beside it. All of it bumps one event, so the attention tasks carry a single wait condition; task
@@ -150,12 +150,12 @@ class Qwen3DecodeLayer:
         slots1 = self.slots1 if self.world > 1 else None
         slots2 = self.slots2 if self.world > 1 else None
         e_y1 = fused.gemm_allreduce(b, self.attn, self.w_o, slots1, self.y1, residual=self.x, a_ready=e_attn,
-                                    w_blocked=self.wb_o)
+                                    w_blocked=self.wb_o, w_static=True)
         e_h2 = b.elementwise(int(TaskType.RMSNORM), self.y1, self.h2, in1=self.w_post, rows=B, cols=H, f0=self.eps,
                              in_ready=[e_y1])
-        e_act = b.gemm_splitk(self.h2, self.w_gate_up, self.act, epilogue="swiglu", a_ready=e_h2, w_blocked=self.wb_gate_up)
+        e_act = b.gemm_splitk(self.h2, self.w_gate_up, self.act, epilogue="swiglu", a_ready=e_h2, w_blocked=self.wb_gate_up, w_static=True)
         e_out = fused.gemm_allreduce(b, self.act, self.w_down, slots2, self.out, residual=self.y1, a_ready=e_act,
-                                     w_blocked=self.wb_down)
+                                     w_blocked=self.wb_down, w_static=True)
         if self.world > 1:
             fused.epoch_fence_signal(b, [(e_out.all_event[0], e_out.all_event[1], False, False)])
         # (a CPU device plans only: the task list stays in ``self.builder`` for host-side schedule checks)

@@ -37,7 +37,7 @@ WORKER_QUEUE_SIZE = 1024
 T_SPLITK_FIN = 118
 
 EPI = {None: 0, "none": 0, "gelu": 1, "swiglu": 2, "f32": 3, "f32_acc": 4, "gelu_bwd": 5, "silu": 6, "residual": 7, "f32_atomic": 8,
-       "splitk_fused": 9, "scatter_rows": 10}
+       "splitk_fused": 9, "scatter_rows": 10, "fewrow": 11}
 
 TASK_DTYPE = np.dtype([
     ("type", "<u2"), ("flags", "<u2"), ("node_id", "<u4"), ("wait_event", "<i4", 2), ("wait_count", "<u4", 2),
@@ -128,6 +128,33 @@ def pick_split_k(n_tiles: int, k_blocks: int, workers: int) -> int:
     def cost(sp: int) -> int:
         return -(-n_tiles * sp // workers) * (-(-k_blocks // sp) + 8)
     return min(range(1, max(1, min(16, k_blocks // 2)) + 1), key=cost)
+
+
+def stream_pieces(n_tiles: int, steps: int, workers: int) -> List[Tuple[int, int, int, int]]:
+    """Cuts the ``n_tiles * steps`` (tile, k-step) pairs of a few-row GEMM into one nearly equal piece per worker, at least
+    two steps (64 KB of weights) each. Returns (tile, first step, steps, worker): a worker's piece is split where it
+    crosses a tile. A cut that would leave less than an eighth of a piece on one side of a tile boundary moves to it
+    (a part costs about a microsecond of reductions and arrival whatever its length)."""
+    total = n_tiles * steps
+    workers = max(1, min(workers, total // 2))
+    slack = total // workers // 8
+    cuts = [0]
+    for i in range(1, workers):
+        c = i * total // workers
+        lo, hi = c % steps, steps - c % steps
+        if lo and min(lo, hi) <= slack:
+            c = c - lo if lo <= hi else c + hi
+        cuts.append(max(cuts[-1], c))
+    cuts.append(total)
+    pieces = []
+    for w in range(workers):
+        pos = cuts[w]
+        while pos < cuts[w + 1]:
+            tile, s0 = divmod(pos, steps)
+            n = min(steps - s0, cuts[w + 1] - pos)
+            pieces.append((tile, s0, n, w))
+            pos += n
+    return pieces
 
 
 def attention_pieces(groups: int, kv_len: int, workers: int) -> List[Tuple[int, int, int, int]]:
@@ -458,7 +485,8 @@ class ProgramBuilder:
     def add_task(self, ttype: int, raw: bytes, waits: Sequence[Tuple[int, int, bool, bool]] = (),
                  signals: Sequence[int] = (), signal_peer: int = -1, signal_peer_event: int = -1, node_id: int = 0,
                  comm_worker: bool = False, signal_sys: bool = False, any_worker: bool = False,
-                 counted: bool = False, worker: Optional[int] = None, pair_half: Optional[int] = None) -> int:
+                 counted: bool = False, worker: Optional[int] = None, pair_half: Optional[int] = None,
+                 b_static: bool = False) -> int:
         """``waits``: up to two (event, count, sys_scope, previous_epoch). ``worker`` pins the task to a compute
         worker's static queue (the dynamic scheduler ignores it)."""
         if len(waits) > 2 or len(signals) > 2:
@@ -479,6 +507,8 @@ class ProgramBuilder:
             flags |= TF_ANY_WORKER
         if counted:
             flags |= TF_COUNTED
+        if b_static:
+            flags |= TF_B_STATIC
         se = list(signals) + [-1] * (2 - len(signals))
         self.tasks.append(dict(type=ttype, flags=flags, node_id=node_id, wait_event=we, wait_count=wc, signal_event=se,
                                signal_peer=signal_peer, signal_peer_event=signal_peer_event, raw=raw, worker=worker,
@@ -541,7 +571,7 @@ class ProgramBuilder:
              aux: Optional[torch.Tensor] = None, alpha: float = 1.0, bn: int = 0,
              a_ready: Optional[RowEvents] = None, extra_waits: Sequence[Tuple[int, int, bool, bool]] = (),
              per_tile=None, m_blocks: Optional[Sequence[int]] = None, signal_sys: bool = False,
-             row_wait=None, group_blocks: Optional[int] = None) -> RowEvents:
+             row_wait=None, group_blocks: Optional[int] = None, b_static: bool = False) -> RowEvents:
         """Adds the tiles of ``out = epilogue(alpha * A · B^T)`` (A logically [M,K], B logically [N,K]).
 
         ``a_ready`` gives row-block events of A (a tile waits only for its 128 rows); ``extra_waits``
@@ -553,6 +583,7 @@ class ProgramBuilder:
         group runs, its A panel (group_blocks x 128 x K) stays in L2 and B streams through once, so DRAM reads
         B once per GROUP: large groups cut the re-reads of a B that does not fit the 126 MB L2. Default: as many
         blocks as keep the A panel near 32 MB (MACO_GEMM_PANEL_MB; at least 8) when the caller did not fix the block order, else 8.
+        ``b_static``: no task of the program writes ``b`` (a weight), so a tile's B loads may run ahead of its wait conditions.
         """
         for t in (a, b):
             if t.dim() != 2 or t.stride(1) != 1 or t.dtype not in (torch.bfloat16, torch.float16):
@@ -632,7 +663,8 @@ class ProgramBuilder:
                              ov.get("count_base", 0), ov.get("count_ptr", 0))
             self.add_task(int(TaskType.LINEAR), raw, waits=waits, signals=[row_events[mb], all_ev],
                           signal_peer=ov.get("signal_peer", -1), signal_peer_event=ov.get("signal_peer_event", -1),
-                          node_id=node_id, signal_sys=signal_sys, counted=bool(ov.get("count_ptr", 0)), pair_half=half)
+                          node_id=node_id, signal_sys=signal_sys, counted=bool(ov.get("count_ptr", 0)), pair_half=half,
+                          b_static=b_static)
 
         def emit_filler(nb: int) -> None:
             # second half of a pair that has only one row block left: rows past the end of A (the loads return
@@ -693,14 +725,91 @@ class ProgramBuilder:
                                     wait_count=list(t["wait_count"]), flags=t["flags"] & mask))
             i = j
 
-    # ------------------------------------------------------------------ split-K GEMM for few rows (decode)
+    # ------------------------------------------------------------------ few-row GEMMs (decode)
+    def _rope_params(self, rope: dict, M: int, Nn: int, device) -> torch.Tensor:
+        """MacoQkRopeParams of a fused QKV projection in device memory (tensors checked and kept alive)."""
+        hq, hkv = int(rope["hq"]), int(rope["hkv"])
+        q_out, kc, vc = rope["q_out"], rope["k_cache"], rope["v_cache"]
+        if Nn != (hq + 2 * hkv) * 128 or kc.shape[-1] != 128 or kc.dim() != 4 or kc.shape[1] != hkv or not kc.is_contiguous() \
+                or not vc.is_contiguous() or vc.shape != kc.shape or tuple(q_out.shape) != (M, hq, 128) or not q_out.is_contiguous() \
+                or rope["cos_sin"].shape != (M, 128) or not (0 <= int(rope["pos"]) < kc.shape[2]):
+            raise ValueError("gemm_splitk: rope tensors do not match (hq + 2 hkv) heads of 128 and caches [M, hkv, S, 128]")
+        blob = struct.pack("<QQQQQQqqiiiifi", q_out.data_ptr(), kc.data_ptr(), vc.data_ptr(), rope["q_norm"].data_ptr(),
+                           rope["k_norm"].data_ptr(), rope["cos_sin"].data_ptr(), kc.stride(0), kc.stride(1), hq, hkv,
+                           int(rope["pos"]), N.DTYPE_CODE[q_out.dtype], float(rope["eps"]), 0)
+        dev = torch.frombuffer(bytearray(blob), dtype=torch.uint8).to(device)
+        self.keepalive += [dev, q_out, kc, vc, rope["q_norm"], rope["k_norm"], rope["cos_sin"]]
+        return dev
+
+    @staticmethod
+    def can_stream(M: int, Nn: int, K: int, epilogue: Optional[str] = None) -> bool:
+        """Shapes ``gemm_stream`` takes: at most 64 rows (a ring stage holds two 64-wide k-blocks of 64 tokens beside two
+        of 128 features), whole tiles of 128 features (256 for the gate / up pairs of SwiGLU), rows of 16-byte multiples."""
+        return 1 <= M <= 64 and Nn % (256 if epilogue == "swiglu" else 128) == 0 and K % 8 == 0 and K >= 128
+
+    def gemm_stream(self, a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], *, epilogue: Optional[str] = None,
+                    aux: Optional[torch.Tensor] = None, a_ready: Optional[RowEvents] = None,
+                    extra_waits: Sequence[Tuple[int, int, bool, bool]] = (), rope: Optional[dict] = None,
+                    w_static: bool = False) -> RowEvents:
+        """``out = op(a @ w.T)`` for at most 64 rows (csrc/fewrow_gemm.cuh): weights on the M side of the MMA, 128
+        features per tile, the whole GEMM cut into one equal piece of the weight stream per worker. Operators as in
+        ``gemm_splitk``: None, "swiglu", "residual" (``aux``), "qk_rope" (``rope``, ``out=None``)."""
+        M, K = a.shape
+        Nn = w.shape[0]
+        mode = {None: 0, "none": 0, "swiglu": 1, "residual": 2, "qk_rope": 3}[epilogue]
+        if self.cta_pair or w.shape[1] != K or not self.can_stream(M, Nn, K, epilogue) or (mode == 3) != (out is None):
+            raise ValueError("gemm_stream: at most 64 rows, whole 128-feature tiles, one-CTA programs")
+        for t in (a, w):
+            if t.dim() != 2 or t.stride(1) != 1 or t.dtype not in (torch.bfloat16, torch.float16) or t.data_ptr() % 16 or (t.stride(0) * 2) % 16:
+                raise ValueError("gemm_stream: row-major 16-bit operands with 16-byte aligned rows")
+        out_dtype = out.dtype if out is not None else a.dtype
+        ld_o = out.stride(0) if out is not None else 0
+        if out is not None and (out.data_ptr() % 16 or (ld_o * 2) % 16 or out_dtype not in (torch.bfloat16, torch.float16)):
+            raise ValueError("gemm_stream: 16-bit output rows, 16-byte aligned")
+        if mode == 2 and (aux is None or aux.stride(0) != ld_o or aux.dtype != out_dtype or aux.data_ptr() % 16):
+            raise ValueError("gemm_stream: aux must have the output's type and row stride")
+        n_tiles, steps = Nn // 128, -(-K // 128)
+        pieces = stream_pieces(n_tiles, steps, self.num_workers)
+        tiles_per_group = 2 if mode == 1 else 1
+        n_groups = n_tiles // tiles_per_group
+        arrivals = collections.Counter(tile // tiles_per_group for tile, _, _, _ in pieces)
+        npad = -(-M // 16) * 16
+        ws = torch.zeros(M, Nn, device=a.device, dtype=torch.float32)
+        counters = torch.zeros(n_groups, device=a.device, dtype=torch.int32)
+        self.launch_state += [ws, counters]
+        par = self._rope_params(rope, M, Nn, a.device) if mode == 3 else aux
+        fin = _pack_elt(ws.data_ptr(), N.ptr(par), 0, N.ptr(out), 0, M, Nn // tiles_per_group, N.DTYPE_CODE[out_dtype], Nn, ld_o, i0=mode, i1=-1)
+        fin_dev = torch.frombuffer(bytearray(fin), dtype=torch.uint8).to(a.device)
+        self.epis.append(_pack_epilogue(ws.data_ptr(), counters.data_ptr(), fin_dev.data_ptr(), Nn, 0, EPI["fewrow"],
+                                        N.DTYPE_CODE[torch.float32], 0, 0, Nn, M, 1.0))
+        epi = len(self.epis) - 1
+        self.keepalive += [t for t in (a, w, out, aux, ws, counters, fin_dev) if t is not None]
+        tw = self._tmap(w, Nn, K, w.stride(0), False, BM)
+        tx = self._tmap(a, M, K, a.stride(0), False, npad)
+        idesc = make_idesc(1 if a.dtype == torch.bfloat16 else 0, BM, npad, 0, 0)
+        node_id = self.new_node_id()
+        waits = list(extra_waits)
+        if a_ready is not None:
+            ev, cnt = a_ready.for_rows(0, M)
+            waits.append((ev, cnt, a_ready.sys, False))
+        waits = self.join(list(dict.fromkeys(waits)), node_id)
+        done = self.new_event()
+        for tile, s0, n, wk in pieces:
+            group = tile // tiles_per_group
+            raw = _pack_gemm(tw, tx, epi, 0, 4, tile * 128, 0, s0 * 128, n, idesc, -1, group, 0, npad, count_base=arrivals[group])
+            self.add_task(int(TaskType.LINEAR), raw, waits=waits, signals=[done], node_id=node_id, worker=wk, b_static=w_static)
+        return RowEvents(rows=M, block=BM, row_events=[(done, n_groups)], all_event=(done, n_groups))
+
     def gemm_splitk(self, a: torch.Tensor, w: torch.Tensor, out: Optional[torch.Tensor], *, split_k: int = 0,
                     epilogue: Optional[str] = None, aux: Optional[torch.Tensor] = None,
                     a_ready: Optional[RowEvents] = None, extra_waits: Sequence[Tuple[int, int, bool, bool]] = (),
                     heap_out_off: Optional[int] = None, ld_out: Optional[int] = None,
                     signal_peer_event: int = -1, rows_per_task: int = 0, fused_finish: Optional[bool] = None,
-                    w_blocked: Optional[torch.Tensor] = None, rope: Optional[dict] = None) -> RowEvents:
+                    w_blocked: Optional[torch.Tensor] = None, rope: Optional[dict] = None, w_static: bool = False) -> RowEvents:
         """``out = op(a @ w.T)`` for at most 128 rows, bound by streaming ``w`` out of HBM.
+
+        Up to 64 rows with a local result (and no explicit ``split_k``, ``fused_finish=False`` or ``w_blocked``) run as
+        ``gemm_stream`` tasks; the rest of this text is about the others. ``w_static``: no task of the program writes ``w``.
 
         The K dimension is cut into ``split_k`` slices (0: enough slices for every worker to hold a tile),
         256-column tcgen05 tiles add their fp32 partial sums into one workspace with vector reductions,
@@ -726,25 +835,19 @@ class ProgramBuilder:
             raise ValueError("split-K GEMMs are not available in two-CTA programs")
         M, K = a.shape
         Nn = w.shape[0]
+        if epilogue == "qk_rope" and (rope is None or out is not None or heap_out_off is not None or fused_finish is False):
+            raise ValueError("gemm_splitk: epilogue 'qk_rope' takes rope=..., out=None, a local result and fused finishing")
+        if (split_k <= 0 and w_blocked is None and heap_out_off is None and signal_peer_event < 0 and fused_finish is not False
+                and ld_out is None and self.can_stream(M, Nn, K, epilogue)):
+            return self.gemm_stream(a, w, out, epilogue=epilogue, aux=aux, a_ready=a_ready, extra_waits=extra_waits, rope=rope,
+                                    w_static=w_static)
         if M > BM or w.shape[1] != K or Nn % 256 or K % BK:
             raise ValueError("gemm_splitk: at most 128 rows, N a multiple of 256, K a multiple of 64")
         mode = {None: 0, "none": 0, "swiglu": 1, "residual": 2, "qk_rope": 3}[epilogue]
         rope_dev = None
         if mode == 3:
-            if rope is None or out is not None or heap_out_off is not None or fused_finish is False:
-                raise ValueError("gemm_splitk: epilogue 'qk_rope' takes rope=..., out=None, a local result and fused finishing")
-            hq, hkv = int(rope["hq"]), int(rope["hkv"])
-            q_out, kc, vc = rope["q_out"], rope["k_cache"], rope["v_cache"]
-            if Nn != (hq + 2 * hkv) * 128 or kc.shape[-1] != 128 or kc.dim() != 4 or kc.shape[1] != hkv or not kc.is_contiguous() \
-                    or not vc.is_contiguous() or vc.shape != kc.shape or tuple(q_out.shape) != (M, hq, 128) or not q_out.is_contiguous() \
-                    or rope["cos_sin"].shape != (M, 128) or not (0 <= int(rope["pos"]) < kc.shape[2]):
-                raise ValueError("gemm_splitk: rope tensors do not match (hq + 2 hkv) heads of 128 and caches [M, hkv, S, 128]")
             fused_finish = True
-            blob = struct.pack("<QQQQQQqqiiiifi", q_out.data_ptr(), kc.data_ptr(), vc.data_ptr(), rope["q_norm"].data_ptr(),
-                               rope["k_norm"].data_ptr(), rope["cos_sin"].data_ptr(), kc.stride(0), kc.stride(1), hq, hkv,
-                               int(rope["pos"]), N.DTYPE_CODE[q_out.dtype], float(rope["eps"]), 0)
-            rope_dev = torch.frombuffer(bytearray(blob), dtype=torch.uint8).to(a.device)
-            self.keepalive += [rope_dev, q_out, kc, vc, rope["q_norm"], rope["k_norm"], rope["cos_sin"]]
+            rope_dev = self._rope_params(rope, M, Nn, a.device)
         n_tiles, k_blocks = Nn // 256, K // BK
         if split_k <= 0:
             split_k = pick_split_k(n_tiles, k_blocks, self.num_workers)
@@ -808,10 +911,10 @@ class ProgramBuilder:
                 raw = _pack_gemm(ta, tb, epi, 0, 2 if w_blocked is not None else 0, 0, nb * 256, kb0 * BK, kb1 - kb0, idesc,
                                  -1, 0, 0, 256, count_base=k_blocks if w_blocked is not None else 0)
                 if fused_finish:
-                    self.add_task(int(TaskType.LINEAR), raw, waits=waits, signals=[e_ws], node_id=node_id,
+                    self.add_task(int(TaskType.LINEAR), raw, waits=waits, signals=[e_ws], node_id=node_id, b_static=w_static,
                                   signal_peer=-2 if signal_peer_event >= 0 else -1, signal_peer_event=signal_peer_event)
                 else:
-                    self.add_task(int(TaskType.LINEAR), raw, waits=waits, signals=[e_ws], node_id=node_id)
+                    self.add_task(int(TaskType.LINEAR), raw, waits=waits, signals=[e_ws], node_id=node_id, b_static=w_static)
                 n_parts += 1
         if fused_finish:
             return RowEvents(rows=M, block=BM, row_events=[(e_ws, n_parts)], all_event=(e_ws, n_parts))
@@ -1017,7 +1120,8 @@ def validate_tasks(b: "ProgramBuilder") -> None:
                 bad(f"destination rank {peer} outside the world of {world}")
             if peer != -1 and out_off >= heap_bytes:
                 bad(f"tile destination offset {out_off} outside the heap of {heap_bytes} bytes")
-            if bn not in (128, 256) or k_blocks < 0:
+            few = raw[7] & 4                          # few-row task: bn = padded token count
+            if k_blocks < 0 or (bn not in (16, 32, 48, 64) if few else bn not in (128, 256)):
                 bad("bad tile width or k-block count")
         elif 200 <= t["type"] < 300 and len(raw) >= 72:
             src_off, dst_off, s_str, d_str, row_bytes, rows, _, peer, op, _, _, local_ptr = struct.unpack_from("<QQQQIIiiiiQQ", raw)
@@ -1319,9 +1423,22 @@ def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None)
     workers = min(graph.num_workers, sms - (1 if mode == "dynamic" else 0))
 
     def _few_rows(n: TaskNode) -> bool:
+        """Decode-shaped linears: a weight stream, cut along K over every SM. Above 64 rows from 4 Mi weights on (split-K
+        tiles of 256 columns), up to 64 rows from 1 Mi weights on (``gemm_stream``): below that a plain tile per 128
+        columns reads its weights in a few microseconds, which the exchange of partial sums would cost again."""
         x2, w = _flat2d(n.inputs[0]), n.inputs[1]
-        return (n.task_type == TaskType.LINEAR and not n.attrs.get("has_bias") and n.attrs.get("activation") in (None, "none", "swiglu")
-                and x2.shape[0] <= BM and w.shape[0] % 256 == 0 and x2.shape[1] % BK == 0 and w.shape[0] * w.shape[1] >= (1 << 22))
+        act = n.attrs.get("activation")
+        if n.task_type != TaskType.LINEAR or n.attrs.get("has_bias") or act not in (None, "none", "swiglu"):
+            return False
+        if ProgramBuilder.can_stream(x2.shape[0], w.shape[0], x2.shape[1], act) and w.numel() >= (1 << 20):
+            return True
+        return x2.shape[0] <= BM and w.shape[0] % 256 == 0 and x2.shape[1] % BK == 0 and w.numel() >= (1 << 22)
+
+    from ..task_graph.graph import _storage_key
+    written = {_storage_key(o) for n in graph._nodes for o in n.outputs}
+
+    def _static(t: torch.Tensor) -> bool:
+        return _storage_key(t) not in written                  # no node of the graph writes this tensor's storage
 
     gemm_nodes = [n for n in graph._nodes if n.task_type in (TaskType.LINEAR, TaskType.MATMUL) and n.outputs and n.outputs[0].numel()]
     # two-CTA tiles pay once the 256-row tiles of every GEMM cover the worker pairs; decode-shaped (split-K)
@@ -1400,11 +1517,9 @@ def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None)
                 produced[rs._node_id] = (rs, out_ev)
                 skip[rs._node_id] = True
                 continue
-            few_rows = (t == TaskType.LINEAR and bias is None and act in (None, "none", "swiglu") and x2.shape[0] <= BM
-                        and w.shape[0] % 256 == 0 and x2.shape[1] % BK == 0 and w.shape[0] * w.shape[1] >= (1 << 22))
-            if few_rows:
-                # decode-shaped linear: a weight stream, cut along K over every SM (csrc/splitk_tasks.cuh)
-                ev = b.gemm_splitk(x2, w, out2, epilogue=act if act == "swiglu" else None, a_ready=aligned, extra_waits=extra)
+            if _few_rows(node):
+                ev = b.gemm_splitk(x2, w, out2, epilogue=act if act == "swiglu" else None, a_ready=aligned, extra_waits=extra,
+                                   w_static=_static(w))
             else:
                 order = None
                 if dist and aligned is not None and aligned.sys and x2.shape[0] % (heap.world * BM) == 0:

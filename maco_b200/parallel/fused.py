@@ -339,18 +339,20 @@ def allreduce_push_tasks(b: ProgramBuilder, buf: torch.Tensor, staging: torch.Te
 def gemm_allreduce(b: ProgramBuilder, a: torch.Tensor, w: torch.Tensor, slots: Optional[torch.Tensor],
                    out: torch.Tensor, *, residual: Optional[torch.Tensor] = None, a_ready: Optional[RowEvents] = None,
                    extra_waits: Sequence[Tuple[int, int, bool, bool]] = (), bn: int = 128,
-                   reduce_rows: Optional[int] = None, w_blocked: Optional[torch.Tensor] = None) -> RowEvents:
+                   reduce_rows: Optional[int] = None, w_blocked: Optional[torch.Tensor] = None,
+                   w_static: bool = False) -> RowEvents:
     """``out = all_reduce(a @ w.T) (+ residual)`` for small row counts (decode): the GEMM epilogue stores
     every partial tile into slot ``rank`` of ALL ranks' ``slots`` [world, M, N] (one-shot exchange) and
     bumps their counters; each rank then sums its slots and the residual. With one rank the residual is
-    added in the GEMM epilogue and nothing is exchanged. ``w_blocked``: ``ops.block_weight(w)`` for the split-K form."""
+    added in the GEMM epilogue and nothing is exchanged. ``w_blocked``: ``ops.block_weight(w)`` for the split-K form.
+    ``w_static``: no task of the program writes ``w``."""
     M, Nn = a.shape[0], w.shape[0]
     heap = b.heap
     splitk = M <= BM and Nn % 256 == 0 and a.shape[1] % 64 == 0 and (residual is None or residual.stride(0) == out.stride(0))
     if heap is None or heap.world == 1:
         if splitk:
             return b.gemm_splitk(a, w, out, epilogue="residual" if residual is not None else None, aux=residual,
-                                 a_ready=a_ready, extra_waits=extra_waits, w_blocked=w_blocked)
+                                 a_ready=a_ready, extra_waits=extra_waits, w_blocked=w_blocked, w_static=w_static)
         return b.gemm(a, w, out, epilogue="residual" if residual is not None else None, aux=residual, a_ready=a_ready,
                       extra_waits=extra_waits, bn=bn)
     rank, world = heap.rank, heap.world
@@ -362,7 +364,7 @@ def gemm_allreduce(b: ProgramBuilder, a: torch.Tensor, w: torch.Tensor, slots: O
     if splitk:
         # split-K tiles over every SM; the finishing tasks write this rank's partial into slot `rank` of every rank
         fin = b.gemm_splitk(a, w, None, a_ready=a_ready, extra_waits=extra_waits, heap_out_off=off + rank * slot_bytes,
-                            ld_out=Nn, signal_peer_event=arrived, w_blocked=w_blocked)
+                            ld_out=Nn, signal_peer_event=arrived, w_blocked=w_blocked, w_static=w_static)
         n_arrive = fin.all_event[1]
     else:
         n_arrive = (Nn + bn - 1) // bn

@@ -264,3 +264,69 @@ def test_attention_decode_node_multi_chunk():
     p = torch.softmax(torch.einsum("bhgd,bhsd->bhgs", q.float().view(B, hkv, G, 128), k[:, :, :kv_len].float()) * 128 ** -0.5, -1)
     ref = torch.einsum("bhgs,bhsd->bhgd", p, v[:, :, :kv_len].float()).reshape(B, hq, 128)
     assert_close(out, ref, dt)
+
+
+@pytest.mark.parametrize("mode", ["static", "dynamic"])
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,K,Nn", [(1, 128, 256), (3, 200, 768), (16, 1536, 1024), (17, 2056, 512), (48, 1024, 2560), (64, 4096, 1280)])
+def test_stream_gemm(mode, dtype, M, K, Nn):
+    """Few-row GEMM with swapped operands: one token to the most a stage holds, padded token counts, K with a ragged last
+    step, tiles shared by several workers and workers with parts of several tiles; three launches (the workspace must be
+    zero and the arrival counters consistent again) of three operators in one program."""
+    from maco_b200.ops import interleave_gate_up, megakernel as mk
+    x = torch.randn(M, K, device="cuda", dtype=dtype)
+    w = torch.randn(Nn, K, device="cuda", dtype=dtype) * K ** -0.5
+    aux = torch.randn(M, Nn, device="cuda", dtype=dtype)
+    plain, res, act = torch.empty_like(aux), torch.empty_like(aux), torch.empty(M, Nn // 2, device="cuda", dtype=dtype)
+    b = mk.ProgramBuilder(torch.device("cuda"), mode=mode)
+    b.gemm_stream(x, w, plain)
+    b.gemm_stream(x, w, res, epilogue="residual", aux=aux, w_static=True)
+    e = b.gemm_stream(x, interleave_gate_up(w[: Nn // 2].contiguous(), w[Nn // 2:].contiguous()), act, epilogue="swiglu", w_static=True)
+    again = torch.empty(M, 256, device="cuda", dtype=dtype)
+    w2 = torch.randn(256, Nn // 2, device="cuda", dtype=dtype) * Nn ** -0.5
+    b.gemm_stream(act, w2, again, a_ready=e, w_static=True)                    # waits for every tile of the one before
+    prog = b.build()
+    for _ in range(3):
+        for t in (plain, res, act, again):
+            t.zero_()
+        prog.run()
+    torch.cuda.synchronize()
+    assert _native.status() == 0
+    acc = x.float() @ w.float().t()
+    assert_close(plain, acc, dtype)
+    assert_close(res, acc + aux.float(), dtype)
+    h = torch.nn.functional.silu(acc[:, : Nn // 2]) * acc[:, Nn // 2:]
+    assert_close(act, h, dtype)
+    assert_close(again, h.to(dtype).float() @ w2.float().t(), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("rows,cols,per", [(1, 64, 1), (3, 8192, 1), (9, 5120, 4), (130, 2048, 8), (37, 16384, 8), (5, 40000, 1)])
+def test_staged_row_and_point_tasks(dtype, rows, cols, per):
+    """Row-wise and point-wise tasks of the persistent kernel: one warp or four per row, parameters staged or read from
+    memory, one or two row buffers, rows too long for the scratch block (the unstaged form)."""
+    from maco_b200.ops import megakernel as mk
+    F = torch.nn.functional
+    x, y = (torch.randn(rows, cols, device="cuda", dtype=dtype) for _ in range(2))
+    w, bias = (torch.randn(cols, device="cuda", dtype=dtype) for _ in range(2))
+    b = mk.ProgramBuilder(torch.device("cuda"), num_workers=7)
+    outs = [torch.empty_like(x) for _ in range(6)]
+    kw = dict(rows=rows, cols=cols, rows_per_task=per)
+    b.elementwise(104, x, outs[0], in1=w, f0=1e-6, **kw)
+    b.elementwise(103, x, outs[1], in1=w, in2=bias, f0=1e-5, **kw)
+    b.elementwise(107, x, outs[2], **kw)
+    b.elementwise(105, x, outs[3], **kw)
+    b.elementwise(114, x, outs[4], in1=y, **kw)
+    b.elementwise(115, x, outs[5], in1=y, f0=0.5, f1=-2.0, **kw)
+    prog = b.build()
+    prog.run()
+    torch.cuda.synchronize()
+    assert _native.status() == 0
+    xf, yf = x.float(), y.float()
+    g = yf.clone().requires_grad_(True)
+    F.gelu(g, approximate="tanh").sum().backward()
+    refs = [xf * torch.rsqrt(xf.pow(2).mean(-1, keepdim=True) + 1e-6) * w.float(),
+            F.layer_norm(xf, (cols,), w.float(), bias.float(), 1e-5), torch.softmax(xf, -1), F.gelu(xf, approximate="tanh"),
+            xf * g.grad, 0.5 * xf - 2.0 * yf]
+    for o, r in zip(outs, refs):
+        assert_close(o, r, dtype)
