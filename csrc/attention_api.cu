@@ -1,5 +1,6 @@
-// Stand-alone split-KV decode attention: one CTA per (batch, kv-head, split) runs the same task body
-// the persistent kernel uses (attention_decode.cuh), a second launch merges the splits.
+// Stand-alone decode attention. Default: one CTA per SM streams an equal share of all (batch, kv-head, 128-key chunk)
+// triples (attn_stream_kernel), a second launch merges the ranges cut by a share's end. With a caller-chosen split count
+// or scratch: one CTA per (batch, kv-head, split) on the CUDA cores and a merge launch.
 //
 // Layouts (row-major, 16-bit):
 //   q   [B, Hq, 128]          Hq = Hkv * G query heads, the G heads of one KV head are adjacent
@@ -55,6 +56,122 @@ __global__ void __launch_bounds__(128) attn_merge_kernel(AttnParams p) {
   attn_merge_task(a, threadIdx.x);
 }
 
+// ---- streaming form --------------------------------------------------------------------------
+// 160 threads: four consumer warps and a TMA warp around a 192 KB ring, one CTA per SM. What bounds it is the HBM stream
+// of K and V; the shares are equal to one 128-key chunk, so no SM runs a second wave, and a share that ends inside a
+// (batch, kv-head) leaves a record of at most 4.2 KB. Batch 16 x 8 kv heads x 8192 keys (537 MB): 117 us through the
+// persistent kernel's former tcgen05 task, see the figures in the repository's design notes for this form.
+struct AttnStreamParams {
+  const void* q; void* out; float* scratch; uint32_t* status;
+  int Hkv, G, S, chunks_per_head, groups;
+  long long total;                                 // groups * chunks_per_head
+  float scale;
+};
+constexpr int kStreamThreads = 160;
+constexpr int kStreamSmem = 1024 + kAttnStages * kAttnStageBytes + kAttnTcScratchBytes + 128;
+
+MACO_DEVICE long long share_begin(const AttnStreamParams& p, int cta, int n) { return p.total * cta / n; }
+
+template <int DTT>
+__global__ void __launch_bounds__(kStreamThreads, 1)
+attn_stream_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV, const AttnStreamParams p) {
+  extern __shared__ uint8_t dyn_smem[];
+  uint8_t* ring = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(dyn_smem) + 1023) & ~uintptr_t(1023));
+  uint8_t* scratch = ring + kAttnStages * kAttnStageBytes;
+  uint64_t* full = reinterpret_cast<uint64_t*>(scratch + kAttnTcScratchBytes);
+  uint64_t* empty = full + kAttnStages;
+  volatile uint32_t* abort_word = reinterpret_cast<volatile uint32_t*>(empty + kAttnStages);
+  asm volatile("griddepcontrol.launch_dependents;");   // the merge waits for this grid's end anyway; its CTAs may take their places now
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < kAttnStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 4); }
+    *abort_word = 0;
+    fence_mbar_init();
+  }
+  __syncthreads();
+  constexpr uint64_t kBudgetNs = 2000000000ull;
+  const long long begin = share_begin(p, blockIdx.x, gridDim.x), end = share_begin(p, blockIdx.x + 1, gridDim.x);
+  uint32_t ait = 0;
+  const int tid = threadIdx.x;
+  bool ok = true;
+  for (long long pos = begin; pos < end && ok;) {
+    const int group = (int)(pos / p.chunks_per_head), c0 = (int)(pos - (long long)group * p.chunks_per_head);
+    const int n = (int)min((long long)(p.chunks_per_head - c0), end - pos);
+    const int key0 = c0 * 128, rows = min(p.S - key0, n * 128);
+    if (tid >= 128) {
+      if (tid == 128) {
+        const uint64_t pol = attn_evict_first();
+        const int b = group / p.Hkv, h = group - b * p.Hkv;
+        for (int i = 0; i < n && ok; ++i)
+          ok = attn_load_chunk(ring, full, empty, &tmK, &tmV, key0 + i * 128, h, b, ait, pol, kBudgetNs, abort_word);
+      }
+    } else {
+      float o[kAttnMaxG], M[kAttnMaxG], L[kAttnMaxG];
+      auto bar = [] { attn_bar(); };
+      const size_t row0 = (size_t)group * p.G * kAttnD * 2;
+      ok = attn_consume_range<DTT>(reinterpret_cast<const uint8_t*>(p.q) + row0, p.G, rows, p.scale * 1.4426950408889634f, ring, full, empty, ait,
+                                   scratch, tid, kBudgetNs, abort_word, bar, o, M, L);
+      if (ok && n == p.chunks_per_head) {
+#pragma unroll
+        for (int g = 0; g < kAttnMaxG; ++g)
+          if (g < p.G) store1(reinterpret_cast<uint8_t*>(p.out) + row0, g * kAttnD + tid, DTT, L[g] > 0.f ? o[g] / L[g] : 0.f);
+      } else if (ok) {
+        // slot 0: the range starts with the share, slot 1: it ends with it (attn_stream_merge_kernel uses the same rule)
+        attn_store_record(p.scratch + ((size_t)blockIdx.x * 2 + (pos == begin ? 0 : 1)) * (p.G * kAttnD + 2 * p.G), p.G, tid, o, M, L);
+      }
+    }
+    pos += n;
+  }
+  if (!ok && tid == 128) {                           // loads in flight land in this CTA's memory
+    const AttnPipe pp{ring, full, empty, kBudgetNs, abort_word};
+    attn_drain_loads(pp, ait);
+  }
+  __syncthreads();
+  if (tid == 0 && *abort_word != 0 && p.status != nullptr) st_relaxed_sys_u32(p.status, MACO_STATUS_TIMEOUT);
+}
+
+template <int DTT>
+__global__ void __launch_bounds__(128) attn_stream_merge_kernel(const AttnStreamParams p, int n_ctas) {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+  const int group = blockIdx.x, tid = threadIdx.x;
+  const long long first = (long long)group * p.chunks_per_head, last = first + p.chunks_per_head - 1;
+  // the CTA whose share holds chunk x: floor estimate, then exact (shares differ by at most one chunk)
+  auto owner = [&](long long x) {
+    int c = (int)(x * n_ctas / p.total);
+    while (c > 0 && share_begin(p, c, n_ctas) > x) --c;
+    while (c + 1 < n_ctas && share_begin(p, c + 1, n_ctas) <= x) ++c;
+    return c;
+  };
+  const int lo = owner(first), hi = owner(last);
+  if (lo == hi) return;                              // one share held the whole group and wrote its rows
+  const int rec = p.G * kAttnD + 2 * p.G;
+  attn_merge_records<DTT>(reinterpret_cast<uint8_t*>(p.out) + (size_t)group * p.G * kAttnD * 2, p.G, hi - lo + 1, tid, [&](int i) {
+    const int c = lo + i, slot = share_begin(p, c, n_ctas) >= first ? 0 : 1;
+    return (const float*)(p.scratch + ((size_t)c * 2 + slot) * rec);
+  });
+}
+
+template <int DTT>
+int launch_stream(const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnStreamParams& p, int grid, cudaStream_t stream) {
+  static bool attr_set[64] = {};
+  int dev = 0;
+  MACO_CHECK_CUDA(cudaGetDevice(&dev));
+  if (!attr_set[dev]) {
+    MACO_CHECK_CUDA(cudaFuncSetAttribute(attn_stream_kernel<DTT>, cudaFuncAttributeMaxDynamicSharedMemorySize, kStreamSmem));
+    attr_set[dev] = true;
+  }
+  attn_stream_kernel<DTT><<<grid, kStreamThreads, kStreamSmem, stream>>>(tmK, tmV, p);
+  MACO_CHECK_CUDA(cudaGetLastError());
+  if (p.total > grid || p.chunks_per_head > 1) {     // else every share is one whole group
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(p.groups); cfg.blockDim = dim3(128); cfg.stream = stream;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = at; cfg.numAttrs = 1;
+    MACO_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_stream_merge_kernel<DTT>, p, grid));
+  }
+  return 0;
+}
+
 int check_and_fill(AttnParams& p, const void* q, const void* k, const void* v, void* out, float* scratch, int B,
                    int Hq, int Hkv, int S, int head_dim, int splits, int dtype, long long kv_batch_stride,
                    long long kv_head_stride, float scale) {
@@ -102,6 +219,30 @@ int maco_attention_decode(const void* q, const void* k, const void* v, void* out
   attn_merge_kernel<<<B * Hkv, 128, 0, stream>>>(p);
   MACO_CHECK_CUDA(cudaGetLastError());
   return 0;
+}
+
+// Streaming form: scratch for 2 records per CTA.
+unsigned long long maco_attention_stream_scratch_bytes(int G) {
+  return (unsigned long long)maco_host::sm_count() * 2 * (G * kAttnD + 2 * G) * sizeof(float);
+}
+
+// Returns -2 when the caches cannot be addressed by a tensor map (use maco_attention_decode).
+int maco_attention_decode_stream(const void* q, const void* k, const void* v, void* out, void* scratch, int B, int Hq, int Hkv, int S,
+                                 int dtype, long long kv_batch_stride, long long kv_head_stride, float scale, void* stream_) {
+  AttnParams c;
+  int rc = check_and_fill(c, q, k, v, out, reinterpret_cast<float*>(scratch), B, Hq, Hkv, S, kAttnD, 1, dtype, kv_batch_stride, kv_head_stride, scale);
+  if (rc != 0) return rc;
+  CUtensorMap tmK, tmV;
+  if (maco_host::encode_kv_tmap(&tmK, k, S, Hkv, B, kv_head_stride, kv_batch_stride) != 0 ||
+      maco_host::encode_kv_tmap(&tmV, v, S, Hkv, B, kv_head_stride, kv_batch_stride) != 0) return -2;
+  AttnStreamParams p;
+  p.q = q; p.out = out; p.scratch = reinterpret_cast<float*>(scratch); p.status = maco_host::status_device_ptr();
+  p.Hkv = Hkv; p.G = Hq / Hkv; p.S = S; p.chunks_per_head = (S + 127) / 128; p.groups = B * Hkv;
+  p.total = (long long)p.groups * p.chunks_per_head; p.scale = scale;
+  const int sms = maco_host::sm_count();
+  const int grid = p.total < sms ? (int)p.total : sms;
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  return dtype == MACO_DT_BF16 ? launch_stream<MACO_DT_BF16>(tmK, tmV, p, grid, stream) : launch_stream<MACO_DT_F16>(tmK, tmV, p, grid, stream);
 }
 
 }  // extern "C"

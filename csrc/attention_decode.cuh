@@ -160,99 +160,279 @@ __device__ __noinline__ void attn_decode_task_t(const MacoEltArgs& ar, int tid, 
   }
 }
 
-// ---- tensor-core form (persistent kernel) -------------------------------------------------------
-// Decode attention of one (sequence, kv head, split) on the 5th-generation tensor cores, fed by the
-// worker's TMA warp:
+// ---- streaming form -----------------------------------------------------------------------------
+// Decode attention of one key range of one (sequence, kv head), bound by streaming K and V out of HBM. A TMA thread
+// brings 128-key chunks of K and V (two boxes of 64 dims x 128 keys each, 128-byte swizzle) through a ring of six 32 KB
+// stages (192 KB in flight per SM); four warps consume it. Warp w owns keys [32 w, 32 w + 32) of every chunk and
+// keeps its own softmax state, so there is no barrier among the warps before the range is done:
 //
-//   per 128-key chunk   S^T[key, head]  = K[key, :] . Q[head, :]^T      tcgen05.mma 128 x 16 x 128
-//                       P = exp(S * scale - m_ref)  (registers -> bf16/fp16 tile in shared memory)
-//                       O^T[dim, head] += V[key, dim]^T . P[head, key]  tcgen05.mma 128 x 16 x 128
+//   S^T[key, head] = K . Q^T       keys on the M = 16 side, the G <= 8 heads are the N = 8 columns
+//   P = exp2(S - m)                m is lazy: it moves only when a score exceeds it by more than kAttnLazyMargin
+//   O^T[dim, head] += V^T . P      V through ldmatrix.trans, P turned into the B operand by movmatrix
 //
-// The keys (then the head dimensions) take the M = 128 rows of the instruction and the G <= 8 query
-// heads of the group, padded to 16, its N columns, so the big operand of both products is the K / V
-// chunk exactly as TMA delivers it: K rows as a K-major A operand (two 64-dim boxes), V rows as an
-// MN-major A operand (four 64 x 64 panels). Only the small operands are built by threads: Q once per
-// task, P once per chunk, both written in the 128-byte-swizzled K-major layout the descriptors expect.
-//
-// Three roles share a task: the worker's TMA warp streams K / V (attn_produce), its MMA warp issues every
-// product (attn_mma), the four general warps do the softmax (attn_consume). A split is read once and nothing is
-// reused, so the K / V chunks go through their own ring of six 32 KB stages over the worker's operand memory
-// (192 KB in flight per SM) with barriers of their own, and the per-chunk dependency chain is kept
-// short:
-//   * scores run one chunk ahead (S double buffered in TMEM columns 0-15 / 16-31);
-//   * the softmax reference m_ref is lazy: it only moves when some score exceeds it by more than
-//     kAttnLazyMargin, which one barrier with an OR-reduction (also the "P complete" barrier) decides.
-//     While it stands still P.V accumulates in TMEM (columns 32-47) across chunks and nothing is read
-//     back; when it moves, the accumulator is drained into registers, rescaled, and restarted;
-//   * the softmax denominator is kept per thread (one key per thread) and summed once per task.
-//
-// The reference has no attention task at all (maco/csrc/maco_types.h:24-40 lists ATTENTION, the
-// worker never implements it).
-struct AttnPipe {
-  uint8_t* ring;
-  uint64_t* full;         // [kAttnStages]
-  uint64_t* empty;        // [kAttnStages]
-  uint64_t budget_ns;
-  volatile uint32_t* abort_word;
-  const CUtensorMap* tmaps;
-  uint64_t* mma_bars;     // [4]: scores ready (two buffers), P.V issued from P buffer 0 / 1 finished
-  uint32_t tmem_base;
-  uint64_t* p_ready;      // [3]: P buffer 0 / 1 staged by the softmax warps; [2]: Q tile staged (once per task)
-  volatile uint32_t* pv_flags;   // [2]: 1 = the P.V product of this buffer adds to the accumulator, 0 = it starts a new sum
-  uint32_t task_idx;      // pipelined attention tasks this worker has run before this one (parity of p_ready[2])
-};
-
+// Warp-level mma.sync on purpose. The op does 4 G flops per byte of K / V read (0.05 of the tensor rate at the HBM rate),
+// so what counts is the latency from "chunk landed" to "stage free". The tcgen05 form of this task (128 x 16 x 128
+// products from shared memory, scores read back from TMEM, P staged for all warps behind a block barrier, one thread
+// issuing) needed about 1.9 us per 64 KB chunk and SM against 1.4 us at the HBM rate; a warp's chain here (16 ldmatrix,
+// 16 + 16 mma, two exponentials per lane and key pair) takes about 0.4 us per chunk with the four warps side by side.
+// Measured for one persistent launch over 537 MB of K / V (batch 16, 8 kv heads, 8192 keys): see attention_api.cu.
 constexpr int kAttnStages = 6;
 constexpr int kAttnStageBytes = 32768;               // one 128-key chunk of K or of V
-constexpr int kAttnTileBytes = 4096;                 // 16 rows x 128 columns of 16-bit values, swizzled
-constexpr int kAttnTcScratchBytes = 1024 + 3 * kAttnTileBytes + 4 * kAttnMaxG * 4;
-constexpr float kAttnLazyMargin = 8.f;               // P <= e^8 between two moves of the reference
+constexpr int kAttnHalfBytes = 16384;                // its 64-dim half
+constexpr float kAttnLazyMargin = 11.5f;             // in log2 units: P <= 2^11.5 (e^8) between two moves of the reference
+constexpr int kAttnTcScratchBytes = 1024 + 4 * kAttnMaxG * kAttnD * 4;
 
-// ld_out carries the tensor-map indices of the K and V caches (+1 each, 16 bits each); row0 is the first
-// key's row in the flattened [rows, 128] view both maps describe.
-MACO_DEVICE bool attn_pipelined(const MacoEltArgs& a) { return a.ld_in == kAttnD && a.rows > 0 && a.ld_out != 0; }
-MACO_DEVICE uint32_t attn_stage_uses(const MacoEltArgs& a) { return 2u * (uint32_t)((a.rows + 127) / 128); }
-
-// Producer side: called by one thread. `ait` counts the stage uses of the attention ring on this worker.
-// Called by all 32 lanes of the producer warp, converged. Lane 0 waits for the two stages of a chunk (K, then V)
-// to be free and arms their barriers; lanes 0-5 then issue the chunk's six boxes with one warp instruction: lanes
-// 0, 1 the two 64-dim halves of the 128 keys of K, lanes 2-5 the (64-key block, 64-dim half) boxes of V. One thread
-// alone issues only a few TMA operations per microsecond, which capped this stream at about 4 TB/s over the GPU.
-// `ait` advances identically in every lane.
-MACO_DEVICE bool attn_produce(const MacoEltArgs& ar, const AttnPipe& pp, uint32_t& ait, uint32_t lane) {
-  const MacoEltArgs a = ar;
-  const CUtensorMap* tmK = pp.tmaps + ((a.ld_out & 0xffff) - 1);
-  const CUtensorMap* tmV = pp.tmaps + (((uint32_t)a.ld_out >> 16) - 1);
-  const bool is_k = lane < 2;
-  const uint32_t vb = lane - 2;                                       // V box: bit 0 dim half, bit 1 key block
-  const CUtensorMap* tm = is_k ? tmK : tmV;
-  const int x = is_k ? (int)lane * 64 : (int)(vb & 1u) * 64;
-  const int y_off = is_k ? 0 : (int)(vb >> 1) * 64;
-  const uint32_t s_off = is_k ? lane * 16384u : (vb >> 1) * 16384u + (vb & 1u) * 8192u;
-  for (int base = 0; base < a.rows; base += 128) {
-    const int y = a.row0 + base;
-    const uint32_t sk = ait % kAttnStages, phk = (ait / kAttnStages) & 1;
-    const uint32_t sv = (ait + 1) % kAttnStages, phv = ((ait + 1) / kAttnStages) & 1;
-    uint32_t good = 1;
-    if (lane == 0) {
-      good = (mbar_wait(&pp.empty[sk], phk ^ 1, pp.budget_ns, pp.abort_word) &&
-              mbar_wait(&pp.empty[sv], phv ^ 1, pp.budget_ns, pp.abort_word)) ? 1u : 0u;
-      if (good) {
-        mbar_arrive_expect_tx(&pp.full[sk], kAttnStageBytes);
-        mbar_arrive_expect_tx(&pp.full[sv], kAttnStageBytes);
-      }
-    }
-    good = __shfl_sync(0xffffffffu, good, 0);
-    if (!good) return false;
-    if (lane < 6) {
-      const uint32_t s = is_k ? sk : sv;
-      tma_load_2d(pp.ring + (size_t)s * kAttnStageBytes + s_off, tm, &pp.full[s], x, y + y_off);
-    }
-    __syncwarp();
-    ait += 2;
+// K / V tensor maps: 4-D (dim, key, head, batch); a chunk that runs past the last key reads zeros.
+MACO_DEVICE void attn_load_box(void* dst, const void* tmap, uint64_t* bar, int x, int key, int head, int batch, uint64_t pol) {
+  asm volatile(
+      "cp.async.bulk.tensor.4d.shared::cta.global.mbarrier::complete_tx::bytes.L2::cache_hint [%0], [%1, {%3, %4, %5, %6}], [%2], %7;"
+      :: "r"(smem_u32(dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(x), "r"(key), "r"(head), "r"(batch), "l"(pol) : "memory");
+}
+MACO_DEVICE uint64_t attn_evict_first() {            // every K / V row is read once
+  uint64_t pol;
+  asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
+  return pol;
+}
+// Both stages of one chunk (K, then V); one thread. `ait` counts stage uses.
+MACO_DEVICE bool attn_load_chunk(uint8_t* ring, uint64_t* full, uint64_t* empty, const void* tmK, const void* tmV, int key, int head, int batch,
+                                 uint32_t& ait, uint64_t pol, uint64_t budget_ns, volatile uint32_t* abort_word) {
+#pragma unroll
+  for (int kv = 0; kv < 2; ++kv, ++ait) {
+    const uint32_t s = ait % kAttnStages;
+    if (!mbar_wait(&empty[s], ((ait / kAttnStages) & 1) ^ 1, budget_ns, abort_word)) return false;
+    mbar_arrive_expect_tx(&full[s], kAttnStageBytes);
+    uint8_t* dst = ring + (size_t)s * kAttnStageBytes;
+    const void* tm = kv == 0 ? tmK : tmV;
+    attn_load_box(dst, tm, &full[s], 0, key, head, batch, pol);
+    attn_load_box(dst + kAttnHalfBytes, tm, &full[s], 64, key, head, batch, pol);
   }
   return true;
 }
+
+MACO_DEVICE float attn_ex2(float x) { float r; asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x)); return r; }
+MACO_DEVICE void ldsm_x4(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+MACO_DEVICE void ldsm_x4_trans(uint32_t addr, uint32_t (&r)[4]) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0, %1, %2, %3}, [%4];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(addr) : "memory");
+}
+MACO_DEVICE uint32_t movmatrix_trans(uint32_t a) {
+  uint32_t d;
+  asm volatile("movmatrix.sync.aligned.m8n8.trans.b16 %0, %1;" : "=r"(d) : "r"(a));
+  return d;
+}
+template <int DTT>
+MACO_DEVICE void mma_16816(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  if constexpr (DTT == MACO_DT_BF16)
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+  else
+    asm volatile("mma.sync.aligned.m16n8k16.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+                 : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
+}
+
+// 128 threads: attention of `rows` keys for the G query rows at `q`. On return (all threads behind a barrier) thread
+// `tid` holds output dimension `tid` of every head: o[g] unnormalised, under the reference M[g] (log2 units) with
+// denominator L[g]. `ait`: ring uses before this range (advanced); `bar`: barrier of the 128 threads.
+template <int DTT, typename BarFn>
+MACO_DEVICE bool attn_consume_range(const void* q, int G, int rows, float scale_log2, uint8_t* ring, uint64_t* full, uint64_t* empty,
+                                    uint32_t& ait, uint8_t* scratch, int tid, uint64_t budget_ns, volatile uint32_t* abort_word, BarFn bar,
+                                    float (&o)[kAttnMaxG], float (&M)[kAttnMaxG], float (&L)[kAttnMaxG]) {
+  const int warp = tid >> 5, lane = tid & 31, hc = 2 * (lane & 3);     // this lane's two heads (columns of S^T and O^T)
+  uint32_t qf[8][2];                                 // Q as the B operand: head lane / 4, dims 16 k + 2 (lane % 4) + {0, 1, 8, 9}
+  {
+    const uint32_t* qrow = reinterpret_cast<const uint32_t*>(q) + (lane >> 2) * (kAttnD / 2) + (lane & 3);
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+#pragma unroll
+      for (int h = 0; h < 2; ++h) qf[k][h] = (lane >> 2) < G ? qrow[k * 8 + h * 4] : 0u;
+  }
+  float acc[8][4];                                   // O^T: dims 16 t + lane / 4 (+ 8), heads hc, hc + 1
+#pragma unroll
+  for (int t = 0; t < 8; ++t)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[t][j] = 0.f;
+  float m0 = -INFINITY, m1 = -INFINITY, l0 = 0.f, l1 = 0.f;
+  // ldmatrix row addresses inside a 64-dim half: K rows in order, V rows with the two 8-key blocks on the upper lanes
+  const uint32_t k_row = (uint32_t)(warp * 32 + (lane & 15)), k_chunk = (uint32_t)(lane >> 4);
+  const uint32_t v_row = (uint32_t)(warp * 32 + (lane & 7) + ((lane >> 4) & 1) * 8), v_chunk = (uint32_t)((lane >> 3) & 1);
+  const uint32_t ring_s = smem_u32(ring);
+  const uint32_t ait_end = ait + 2u * (uint32_t)((rows + 127) / 128);
+  bool ok;
+#pragma unroll 1
+  for (int base = 0; base < rows; base += 128, ait += 2) {
+    const int n_w = rows - base - warp * 32;         // keys of this warp in the chunk (may be <= 0 or more than 32)
+    const uint32_t sk = ait % kAttnStages, sv = (ait + 1) % kAttnStages;
+    if (!mbar_wait(&full[sk], (ait / kAttnStages) & 1, budget_ns, abort_word)) break;
+    uint32_t pb[2][2];
+    if (n_w > 0) {
+      float s[2][4];
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) s[t][j] = 0.f;
+      const uint32_t kb = ring_s + sk * kAttnStageBytes + k_row * 128;
+#pragma unroll
+      for (int k = 0; k < 8; ++k) {
+        const uint32_t off = (uint32_t)(k >> 2) * kAttnHalfBytes + (((((uint32_t)k & 3) * 2 + k_chunk) ^ (k_row & 7)) << 4);
+#pragma unroll
+        for (int t = 0; t < 2; ++t) {
+          uint32_t a[4];
+          ldsm_x4(kb + t * 2048 + off, a);
+          mma_16816<DTT>(s[t], a, qf[k][0], qf[k][1]);
+        }
+      }
+      __syncwarp();
+      if (lane == 0) mbar_arrive(&empty[sk]);
+      float mx0 = -INFINITY, mx1 = -INFINITY;
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int key = t * 16 + (lane >> 2) + (j >> 1) * 8;
+          s[t][j] = key < n_w ? s[t][j] * scale_log2 : -INFINITY;
+          if (j & 1) mx1 = fmaxf(mx1, s[t][j]); else mx0 = fmaxf(mx0, s[t][j]);
+        }
+      if (__any_sync(0xffffffffu, mx0 > m0 + kAttnLazyMargin || mx1 > m1 + kAttnLazyMargin)) {
+#pragma unroll
+        for (int d = 4; d < 32; d <<= 1) {
+          mx0 = fmaxf(mx0, __shfl_xor_sync(0xffffffffu, mx0, d));
+          mx1 = fmaxf(mx1, __shfl_xor_sync(0xffffffffu, mx1, d));
+        }
+        const float n0 = fmaxf(m0, mx0), n1 = fmaxf(m1, mx1);
+        const float c0 = m0 == -INFINITY ? 0.f : attn_ex2(m0 - n0), c1 = m1 == -INFINITY ? 0.f : attn_ex2(m1 - n1);
+        l0 *= c0; l1 *= c1;
+#pragma unroll
+        for (int t = 0; t < 8; ++t) { acc[t][0] *= c0; acc[t][1] *= c1; acc[t][2] *= c0; acc[t][3] *= c1; }
+        m0 = n0; m1 = n1;
+      }
+#pragma unroll
+      for (int t = 0; t < 2; ++t)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          // the product uses the rounded probabilities; the denominator sums the same ones
+          const float p0 = attn_ex2(s[t][2 * h] - m0), p1 = attn_ex2(s[t][2 * h + 1] - m1);
+          uint32_t w;
+          float2 r;
+          if constexpr (DTT == MACO_DT_BF16) { w = pack_bf16x2(p0, p1); r = unpack_bf16x2(w); }
+          else { const __half2 hh = __floats2half2_rn(p0, p1); w = *reinterpret_cast<const uint32_t*>(&hh); r = __half22float2(hh); }
+          l0 += r.x; l1 += r.y;
+          pb[t][h] = movmatrix_trans(w);             // (key, head pair) -> (head, key pair): the B operand
+        }
+    } else if (lane == 0) {
+      mbar_arrive(&empty[sk]);
+    }
+    if (!mbar_wait(&full[sv], ((ait + 1) / kAttnStages) & 1, budget_ns, abort_word)) break;
+    if (n_w > 0) {
+      const uint32_t vb = ring_s + sv * kAttnStageBytes + v_row * 128;
+#pragma unroll
+      for (int t = 0; t < 8; ++t) {
+        const uint32_t off = (uint32_t)(t >> 2) * kAttnHalfBytes + (((((uint32_t)t & 3) * 2 + v_chunk) ^ (v_row & 7)) << 4);
+#pragma unroll
+        for (int kt = 0; kt < 2; ++kt) {
+          uint32_t a[4];
+          ldsm_x4_trans(vb + kt * 2048 + off, a);
+          mma_16816<DTT>(acc[t], a, pb[kt][0], pb[kt][1]);
+        }
+      }
+      __syncwarp();
+    }
+    if (lane == 0) mbar_arrive(&empty[sv]);
+  }
+  ait = ait_end;
+  // combine the four warps: {m, l} per head and O per (head, dim) through shared memory
+#pragma unroll
+  for (int d = 4; d < 32; d <<= 1) {
+    l0 += __shfl_xor_sync(0xffffffffu, l0, d);
+    l1 += __shfl_xor_sync(0xffffffffu, l1, d);
+  }
+  float* red = reinterpret_cast<float*>(scratch);    // [4 warps][8 heads] m, then l; O behind it
+  float* ro = red + 256;
+  if (lane < 4) {
+    red[warp * 8 + hc] = m0; red[warp * 8 + hc + 1] = m1;
+    red[32 + warp * 8 + hc] = l0; red[32 + warp * 8 + hc + 1] = l1;
+  }
+#pragma unroll
+  for (int t = 0; t < 8; ++t)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      ro[(warp * kAttnMaxG + hc + (j & 1)) * kAttnD + t * 16 + (lane >> 2) + (j >> 1) * 8] = acc[t][j];
+  bar();
+  // one verdict for all threads (a wait that ran out has set the abort word): callers leave or go on together
+  if (tid == 0) red[128] = *abort_word != 0 ? 1.f : 0.f;
+#pragma unroll
+  for (int g = 0; g < kAttnMaxG; ++g) {
+    M[g] = fmaxf(fmaxf(red[g], red[8 + g]), fmaxf(red[16 + g], red[24 + g]));
+    o[g] = 0.f; L[g] = 0.f;
+#pragma unroll
+    for (int w = 0; w < 4; ++w) {
+      const float c = red[w * 8 + g] == -INFINITY ? 0.f : attn_ex2(red[w * 8 + g] - M[g]);
+      L[g] += red[32 + w * 8 + g] * c;
+      o[g] += ro[(w * kAttnMaxG + g) * kAttnD + tid] * c;
+    }
+  }
+  bar();
+  ok = red[128] == 0.f;
+  bar();                                             // scratch may be used again
+  return ok;
+}
+
+// One record {o[G][128], m[G], l[G]} (m in log2 units) of a key range.
+MACO_DEVICE void attn_store_record(float* rec, int G, int tid, const float (&o)[kAttnMaxG], const float (&M)[kAttnMaxG], const float (&L)[kAttnMaxG]) {
+#pragma unroll
+  for (int g = 0; g < kAttnMaxG; ++g) {
+    if (g < G) {
+      rec[g * kAttnD + tid] = o[g];
+      if (tid == g) { rec[G * kAttnD + g] = M[g]; rec[G * kAttnD + G + g] = L[g]; }
+    }
+  }
+}
+// Output rows from n records; `rec_of(i)` is the address of record i. Loads of one record are independent of each other.
+template <int DTT, typename RecFn>
+MACO_DEVICE void attn_merge_records(void* out, int G, int n, int tid, RecFn rec_of) {
+  float M[kAttnMaxG], L[kAttnMaxG], acc[kAttnMaxG];
+#pragma unroll
+  for (int g = 0; g < kAttnMaxG; ++g) { M[g] = -INFINITY; L[g] = 0.f; acc[g] = 0.f; }
+#pragma unroll 1
+  for (int i = 0; i < n; ++i) {
+    const float* r = rec_of(i);
+    float ms[kAttnMaxG], ls[kAttnMaxG], os[kAttnMaxG];
+#pragma unroll
+    for (int g = 0; g < kAttnMaxG; ++g) {
+      ms[g] = g < G ? __ldcg(r + G * kAttnD + g) : -INFINITY;
+      ls[g] = g < G ? __ldcg(r + G * kAttnD + G + g) : 0.f;
+      os[g] = g < G ? __ldcg(r + g * kAttnD + tid) : 0.f;
+    }
+#pragma unroll
+    for (int g = 0; g < kAttnMaxG; ++g) {
+      const float m = fmaxf(M[g], ms[g]);
+      const float a = M[g] == -INFINITY ? 0.f : attn_ex2(M[g] - m), b = ms[g] == -INFINITY ? 0.f : attn_ex2(ms[g] - m);
+      L[g] = L[g] * a + ls[g] * b;
+      acc[g] = acc[g] * a + os[g] * b;
+      M[g] = m;
+    }
+  }
+#pragma unroll
+  for (int g = 0; g < kAttnMaxG; ++g)
+    if (g < G) store1(out, g * kAttnD + tid, DTT, L[g] > 0.f ? acc[g] / L[g] : 0.f);
+}
+
+// ---- the task of the persistent kernel: one key range of one (sequence, kv head) ----------------------------------
+//   in0 = q rows, in1 = arrival counter of the (sequence, kv head), in2 = output rows, out = this range's record
+//   row0 = first key, rows = keys, cols = index of the (sequence, kv head), f0 = softmax scale, f1 = index of the range,
+//   i0 = G | first key a task of this program writes << 8 (0: every key waits for the task's conditions), i1 = ranges
+//   ld_in = 128 and ld_out = tensor-map indices of K and V (+1 each, 16 bits each) mark this form
+struct AttnPipe {
+  uint8_t* ring;
+  uint64_t* full;         // [kAttnStages]
+  uint64_t* empty;        // [kAttnStages], four arrivals (one per consumer warp)
+  uint64_t budget_ns;
+  volatile uint32_t* abort_word;
+};
+MACO_DEVICE bool attn_pipelined(const MacoEltArgs& a) { return a.ld_in == kAttnD && a.rows > 0 && a.ld_out != 0; }
+MACO_DEVICE uint32_t attn_stage_uses(const MacoEltArgs& a) { return 2u * (uint32_t)((a.rows + 127) / 128); }
 
 // Waits (bounded) until the last uses of the attention ring have been released by the consumer: the
 // operand memory may then be handed to another pipeline.
@@ -272,282 +452,38 @@ MACO_DEVICE void attn_drain_loads(const AttnPipe& pp, uint32_t ait) {
   }
 }
 
-// Byte offset of element (row, col) inside a 16-row x 128-column K-major tile of 16-bit values stored
-// as two 64-column atoms with the 128-byte swizzle (the tile's base is 1024-byte aligned).
-MACO_DEVICE uint32_t attn_tile_off(int row, int col) {
-  return (uint32_t)((col >> 6) * 2048 + (row >> 3) * 1024 + (row & 7) * 128 + ((((col & 63) >> 3) ^ (row & 7)) << 4) + (col & 7) * 2);
-}
-
-// Maximum over the warp in one instruction (sm_100a).
-MACO_DEVICE float warp_max_redux(float v) {
-  float r;
-  asm volatile("redux.sync.max.f32 %0, %1, 0xffffffff;" : "=f"(r) : "f"(v));
-  return r;
-}
-
-// Barrier of the 128 general threads that also ORs a predicate over them.
-MACO_DEVICE bool attn_bar_or(bool pred) {
-  uint32_t r;
-  asm volatile("{\n .reg .pred p, q;\n setp.ne.u32 q, %1, 0;\n bar.red.or.pred p, 1, 128, q;\n selp.u32 %0, 1, 0, p;\n}"
-               : "=r"(r) : "r"((uint32_t)pred) : "memory");
-  return r != 0;
-}
-
-// Softmax side: all 128 general threads; they wait for scores, stage P and post "P staged", and never issue a
-// tensor-core product themselves (attn_mma does, on the MMA warp). `ait`: this task's first use of the attention
-// ring (kept for symmetry with the other two roles). `chunk_seq` counts the chunks this worker has processed
-// (buffer index and parity of the MMA barriers); every thread keeps its own copy.
-template <int DTT>
-__device__ __noinline__ bool attn_consume_t(const MacoEltArgs& ar, int tid, uint8_t* scratch, const AttnPipe& pp, uint32_t ait,
-                                            uint32_t& chunk_seq) {
+// 128 general threads. The range that arrives last at the group's counter combines all of them (no separate merge task,
+// no extra dependency hop); the counter only grows: i1 arrivals per launch.
+template <int DTT, typename BarFn>
+__device__ __noinline__ bool attn_task_t(const MacoEltArgs& ar, int tid, uint8_t* scratch, const AttnPipe& pipe, uint32_t& ait, volatile uint32_t* word,
+                                         BarFn bar) {
   const MacoEltArgs a = ar;
-  const int G = a.i0 < kAttnMaxG ? a.i0 : kAttnMaxG;
-  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(scratch) + 1023) & ~uintptr_t(1023));
-  uint8_t* q_t = tiles;                                  // Q  [16 heads][128 dims]
-  uint8_t* p_t = tiles + kAttnTileBytes;                 // P  [2][16 heads][128 keys]
-  float* red_m = reinterpret_cast<float*>(tiles + 3 * kAttnTileBytes);
-  const int lane = tid & 31;
-  const int quarter = ((tid >> 5) + 2) & 3;              // TMEM lane quarter this warp may read (warp id mod 4)
-  const int row = quarter * 32 + lane;                   // key of the chunk, then output dimension, of this thread
-  const int wslot = tid >> 5;
-  // Q: 16 x 16 vectors of 16 bytes; rows >= G are zero. P: zero everywhere (rows >= G stay zero).
-  for (int i = tid; i < 256; i += 128) {
-    const int r = i >> 4, v = i & 15;
-    uint4 u = make_uint4(0, 0, 0, 0);
-    if (r < G) u = reinterpret_cast<const uint4*>(a.in0)[r * 16 + v];
-    *reinterpret_cast<uint4*>(q_t + attn_tile_off(r, v * 8)) = u;
-    *reinterpret_cast<uint4*>(p_t + i * 16) = make_uint4(0, 0, 0, 0);
-    *reinterpret_cast<uint4*>(p_t + kAttnTileBytes + i * 16) = make_uint4(0, 0, 0, 0);
-  }
-  fence_proxy_async_smem();
-  float m_ref[kAttnMaxG], l_thr[kAttnMaxG], o[kAttnMaxG];
+  const AttnPipe pp = pipe;
+  const int G = a.i0 & 0xff, S = a.i1;
+  float o[kAttnMaxG], M[kAttnMaxG], L[kAttnMaxG];
+  if (!attn_consume_range<DTT>(a.in0, G, a.rows, a.f0 * 1.4426950408889634f, pp.ring, pp.full, pp.empty, ait, scratch, tid, pp.budget_ns,
+                               pp.abort_word, bar, o, M, L)) return false;
+  void* out = const_cast<void*>(a.in2);
+  if (S <= 1) {
 #pragma unroll
-  for (int g = 0; g < kAttnMaxG; ++g) { m_ref[g] = -INFINITY; l_thr[g] = 0.f; o[g] = 0.f; }
-  attn_bar();
-  if (tid == 0) mbar_arrive(&pp.p_ready[2]);             // Q and the zeroed P buffers are in place: the MMA warp may start
-  bool ok = true;
-  bool acc_live = false;                                 // TMEM holds P.V sums not yet drained (same in every thread)
-  const uint32_t t_lane = (uint32_t)(quarter * 32) << 16;
-  const uint32_t t_o = pp.tmem_base + 32;
-  const int chunks = (a.rows + 127) / 128;
-
-  // every thread: waits for the P.V of chunk `seq` (and all before it), then o += accumulator
-  auto drain_output = [&](uint32_t seq) {
-    if (!mbar_wait(&pp.mma_bars[2 + (seq & 1)], (seq >> 1) & 1, pp.budget_ns, pp.abort_word)) ok = false;
-    tc_fence_after();
-    uint32_t r[16];
-    if (ok) { tmem_ld_32x16(t_o + t_lane, r); tmem_ld_wait(); }
-#pragma unroll
-    for (int g = 0; g < kAttnMaxG; ++g) o[g] += (ok && g < G) ? __uint_as_float(r[g]) : 0.f;
-    tc_fence_before();
-  };
-  // every thread: P[g][row] = exp(s - m_ref) rounded to the operand type; returns the rounded values
-  auto store_p = [&](uint8_t* p_buf, const float (&s)[kAttnMaxG], float (&pr)[kAttnMaxG]) {
-#pragma unroll
-    for (int g = 0; g < kAttnMaxG; ++g) {
-      float pj = (g < G && m_ref[g] != -INFINITY) ? __expf(s[g] - m_ref[g]) : 0.f;
-      if (g < G) {
-        // the product uses the rounded value; the denominator sums the same one, so the two agree
-        if (DTT == MACO_DT_BF16) {
-          const __nv_bfloat16 h = __float2bfloat16_rn(pj);
-          *reinterpret_cast<__nv_bfloat16*>(p_buf + attn_tile_off(g, row)) = h;
-          pj = __bfloat162float(h);
-        } else {
-          const __half h = __float2half_rn(pj);
-          *reinterpret_cast<__half*>(p_buf + attn_tile_off(g, row)) = h;
-          pj = __half2float(h);
-        }
-      }
-      pr[g] = pj;
-    }
-    fence_proxy_async_smem();
-  };
-
-  for (int c = 0; c < chunks; ++c, ++chunk_seq) {
-    const int nk = min(128, a.rows - c * 128);
-    const bool valid = row < nk;
-    const uint32_t seq = chunk_seq, buf = seq & 1, par = (seq >> 1) & 1;
-    if (!mbar_wait(&pp.mma_bars[buf], par, pp.budget_ns, pp.abort_word)) ok = false;
-    tc_fence_after();
-    float s[kAttnMaxG], pr[kAttnMaxG];
-    {
-      uint32_t r[16];
-      if (ok) { tmem_ld_32x16(pp.tmem_base + buf * 16 + t_lane, r); tmem_ld_wait(); }
-#pragma unroll
-      for (int g = 0; g < kAttnMaxG; ++g) s[g] = (ok && valid && g < G) ? __uint_as_float(r[g]) * a.f0 : -INFINITY;
-    }
-    tc_fence_before();
-    // the P buffer is free once the product issued from it two chunks ago has finished
-    if (c >= 2 && !mbar_wait(&pp.mma_bars[2 + buf], ((seq - 2) >> 1) & 1, pp.budget_ns, pp.abort_word)) ok = false;
-    uint8_t* p_buf = p_t + buf * kAttnTileBytes;
-    bool exceed = false;
-#pragma unroll
-    for (int g = 0; g < kAttnMaxG; ++g) exceed |= s[g] > m_ref[g] + kAttnLazyMargin;
-    store_p(p_buf, s, pr);
-    if (attn_bar_or(exceed)) {                    // P complete, and: does the reference have to move?
-#pragma unroll
-      for (int g = 0; g < kAttnMaxG; ++g) {
-        const float mx = warp_max_redux(s[g]);
-        if (lane == g) red_m[wslot * kAttnMaxG + g] = mx;
-      }
-      if (acc_live) drain_output(seq - 1);        // sums under the old reference leave TMEM
-      attn_bar();
-#pragma unroll
-      for (int g = 0; g < kAttnMaxG; ++g) {
-        const float cm = fmaxf(fmaxf(red_m[g], red_m[kAttnMaxG + g]), fmaxf(red_m[2 * kAttnMaxG + g], red_m[3 * kAttnMaxG + g]));
-        const float m_new = fmaxf(m_ref[g], cm);
-        const float corr = (m_ref[g] == -INFINITY) ? 0.f : __expf(m_ref[g] - m_new);
-        o[g] *= corr;
-        l_thr[g] *= corr;
-        m_ref[g] = m_new;
-      }
-      store_p(p_buf, s, pr);
-      acc_live = false;
-      attn_bar();                                 // P complete under the new reference; red_m free
-    }
-#pragma unroll
-    for (int g = 0; g < kAttnMaxG; ++g) l_thr[g] += pr[g];
-    // P of this chunk is staged (the barrier above ordered every thread's stores and proxy fence): hand it to
-    // the MMA warp, which issues the P.V product as soon as the chunk's V rows have landed
-    if (tid == 0) {
-      pp.pv_flags[buf] = acc_live ? 1u : 0u;
-      mbar_arrive(&pp.p_ready[buf]);
-    }
-    acc_live = true;
-  }
-  drain_output(chunk_seq - 1);
-  // softmax denominator: one CTA-wide sum per head
-#pragma unroll
-  for (int g = 0; g < kAttnMaxG; ++g) {
-    const float sm = warp_sum(l_thr[g]);
-    if (lane == 0) red_m[wslot * kAttnMaxG + g] = sm;
-  }
-  attn_bar();
-  float* out = reinterpret_cast<float*>(a.out);
-  const int S = a.i1;                              // splits of this (sequence, kv head); the last one to finish merges
-  uint32_t* counter = reinterpret_cast<uint32_t*>(const_cast<void*>(a.in1));
-  if (S <= 1 && counter != nullptr) {
-    // a single split: normalise and write the final rows directly
-#pragma unroll
-    for (int g = 0; g < kAttnMaxG; ++g) {
-      if (g < G) {
-        const float l = red_m[g] + red_m[kAttnMaxG + g] + red_m[2 * kAttnMaxG + g] + red_m[3 * kAttnMaxG + g];
-        store1(const_cast<void*>(a.in2), g * kAttnD + row, DTT, l > 0.f ? o[g] / l : 0.f);
-      }
-    }
-  } else {
-#pragma unroll
-    for (int g = 0; g < kAttnMaxG; ++g) if (g < G) out[g * kAttnD + row] = o[g];
-    if (tid < G) {
-      float mg = -INFINITY;
-#pragma unroll
-      for (int g = 0; g < kAttnMaxG; ++g) if (g == tid) mg = m_ref[g];
-      out[G * kAttnD + tid] = mg;
-      out[G * kAttnD + G + tid] = red_m[tid] + red_m[kAttnMaxG + tid] + red_m[2 * kAttnMaxG + tid] + red_m[3 * kAttnMaxG + tid];
-    }
-    if (counter != nullptr) {
-      // The split that arrives last at the group's counter combines all S records (no separate merge
-      // task, no extra dependency hop). The counter only grows: S arrivals per launch.
-      __threadfence();                             // this thread's part of the record is visible GPU-wide
-      attn_bar();
-      __shared__ uint32_t s_last;
-      if (tid == 0) s_last = ((atomicAdd(counter, 1u) + 1u) % (uint32_t)S) == 0u ? 1u : 0u;
-      attn_bar();
-      if (s_last != 0u) {
-        __threadfence();
-        const int rec = G * kAttnD + 2 * G;
-        const float* part = out - (size_t)(int)a.f1 * rec;      // record of split 0 of this group
-        float M[kAttnMaxG], L[kAttnMaxG], acc[kAttnMaxG];
-#pragma unroll
-        for (int g = 0; g < kAttnMaxG; ++g) { M[g] = -INFINITY; L[g] = 0.f; acc[g] = 0.f; }
-        for (int sp = 0; sp < S; ++sp) {
-#pragma unroll
-          for (int g = 0; g < kAttnMaxG; ++g) if (g < G) M[g] = fmaxf(M[g], __ldcg(part + sp * rec + G * kAttnD + g));
-        }
-        for (int sp = 0; sp < S; ++sp) {
-          float ms[kAttnMaxG], ls[kAttnMaxG], os[kAttnMaxG];
-#pragma unroll
-          for (int g = 0; g < kAttnMaxG; ++g) {
-            ms[g] = g < G ? __ldcg(part + sp * rec + G * kAttnD + g) : -INFINITY;
-            ls[g] = g < G ? __ldcg(part + sp * rec + G * kAttnD + G + g) : 0.f;
-            os[g] = g < G ? __ldcg(part + sp * rec + g * kAttnD + row) : 0.f;
-          }
-#pragma unroll
-          for (int g = 0; g < kAttnMaxG; ++g) {
-            const float w = (ms[g] == -INFINITY) ? 0.f : __expf(ms[g] - M[g]);
-            L[g] += ls[g] * w;
-            acc[g] += os[g] * w;
-          }
-        }
-#pragma unroll
-        for (int g = 0; g < kAttnMaxG; ++g)
-          if (g < G) store1(const_cast<void*>(a.in2), g * kAttnD + row, DTT, L[g] > 0.f ? acc[g] / L[g] : 0.f);
-      }
-    }
-  }
-  attn_bar();                                     // red_m is free again
-  return ok;
-}
-
-// MMA side of the task: one thread (the worker's MMA warp, idle during an attention task otherwise) issues every
-// tensor-core product, so the softmax warps never issue one. Per chunk c: scores S(c+1) = K(c+1) Q^T as soon as the
-// chunk's K rows have landed (into the score buffer the softmax warps left two chunks ago), then, when the softmax
-// warps have staged P(c), O (+)= V(c)^T P(c). With the issue inside the softmax loop, one thread's instruction stream
-// (two waits, 16 descriptor pairs, 16 MMAs, 4 commits per chunk) sat on the critical path of all 128 threads and
-// held a worker at about 23 GB/s of K/V.
-// `ait`, `chunk_seq`: this worker's ring uses and chunks before this task (same counts as the consumer's).
-MACO_DEVICE bool attn_mma(const MacoEltArgs& ar, uint8_t* scratch, const AttnPipe& pp, uint32_t ait, uint32_t chunk_seq) {
-  const MacoEltArgs a = ar;
-  uint8_t* tiles = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(scratch) + 1023) & ~uintptr_t(1023));
-  const uint32_t q_addr = smem_u32(tiles), p_addr = smem_u32(tiles + kAttnTileBytes);
-  const uint32_t fmt = a.dtype == MACO_DT_BF16 ? 1u : 0u;
-  const uint32_t idesc_s = make_idesc(fmt, 128, 16, 0, 0);
-  const uint32_t idesc_o = make_idesc(fmt, 128, 16, 1, 0);
-  const uint32_t t_o = pp.tmem_base + 32;
-  const int chunks = (a.rows + 127) / 128;
-  if (!mbar_wait(&pp.p_ready[2], pp.task_idx & 1u, pp.budget_ns, pp.abort_word)) return false;
-  auto issue_scores = [&](int c, uint32_t seq) -> bool {
-    const uint32_t u = ait + 2u * (uint32_t)c, sk = u % kAttnStages, phk = (u / kAttnStages) & 1;
-    if (!mbar_wait(&pp.full[sk], phk, pp.budget_ns, pp.abort_word)) return false;
-    tc_fence_after();
-    const uint32_t k_addr = smem_u32(pp.ring + (size_t)sk * kAttnStageBytes);
-    const uint32_t t_s = pp.tmem_base + (seq & 1) * 16;
-#pragma unroll
-    for (int k = 0; k < kAttnD / 16; ++k) {
-      const uint64_t adesc = make_smem_desc(k_addr + (k >> 2) * 16384 + (k & 3) * 32, 16, 1024, 2);
-      const uint64_t bdesc = make_smem_desc(q_addr + (k >> 2) * 2048 + (k & 3) * 32, 16, 1024, 2);
-      tc_mma_f16(t_s, adesc, bdesc, idesc_s, k != 0 ? 1u : 0u);
-    }
-    tc_commit(&pp.empty[sk]);
-    tc_commit(&pp.mma_bars[seq & 1]);
+    for (int g = 0; g < kAttnMaxG; ++g)
+      if (g < G) store1(out, g * kAttnD + tid, DTT, L[g] > 0.f ? o[g] / L[g] : 0.f);
     return true;
-  };
-  if (!issue_scores(0, chunk_seq)) return false;
-  for (int c = 0; c < chunks; ++c) {
-    const uint32_t seq = chunk_seq + (uint32_t)c, buf = seq & 1, par = (seq >> 1) & 1;
-    if (c + 1 < chunks && !issue_scores(c + 1, seq + 1)) return false;
-    if (!mbar_wait(&pp.p_ready[buf], par, pp.budget_ns, pp.abort_word)) return false;
-    const uint32_t accum = pp.pv_flags[buf];
-    const uint32_t u = ait + 2u * (uint32_t)c + 1u, sv = u % kAttnStages, phv = (u / kAttnStages) & 1;
-    if (!mbar_wait(&pp.full[sv], phv, pp.budget_ns, pp.abort_word)) return false;
-    tc_fence_after();
-    const uint32_t v_addr = smem_u32(pp.ring + (size_t)sv * kAttnStageBytes);
-    const uint32_t pb = p_addr + buf * kAttnTileBytes;
-#pragma unroll
-    for (int k = 0; k < 128 / 16; ++k) {
-      const uint64_t adesc = make_smem_desc(v_addr + (k >> 2) * 16384 + (k & 3) * 2048, 8192, 1024, 2);
-      const uint64_t bdesc = make_smem_desc(pb + (k >> 2) * 2048 + (k & 3) * 32, 16, 1024, 2);
-      tc_mma_f16(t_o, adesc, bdesc, idesc_o, (k != 0 || accum != 0) ? 1u : 0u);
-    }
-    tc_commit(&pp.empty[sv]);
-    tc_commit(&pp.mma_bars[2 + buf]);
+  }
+  float* rec = reinterpret_cast<float*>(a.out);
+  attn_store_record(rec, G, tid, o, M, L);
+  bar();
+  if (tid == 0) {
+    uint32_t* counter = reinterpret_cast<uint32_t*>(const_cast<void*>(a.in1));
+    *word = ((atom_add_acq_rel_gpu_u32(counter, 1u) + 1u) % (uint32_t)S) == 0u ? 1u : 0u;
+  }
+  bar();
+  if (*word != 0u) {
+    const int n = G * kAttnD + 2 * G;
+    const float* first = rec - (size_t)(int)a.f1 * n;
+    attn_merge_records<DTT>(out, G, S, tid, [=](int i) { return first + (size_t)i * n; });
   }
   return true;
-}
-
-MACO_DEVICE bool attn_consume(const MacoEltArgs& a, int tid, uint8_t* scratch, const AttnPipe& pp, uint32_t it, uint32_t& chunk_seq) {
-  if (a.dtype == MACO_DT_BF16) return attn_consume_t<MACO_DT_BF16>(a, tid, scratch, pp, it, chunk_seq);
-  return attn_consume_t<MACO_DT_F16>(a, tid, scratch, pp, it, chunk_seq);
 }
 
 MACO_DEVICE void attn_decode_task(const MacoEltArgs& a, int tid, uint8_t* scratch) {

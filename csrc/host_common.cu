@@ -54,6 +54,25 @@ int encode_tmap_2d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t 
   return 0;
 }
 
+int encode_kv_tmap(CUtensorMap* out, const void* base, int keys, int heads, int batch, long long head_stride, long long batch_stride) {
+  EncodeTiledFn enc = get_encode();
+  if (enc == nullptr) { set_error("cuTensorMapEncodeTiled is not available (no CUDA driver?)"); return -1; }
+  if ((reinterpret_cast<uintptr_t>(base) & 15) != 0 || head_stride % 8 != 0 || batch_stride % 8 != 0) {
+    set_error("K / V tensor map: base address and strides must be multiples of 16 bytes");
+    return -2;
+  }
+  cuuint64_t dims[4] = {128, (cuuint64_t)keys, (cuuint64_t)heads, (cuuint64_t)batch};
+  cuuint64_t strides[3] = {256, (cuuint64_t)head_stride * 2, (cuuint64_t)batch_stride * 2};
+  cuuint32_t box[4] = {64, 128, 1, 1}, estr[4] = {1, 1, 1, 1};
+  CUresult r = enc(out, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 4, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                   CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) {
+    set_error("cuTensorMapEncodeTiled failed with " + std::to_string((int)r) + " (K / V map)");
+    return -3;
+  }
+  return 0;
+}
+
 // One status block per device, allocated on first use in host-mapped pinned memory so the host
 // can read what a kernel reported without a copy.
 static MacoStatusBlock* g_status_host[64] = {};

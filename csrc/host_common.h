@@ -28,6 +28,10 @@ const char* last_error();
 int encode_tmap_2d(CUtensorMap* out, const void* base, int elem_bytes, uint64_t rows, uint64_t cols,
                    uint64_t row_stride_bytes, uint32_t box_cols, uint32_t box_rows);
 
+// 4-D map (dim 128, key, head, batch) over a K or V cache of 16-bit elements with contiguous 128-element rows; strides in
+// elements. A box is 64 dims x 128 keys of one head, 128-byte swizzle; keys past the end read as zeros.
+int encode_kv_tmap(CUtensorMap* out, const void* base, int keys, int heads, int batch, long long head_stride, long long batch_stride);
+
 // Device pointer of the per-process status block (host-mapped, zero-copy) and its host view.
 uint32_t* status_device_ptr();
 MacoStatusBlock* status_host_ptr();

@@ -321,12 +321,7 @@ __device__ void mma_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_base,
   }
 }
 
-// ---- producer warp ------------------------------------------------------------------------------
-// All 32 lanes walk the task sequence together. Lane 0 owns every decision and every side effect (queue reads,
-// dependency waits, GEMM loads); its verdicts are broadcast with shuffles. The other lanes exist for one thing:
-// the K / V stream of a decode-attention task is six TMA boxes per 64 KB chunk, and one thread issues a few TMA
-// operations per microsecond only; lanes 0-5 issue the six boxes with ONE warp instruction.
-
+// ---- producer warp (lane 0) ---------------------------------------------------------------------
 // A few-row GEMM task on lane 0: the weights (operand A here) of up to a whole ring go out before the task waits for its
 // tokens, unless a task of the program writes them.
 __device__ int producer_few_task(const MacoProgram& p, const MacoTaskDesc& d, uint32_t task, uint8_t* smem, const GemmCtrl& c,
@@ -400,70 +395,65 @@ __device__ int producer_gemm_task(const MacoProgram& p, const MacoTaskDesc& d, u
   return ok ? 1 : 0;
 }
 
+// The K / V stream of a decode-attention task: chunks below the first key that a task of the program writes (the new
+// token's cache row) go out before the task's conditions hold. 1 = carry on, 0 = stop.
+__device__ int producer_attn_task(const MacoProgram& p, const MacoTaskDesc& d, uint32_t task, const CUtensorMap* tmaps, const AttnPipe& pp,
+                                  uint32_t& ait) {
+  const MacoEltArgs& a = d.u.elt;
+  const CUtensorMap* tmK = tmaps + ((a.ld_out & 0xffff) - 1);
+  const CUtensorMap* tmV = tmaps + (((uint32_t)a.ld_out >> 16) - 1);
+  const uint64_t pol = attn_evict_first();
+  const int fixed = a.i0 >> 8, row0 = a.row0, rows = a.rows, bh = a.cols;
+  bool waited = false, ok = true;
+  for (int base = 0; ok && base < rows; base += 128) {
+    if (!waited && row0 + min(base + 128, rows) > fixed) {
+      if (!wait_deps(p, d, task, pp.abort_word, nullptr)) return 0;
+      fence_proxy_async_all();
+      waited = true;
+    }
+    ok = attn_load_chunk(pp.ring, pp.full, pp.empty, tmK, tmV, row0 + base, bh, 0, ait, pol, pp.budget_ns, pp.abort_word);
+  }
+  if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, pp.abort_word);
+  return ok ? 1 : 0;
+}
+
 __device__ void producer_role(const MacoProgram& p, uint32_t w, uint32_t q_base, uint8_t* smem, const GemmCtrl& c,
                               uint64_t* attn_ring_bars, MacoTaskDesc* desc_slots) {
-  const uint32_t lane = threadIdx.x & 31;
   TaskStream ts;
-  if (lane == 0) ts.start(p, desc_slots, w, q_base);
-  uint32_t it = 0;                   // stage uses of the GEMM ring (lane 0)
-  uint32_t ait = 0;                  // stage uses of the attention ring (same memory); every lane keeps the same count
-  int owner = 0;                     // lane 0: which pipeline used the operand memory last: 1 GEMM, 2 attention
-  bool ok = true;                    // uniform over the warp
+  ts.start(p, desc_slots, w, q_base);
+  uint32_t it = 0;                   // stage uses of the GEMM ring
+  uint32_t ait = 0;                  // stage uses of the attention ring (same memory)
+  int owner = 0;                     // which pipeline used the operand memory last: 1 GEMM, 2 attention
+  bool ok = true;
   const CUtensorMap* tmaps = reinterpret_cast<const CUtensorMap*>(p.tmaps);
-  const AttnPipe apipe{smem, attn_ring_bars, attn_ring_bars + kAttnStages, p.budget_ns, c.abort_word, tmaps, nullptr, 0,
-                       nullptr, nullptr, 0};
-  for (uint32_t i = 0; ok; ++i) {
-    uint32_t task = 0, verdict = 0;  // 0 run, 1 end of queue, 2 failure
-    if (lane == 0) {
-      bool failed = false;
-      if (ts.next(p, task, failed, c.abort_word) == nullptr) verdict = failed ? 2u : 1u;
-    }
-    verdict = __shfl_sync(0xffffffffu, verdict, 0);
-    if (verdict == 2) { ok = false; break; }
-    if (verdict == 1) break;
-    const MacoTaskDesc& d = desc_slots[i & (kStreamSlots - 1)];
+  const AttnPipe apipe{smem, attn_ring_bars, attn_ring_bars + kAttnStages, p.budget_ns, c.abort_word};
+  while (ok) {
+    uint32_t task;
+    bool failed = false;
+    const MacoTaskDesc* dp = ts.next(p, task, failed, c.abort_word);
+    if (dp == nullptr) { ok = !failed; break; }
+    const MacoTaskDesc& d = *dp;
     if (d.type == MACO_TASK_ATTENTION && attn_pipelined(d.u.elt)) {
-      // K / V rows of the split stream through the operand ring; the general warps consume them
-      uint32_t go = 1;               // 1 produce, 0 stop silently (the wait reported), 2 stop and report
-      if (lane == 0) {
-        if (!wait_deps(p, d, task, c.abort_word, nullptr)) {
-          go = 0;
-        } else {
-          fence_proxy_async_all();
-          if (owner == 1) {          // the MMA warp may still be reading the last GEMM stages out of this memory
-            bool free_ok = true;
-            for (uint32_t u = it > (uint32_t)kMkStages ? it - kMkStages : 0; u < it && free_ok; ++u)
-              free_ok = mbar_wait(&c.empty[u % kMkStages], (u / kMkStages) & 1, p.budget_ns, c.abort_word);
-            if (!free_ok) go = 2;
-          }
-          owner = 2;
-        }
+      if (owner == 1) {              // the MMA warp may still be reading the last GEMM stages out of this memory
+        for (uint32_t u = it > (uint32_t)kMkStages ? it - kMkStages : 0; u < it && ok; ++u)
+          ok = mbar_wait(&c.empty[u % kMkStages], (u / kMkStages) & 1, p.budget_ns, c.abort_word);
+        if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
       }
-      go = __shfl_sync(0xffffffffu, go, 0);
-      if (go == 1 && !attn_produce(d.u.elt, apipe, ait, lane)) go = 2;
-      if (go != 1) {
-        if (go == 2 && lane == 0) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
-        ok = false;
-      }
-      continue;
+      owner = 2;
+      ok = ok && producer_attn_task(p, d, task, tmaps, apipe, ait) != 0;
+    } else if (is_gemm_type(d.type)) {
+      ok = producer_gemm_task(p, d, task, smem, c, tmaps, apipe, ait, it, owner) != 0;
     }
-    if (!is_gemm_type(d.type)) continue;
-    uint32_t carry_on = 1;
-    if (lane == 0) carry_on = (uint32_t)producer_gemm_task(p, d, task, smem, c, tmaps, apipe, ait, it, owner);
-    carry_on = __shfl_sync(0xffffffffu, carry_on, 0);
-    if (carry_on == 0) ok = false;
   }
-  if (!ok && lane == 0) { gemm_drain_loads<kMkStages>(c, it); attn_drain_loads(apipe, ait); }
+  if (!ok) { gemm_drain_loads<kMkStages>(c, it); attn_drain_loads(apipe, ait); }
 }
 
 // ---- MMA warp (lane 0) --------------------------------------------------------------------------
 __device__ void mma_role(const MacoProgram& p, uint32_t w, uint32_t q_base, uint8_t* smem, const GemmCtrl& c,
-                         uint32_t tmem_base, volatile uint32_t* attn_done, uint64_t* attn_bars, uint64_t* p_ready,
-                         volatile uint32_t* pv_flags, uint8_t* scratch_smem, MacoTaskDesc* desc_slots) {
+                         uint32_t tmem_base, MacoTaskDesc* desc_slots) {
   TaskStream ts;
   ts.start(p, desc_slots, w, q_base);
-  uint32_t it = 0, seq = 0, attn_seen = 0;
-  uint32_t ait = 0, attn_chunks = 0;   // attention ring uses / chunks so far: the same counts the general warps keep
+  uint32_t it = 0, seq = 0;
   bool ok = true;
   while (ok) {
     uint32_t task;
@@ -471,30 +461,6 @@ __device__ void mma_role(const MacoProgram& p, uint32_t w, uint32_t q_base, uint
     const MacoTaskDesc* dp = ts.next(p, task, failed, c.abort_word);
     if (dp == nullptr) break;
     const MacoTaskDesc& d = *dp;
-    if (d.type == MACO_TASK_ATTENTION && attn_pipelined(d.u.elt)) {
-      // The attention task issues its own tensor-core products into the low TMEM columns: this warp must
-      // not start the next GEMM tile's accumulator there before the general warps have finished the task
-      // (CTA-local counter).
-      {
-        // this warp issues the task's tensor-core products (scores and P.V), the general warps do the softmax
-        const AttnPipe pipe{smem, attn_bars + 4, attn_bars + 4 + kAttnStages, p.budget_ns, c.abort_word, nullptr, attn_bars,
-                            tmem_base, p_ready, pv_flags, attn_seen};
-        if (!attn_mma(d.u.elt, scratch_smem, pipe, ait, attn_chunks)) {
-          report_failure(p, MACO_STATUS_TIMEOUT, task, 0xfffffffeu, c.abort_word);
-          ok = false;
-          break;
-        }
-        ait += attn_stage_uses(d.u.elt);
-        attn_chunks += (uint32_t)((d.u.elt.rows + 127) / 128);
-      }
-      ++attn_seen;
-      const uint64_t t0 = globaltimer_ns();
-      while ((int32_t)(*attn_done - attn_seen) < 0) {
-        if (*c.abort_word != 0 || globaltimer_ns() - t0 > p.budget_ns) { ok = false; break; }
-        __nanosleep(64);
-      }
-      continue;
-    }
     if (!is_gemm_type(d.type)) continue;
     const MacoGemmArgs& g = d.u.gemm;
     if (d.flags & MACO_TF_COUNTED) {
@@ -545,7 +511,7 @@ __device__ __noinline__ void run_moe(const MacoProgram& p, uint32_t type, const 
 template <int CG>
 __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, const GemmCtrl& c, uint32_t tmem_base,
                              volatile uint32_t* slots, uint8_t* scratch_smem, uint8_t* ring_smem, uint64_t* bulk_bars,
-                             uint64_t* attn_bars, uint64_t* attn_p_ready, MacoTaskDesc* desc_slots) {
+                             uint64_t* attn_bars, MacoTaskDesc* desc_slots) {
   const int tid = threadIdx.x - 64;          // 0..127
   // two-CTA programs: the epilogue warps of both CTAs report "accumulator drained" to the leader's barrier
   uint32_t pair_empty_bar = 0;
@@ -556,9 +522,7 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
   // Communication workers never get GEMM tasks, so their operand ring is free to stage bulk copies.
   const bool comm_worker = p.num_comm_workers > 0 && w >= p.num_workers - p.num_comm_workers;
   BulkCtx bulk{ring_smem, bulk_bars, kBulkBuffers, kBulkBufBytes, slots + 12};   // phase word: zeroed at kernel start
-  uint32_t seq = 0, done = 0, it = 0;      // it: ring stages consumed so far (kept in step with the TMA and MMA warps)
-  uint32_t attn_chunks = 0, ait = 0;       // attention chunks done (parity of its MMA barriers), uses of its ring
-  uint32_t attn_tasks = 0;                 // pipelined attention tasks done (parity of the "Q staged" barrier)
+  uint32_t seq = 0, done = 0, ait = 0;     // accumulators drained, tasks done, uses of the attention ring
   enum : uint32_t { kEnd = 0, kRun = 1, kSkip = 2, kStop = 3 };
   for (uint32_t i = 0;; ++i) {
     volatile uint32_t* cur = slots + (i & 1u) * 4;     // [0] verdict on the task, [2] failure, [3] last arrival
@@ -620,7 +584,6 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
       else ok = gemm_epilogue_tile<256, kMkBN>(c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, bcp, stage, pair_empty_bar, row_limit);
       if (!ok) cur[2] = 1;
       ++seq;
-      it += (uint32_t)g.k_blocks;
       if (e.mode == MACO_EPI_SPLITK_FUSED) {
         // Split-K with the finishing pass folded in: every tile adds its partial sums to the workspace and then
         // arrives at its column tile's counter; whoever arrives last finds all K slices summed and finishes the
@@ -658,16 +621,13 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
       }
     } else if (d.type == MACO_TASK_ATTENTION && attn_pipelined(d.u.elt)) {
       if constexpr (CG == 1) {
-        const AttnPipe pipe{ring_smem, attn_bars + 4, attn_bars + 4 + kAttnStages, p.budget_ns, c.abort_word,
-                            nullptr, attn_bars, tmem_base, attn_p_ready, slots + 20, attn_tasks};
-        if (!attn_consume(d.u.elt, tid, scratch_smem, pipe, ait, attn_chunks)) cur[2] = 1;
-        ait += attn_stage_uses(d.u.elt);
-        ++attn_tasks;
-        general_bar();
-        if (leader) slots[13] = slots[13] + 1;                 // lets the MMA warp move past this task
+        const AttnPipe pipe{ring_smem, attn_bars, attn_bars + kAttnStages, p.budget_ns, c.abort_word};
+        auto bar = [] { general_bar(); };
+        const bool ok = d.u.elt.dtype == MACO_DT_BF16 ? attn_task_t<MACO_DT_BF16>(d.u.elt, tid, scratch_smem, pipe, ait, cur + 3, bar)
+                                                      : attn_task_t<MACO_DT_F16>(d.u.elt, tid, scratch_smem, pipe, ait, cur + 3, bar);
+        if (!ok) cur[2] = 1;
       } else {
-        // the tensor-core attention task issues one-CTA MMAs; a kernel has one cta_group (the builder
-        // keeps such tasks out of two-CTA programs)
+        // (the builder keeps attention tasks out of two-CTA programs: their producer role has no K / V stream)
         cur[2] = 1;
         if (leader) report_failure(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word);
       }
@@ -802,16 +762,12 @@ __device__ __forceinline__ void persistent_body(const MacoProgram& p) {
     const uint32_t w = blockIdx.x;
     // All roles must start from the same ring position: one thread reads it before anyone can move it.
     uint64_t* bulk_bars = reinterpret_cast<uint64_t*>(extra + 32);          // bytes 128.. of the extra block
-    uint64_t* attn_bars = reinterpret_cast<uint64_t*>(extra + 64);          // bytes 256..383: 4 MMA barriers, then full[6], empty[6] of the K/V ring
-    uint64_t* attn_p_ready = reinterpret_cast<uint64_t*>(extra + 96);       // bytes 384..407: P staged (two buffers), Q staged; words 20, 21: P.V accumulate flags
+    uint64_t* attn_bars = reinterpret_cast<uint64_t*>(extra + 64);          // bytes 256..351: full[6], empty[6] of the K / V ring
     if (threadIdx.x == 0) {
       extra[16] = p.mode == MACO_MODE_DYNAMIC ? ld_relaxed_gpu_u32(&p.tails[w]) : 0;
       extra[12] = 0;                                                     // parity bits of the bulk barriers
-      extra[13] = 0;                                                     // pipelined attention tasks finished
       for (uint32_t b = 0; b < kBulkBuffers; ++b) mbar_init(&bulk_bars[b], 1);
-      for (int b = 0; b < 4 + 2 * kAttnStages; ++b) mbar_init(&attn_bars[b], 1);   // attention: 4 MMA barriers, ring full / empty
-      for (int b = 0; b < 3; ++b) mbar_init(&attn_p_ready[b], 1);
-      extra[20] = 0; extra[21] = 0;
+      for (int b = 0; b < kAttnStages; ++b) { mbar_init(&attn_bars[b], 1); mbar_init(&attn_bars[kAttnStages + b], 4); }
       fence_mbar_init();
     }
     __syncthreads();
@@ -821,19 +777,18 @@ __device__ __forceinline__ void persistent_body(const MacoProgram& p) {
       if constexpr (CG == 2) {
         if (lane == 0) producer_role_pair(p, w, q_base, smem, c, desc_slots);
       } else {
-        producer_role(p, w, q_base, smem, c, attn_bars + 4, desc_slots);          // all 32 lanes (see the role)
+        if (lane == 0) producer_role(p, w, q_base, smem, c, attn_bars, desc_slots);
       }
       __syncwarp();
     } else if (warp == 1) {
       if (lane == 0) {
         if constexpr (CG == 2) { if (cluster_ctarank() == 0) mma_role_pair(p, w, q_base, smem, c, tmem_base, desc_slots + kStreamSlots); }
-        else mma_role(p, w, q_base, smem, c, tmem_base, extra + 13, attn_bars, attn_p_ready, extra + 20,
-                      reinterpret_cast<uint8_t*>(extra) + kMkExtraSmem, desc_slots + kStreamSlots);
+        else mma_role(p, w, q_base, smem, c, tmem_base, desc_slots + kStreamSlots);
       }
       __syncwarp();
     } else {
       general_role<CG>(p, w, q_base, c, tmem_base, extra, reinterpret_cast<uint8_t*>(extra) + kMkExtraSmem, smem, bulk_bars, attn_bars,
-                       attn_p_ready, desc_slots + 2 * kStreamSlots);
+                       desc_slots + 2 * kStreamSlots);
     }
   } else {
     if constexpr (CG == 1) { if (warp == 0) scheduler_role(p, extra); }
@@ -907,6 +862,11 @@ int maco_encode_operand_tmap(void* out, const void* base, int rows_or_k, int col
   // K-major operand [rows, K]: box = 64 (K) x box_rows. MN-major operand stored [K, rows]: box = 64 (rows) x 64 (K).
   if (!mn_major) return maco_host::encode_tmap_2d(tm, base, 2, rows_or_k, cols, ld_elems * 2, kBK, box_rows);
   return maco_host::encode_tmap_2d(tm, base, 2, rows_or_k, cols, ld_elems * 2, 64, kBK);
+}
+
+// K or V cache of a decode-attention task: [groups, keys, 128], rows of 256 bytes, groups `group_stride` elements apart.
+int maco_encode_kv_tmap(void* out, const void* base, int keys, int groups, long long group_stride) {
+  return maco_host::encode_kv_tmap(reinterpret_cast<CUtensorMap*>(out), base, keys, groups, 1, group_stride, group_stride * groups);
 }
 
 int maco_program_launch(const MacoProgram* prog, void* stream_) {

@@ -79,6 +79,8 @@ def _lib():
         lib.maco_abi_sizes.argtypes = [ctypes.POINTER(I)] * 6
         lib.maco_encode_operand_tmap.restype = I
         lib.maco_encode_operand_tmap.argtypes = [P, P, I, I, LL, I, I]
+        lib.maco_encode_kv_tmap.restype = I
+        lib.maco_encode_kv_tmap.argtypes = [P, P, I, I, LL]
         lib.maco_program_launch.restype = I
         lib.maco_program_launch.argtypes = [ctypes.POINTER(_ProgramStruct), P]
         lib.maco_persistent_smem_bytes.restype = I
@@ -547,6 +549,20 @@ class ProgramBuilder:
         self._tmap_cache[key] = len(self.tmaps) - 1
         return len(self.tmaps) - 1
 
+    def _kv_tmap(self, cache: torch.Tensor, kv_len: int) -> int:
+        """Tensor map of a contiguous K or V cache [B, hkv, S, 128] whose first ``kv_len`` rows per head are valid (rows past
+        them read as zeros)."""
+        B, hkv, S, D = cache.shape
+        key = ("kv", cache.data_ptr(), B * hkv, S, kv_len)
+        idx = self._tmap_cache.get(key)
+        if idx is None:
+            buf = ctypes.create_string_buffer(128)
+            if self.device.type == "cuda":                 # (planning mode: the contents do not matter)
+                N.check(_lib().maco_encode_kv_tmap(buf, cache.data_ptr(), kv_len, B * hkv, S * D), "maco_encode_kv_tmap")
+            self.tmaps.append(buf.raw)
+            idx = self._tmap_cache[key] = len(self.tmaps) - 1
+        return idx
+
     # ------------------------------------------------------------------ GEMM node
     def add_epilogue(self, out_ptr: int, ld_out: int, out_dtype: torch.dtype, M: int, Nn: int, *, mode: str = None,
                      aux_ptr: int = 0, ld_aux: int = 0, aux_dtype: Optional[torch.dtype] = None, alpha: float = 1.0,
@@ -948,12 +964,15 @@ class ProgramBuilder:
     # ------------------------------------------------------------------ decode attention node
     def attention_decode(self, q: torch.Tensor, k_cache: torch.Tensor, v_cache: torch.Tensor, out: torch.Tensor, *,
                          kv_len: Optional[int] = None, splits: int = 1, scale: Optional[float] = None,
-                         waits: Sequence[Tuple[int, int, bool, bool]] = (), balance: bool = False) -> Tuple[int, int]:
+                         waits: Sequence[Tuple[int, int, bool, bool]] = (), balance: bool = False,
+                         new_from: Optional[int] = None) -> Tuple[int, int]:
         """Split-KV decode attention: q [B, hq, D] against caches [B, hkv, S, D] -> out [B, hq, D].
 
+        ``new_from``: first key position that a task of this program writes (the new token's cache row): chunks below it are
+        loaded before ``waits`` hold. None: every key may be written by the program.
         One ATTENTION task per (sequence, kv head, split) writes an fp32 partial {o, m, l}. 16-bit caches
         run on the tensor cores (csrc/attention_decode.cuh), fed by TMA through tensor maps over the
-        flattened caches, and the split that finishes last for a (sequence, kv head) combines the records
+        caches, and the split that finishes last for a (sequence, kv head) combines the records
         itself; other element types use the CUDA-core task plus one ATTN_MERGE task per (sequence, kv
         head), emitted after all attention tasks (with static queues a merge placed right behind its
         splits would hold its worker idle until the neighbours finish theirs).
@@ -978,10 +997,9 @@ class ProgramBuilder:
         self.keepalive += [q, k_cache, v_cache, out, partials]
         tm_kv = 0
         if es == 2:
-            rows_total = B * hkv * S
-            tk = self._tmap(k_cache.view(rows_total, D), rows_total, D, D, False, BM)
-            tv = self._tmap(v_cache.view(rows_total, D), rows_total, D, D, True, 64)
-            tm_kv = (tk + 1) | ((tv + 1) << 16)
+            tm_kv = (self._kv_tmap(k_cache, kv_len) + 1) | ((self._kv_tmap(v_cache, kv_len) + 1) << 16)
+            if not 0 <= (new_from or 0) < (1 << 23):
+                raise ValueError("attention_decode: new_from out of range")
         waits = self.join(list(waits))
         per = -(-kv_len // splits)
         splits = -(-kv_len // per)                         # every split holds at least one key
@@ -1009,11 +1027,10 @@ class ProgramBuilder:
                 bi, j = divmod(bh, hkv)
                 sp = idx_in_group[bh]
                 idx_in_group[bh] += 1
-                row = (bi * hkv + j) * S + s0
                 # records of a group are consecutive: the piece index minus its position is the group's first record
                 raw = _pack_elt(q.data_ptr() + (bi * hq + j * G) * D * es, counters.data_ptr() + bh * 4,
                                 out.data_ptr() + (bi * hq + j * G) * D * es, partials.data_ptr() + pi * rec * 4,
-                                row, keys, D, dt, D, tm_kv, f0=scale, f1=float(sp), i0=G, i1=n_of[bh])
+                                s0, keys, bh, dt, D, tm_kv, f0=scale, f1=float(sp), i0=G | ((new_from or 0) << 8), i1=n_of[bh])
                 self.add_task(int(TaskType.ATTENTION), raw, waits=waits, signals=[merged], worker=wk)
             return merged, len(pieces)
         merges = []

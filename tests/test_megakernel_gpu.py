@@ -330,3 +330,33 @@ def test_staged_row_and_point_tasks(dtype, rows, cols, per):
             xf * g.grad, 0.5 * xf - 2.0 * yf]
     for o, r in zip(outs, refs):
         assert_close(o, r, dtype)
+
+
+@pytest.mark.parametrize("mode", ["static", "dynamic"])
+@pytest.mark.parametrize("kv_len,balance", [(1, True), (127, False), (300, True), (1037, True)])
+def test_attention_task_with_keys_written_by_the_program(mode, kv_len, balance):
+    """The last key's cache row is written by a task of the same program (everything below it may be loaded before that);
+    cache rows past kv_len hold NaN."""
+    from maco_b200.ops import megakernel as mk
+    dt = torch.bfloat16
+    B, hq, hkv, S = 3, 16, 2, 1100
+    q = torch.randn(B, hq, 128, device="cuda", dtype=dt)
+    k, v = (torch.randn(B, hkv, S, 128, device="cuda", dtype=dt) for _ in range(2))
+    k[:, :, kv_len - 1:], v[:, :, kv_len - 1:] = float("nan"), float("nan")
+    new_k, new_v = (torch.randn(B * hkv, 128, device="cuda", dtype=dt) for _ in range(2))
+    out = torch.empty_like(q)
+    b = mk.ProgramBuilder(torch.device("cuda"), mode=mode)
+    ev = b.new_event()
+    for src, cache in ((new_k, k), (new_v, v)):
+        b.elementwise(300, src, cache.view(B * hkv, S, 128)[:, kv_len - 1], rows=B * hkv, cols=128, ld_in=128, ld_out=S * 128,
+                      rows_per_task=B * hkv, all_event=ev)
+    b.attention_decode(q, k, v, out, kv_len=kv_len, splits=2, waits=[(ev, 2, False, False)], balance=balance, new_from=kv_len - 1)
+    prog = b.build()
+    for _ in range(3):
+        out.zero_()
+        prog.run()
+    torch.cuda.synchronize()
+    assert _native.status() == 0
+    kk, vv = k[:, :, :kv_len].float(), v[:, :, :kv_len].float()
+    p = torch.softmax(torch.einsum("bhgd,bhsd->bhgs", q.float().view(B, hkv, 8, 128), kk) * 128 ** -0.5, -1)
+    assert_close(out, torch.einsum("bhgs,bhsd->bhgd", p, vv).reshape(B, hq, 128), dt)

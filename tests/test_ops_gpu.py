@@ -193,3 +193,28 @@ def test_attention_decode(dtype, cfg):
         ops.attention_decode(q, k, v, out=out2)
         torch.cuda.synchronize()
         assert_close(out2, ref, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("B,Hkv,G,S,extra", [(1, 1, 8, 1, 0), (2, 2, 4, 127, 3), (1, 4, 1, 128, 0), (3, 2, 7, 129, 200), (2, 8, 8, 1300, 36),
+                                             (70, 4, 2, 40, 5), (1, 1, 4, 40000, 0), (5, 3, 8, 513, 0)])
+def test_attention_decode_streaming(dtype, B, Hkv, G, S, extra):
+    """Shares that cover several heads, one head, a part of one; ragged chunks; the filled part of a longer cache whose other
+    rows hold NaN; scores that make the lazy softmax reference move late."""
+    ops = _ops()
+    q = torch.randn(B, Hkv * G, 128, device="cuda", dtype=dtype)
+    k = torch.randn(B, Hkv, S + extra, 128, device="cuda", dtype=dtype)
+    v = torch.randn(B, Hkv, S + extra, 128, device="cuda", dtype=dtype)
+    k[:, :, S - S // 8 - 1: S] *= 4.0
+    if extra:
+        k[:, :, S:], v[:, :, S:] = float("nan"), float("nan")
+    k, v = k[:, :, :S], v[:, :, :S]
+    s = torch.einsum("bhgd,bhsd->bhgs", q.float().view(B, Hkv, G, 128), k.float()) * 128 ** -0.5
+    ref = torch.einsum("bhgs,bhsd->bhgd", torch.softmax(s, -1), v.float()).reshape(B, Hkv * G, 128)
+    out = torch.empty_like(q)
+    for res in (ops.attention_decode(q, k, v), ops.attention_decode(q, k, v, out=out), out):
+        # bf16 / fp16 probabilities and output: 2^-8 / 2^-11 of the result, the sums are fp32
+        rel = ((res.float() - ref).norm() / ref.norm()).item()
+        assert rel < (1e-2 if dtype == torch.bfloat16 else 2e-3), rel
+    from maco_b200 import _native
+    assert _native.status() == 0
