@@ -1,11 +1,11 @@
 // Host launchers for the GEMM operators.
 //
 //   maco_gemm        tcgen05 / TMEM / TMA pipeline (bf16 or fp16 inputs, 16-byte aligned rows)
-//   maco_gemm_simt   CUDA-core tiled GEMM for fp32 inputs and for shapes TMA cannot address
+//   maco_gemm_simt   CUDA cores: fp32 inputs (gemm_f32.cuh), and 16-bit inputs that TMA cannot address
 //
 // Both compute D = epilogue(alpha * op(A) · op(B)^T) with A logically [M,K] and B logically
 // [N,K]; `a_mn` / `b_mn` say that the operand is stored transposed ([K,M] / [K,N] row-major).
-#include "gemm_tcgen05.cuh"
+#include "gemm_f32.cuh"
 #include "host_common.h"
 
 using namespace maco;
@@ -104,9 +104,8 @@ int dispatch_major_pair(bool a_mn, bool b_mn, const CUtensorMap& tmA, const CUte
   return launch_gemm_pair<BN, true, true>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
 }
 
-// ---- CUDA-core GEMM: 64x64 tile, 256 threads, 4x4 outputs per thread ---------------------------
+// ---- CUDA-core GEMM for 16-bit operands without TMA alignment: 64x64 tile, 256 threads, 4x4 outputs per thread --------
 template <typename T> __device__ __forceinline__ float to_f32(T v);
-template <> __device__ __forceinline__ float to_f32<float>(float v) { return v; }
 template <> __device__ __forceinline__ float to_f32<__nv_bfloat16>(__nv_bfloat16 v) { return __bfloat162float(v); }
 template <> __device__ __forceinline__ float to_f32<__half>(__half v) { return __half2float(v); }
 
@@ -145,23 +144,51 @@ gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ B, long long sam
     for (int j = 0; j < 4; ++j) {
       const int n = n0 + tx * 4 + j;
       if (n >= e.N) continue;
-      float v = acc[i][j] * e.alpha;
-      if (e.bias != nullptr) v += epi_bias(e, n);
-      if (e.mode == MACO_EPI_GELU) v = gelu_tanh(v);
-      else if (e.mode == MACO_EPI_SILU) v = silu(v);
-      else if (e.mode == MACO_EPI_GELU_BWD) v *= gelu_tanh_grad(epi_load_aux(e, m, n));
-      else if (e.mode == MACO_EPI_RESIDUAL) v += epi_load_aux(e, m, n);
-      const long long o = (long long)m * e.ld_out + n;
-      if (e.out_type == MACO_DT_F32) {
-        float* p = reinterpret_cast<float*>(e.out) + o;
-        *p = (e.mode == MACO_EPI_F32_ACC) ? *p + v : v;
-      } else if (e.out_type == MACO_DT_F16) {
-        reinterpret_cast<__half*>(e.out)[o] = __float2half_rn(v);
-      } else {
-        reinterpret_cast<__nv_bfloat16*>(e.out)[o] = __float2bfloat16_rn(v);
-      }
+      simt_store(e, m, n, acc[i][j]);
     }
   }
+}
+
+template <int BM, int BN, int TM, int TN>
+int launch_gemm_f32(const F32Operand& A, const F32Operand& B, const GemmEpilogue& e, int K, int split, cudaStream_t stream) {
+  using T = F32Tile<BM, BN, TM, TN>;
+  auto kern = gemm_f32_kernel<BM, BN, TM, TN>;
+  static bool attr_set[64] = {};
+  int dev = 0;
+  MACO_CHECK_CUDA(cudaGetDevice(&dev));
+  if (!attr_set[dev]) {
+    MACO_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, T::kSmemBytes));
+    attr_set[dev] = true;
+  }
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((e.N + BN - 1) / BN * split, (e.M + BM - 1) / BM);
+  cfg.blockDim = dim3(T::kThreads);
+  cfg.dynamicSmemBytes = T::kSmemBytes;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim = {(unsigned)split, 1, 1};
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  MACO_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, A, B, e, K, split));
+  return 0;
+}
+
+// Tile and K split of an fp32 GEMM. 64 x 64 tiles (half an LDS per FMA of the 32 x 32 ones) as soon as they give every SM
+// one; below that 32 x 32, and 8 x 64 for at most eight rows, where a 32-row tile would spend three quarters of its
+// FMAs on padding. While the tiles leave SMs idle the split doubles, as long as each block keeps two k-steps.
+int dispatch_gemm_f32(const F32Operand& A, const F32Operand& B, const GemmEpilogue& e, int K, cudaStream_t stream) {
+  const long long sms = maco_host::sm_count();
+  auto tiles = [&](int bm, int bn) { return (long long)((e.M + bm - 1) / bm) * ((e.N + bn - 1) / bn); };
+  auto split_for = [&](long long t) {
+    int s = 1;
+    const int steps = (K + kF32BK - 1) / kF32BK;
+    while (s < kF32MaxSplit && t * s < sms && steps >= 4 * s) s *= 2;
+    return s;
+  };
+  if (e.M <= 8) return launch_gemm_f32<8, 64, 1, 4>(A, B, e, K, split_for(tiles(8, 64)), stream);
+  if (tiles(64, 64) >= sms) return launch_gemm_f32<64, 64, 4, 4>(A, B, e, K, 1, stream);
+  return launch_gemm_f32<32, 32, 2, 4>(A, B, e, K, split_for(tiles(32, 32)), stream);
 }
 
 }  // namespace
@@ -260,10 +287,15 @@ int maco_gemm_simt(const void* A, const void* B, void* D, int M, int N, int K, l
   GemmEpilogue e;
   e.out = D; e.bias = bias; e.aux = aux; e.ld_out = ldd; e.ld_aux = ld_aux; e.mode = mode; e.out_type = out_type;
   e.bias_type = bias_type; e.aux_type = aux_type; e.M = M; e.N = N; e.alpha = alpha; e.aux_pack = 0;
+  if (ab_type == MACO_DT_F32) {
+    auto operand = [](const void* p, long long s_row, long long s_k, int rows) {
+      const bool vec = s_k == 1 && s_row % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+      return F32Operand{(const float*)p, s_row, s_k, rows, vec ? 1 : 0};
+    };
+    return dispatch_gemm_f32(operand(A, sam, sak, M), operand(B, sbn, sbk, N), e, K, stream);
+  }
   dim3 grid((N + 63) / 64, (M + 63) / 64);
-  if (ab_type == MACO_DT_F32)
-    gemm_simt_kernel<float><<<grid, 256, 0, stream>>>((const float*)A, (const float*)B, sam, sak, sbn, sbk, e, K);
-  else if (ab_type == MACO_DT_F16)
+  if (ab_type == MACO_DT_F16)
     gemm_simt_kernel<__half><<<grid, 256, 0, stream>>>((const __half*)A, (const __half*)B, sam, sak, sbn, sbk, e, K);
   else
     gemm_simt_kernel<__nv_bfloat16><<<grid, 256, 0, stream>>>((const __nv_bfloat16*)A, (const __nv_bfloat16*)B, sam, sak, sbn, sbk, e, K);

@@ -134,6 +134,26 @@ def test_gemm_fp32_simt_and_odd_shapes():
     assert_close(ops.linear(ah, bh), ah.float() @ bh.float().t(), torch.float16)
 
 
+@pytest.mark.parametrize("shape", [(1, 1, 1), (8, 65, 31), (9, 33, 300), (32, 512, 1024), (31, 70, 2047), (100, 333, 777),
+                                   (640, 1024, 40)])
+def test_gemm_fp32_tiles_and_k_split(shape):
+    """Every tile of the fp32 GEMM (8 x 64, 32 x 32, 64 x 64), split and whole K, K remainders, both majors of both operands,
+    rows that are and are not 16-byte aligned. Bound: each of K products and sums rounds once (2^-24, relative)."""
+    ops = _ops()
+    M, N, K = shape
+    g = torch.Generator(device="cuda").manual_seed(M + N + K)
+    a = torch.randn(M, K, device="cuda", generator=g)
+    b = torch.randn(N, K, device="cuda", generator=g)
+    ref = a.double() @ b.double().t()
+    bound = (K + 8) * 2.0 ** -24 * (a.double().abs() @ b.double().abs().t()) + 1e-30
+    for ta, tb in [(False, False), (False, True), (True, False), (True, True)]:
+        out = ops.gemm(a.t().contiguous() if ta else a, b.t().contiguous() if tb else b, trans_a=ta, trans_b=tb)
+        assert ((out.double() - ref).abs() <= bound).all(), (ta, tb)
+    bias = torch.randn(N, device="cuda", generator=g)
+    out = ops.gemm(a, b, bias=bias)
+    assert ((out.double() - ref - bias.double()).abs() <= bound + 2.0 ** -22 * (ref.abs() + bias.double().abs())).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
 @pytest.mark.parametrize("shape", [(37, 256), (513, 1000), (4, 8192)])
 def test_elementwise_and_rowwise(dtype, shape):
