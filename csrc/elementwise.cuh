@@ -124,7 +124,7 @@ MACO_DEVICE float elt_apply(uint32_t type, float x, float y, const MacoEltArgs& 
   }
 }
 
-MACO_DEVICE bool elt_is_binary(uint32_t type) {
+MACO_DEVICE constexpr bool elt_is_binary(uint32_t type) {
   return type == MACO_TASK_ADD || type == MACO_TASK_SILU_GATE || type == MACO_TASK_GELU_BWD || type == MACO_TASK_AXPBY;
 }
 

@@ -238,3 +238,27 @@ def test_attention_decode_streaming(dtype, B, Hkv, G, S, extra):
         assert rel < (1e-2 if dtype == torch.bfloat16 else 2e-3), rel
     from maco_b200 import _native
     assert _native.status() == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("cols", [8, 256, 264, 512, 520, 1000, 1024, 2056, 4096, 4104, 6152, 8192, 8200, 16, 777, 16384])
+def test_row_and_point_operators_every_row_length(dtype, cols):
+    """Edges of the row kernels' team and vector counts, rows that are not whole vectors, a base that is not 16-byte aligned,
+    and the last elements of a tensor that is not whole vectors. Bounds: the output's rounding plus fp32 sums."""
+    ops = _ops()
+    rows = 5
+    g = torch.Generator(device="cuda").manual_seed(cols)
+    tol = {torch.float32: 2e-6, torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -11 * 1.01}[dtype]
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g).to(dtype)
+    w, b = rnd(cols), rnd(cols)
+    for offset in (0, 1):
+        x, y = (rnd(rows * cols + offset)[offset:].view(rows, cols) for _ in range(2))
+        xd, yd, wd, bd = x.double(), y.double(), w.double(), b.double()
+        F = torch.nn.functional
+        pairs = [(ops.rmsnorm(x, w, 1e-6), xd * torch.rsqrt(xd.pow(2).mean(-1, keepdim=True) + 1e-6) * wd),
+                 (ops.layernorm(x, w, b, 1e-5), F.layer_norm(xd, (cols,), wd, bd, 1e-5)),
+                 (ops.softmax(x), torch.softmax(xd, -1)), (ops.add(x, y), xd + yd), (ops.silu_gate(x, y), F.silu(xd) * yd),
+                 (ops.gelu(x), F.gelu(xd, approximate="tanh"))]
+        for i, (out, ref) in enumerate(pairs):
+            scale = ref.abs() if i >= 3 else ref.abs() + (wd.abs() + bd.abs() if i == 1 else 0)
+            assert ((out.double() - ref).abs() <= tol * scale + 4e-6).all(), (offset, i)
