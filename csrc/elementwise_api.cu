@@ -172,6 +172,28 @@ __global__ void __launch_bounds__(256) flat_kernel(const void* in0, const void* 
     store1(out, rest, DT, elt_op<DT, OP>(load1(in0, rest, DT), bin ? load1(in1, rest, DT) : 0.f, f0, f1));
 }
 
+// Start of an MLP's backward pass, dz = f * (a - target) * gelu'(z), bound by memory (four tensors once each).
+// It was two passes of tasks in the persistent kernel with a rounded tensor in between, whose 28 KB of staging per SM held each at
+// about 2 TB/s: 320 us of the backward pass for 8192 x 4096.
+template <int DT>
+__global__ void __launch_bounds__(256) mse_gelu_bwd_kernel(const uint4* a, const uint4* target, const uint4* z, uint4* dz, long long nvec, float f) {
+  using Vec = VecOf<DT>;
+  const long long first = (long long)blockIdx.x * (256 * 2) + threadIdx.x;
+  uint4 ar[2], tr[2], zr[2];
+#pragma unroll
+  for (int u = 0; u < 2; ++u) if (first + u * 256 < nvec) { ar[u] = a[first + u * 256]; tr[u] = target[first + u * 256]; zr[u] = z[first + u * 256]; }
+#pragma unroll
+  for (int u = 0; u < 2; ++u) {
+    if (first + u * 256 < nvec) {
+      const Vec av = vec_unpack<DT>(ar[u]), tv = vec_unpack<DT>(tr[u]);
+      Vec v = vec_unpack<DT>(zr[u]);
+#pragma unroll
+      for (int j = 0; j < Vec::kN; ++j) v.v[j] = f * (av.v[j] - tv.v[j]) * gelu_tanh_grad(v.v[j]);
+      dz[first + u * 256] = vec_pack<DT>(v);
+    }
+  }
+}
+
 template <int DT>
 bool launch_flat(uint32_t type, const MacoEltArgs& a, cudaStream_t stream) {
   const long long total = (long long)a.rows * a.cols, per = 256ll * kFlatU * VecOf<DT>::kN;
@@ -234,6 +256,23 @@ extern "C" int maco_elementwise(int type, const void* in0, const void* in1, cons
   if (rows_per_cta < 1) rows_per_cta = 1;
   int grid = (rows + rows_per_cta - 1) / rows_per_cta;
   elt_kernel<<<grid, 128, 0, stream>>>((uint32_t)type, a, rows_per_cta);
+  MACO_CHECK_CUDA(cudaGetLastError());
+  return 0;
+}
+
+// `total` elements of 16-bit tensors, a multiple of 8; all four bases 16-byte aligned.
+extern "C" int maco_mse_gelu_bwd(const void* a, const void* target, const void* z, void* dz, long long total, int dtype, float f, void* stream_) {
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  if (total <= 0) return 0;
+  const uintptr_t bases = reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(target) | reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(dz);
+  const long long nvec = total / 8, grid = (nvec + 511) / 512;
+  if (total % 8 != 0 || (bases & 15) != 0 || grid > 0x7fffffffll || (dtype != MACO_DT_BF16 && dtype != MACO_DT_F16)) {
+    maco_host::set_error("maco_mse_gelu_bwd: 16-bit tensors of whole, aligned 16-byte vectors only");
+    return -1;
+  }
+  auto v = [](const void* p) { return reinterpret_cast<const uint4*>(p); };
+  if (dtype == MACO_DT_BF16) mse_gelu_bwd_kernel<MACO_DT_BF16><<<(unsigned)grid, 256, 0, stream>>>(v(a), v(target), v(z), reinterpret_cast<uint4*>(dz), nvec, f);
+  else mse_gelu_bwd_kernel<MACO_DT_F16><<<(unsigned)grid, 256, 0, stream>>>(v(a), v(target), v(z), reinterpret_cast<uint4*>(dz), nvec, f);
   MACO_CHECK_CUDA(cudaGetLastError());
   return 0;
 }

@@ -77,7 +77,10 @@ enum MacoEpilogueMode {
   /* Few-row GEMM with swapped operands (csrc/fewrow_gemm.cuh): `out` = fp32 workspace [tokens, features] (ld_out), N =
      tokens, `bias` = uint32 arrival counters (one per finished tile, never reset), `aux` = a MacoEltArgs in device memory:
      in0 / ld_in the workspace, rows = tokens, in1 = residual rows or MacoQkRopeParams, out / ld_out / dtype, i0 = operator. */
-  MACO_EPI_FEWROW = 11
+  MACO_EPI_FEWROW = 11,
+  /* A layer's forward: out = alpha * acc + bias (16-bit), and `aux`[row, col] (written here, ld_aux / aux_type) = gelu of the
+     ROUNDED out: both tensors that the backward pass reads, in one pass. */
+  MACO_EPI_GELU_DUAL = 12
 };
 
 struct GemmEpilogue {

@@ -51,8 +51,9 @@ class DPMLPStackBackward:
         self.target = torch.randn(tokens, hidden, generator=gx).to(dtype).to(dev)
         self.z = [torch.empty(tokens, hidden, device=dev, dtype=dtype) for _ in range(layers)]
         self.a = [torch.empty(tokens, hidden, device=dev, dtype=dtype) for _ in range(layers)]
-        self.dz = [torch.empty(tokens, hidden, device=dev, dtype=dtype) for _ in range(2)]   # ping-pong
-        self.da = torch.empty(tokens, hidden, device=dev, dtype=dtype)
+        # In turn: dgrad of layer l writes the buffer that wgrad of layer l + 2 has read, two GEMMs back in every queue. (With two
+        # buffers it was the wgrad directly in front of it, whose last tiles held the whole GPU up for 100-130 us a layer.)
+        self.dz = [torch.empty(tokens, hidden, device=dev, dtype=dtype) for _ in range(3)]
         if world > 1:
             if (hidden // BM) % world:
                 raise ValueError("hidden / 128 must be a multiple of world")
@@ -71,8 +72,7 @@ class DPMLPStackBackward:
     def forward(self) -> torch.Tensor:
         cur = self.x
         for l in range(self.layers):
-            ops.gemm(cur, self.weights[l], out=self.z[l])
-            ops.gelu(self.z[l], out=self.a[l])
+            ops.gemm(cur, self.weights[l], out=self.z[l], aux=self.a[l], epilogue="gelu_dual")
             cur = self.a[l]
         return cur
 
@@ -81,26 +81,21 @@ class DPMLPStackBackward:
         L, H, T, world, rank = self.layers, self.hidden, self.tokens, self.world, self.rank
         b = ProgramBuilder(self.device, mode=mode, heap=self.heap, trace=trace, num_comm_workers=comm_workers,
                            cta_pair=self.cta_pair)
-        numel = float(T * H)
-        e_da = b.elementwise(int(TaskType.AXPBY), self.a[L - 1], self.da, in1=self.target, rows=T, cols=H,
-                             f0=2.0 / numel, f1=-2.0 / numel)
-        e_dz = b.elementwise(int(TaskType.GELU_BWD), self.da, self.dz[(L - 1) & 1], in1=self.z[L - 1], rows=T, cols=H,
-                             in_ready=[e_da])
+        e_dz = None                  # dz of the last layer is written by a launch of its own, in front of the program
         n_blocks = H // BM
         n_tiles_w = (H + 255) // 256
         done_events: List[tuple] = []
         row_bytes = H * 4
         split = 4
-        prev_readers = None          # tasks that still read the ping-pong buffer about to be overwritten
+        readers: List[tuple] = []    # completion of each wgrad so far: what may still read a buffer of ``self.dz``
         for l in range(L - 1, -1, -1):
-            dz_l = self.dz[l & 1]
+            dz_l = self.dz[l % 3]
             inp = self.a[l - 1] if l > 0 else self.x
             e_next = None
             if l > 0:
-                # dgrad first: it is the critical path. Overwrites the other ping-pong buffer, which the
-                # wgrad of layer l+1 may still be reading: order it behind that wgrad.
-                extra = [prev_readers] if prev_readers is not None else []
-                e_next = b.gemm(dz_l, self.weights[l], self.dz[(l - 1) & 1], trans_b=True, epilogue="gelu_bwd",
+                # dgrad first: it is the critical path. Its buffer was last read by the wgrad (and dgrad) of layer l + 2.
+                extra = readers[-2:-1]
+                e_next = b.gemm(dz_l, self.weights[l], self.dz[(l - 1) % 3], trans_b=True, epilogue="gelu_bwd",
                                 aux=self.z[l - 1], a_ready=e_dz, bn=256, extra_waits=extra)
             ready = [b.new_event() for _ in range(n_blocks)] if world > 1 else None
             if world > 1:
@@ -116,8 +111,9 @@ class DPMLPStackBackward:
                             signal_peer=mb % world, signal_peer_event=ready[mb])
 
             e_w = b.gemm(dz_l, inp, self.dw[l], trans_a=True, trans_b=True, epilogue="f32", alpha=1.0 / world, bn=256,
-                         extra_waits=[(e_dz.all_event[0], e_dz.all_event[1], False, False)], per_tile=per_tile)
-            prev_readers = (e_w.all_event[0], e_w.all_event[1], False, False)
+                         extra_waits=[(e_dz.all_event[0], e_dz.all_event[1], False, False)] if e_dz is not None else [],
+                         per_tile=per_tile)
+            readers.append((e_w.all_event[0], e_w.all_event[1], False, False))
             if world > 1:
                 off = self.heap.offset_of(self.dw[l])
                 done = b.new_event()
@@ -147,7 +143,10 @@ class DPMLPStackBackward:
         self.program = b.build() if self.device.type == "cuda" else None
 
     def backward(self, stream=None) -> torch.Tensor:
-        """One persistent launch: all dgrad / wgrad GEMMs plus the averaged gradient all-reduce."""
+        """The loss gradient (one point-wise launch), then one persistent launch: all dgrad / wgrad GEMMs plus the averaged
+        gradient all-reduce."""
+        last, f = self.layers - 1, 2.0 / float(self.tokens * self.hidden)
+        ops.mse_gelu_bwd(self.a[last], self.target, self.z[last], self.dz[last % 3], f, stream=stream)
         self.program.run(stream=stream)
         return self.dw
 

@@ -87,3 +87,20 @@ def qknorm_rope(x: torch.Tensor, weight: torch.Tensor, cos_sin: torch.Tensor, ep
     tokens, heads, hd = x.shape
     return _launch(T_ROPE, x, in1=weight, in2=cos_sin.to(x.dtype), out=out, f0=eps, f1=1.0, i0=heads,
                    i1=token_offset, rows=tokens * heads, cols=hd, ld=heads * hd)
+
+
+def mse_gelu_bwd(a: torch.Tensor, target: torch.Tensor, z: torch.Tensor, out: torch.Tensor, factor: float,
+                 stream: Optional[torch.cuda.Stream] = None) -> torch.Tensor:
+    """``out = factor * (a - target) * gelu'(z)``: gradient of a mean-squared error through the last layer's GELU, in one pass.
+    Contiguous 16-bit tensors of one shape and type."""
+    for t in (target, z, out):
+        if t.shape != a.shape or t.dtype != a.dtype or t.device != a.device:
+            raise ValueError("mse_gelu_bwd: tensors of one shape, type and device")
+    if not a.is_cuda or not all(t.is_contiguous() for t in (a, target, z, out)):
+        raise ValueError("mse_gelu_bwd: contiguous CUDA tensors only")
+    lib = N.lib()
+    rc = lib.maco_mse_gelu_bwd(ctypes.c_void_p(a.data_ptr()), ctypes.c_void_p(target.data_ptr()), ctypes.c_void_p(z.data_ptr()),
+                               ctypes.c_void_p(out.data_ptr()), ctypes.c_longlong(a.numel()), N.DTYPE_CODE[a.dtype], ctypes.c_float(factor),
+                               ctypes.c_void_p(N.current_stream_ptr(stream)))
+    N.check(rc, "maco_mse_gelu_bwd")
+    return out

@@ -16,8 +16,9 @@ EPI_STORE, EPI_GELU, EPI_SWIGLU, EPI_F32_STORE, EPI_F32_ACC, EPI_GELU_BWD, EPI_S
 
 _MODES = {
     None: EPI_STORE, "none": EPI_STORE, "gelu": EPI_GELU, "swiglu": EPI_SWIGLU, "f32": EPI_F32_STORE,
-    "f32_acc": EPI_F32_ACC, "gelu_bwd": EPI_GELU_BWD, "silu": EPI_SILU, "residual": EPI_RESIDUAL,
+    "f32_acc": EPI_F32_ACC, "gelu_bwd": EPI_GELU_BWD, "silu": EPI_SILU, "residual": EPI_RESIDUAL, "gelu_dual": 12,
 }
+EPI_GELU_DUAL = _MODES["gelu_dual"]
 
 
 def _row_major_2d(t: torch.Tensor) -> torch.Tensor:
@@ -58,6 +59,8 @@ def gemm(
     either layout: the MMA reads MN-major operands directly from shared memory.
     ``cta_pair``: True runs two-CTA tiles (``tcgen05.mma.cta_group::2``, 256 x bn per CTA pair), False one-CTA
     tiles (128 x bn), None lets the launcher choose (pairs once the tiles cover every SM pair).
+    ``epilogue="gelu_dual"``: ``aux`` [M, N] is an output too, the GELU of ``out`` (as rounded): a layer's pre-activation
+    and activation in one pass. 16-bit, 16-byte aligned operands and outputs only.
     """
     if not a.is_cuda:
         raise ValueError("maco_b200.ops.gemm needs CUDA tensors")
@@ -82,6 +85,9 @@ def gemm(
         if mode != EPI_F32_ACC:
             out.zero_()
         return out
+    if mode == EPI_GELU_DUAL and (aux is None or tuple(aux.shape) != (M, Nn) or aux.stride(1) != 1 or aux.dtype not in (torch.bfloat16, torch.float16)
+                                  or out.dtype not in (torch.bfloat16, torch.float16)):
+        raise ValueError(f"the gelu_dual epilogue needs 16-bit outputs and aux, a row-major [{M}, {Nn}] tensor")
     lib = N.lib()
     st = N.current_stream_ptr(stream)
     bias_t = N.DTYPE_CODE[bias.dtype] if bias is not None else 0
@@ -103,6 +109,8 @@ def gemm(
             return out
         if rc != -2:
             N.check(rc, "maco_gemm")
+    if mode == EPI_GELU_DUAL:
+        raise ValueError("the gelu_dual epilogue needs 16-bit, 16-byte aligned operands")
     from ..config import config
     if (config.allow_tf32 and a.dtype == torch.float32 and not trans_a and not trans_b and mode != EPI_SWIGLU
             and _tma_ok(a) and _tma_ok(b) and out.data_ptr() % 16 == 0 and (out.stride(0) * out.element_size()) % 16 == 0):
