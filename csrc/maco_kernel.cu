@@ -33,6 +33,7 @@
 #include "comm_tasks.cuh"
 #include "attention_decode.cuh"
 #include "moe_tasks.cuh"
+#include "moe_experts.cuh"
 #include "splitk_tasks.cuh"
 #include "fewrow_gemm.cuh"
 #include "host_common.h"
@@ -446,6 +447,15 @@ __device__ void producer_role(const MacoProgram& p, uint32_t w, uint32_t q_base,
       ok = ok && producer_attn_task(p, d, task, tmaps, apipe, ait) != 0;
     } else if (is_gemm_type(d.type)) {
       ok = producer_gemm_task(p, d, task, smem, c, tmaps, apipe, ait, it, owner) != 0;
+    } else if (d.type == MACO_TASK_MOE_EXPERTS) {
+      ok = wait_deps(p, d, task, c.abort_word, nullptr) && (owner != 2 || attn_ring_drained(apipe, ait));
+      owner = 1;
+      if (ok) {
+        fence_proxy_async_all();       // rows and activations are written by other CTAs (bulk copies and generic stores)
+        ok = experts_produce<kMkStages>(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, smem, c, tmaps, it,
+                                        [&p](const uint32_t* flag, uint32_t expect) { return mk_wait(p, flag, expect, false); });
+        if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
+      }
     }
   }
   if (!ok) { gemm_drain_loads<kMkStages>(c, it); attn_drain_loads(apipe, ait); }
@@ -464,6 +474,11 @@ __device__ void mma_role(const MacoProgram& p, uint32_t w, uint32_t q_base, uint
     const MacoTaskDesc* dp = ts.next(p, task, failed, c.abort_word);
     if (dp == nullptr) break;
     const MacoTaskDesc& d = *dp;
+    if (d.type == MACO_TASK_MOE_EXPERTS) {
+      ok = wait_deps(p, d, task, c.abort_word, nullptr) &&
+           experts_mma<kMkStages>(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, smem, c, tmem_base, it, seq);
+      continue;
+    }
     if (!is_gemm_type(d.type)) continue;
     const MacoGemmArgs& g = d.u.gemm;
     if (d.flags & MACO_TF_COUNTED) {
@@ -503,9 +518,11 @@ __device__ __noinline__ void run_moe(const MacoProgram& p, uint32_t type, const 
                                     BulkCtx* bulk) {
   if (type == MACO_TASK_SPLITK_FIN) splitk_finalize(p, a, tid);
   else if (type == MACO_TASK_MOE_COMBINE) moe_combine(p, a, tid, bulk);
-  else if (type == MACO_TASK_TOPK) moe_topk_dispatch(p, a, tid, scratch);
   else if (type == MACO_TASK_MOE_COUNTS) moe_publish_counts(p, a, tid);
   else moe_return(p, a, tid, scratch);
+}
+__device__ __noinline__ bool run_topk(const MacoProgram& p, const MacoEltArgs& a, int tid, const BulkCtx* bulk) {
+  return moe_topk_dispatch(p, a, tid, bulk);
 }
 
 // The epilogue of a tile that is not a lean one (gemm_epilogue_lean), out of line.
@@ -539,7 +556,11 @@ __device__ __noinline__ int run_task(const MacoProgram& p, const MacoTaskDesc& d
     }
   } else if (d.type == MACO_TASK_ATTENTION || d.type == MACO_TASK_ATTN_MERGE) {
     run_attn(d.type, d.u.elt, tid, scratch_smem);
-  } else if (d.type == MACO_TASK_TOPK || d.type == MACO_TASK_MOE_COUNTS || d.type == MACO_TASK_MOE_RETURN ||
+  } else if (d.type == MACO_TASK_TOPK) {
+    // rows wait in the operand ring where nothing uses it before dispatch has ended, else in the scratch block
+    if (!ring_free) { bulk.buf = scratch_smem; bulk.nbuf = 1; bulk.buf_bytes = kMkScratchSmem; }
+    return run_topk(p, d.u.elt, tid, &bulk) ? kTaskDone : kTaskAborted;
+  } else if (d.type == MACO_TASK_MOE_COUNTS || d.type == MACO_TASK_MOE_RETURN ||
              d.type == MACO_TASK_SPLITK_FIN || d.type == MACO_TASK_MOE_COMBINE) {
     run_moe(p, d.type, d.u.elt, tid, scratch_smem, ring_free ? &bulk : nullptr);
   } else if (d.type != MACO_TASK_NOP) {
@@ -660,6 +681,10 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
           }
         }
       }
+    } else if (CG == 1 && d.type == MACO_TASK_MOE_EXPERTS) {
+      const int r = experts_epilogue(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, c, tmem_base, seq);
+      if (r < 0) cur[2] = 1;
+      else seq += (uint32_t)r;
     } else {
       const int r = run_task<CG>(p, d, tid, scratch_smem, ring_smem, bulk_bars, attn_bars, slots, c.abort_word, ait, cur + 3, ring_free);
       if (CG == 1 && d.type == MACO_TASK_ATTENTION && attn_pipelined(d.u.elt)) ait += attn_stage_uses(d.u.elt);

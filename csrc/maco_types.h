@@ -40,6 +40,7 @@ enum MacoTaskType {
   MACO_TASK_MOE_COUNTS = 117,    /* publish this rank's per-expert token counts to the expert owners */
   MACO_TASK_MOE_COMBINE = 119,   /* out[token] = sum of the token's k returned rows (bulk-staged when the operand ring is idle) */
   MACO_TASK_SPLITK_FIN = 118,    /* split-K GEMM: fp32 partial-sum buffer -> epilogue op -> 16-bit output (local or every rank) */
+  MACO_TASK_MOE_EXPERTS = 120,   /* one worker's share of a layer's expert GEMMs: in2 = MacoExpertArgs, i0 = share */
   MACO_TASK_CUSTOM_COMPUTE = 150,
   MACO_TASK_ALLREDUCE = 200,     /* reduce one chunk over all peers' buffers, write to all */
   MACO_TASK_ALLGATHER = 201,     /* push one chunk of the local shard to every peer */
@@ -274,7 +275,8 @@ static_assert(sizeof(MacoTaskDesc) == 128, "task descriptor must stay 128 bytes"
 struct MacoMoeParams {
   const void* logits;             /* [tokens, experts] router output (16-bit) */
   const void* x;                  /* [tokens, hidden] */
-  uint32_t* counts;               /* [experts] slots handed out by this rank, zero at launch start */
+  uint32_t* counts;               /* [experts] slots handed out by this rank, zero at launch start; then the dropped pairs of the last
+                                     launch and of this one */
   void* comb;                     /* [tokens, top_k, hidden] combine buffer of this rank (inside the heap) */
   unsigned long long recv_off;    /* heap offset: recv [experts_per_rank][world][capacity][hidden] */
   unsigned long long meta_off;    /* heap offset: meta [experts_per_rank][world][capacity] x {token, k, weight, -} */
@@ -282,6 +284,19 @@ struct MacoMoeParams {
   unsigned long long comb_off;    /* heap offset of comb */
   const void* y;                  /* [experts_per_rank][world][capacity][hidden] expert outputs (local) */
   int32_t hidden, experts, top_k, experts_per_rank, capacity, tokens, dtype, _pad;
+};
+
+/* The expert GEMMs of one layer (MACO_TASK_MOE_EXPERTS, csrc/moe_experts.cuh): slab (expert, source rank) holds `capacity` rows. */
+struct MacoExpertArgs {
+  const uint32_t* counts;         /* [world][experts] rows received per slab */
+  uint32_t* ready;                /* [experts][world][capacity / 128] epilogue warps that have finished a gate / up tile; zero at launch start */
+  const void* meta;               /* [experts][world][capacity] {token, k, weight, -} */
+  void* act;                      /* [experts][world][capacity][inter] */
+  unsigned long long comb_off;    /* heap offset of the combine buffer */
+  int32_t experts, world, capacity, hidden, inter, top_k, shares, dtype;   /* local experts; workers that share the tiles */
+  uint32_t idesc;
+  uint16_t tmap_x, tmap_w1, tmap_act, tmap_w2;
+  int32_t _pad;
 };
 
 /* ---- device trace ring ----------------------------------------------------------------------- */

@@ -8,11 +8,12 @@ Per rank, inside the persistent kernel:
    copy per expert, straight into that slab on the GPU that owns the expert (dispatch all-to-all
    fused with the router permute), with a {token, k, weight} record beside it
 3. the per-expert counts are published to the expert owners
-4. grouped expert GEMMs over the slabs: gate/up with SwiGLU in the epilogue, then down; tiles whose
-   128-row block holds no tokens are skipped by all roles of the worker (run-time counted tiles)
+   (one rank: the experts read them where dispatch counted)
+4. grouped expert GEMMs over the slabs: gate/up with SwiGLU in the epilogue, then down; every worker takes its share of
+   the tiles that the received counts leave (csrc/moe_experts.cuh)
 5. the down projection's epilogue scales every valid output row by its routing weight and sends it back into the
    source rank's combine buffer at [token, k] (combine all-to-all fused into the GEMM; ``fused_return=False``: separate
-   MOE_RETURN tasks do it from a slab of outputs)
+   MOE_RETURN tasks do it from a slab of outputs, and a task per tile of every slab, skipped at run time where no tokens are)
 6. the source sums the k rows of every token.
 
 Receive slabs have a fixed capacity per (source rank, expert); routed pairs that do not fit are
@@ -33,12 +34,12 @@ import torch
 
 from .. import _native as N
 from ..ops import interleave_gate_up
-from ..ops.megakernel import BM, COMM_REDUCE_LOCAL, ProgramBuilder, RowEvents, _pack_comm, _pack_elt
+from ..ops.megakernel import BM, MODE_STATIC, T_MOE_EXPERTS, ProgramBuilder, _pack_elt, make_idesc
 from ..parallel import fused
 from ..parallel.symm_heap import LocalHeap
 from ..task_graph.nodes import TaskType
 
-T_TOPK, T_MOE_RETURN, T_MOE_COUNTS, T_MOE_COMBINE, T_FILL = 110, 116, 117, 119, 301
+T_TOPK, T_MOE_RETURN, T_MOE_COUNTS, T_MOE_COMBINE = 110, 116, 117, 119
 
 
 def heap_bytes_needed(hidden: int, experts: int, top_k: int, tokens: int, world: int, capacity: int) -> int:
@@ -61,6 +62,8 @@ class MoEEPLayer:
             raise ValueError("experts % world, tokens % 128, inter % 128 and hidden % 256 must be 0")
         if top_k > 8 or experts > 256 or hidden * 2 * 4 > 20480:
             raise ValueError("supported: top_k <= 8, experts <= 256, hidden <= 2560")
+        if top_k > experts:
+            raise ValueError("top_k must not exceed experts")
         dev = self.device = torch.device(device) if device is not None else torch.device("cuda", torch.cuda.current_device())
         self.hidden, self.experts, self.top_k, self.inter, self.tokens = hidden, experts, top_k, inter, tokens
         self.rank, self.world, self.dtype = rank, world, dtype
@@ -88,7 +91,8 @@ class MoEEPLayer:
         self.w2 = torch.stack(w2)                                   # [EL, H, I]
         self.x = torch.empty(T, H, device=dev, dtype=dtype)
         self.logits = torch.empty(T, experts, device=dev, dtype=dtype)
-        self.counts = torch.zeros(experts + 1, device=dev, dtype=torch.int32)
+        # per expert the slots handed out in this launch (cleared at its end); the pairs dropped by the last launch; by this one
+        self.counts = torch.zeros(experts + 2, device=dev, dtype=torch.int32)
         self.recv = heap.alloc((EL, W, C, H), dtype)
         self.meta = heap.alloc((EL, W, C, 4), torch.int32)
         self.cnt = heap.alloc((W, EL), torch.int32)
@@ -110,6 +114,7 @@ class MoEEPLayer:
         self._drop_pending = False
         self.total_dropped = 0
         self.on_drop = on_drop
+        self.ready = None
         self._build(mode, trace)
 
     def expert_weights(self, e: int):
@@ -124,29 +129,73 @@ class MoEEPLayer:
         b = ProgramBuilder(self.device, mode=mode, heap=self.heap, trace=trace)
         pp = self.d_params.data_ptr()
         fence = fused.epoch_fence_event(b)
-        # 0. clear this rank's slot counters (first task of the launch; everything that follows is ordered behind it)
-        e_fill = b.new_event()
-        b.add_task(T_FILL, _pack_elt(0, 0, 0, self.counts.data_ptr(), 0, 1, self.experts + 1, 2, 0, 0, i0=0), waits=[fence],
-                   signals=[e_fill])
+        b.launch_state.append(self.counts)
         # 1. router
-        e_log = b.gemm(self.x, self.w_router, self.logits, bn=128, extra_waits=[(e_fill, 1, False, False)])
-        # 2. top-k + dispatch: about one task per worker, a multiple of 4 tokens (one warp per token)
+        e_log = b.gemm(self.x, self.w_router, self.logits, bn=128)
+        # 2. top-k + dispatch: about one task per worker, a multiple of 4 tokens (one warp per token). Static queues: the worker's
+        # router tile is done by then and the expert tiles wait for the end of dispatch, so the operand ring is free.
         e_disp_local = b.new_event()
         n_disp = 0
         tok_per = max(4, -(-(-(-T // b.num_workers)) // 4) * 4)
+        static = b.mode == MODE_STATIC
         for t0 in range(0, T, tok_per):
             nt = min(tok_per, T - t0)
             ev, cnt = e_log.for_rows(t0, t0 + nt)
-            b.add_task(T_TOPK, _pack_elt(0, 0, pp, 0, t0, nt, H, dt, 0, 0), waits=[(ev, cnt, False, False)],
-                       signals=[e_disp_local])
+            b.add_task(T_TOPK, _pack_elt(0, 0, pp, 0, t0, nt, H, dt, 0, 0), waits=[(ev, cnt, False, False)] + ([fence] if W > 1 else []),
+                       signals=[e_disp_local], ring_free=static)
             n_disp += 1
+        grouped = self.fused_return and static
         # 3. counts to the expert owners; every rank learns that every rank has dispatched
-        e_disp = b.new_event()
-        b.add_task(T_MOE_COUNTS, _pack_elt(0, 0, pp, 0, 0, 0, 0, dt, 0, 0), waits=[(e_disp_local, n_disp, False, False)],
-                   signal_peer=-2, signal_peer_event=e_disp)
-        arrived = (e_disp, W, True, False)
-        # 4. expert GEMMs over the slabs, tiles guarded by the received counts; 5. weighted return
+        arrived = (e_disp_local, n_disp, False, False)
+        if W > 1 or not grouped:
+            e_disp = b.new_event()
+            b.add_task(T_MOE_COUNTS, _pack_elt(0, 0, pp, 0, 0, 0, 0, dt, 0, 0), waits=[arrived], signal_peer=-2, signal_peer_event=e_disp)
+            arrived = (e_disp, W, True, False)
+        # 4. expert GEMMs; 5. weighted return
         e_ret = b.new_event()
+        if grouped:
+            n_ret = self._expert_shares(b, arrived, e_ret)
+        else:
+            n_ret = self._expert_tiles(b, arrived, e_ret, pp)
+        # 6. combine: sum the k rows of every token (token blocks streamed through the idle operand ring)
+        e_out = b.new_event()
+        n_out = 0
+        per = max(8, -(-T // b.num_workers))
+        for t0 in range(0, T, per):
+            b.add_task(T_MOE_COMBINE, _pack_elt(0, 0, pp, self.out.data_ptr(), t0, min(per, T - t0), H, dt, 0, 0),
+                       waits=[(e_ret, n_ret, True, False)], signals=[e_out])
+            n_out += 1
+        b.add_task(T_MOE_COUNTS, _pack_elt(0, 0, pp, N.ptr(self.ready), 0, 0, self.ready.numel() if grouped else 0, dt, 0, 0, i0=1),
+                   waits=[(e_ret, n_ret, True, False)], signals=[e_out])
+        fused.epoch_fence_signal(b, [(e_out, n_out + 1, False, False)])
+        # (a CPU device plans only: the task list stays in ``self.builder`` for host-side schedule checks)
+        self.builder = b
+        self.program = b.build() if self.device.type == "cuda" else None
+
+    def _expert_shares(self, b: ProgramBuilder, arrived, e_ret: int) -> int:
+        """The expert GEMMs and the weighted return as one task per worker. Returns the signals of ``e_ret`` on every rank."""
+        EL, W, C, H, I = self.el, self.world, self.capacity, self.hidden, self.inter
+        slabs, shares = EL * W, b.num_workers
+        self.ready = torch.zeros(slabs * (C // BM), device=self.device, dtype=torch.int32)
+        b.launch_state.append(self.ready)
+        tm = [b._tmap(t.view(-1, cols), rows, cols, cols, False, box) for t, rows, cols, box in
+              ((self.recv, slabs * C, H, BM), (self.w1, EL * 2 * I, H, 256), (self.act, slabs * C, I, BM), (self.w2, EL * H, I, 256))]
+        counts = self.cnt if W > 1 else self.counts
+        blob = struct.pack("<QQQQQiiiiiiiiIHHHHi", counts.data_ptr(), self.ready.data_ptr(), self.meta.data_ptr(), self.act.data_ptr(),
+                           self.heap.offset_of(self.comb), EL, W, C, H, I, self.top_k, shares, N.DTYPE_CODE[self.dtype],
+                           make_idesc(1 if self.dtype == torch.bfloat16 else 0, BM, 256, 0, 0), *tm, 0)
+        self.d_experts = torch.from_numpy(np.frombuffer(blob, dtype=np.uint8).copy()).to(self.device)
+        b.keepalive += [self.d_experts, self.ready, self.recv, self.w1, self.act, self.w2]
+        for w in range(shares):
+            b.add_task(T_MOE_EXPERTS, _pack_elt(0, 0, self.d_experts.data_ptr(), 0, 0, 0, 0, 0, 0, 0, i0=w), waits=[arrived], signal_peer=-2,
+                       signal_peer_event=e_ret, worker=w)
+        return W * shares
+
+    def _expert_tiles(self, b: ProgramBuilder, arrived, e_ret: int, pp: int) -> int:
+        """A task per tile of every slab, skipped at run time where the slab holds no rows (dynamic scheduler, or a slab of outputs
+        with separate return tasks)."""
+        EL, W, C, H, K = self.el, self.world, self.capacity, self.hidden, self.top_k
+        dt = N.DTYPE_CODE[self.dtype]
         cnt_base = self.cnt.data_ptr()
         # Phase order matters with static queues: a worker that is handed a down-projection tile right
         # behind the gate/up tiles of the same slab would idle until those finish. All gate/up tiles come
@@ -190,18 +239,7 @@ class MoEEPLayer:
             for el, s in pairs:
                 emit_return(el, s)
             n_ret = W * EL * (C // BM)
-        # 6. combine: sum the k rows of every token (token blocks streamed through the idle operand ring)
-        e_out = b.new_event()
-        n_out = 0
-        per = max(8, -(-T // b.num_workers))
-        for t0 in range(0, T, per):
-            b.add_task(T_MOE_COMBINE, _pack_elt(0, 0, pp, self.out.data_ptr(), t0, min(per, T - t0), H, dt, 0, 0),
-                       waits=[(e_ret, n_ret, True, False)], signals=[e_out])
-            n_out += 1
-        fused.epoch_fence_signal(b, [(e_out, n_out, False, False)])
-        # (a CPU device plans only: the task list stays in ``self.builder`` for host-side schedule checks)
-        self.builder = b
-        self.program = b.build() if self.device.type == "cuda" else None
+        return n_ret
 
     def forward(self, x: Optional[torch.Tensor] = None, stream=None) -> torch.Tensor:
         """One step. ``on_drop`` ("warn", "raise", "ignore") says what happens when an EARLIER step turns out to have

@@ -35,6 +35,7 @@ COMM_PUSH, COMM_REDUCE_LOCAL, COMM_REDUCE_PULL, COMM_ALLREDUCE, COMM_ALLREDUCE_M
 MAX_PEERS = 16
 WORKER_QUEUE_SIZE = 1024
 T_SPLITK_FIN = 118
+T_MOE_EXPERTS = 120
 
 EPI = {None: 0, "none": 0, "gelu": 1, "swiglu": 2, "f32": 3, "f32_acc": 4, "gelu_bwd": 5, "silu": 6, "residual": 7, "f32_atomic": 8,
        "splitk_fused": 9, "scatter_rows": 10, "fewrow": 11}
@@ -511,9 +512,10 @@ class ProgramBuilder:
                  signals: Sequence[int] = (), signal_peer: int = -1, signal_peer_event: int = -1, node_id: int = 0,
                  comm_worker: bool = False, signal_sys: bool = False, any_worker: bool = False,
                  counted: bool = False, worker: Optional[int] = None, pair_half: Optional[int] = None,
-                 b_static: bool = False) -> int:
+                 b_static: bool = False, ring_free: bool = False) -> int:
         """``waits``: up to two (event, count, sys_scope, previous_epoch). ``worker`` pins the task to a compute
-        worker's static queue (the dynamic scheduler ignores it)."""
+        worker's static queue (the dynamic scheduler ignores it). ``ring_free``: the caller knows that nothing uses the worker's operand
+        ring while the task runs (tasks behind the last user of a worker's queue are marked when the program is built)."""
         if len(waits) > 2 or len(signals) > 2:
             raise ValueError("a task takes at most two wait conditions and two local signals")
         flags = 0
@@ -534,6 +536,8 @@ class ProgramBuilder:
             flags |= TF_COUNTED
         if b_static:
             flags |= TF_B_STATIC
+        if ring_free:
+            flags |= TF_RING_FREE
         se = list(signals) + [-1] * (2 - len(signals))
         self.tasks.append(dict(type=ttype, flags=flags, node_id=node_id, wait_event=we, wait_count=wc, signal_event=se,
                                signal_peer=signal_peer, signal_peer_event=signal_peer_event, raw=raw, worker=worker,
@@ -1230,7 +1234,7 @@ class Program:
             # tasks behind the queue's last ring user (GEMM tiles, pipelined attention): the worker's operand ring
             # is idle from there on, and communication tasks may stage bulk copies in it
             for w, q in enumerate(queues):
-                last_gemm = max((k for k, t in enumerate(q) if b.tasks[t]["type"] in (100, 101, 102)), default=-1)
+                last_gemm = max((k for k, t in enumerate(q) if b.tasks[t]["type"] in (100, 101, 102, T_MOE_EXPERTS)), default=-1)
                 tasks["flags"][int(queue_begin[w]) + last_gemm + 1: int(queue_begin[w + 1])] |= TF_RING_FREE
         self._order = np.asarray(order, dtype=np.int64)          # position in the uploaded table -> index in the builder's list
         self.task_types = np.array([t["type"] for t in b.tasks], dtype=TASK_DTYPE["type"])
