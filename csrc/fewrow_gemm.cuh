@@ -148,7 +148,7 @@ MACO_DEVICE void few_finish_rows(const MacoEltArgs& fa, int m0, int tid, uint8_t
         const float4 c = few_lds_f4(s + 4096u), d = few_lds_f4(s + 6144u);
         const float up[8] = {c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
 #pragma unroll
-        for (int j = 0; j < 8; ++j) v[j] = silu(v[j]) * up[j];
+        for (int j = 0; j < 8; ++j) v[j] = __fdividef(v[j], 1.f + __expf(-v[j])) * up[j];      // (16-bit results: 2 ulp of fp32 are far below)
       } else if (mode == 2) {
         const uint4 r = lds_v4(s + 4096u);
         const uint32_t rw[4] = {r.x, r.y, r.z, r.w};

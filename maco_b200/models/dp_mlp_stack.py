@@ -34,8 +34,14 @@ class DPMLPStackBackward:
                  heap=None, device: Optional[torch.device] = None, dtype: torch.dtype = torch.bfloat16, seed: int = 0,
                  mode: str = "static", trace: bool = False, comm_workers: Optional[int] = None, weight_std: float = 0.02,
                  cta_pair: bool = False):
-        # two-CTA tiles measured slower here (8.5 ms against 8.0 ms on one GPU: both operands of the wgrad tiles are
-        # MN-major, 64-column TMA boxes), so the one-CTA form is the default
+        # ``cta_pair``: two-CTA tiles whatever the size. Without it they are taken on one GPU where both GEMM kinds have about one
+        # 256 x 256 tile per worker or more (two per pair: below that the last wave costs more than the smaller operand traffic
+        # gains). Backward pass, one- / two-CTA, one B200: 4 layers of 4096 x 8192 tokens 1650 / 1535 us, 2 of 3072 x 6144 342 / 319,
+        # 4 of 2304 x 2304 271 / 297, 3 of 1024 x 8192 197 / 213. (More ranks: not measured, one-CTA.)
+        if not cta_pair and world == 1 and mode == "static":
+            sms = torch.cuda.get_device_properties(device if device is not None else torch.cuda.current_device()).multi_processor_count \
+                if torch.cuda.is_available() and (device is None or torch.device(device).type == "cuda") else 148
+            cta_pair = 20 * min((hidden // 256) ** 2, (tokens // 256) * (hidden // 256)) >= 19 * sms
         self.cta_pair = cta_pair and mode == "static"
         if tokens % BM or hidden % 256:
             raise ValueError("tokens must be a multiple of 128 and hidden of 256")

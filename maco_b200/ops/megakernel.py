@@ -139,6 +139,13 @@ def stream_pieces(n_tiles: int, steps: int, workers: int) -> List[Tuple[int, int
     crosses a tile. A cut that would leave less than an eighth of a piece on one side of a tile boundary moves to it
     (a part costs about a microsecond of reductions and arrival whatever its length)."""
     total = n_tiles * steps
+    parts = min(workers // n_tiles, max(1, steps // 2)) if n_tiles else 0
+    if 5 * parts * n_tiles >= 3 * workers or 0 < parts == steps // 2:
+        # One part per worker. A second one on a worker costs its own reductions and arrival, 4 us, and stands behind the finishing
+        # pass of the first, 3-7 us, so that the tiles of a phase completed one after the other; and 90 SMs with a full ring each keep
+        # enough of the stream in flight. (64 tokens: a QKV projection of 20 tiles ended 20 us after its last MMA, an output
+        # projection of 40 tiles 16 us.)
+        return [(t, i * steps // parts, (i + 1) * steps // parts - i * steps // parts, t * parts + i) for t in range(n_tiles) for i in range(parts)]
     workers = max(1, min(workers, total // 2))
     slack = total // workers // 8
     cuts = [0]
@@ -162,7 +169,12 @@ def stream_pieces(n_tiles: int, steps: int, workers: int) -> List[Tuple[int, int
 
 def attention_pieces(groups: int, kv_len: int, workers: int) -> List[Tuple[int, int, int, int]]:
     """Cuts ``groups`` key ranges of ``kv_len`` keys into one (nearly) equal share per worker.
-    Returns (group, first key, keys, worker); cuts inside a group sit on 128-key boundaries."""
+    Returns (group, first key, keys, worker); cuts inside a group sit on 128-key boundaries. A cache of no more 128-key pieces
+    than workers has one piece per worker: shares counted in keys would put a group's short last piece and the next group's first
+    one on the same worker, and a piece is mostly latency."""
+    chunks = -(-kv_len // 128)
+    if groups * chunks <= workers:
+        return [(g, c * 128, min(128, kv_len - c * 128), g * chunks + c) for g in range(groups) for c in range(chunks)]
     target = -(-(groups * kv_len) // workers)
     target = -(-target // 128) * 128
     pieces, wk, acc = [], 0, 0
