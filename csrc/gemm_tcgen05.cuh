@@ -388,7 +388,7 @@ MACO_DEVICE bool gemm_epilogue_lean(int bn, const GemmCtrl& c, uint32_t tmem_bas
       tmem_ld_32x32(t_row + cols + col, u);
       tmem_ld_wait();
 #pragma unroll
-      for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(silu(__uint_as_float(r[j])) * __uint_as_float(u[j]));
+      for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(silu_16(__uint_as_float(r[j])) * __uint_as_float(u[j]));
     } else {
       tmem_ld_wait();
 #pragma unroll

@@ -45,7 +45,7 @@ namespace {
 constexpr int kMkBN = 256;
 constexpr int kMkStages = 4;
 using MkLayout = GemmSmemLayout<kMkBN, kMkStages>;
-constexpr int kMkExtraSmem = 3072;     // scheduler heads / current-task slots, then the three roles' descriptor slots
+constexpr int kMkExtraSmem = 4608;     // scheduler heads / current-task slots, the three roles' descriptor slots and expert tables
 constexpr int kStreamOffset = 1024;    // byte offset of the descriptor slots inside that block
 constexpr uint32_t kStreamSlots = 4;   // descriptors per role: the current one, up to kStreamAhead on their way
 constexpr uint32_t kStreamAhead = 3;
@@ -53,7 +53,8 @@ constexpr int kMkScratchSmem = 28672;  // scratch of non-GEMM tasks (the operand
                                        // the producer warp may already be filling it for the next GEMM task)
 constexpr int kMkSmemBytes = MkLayout::kTotalBytes + kMkExtraSmem + kMkScratchSmem;
 static_assert(kFewWBytes + 64 * kFewK * 2 <= (uint32_t)MkLayout::kStageBytes, "a few-row stage must fit a ring stage");
-static_assert(kStreamOffset + 3 * kStreamSlots * sizeof(MacoTaskDesc) <= kMkExtraSmem, "descriptor slots");
+constexpr int kExpertOffset = kStreamOffset + 3 * kStreamSlots * sizeof(MacoTaskDesc);   // ... of the expert tables, one per role
+static_assert(kExpertOffset + 3 * kMaxSlabs * 2 <= kMkExtraSmem, "descriptor slots and expert tables");
 static_assert(kMkScratchSmem >= (int)kRowScratch, "staged row tasks must fit the scratch block");
 static_assert(kMkScratchSmem >= kEpiStageBytes, "epilogue staging must fit the scratch block");
 static_assert(kMkScratchSmem >= kAttnScratchBytes && kMkScratchSmem >= kAttnTcScratchBytes, "attention scratch must fit the scratch block");
@@ -245,6 +246,11 @@ struct TaskStream {
     return slot;
   }
 };
+
+// A role's table of row blocks per slab, behind the descriptor slots of all three (`desc_slots`: this role's).
+__device__ __forceinline__ uint16_t* expert_table(MacoTaskDesc* desc_slots, int role) {
+  return reinterpret_cast<uint16_t*>(desc_slots + (3 - role) * kStreamSlots) + role * kMaxSlabs;
+}
 
 // ---- producer warp (lane 0), two-CTA programs ----------------------------------------------------
 // Every GEMM task of such a program is one half (128 rows) of a 256 x BN tile; the two halves sit at the same
@@ -452,7 +458,7 @@ __device__ void producer_role(const MacoProgram& p, uint32_t w, uint32_t q_base,
       owner = 1;
       if (ok) {
         fence_proxy_async_all();       // rows and activations are written by other CTAs (bulk copies and generic stores)
-        ok = experts_produce<kMkStages>(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, smem, c, tmaps, it,
+        ok = experts_produce<kMkStages>(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, expert_table(desc_slots, 0), smem, c, tmaps, it,
                                         [&p](const uint32_t* flag, uint32_t expect) { return mk_wait(p, flag, expect, false); });
         if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
       }
@@ -476,7 +482,7 @@ __device__ void mma_role(const MacoProgram& p, uint32_t w, uint32_t q_base, uint
     const MacoTaskDesc& d = *dp;
     if (d.type == MACO_TASK_MOE_EXPERTS) {
       ok = wait_deps(p, d, task, c.abort_word, nullptr) &&
-           experts_mma<kMkStages>(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, smem, c, tmem_base, it, seq);
+           experts_mma<kMkStages>(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, expert_table(desc_slots, 1), smem, c, tmem_base, it, seq);
       continue;
     }
     if (!is_gemm_type(d.type)) continue;
@@ -628,9 +634,9 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
       // counted tile without rows: nothing to compute (it still signals below)
     } else if (CG == 1 && is_gemm_type(d.type) && (d.u.gemm.b_mn & kFewFlag)) {
       const int r = few_epilogue<kMkBN>(c, tmem_base, p.epis[d.u.gemm.epi], d.u.gemm, tid, seq, p.budget_ns, scratch_smem, cur + 3,
-                                        [] { general_bar(); });
+                                        [] { general_bar(); }, [&p, &d] { signal_done(p, d); });
       if (r == 0) cur[2] = 1;
-      signals = r == 2;                                // the tile's event counts finished tiles, not parts
+      signals = false;                                 // (the tile's event counts finished tiles, not parts)
       ++seq;
     } else if (is_gemm_type(d.type)) {
       const MacoGemmArgs& g = d.u.gemm;
@@ -682,7 +688,8 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
         }
       }
     } else if (CG == 1 && d.type == MACO_TASK_MOE_EXPERTS) {
-      const int r = experts_epilogue(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, c, tmem_base, seq);
+      const int r = experts_epilogue(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, expert_table(desc_slots, 2), tid, c, tmem_base, seq,
+                                     [] { general_bar(); });
       if (r < 0) cur[2] = 1;
       else seq += (uint32_t)r;
     } else {
