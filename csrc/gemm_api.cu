@@ -150,7 +150,7 @@ gemm_simt_kernel(const T* __restrict__ A, const T* __restrict__ B, long long sam
 }
 
 template <int BM, int BN, int TM, int TN>
-int launch_gemm_f32(const F32Operand& A, const F32Operand& B, const GemmEpilogue& e, int K, int split, cudaStream_t stream) {
+int launch_gemm_f32(const F32Operand& A, const F32Operand& B, const GemmEpilogue& e, int K, int split, bool chained, cudaStream_t stream) {
   using T = F32Tile<BM, BN, TM, TN>;
   auto kern = gemm_f32_kernel<BM, BN, TM, TN>;
   static bool attr_set[64] = {};
@@ -165,11 +165,13 @@ int launch_gemm_f32(const F32Operand& A, const F32Operand& B, const GemmEpilogue
   cfg.blockDim = dim3(T::kThreads);
   cfg.dynamicSmemBytes = T::kSmemBytes;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim = {(unsigned)split, 1, 1};
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // set up while the launch in front of it ends
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = chained ? 2 : 1;
   MACO_CHECK_CUDA(cudaLaunchKernelEx(&cfg, kern, A, B, e, K, split));
   return 0;
 }
@@ -177,7 +179,7 @@ int launch_gemm_f32(const F32Operand& A, const F32Operand& B, const GemmEpilogue
 // Tile and K split of an fp32 GEMM. 64 x 64 tiles (half an LDS per FMA of the 32 x 32 ones) as soon as they give every SM
 // one; below that 32 x 32, and 8 x 64 for at most eight rows, where a 32-row tile would spend three quarters of its
 // FMAs on padding. While the tiles leave SMs idle the split doubles, as long as each block keeps two k-steps.
-int dispatch_gemm_f32(const F32Operand& A, const F32Operand& B, const GemmEpilogue& e, int K, cudaStream_t stream) {
+int dispatch_gemm_f32(const F32Operand& A, const F32Operand& B, const GemmEpilogue& e, int K, cudaStream_t stream, bool chained = false) {
   const long long sms = maco_host::sm_count();
   auto tiles = [&](int bm, int bn) { return (long long)((e.M + bm - 1) / bm) * ((e.N + bn - 1) / bn); };
   auto split_for = [&](long long t) {
@@ -186,14 +188,43 @@ int dispatch_gemm_f32(const F32Operand& A, const F32Operand& B, const GemmEpilog
     while (s < kF32MaxSplit && t * s < sms && steps >= 4 * s) s *= 2;
     return s;
   };
-  if (e.M <= 8) return launch_gemm_f32<8, 64, 1, 4>(A, B, e, K, split_for(tiles(8, 64)), stream);
-  if (tiles(64, 64) >= sms) return launch_gemm_f32<64, 64, 4, 4>(A, B, e, K, 1, stream);
-  return launch_gemm_f32<32, 32, 2, 4>(A, B, e, K, split_for(tiles(32, 32)), stream);
+  if (e.M <= 8) return launch_gemm_f32<8, 64, 1, 4>(A, B, e, K, split_for(tiles(8, 64)), chained, stream);
+  if (tiles(64, 64) >= sms) return launch_gemm_f32<64, 64, 4, 4>(A, B, e, K, 1, chained, stream);
+  return launch_gemm_f32<32, 32, 2, 4>(A, B, e, K, split_for(tiles(32, 32)), chained, stream);
+}
+
+F32Operand f32_operand(const void* p, long long s_row, long long s_k, int rows) {
+  const bool vec = s_k == 1 && s_row % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
+  return F32Operand{(const float*)p, s_row, s_k, rows, vec ? 1 : 0};
 }
 
 }  // namespace
 
 extern "C" {
+
+// One fp32 GEMM of a chain (arguments as in maco_gemm_simt).
+struct MacoF32Gemm {
+  const void *A, *B;
+  void* D;
+  const void* bias;
+  long long sam, sak, sbn, sbk, ldd;
+  int M, N, K, mode, bias_type, out_type;
+};
+
+// The fp32 GEMMs of a graph in order on one stream, each behind the one in front of it: one call for the host, and the set-up of a
+// launch under the end of the previous one. (Two layers of 32 rows through one Python call each: 41 us, 17 us of host time a launch.)
+int maco_gemm_f32_chain(const MacoF32Gemm* g, int n, void* stream_) {
+  cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
+  for (int i = 0; i < n; ++i) {
+    GemmEpilogue e = {};
+    e.out = g[i].D; e.bias = g[i].bias; e.ld_out = g[i].ldd; e.mode = g[i].mode; e.out_type = g[i].out_type;
+    e.bias_type = g[i].bias_type; e.M = g[i].M; e.N = g[i].N; e.alpha = 1.f;
+    const int rc = dispatch_gemm_f32(f32_operand(g[i].A, g[i].sam, g[i].sak, g[i].M), f32_operand(g[i].B, g[i].sbn, g[i].sbk, g[i].N), e, g[i].K,
+                                     stream, i > 0);
+    if (rc != 0) return rc;
+  }
+  return 0;
+}
 
 // Cycle counters of the stand-alone GEMM kernels: `buf` (device memory, 8 x int64 per CTA, or null to switch
 // them off) receives per CTA [0] producer cycles waiting for a free stage, [1] MMA warp waiting for a free
@@ -288,11 +319,7 @@ int maco_gemm_simt(const void* A, const void* B, void* D, int M, int N, int K, l
   e.out = D; e.bias = bias; e.aux = aux; e.ld_out = ldd; e.ld_aux = ld_aux; e.mode = mode; e.out_type = out_type;
   e.bias_type = bias_type; e.aux_type = aux_type; e.M = M; e.N = N; e.alpha = alpha; e.aux_pack = 0;
   if (ab_type == MACO_DT_F32) {
-    auto operand = [](const void* p, long long s_row, long long s_k, int rows) {
-      const bool vec = s_k == 1 && s_row % 4 == 0 && (reinterpret_cast<uintptr_t>(p) & 15) == 0;
-      return F32Operand{(const float*)p, s_row, s_k, rows, vec ? 1 : 0};
-    };
-    return dispatch_gemm_f32(operand(A, sam, sak, M), operand(B, sbn, sbk, N), e, K, stream);
+    return dispatch_gemm_f32(f32_operand(A, sam, sak, M), f32_operand(B, sbn, sbk, N), e, K, stream);
   }
   dim3 grid((N + 63) / 64, (M + 63) / 64);
   if (ab_type == MACO_DT_F16)

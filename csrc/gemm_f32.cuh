@@ -80,6 +80,7 @@ gemm_f32_kernel(F32Operand A, F32Operand B, GemmEpilogue e, int K, int split) {
   using T = F32Tile<BM, BN, TM, TN>;
   constexpr int NT = T::kThreads;
   extern __shared__ __align__(16) float f32_smem[];
+  asm volatile("griddepcontrol.wait;" ::: "memory");   // (launched behind another one of a chain: its results are complete)
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int tx = (lane & 7) + 8 * (warp % (T::kTX / 8)), ty = (lane >> 3) + 4 * (warp / (T::kTX / 8));
   const int rank = blockIdx.x % split;

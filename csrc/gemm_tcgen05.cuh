@@ -430,25 +430,28 @@ MACO_DEVICE bool gemm_epilogue_lean(int bn, const GemmCtrl& c, uint32_t tmem_bas
   return true;
 }
 
-// Tiles of an MLP's training step: 16-bit result times gelu'(aux) (MACO_EPI_GELU_BWD), or the result and its GELU
-// (MACO_EPI_GELU_DUAL), whole columns, no bias, 16-byte rows. A tile of 64 k-blocks leaves the tensor cores after about 24 us; in
+// Tiles with a second tensor beside the result, 16-bit, whole columns, no bias, 16-byte rows: the result times gelu'(aux)
+// (MACO_EPI_GELU_BWD), the result and its GELU (MACO_EPI_GELU_DUAL), the result and its sum with aux (MACO_EPI_RESIDUAL_DUAL). A tile of 64 k-blocks leaves the tensor cores after about 24 us; in
 // the general epilogue, whose element type and operator are asked for per element, its 32,768 derivatives took 50 us and the
 // backward pass of 8192 x 4096 layers ran at that rate. Here the operator is one branch per chunk of 32 columns and the
 // aux values of the next chunk are on their way while this one is computed.
-MACO_DEVICE bool epi_is_gelu(const GemmEpilogue& e, int n0, int bn) {
-  return (e.mode == MACO_EPI_GELU_BWD || e.mode == MACO_EPI_GELU_DUAL) && e.bias == nullptr && n0 + bn <= e.N && e.out_type != MACO_DT_F32 &&
-         ((reinterpret_cast<uintptr_t>(e.aux) | (uintptr_t)(e.ld_aux * 2)) & 15) == 0;
+MACO_DEVICE bool epi_is_beside(const GemmEpilogue& e, int n0, int bn) {
+  const bool res = e.mode == MACO_EPI_RESIDUAL_DUAL;
+  const uintptr_t p = reinterpret_cast<uintptr_t>(e.aux) | (uintptr_t)(e.ld_aux * 2) | (res ? reinterpret_cast<uintptr_t>(e.bias) : 0);
+  return (e.mode == MACO_EPI_GELU_BWD || e.mode == MACO_EPI_GELU_DUAL || res) && (res || e.bias == nullptr) && n0 + bn <= e.N &&
+         e.out_type != MACO_DT_F32 && (p & 15) == 0;
 }
 template <int SBN>
-__device__ __noinline__ bool gemm_epilogue_gelu(int bn, const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e_in, void* out_base,
+__device__ __noinline__ bool gemm_epilogue_beside(int bn, const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e_in, void* out_base,
                                                 long long row_off, int m0, int n0, uint32_t tile_seq, uint64_t budget_ns,
                                                 uint32_t pair_empty_bar) {
   const uint32_t q = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, acc = tile_seq & 1;
   const int row = m0 + (int)(q * 32 + lane), dt = e_in.out_type, at = e_in.aux_type;
-  const bool row_ok = row < e_in.M, dual = e_in.mode == MACO_EPI_GELU_DUAL;
+  const bool row_ok = row < e_in.M, dual = e_in.mode == MACO_EPI_GELU_DUAL, res = e_in.mode == MACO_EPI_RESIDUAL_DUAL;
   const float alpha = e_in.alpha;
   uint16_t* dst = reinterpret_cast<uint16_t*>(out_base) + (row + row_off) * e_in.ld_out + n0;
   uint16_t* aux = reinterpret_cast<uint16_t*>(const_cast<void*>(e_in.aux)) + (long long)row * e_in.ld_aux + n0;
+  uint16_t* second = dual ? aux : reinterpret_cast<uint16_t*>(const_cast<void*>(e_in.bias)) + (row + row_off) * e_in.ld_out + n0;
   uint4 ax[4];
   auto fetch = [&](int col) {
     if (row_ok && !dual) {
@@ -473,16 +476,21 @@ __device__ __noinline__ bool gemm_epilogue_gelu(int bn, const GemmCtrl& c, uint3
     for (int i = 0; i < 4; ++i) { g[4 * i] = ax[i].x; g[4 * i + 1] = ax[i].y; g[4 * i + 2] = ax[i].z; g[4 * i + 3] = ax[i].w; }
     if (col + 32 < bn) fetch(col + 32);
     tmem_ld_wait();
-    if (dual) {
+    if (dual || res) {
 #pragma unroll
       for (int j = 0; j < 16; ++j) {
         w[j] = epi_pack(dt, __uint_as_float(r[2 * j]) * alpha, __uint_as_float(r[2 * j + 1]) * alpha);
         const float2 z = dt == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[j])) : unpack_bf16x2(w[j]);
-        g[j] = epi_pack(at, gelu_tanh(z.x), gelu_tanh(z.y));
+        if (dual) {
+          g[j] = epi_pack(at, gelu_tanh(z.x), gelu_tanh(z.y));
+        } else {
+          const float2 x = at == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&g[j])) : unpack_bf16x2(g[j]);
+          g[j] = epi_pack(dt, z.x + x.x, z.y + x.y);
+        }
       }
       if (row_ok) {
 #pragma unroll
-        for (int j = 0; j < 16; j += 4) reinterpret_cast<uint4*>(aux + col)[j >> 2] = make_uint4(g[j], g[j + 1], g[j + 2], g[j + 3]);
+        for (int j = 0; j < 16; j += 4) reinterpret_cast<uint4*>(second + col)[j >> 2] = make_uint4(g[j], g[j + 1], g[j + 2], g[j + 3]);
       }
     } else {
 #pragma unroll
@@ -603,7 +611,7 @@ MACO_DEVICE bool gemm_epilogue_tile(const GemmCtrl& c, uint32_t tmem_base, const
           v[j] = f.x * row_weight; v[j + 1] = f.y * row_weight;
         }
       }
-      if (e.bias != nullptr && e.mode != MACO_EPI_SPLITK_FUSED) {     // (that mode keeps its arrival counters there)
+      if (e.bias != nullptr && e.mode != MACO_EPI_SPLITK_FUSED && e.mode != MACO_EPI_RESIDUAL_DUAL) {     // (those keep counters / an output there)
 #pragma unroll
         for (int j = 0; j < 32; ++j) if (j < valid) v[j] += epi_bias(e, col0 + j);
       }
@@ -624,6 +632,13 @@ MACO_DEVICE bool gemm_epilogue_tile(const GemmCtrl& c, uint32_t tmem_base, const
         } else {
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] *= gelu_tanh_grad(ax[j]);
+        }
+      } else if (e.mode == MACO_EPI_RESIDUAL_DUAL) {
+        uint16_t* sum = reinterpret_cast<uint16_t*>(const_cast<void*>(e.bias)) + out_row * e.ld_out + col0;
+        for (int j = 0; j < valid; ++j) {
+          const uint32_t z = epi_pack(e.out_type, v[j], 0.f);
+          const float f = e.out_type == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&z)).x : unpack_bf16x2(z).x;
+          sum[j] = (uint16_t)(epi_pack(e.out_type, f + epi_load_aux(e, row, col0 + j), 0.f) & 0xffffu);
         }
       } else if (e.mode == MACO_EPI_GELU_DUAL) {
         uint16_t* act = reinterpret_cast<uint16_t*>(const_cast<void*>(e.aux)) + row * e.ld_aux + col0;
@@ -941,8 +956,8 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         if (lane == 0) mbar_arrive_cluster(tempty_leader + (seq & 1) * 8);
         continue;
       }
-      if (epi_is_gelu(epi, nb * BN, BN))
-        ok = gemm_epilogue_gelu<256>(BN, c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns, tempty_leader);
+      if (epi_is_beside(epi, nb * BN, BN))
+        ok = gemm_epilogue_beside<256>(BN, c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns, tempty_leader);
       else
         ok = gemm_epilogue_tile<BN, 256>(c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns,
                                          nullptr, nullptr, tempty_leader);
@@ -1007,8 +1022,8 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         mbar_arrive(&c.tmem_empty[seq & 1]);
         continue;
       }
-      if (epi_is_gelu(epi, nb * BN, BN))
-        ok = gemm_epilogue_gelu<BN>(BN, c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns, 0);
+      if (epi_is_beside(epi, nb * BN, BN))
+        ok = gemm_epilogue_beside<BN>(BN, c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns, 0);
       else
         ok = gemm_epilogue_tile<BN>(c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns);
     }

@@ -649,8 +649,8 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
       uint8_t* stage = g.peer != -1 ? scratch_smem : nullptr;  // tiles that leave the GPU go through the bulk engine
       // run-time row count of a counted tile's operand block (rows at or beyond it hold no tokens)
       const int row_limit = (d.flags & MACO_TF_COUNTED) ? (int)ld_relaxed_gpu_u32(g.count_ptr) : 0x7fffffff;
-      if (g.peer == -1 && epi_is_gelu(e, g.n0, (int)g.bn))
-        ok = gemm_epilogue_gelu<kMkBN>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, pair_empty_bar);
+      if (g.peer == -1 && epi_is_beside(e, g.n0, (int)g.bn))
+        ok = gemm_epilogue_beside<kMkBN>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, pair_empty_bar);
       else if (g.peer == -1 && epi_is_lean(e, g.n0, (int)g.bn))
         ok = gemm_epilogue_lean<kMkBN>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, pair_empty_bar, row_limit);
       else

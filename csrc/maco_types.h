@@ -81,7 +81,10 @@ enum MacoEpilogueMode {
   MACO_EPI_FEWROW = 11,
   /* A layer's forward: out = alpha * acc + bias (16-bit), and `aux`[row, col] (written here, ld_aux / aux_type) = gelu of the
      ROUNDED out: both tensors that the backward pass reads, in one pass. */
-  MACO_EPI_GELU_DUAL = 12
+  MACO_EPI_GELU_DUAL = 12,
+  /* A product that is needed itself and with a residual added: out = alpha * acc (16-bit), and the tensor at `bias` (written here,
+     laid out and typed like out) = the ROUNDED out + `aux`. No bias. */
+  MACO_EPI_RESIDUAL_DUAL = 13
 };
 
 struct GemmEpilogue {

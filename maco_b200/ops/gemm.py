@@ -6,6 +6,7 @@ runs as its own launch; they replace the ``torch.mm`` calls of the reference's l
 """
 from __future__ import annotations
 
+import ctypes
 from typing import Optional
 
 import torch
@@ -133,6 +134,54 @@ def gemm(
     )
     N.check(rc, "maco_gemm_simt")
     return out
+
+
+class _F32Gemm(ctypes.Structure):
+    _fields_ = [(n, ctypes.c_void_p) for n in ("A", "B", "D", "bias")] + [(n, ctypes.c_longlong) for n in ("sam", "sak", "sbn", "sbk", "ldd")] + \
+               [(n, ctypes.c_int) for n in ("M", "N", "K", "mode", "bias_type", "out_type")]
+
+
+class F32Chain:
+    """Linear layers and matrix products in fp32, in order, as one native call (``maco_gemm_f32_chain``). ``calls``: (x, weight, bias or
+    None, out, epilogue, ``weight`` stored [K, N]). ``make`` returns None when one of them needs what only ``gemm`` does
+    (other types, copies, empty operands); ``run`` returns False, with nothing launched, when a tensor is no longer where or
+    what it was when the chain was made."""
+
+    def __init__(self, tensors, key, table):
+        self.tensors, self.key, self.table = tensors, key, table
+
+    @staticmethod
+    def layout(tensors) -> list:
+        return [(t.data_ptr(), t.shape, t.stride()) for t in tensors]
+
+    @classmethod
+    def make(cls, calls) -> Optional["F32Chain"]:
+        rows, tensors = [], []
+        for x, w, bias, out, epilogue, kn in calls:
+            if epilogue not in (None, "none", "gelu", "silu") or x.dim() < 1 or w.dim() != 2 or out is None:
+                return None
+            if any(not t.is_cuda or t.dtype != torch.float32 or t.device != x.device for t in (x, w, out)) or not out.is_contiguous() or not x.is_contiguous():
+                return None
+            K, n = (w.shape[0], w.shape[1]) if kn else (w.shape[1], w.shape[0])
+            if w.stride(1) != 1 or x.shape[-1] != K or out.shape[-1] != n or 0 in (K, n, x.numel()) or out.numel() // n != x.numel() // K:
+                return None
+            if bias is not None and (not bias.is_cuda or bias.dtype not in N.DTYPE_CODE or bias.dim() != 1 or bias.stride(0) != 1):
+                return None
+            sbn, sbk = (1, w.stride(0)) if kn else (w.stride(0), 1)
+            rows.append(_F32Gemm(x.data_ptr(), w.data_ptr(), out.data_ptr(), N.ptr(bias), K, 1, sbn, sbk, n, x.numel() // K, n, K, _MODES[epilogue],
+                                 N.DTYPE_CODE[bias.dtype] if bias is not None else 0, N.DT_F32))
+            tensors += [t for t in (x, w, bias, out) if t is not None]
+        if not rows:
+            return None
+        fn = N.lib().maco_gemm_f32_chain
+        fn.restype, fn.argtypes = ctypes.c_int, [ctypes.c_void_p, ctypes.c_int, ctypes.c_void_p]
+        return cls(tensors, cls.layout(tensors), (_F32Gemm * len(rows))(*rows))
+
+    def run(self) -> bool:
+        if self.layout(self.tensors) != self.key:
+            return False
+        N.check(N.lib().maco_gemm_f32_chain(ctypes.addressof(self.table), len(self.table), N.current_stream_ptr()), "maco_gemm_f32_chain")
+        return True
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None,

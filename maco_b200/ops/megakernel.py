@@ -38,7 +38,7 @@ T_SPLITK_FIN = 118
 T_MOE_EXPERTS = 120
 
 EPI = {None: 0, "none": 0, "gelu": 1, "swiglu": 2, "f32": 3, "f32_acc": 4, "gelu_bwd": 5, "silu": 6, "residual": 7, "f32_atomic": 8,
-       "splitk_fused": 9, "scatter_rows": 10, "fewrow": 11}
+       "splitk_fused": 9, "scatter_rows": 10, "fewrow": 11, "residual_dual": 13}
 
 TASK_DTYPE = np.dtype([
     ("type", "<u2"), ("flags", "<u2"), ("node_id", "<u4"), ("wait_event", "<i4", 2), ("wait_count", "<u4", 2),
@@ -626,7 +626,7 @@ class ProgramBuilder:
              aux: Optional[torch.Tensor] = None, alpha: float = 1.0, bn: int = 0,
              a_ready: Optional[RowEvents] = None, extra_waits: Sequence[Tuple[int, int, bool, bool]] = (),
              per_tile=None, m_blocks: Optional[Sequence[int]] = None, signal_sys: bool = False,
-             row_wait=None, group_blocks: Optional[int] = None) -> RowEvents:
+             row_wait=None, group_blocks: Optional[int] = None, second: Optional[torch.Tensor] = None) -> RowEvents:
         """Adds the tiles of ``out = epilogue(alpha * A · B^T)`` (A logically [M,K], B logically [N,K]).
 
         ``a_ready`` gives row-block events of A (a tile waits only for its 128 rows); ``extra_waits``
@@ -638,6 +638,7 @@ class ProgramBuilder:
         group runs, its A panel (group_blocks x 128 x K) stays in L2 and B streams through once, so DRAM reads
         B once per GROUP: large groups cut the re-reads of a B that does not fit the 126 MB L2. Default: as many
         blocks as keep the A panel near 32 MB (MACO_GEMM_PANEL_MB; at least 8) when the caller did not fix the block order, else 8.
+        ``epilogue="residual_dual"``: ``second`` (laid out like ``out``) receives ``out`` (as rounded) + ``aux``.
         """
         for t in (a, b):
             if t.dim() != 2 or t.stride(1) != 1 or t.dtype not in (torch.bfloat16, torch.float16):
@@ -649,6 +650,10 @@ class ProgramBuilder:
         if K != Kb:
             raise ValueError("inner dimensions differ")
         mode = EPI[epilogue]
+        if (mode == EPI["residual_dual"]) != (second is not None) or (second is not None and (
+                bias is not None or aux is None or second.dtype != out.dtype or second.shape != out.shape or second.stride() != out.stride()
+                or aux.shape != out.shape or aux.stride(1) != 1 or out.element_size() != 2 or aux.element_size() != 2)):
+            raise ValueError("residual_dual: 16-bit out, aux and second of one shape, second laid out like out, no bias")
         if bn == 0:
             m_tiles = (M + BM - 1) // BM
             # the SwiGLU epilogue needs the weight interleaved for the tile width; 256 unless told otherwise
@@ -664,13 +669,13 @@ class ProgramBuilder:
         out_ptr = out.data_ptr() if out is not None else 0
         ld_out = out.stride(0) if out is not None else 0
         out_type = N.DTYPE_CODE[out.dtype] if out is not None else N.DTYPE_CODE[a.dtype]
-        self.epis.append(_pack_epilogue(out_ptr, N.ptr(bias), N.ptr(aux), ld_out, aux.stride(0) if aux is not None else 0,
+        self.epis.append(_pack_epilogue(out_ptr, N.ptr(bias if second is None else second), N.ptr(aux), ld_out, aux.stride(0) if aux is not None else 0,
                                         mode, out_type, N.DTYPE_CODE[bias.dtype] if bias is not None else 0,
                                         N.DTYPE_CODE[aux.dtype] if aux is not None else 0, M, Nn, float(alpha)))
         epi = len(self.epis) - 1
         if epi > 0xFFFF or len(self.tmaps) > 0xFFFF:
             raise ValueError("too many epilogues / tensor maps in one program")
-        self.keepalive += [t for t in (a, b, out, bias, aux) if t is not None]
+        self.keepalive += [t for t in (a, b, out, bias, aux, second) if t is not None]
         node_id = self.new_node_id()
         m_tiles, n_tiles, k_blocks = (M + BM - 1) // BM, (Nn + bn - 1) // bn, (K + BK - 1) // BK
         mbs = list(m_blocks) if m_blocks is not None else list(range(m_tiles))
@@ -1121,6 +1126,10 @@ class ProgramBuilder:
             rows_per_task = 1
             while rows_per_task * 2 <= min(target, BM):
                 rows_per_task *= 2
+            # rounded down, a second wave of a few tasks would double the phase (1003 rows of 2048: 251 tasks of 4 rows ended at 17.5 us,
+            # the first 148 at 7)
+            if rows * cols * esz <= (4 << 20) and rows_per_task < BM and -(-rows // rows_per_task) > self.num_workers >= -(-rows // (2 * rows_per_task)):
+                rows_per_task *= 2
         self.keepalive += [t for t in (in0, in1, in2, out) if t is not None]
         node_id = self.new_node_id()
         all_ev = self.new_event() if all_event is None else all_event
@@ -1484,6 +1493,38 @@ def can_lower(graph) -> bool:
     return True
 
 
+def _residual_adds(graph, few_rows, static) -> Dict[int, Tuple[TaskNode, torch.Tensor]]:
+    """Adds that the linear in front of them does in its epilogue (``residual_dual``): the add depends on that linear alone, its other
+    operand is written by no node of the graph, and all three tensors are contiguous 16-bit rows of 16-byte vectors. Both outputs are
+    written as before; what goes is a phase of the graph and a read of the product."""
+    found: Dict[int, Tuple[TaskNode, torch.Tensor]] = {}
+    for add in graph._nodes:
+        deps = list(dict.fromkeys(add.depends_on))
+        if add.task_type != TaskType.ADD or len(deps) != 1 or deps[0]._node_id in found:
+            continue
+        lin = deps[0]
+        if (lin.task_type not in (TaskType.LINEAR, TaskType.MATMUL) or few_rows(lin) or lin.attrs.get("has_bias")
+                or lin.attrs.get("activation") not in (None, "none")):
+            continue
+        y, z = lin.outputs[0], add.outputs[0]
+        if any(n.outputs and n is not add and n.outputs[0].untyped_storage().data_ptr() == z.untyped_storage().data_ptr() for n in graph._nodes):
+            continue
+        same = [t.data_ptr() == y.data_ptr() and t.shape == y.shape for t in add.inputs]
+        if same.count(True) != 1:
+            continue
+        res = add.inputs[same.index(False)]
+        if (static(res) and _vector_rows(y, z, res) and res.untyped_storage().data_ptr() != z.untyped_storage().data_ptr()):
+            found[lin._node_id] = (add, res)
+    return found
+
+
+def _vector_rows(*tensors: torch.Tensor) -> bool:
+    """Contiguous 16-bit tensors of one shape and type whose rows are whole, aligned 16-byte vectors."""
+    t0 = tensors[0]
+    return all(t.dtype == t0.dtype and t.dtype in _F16 and t.shape == t0.shape and t.is_contiguous() and t.numel() > 0
+               and t.data_ptr() % 16 == 0 and (t.shape[-1] * 2) % 16 == 0 for t in tensors)
+
+
 def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None) -> Program:
     """Lowers a TaskGraph (dependencies already inferred) to a persistent-kernel program."""
     import os
@@ -1519,10 +1560,25 @@ def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None)
         return _storage_key(t) not in written                  # no node of the graph writes this tensor's storage
 
     gemm_nodes = [n for n in graph._nodes if n.task_type in (TaskType.LINEAR, TaskType.MATMUL) and n.outputs and n.outputs[0].numel()]
-    # two-CTA tiles pay once the 256-row tiles of every GEMM cover the worker pairs; few-row nodes keep the graph on one-CTA tiles
-    cta_pair = (mode == "static" and workers >= 4 and bool(gemm_nodes) and not any(_few_rows(n) for n in gemm_nodes)
-                and all(-(-_flat2d(n.inputs[0]).shape[0] // (2 * BM)) * -(-n.outputs[0].shape[-1] // 256) >= workers // 2
-                        for n in gemm_nodes))
+    def _waves(n: TaskNode, pair: bool) -> int:
+        """Rounds of tiles times their length, in k-blocks of 128 columns (``ProgramBuilder.gemm`` takes 128-column tiles where 256 leave
+        workers idle)."""
+        x2, w = _flat2d(n.inputs[0]), n.inputs[1]
+        rows, (cols, k) = x2.shape[0], (w.shape if n.task_type == TaskType.LINEAR else w.shape[::-1])
+        bn = 256 if n.attrs.get("activation") == "swiglu" or -(-rows // BM) * -(-cols // 256) >= workers else 128
+        tiles = -(-rows // (2 * BM if pair else BM)) * -(-cols // bn)
+        return -(-tiles // (workers // 2 if pair else workers)) * -(-k // BK) * (bn // 128)
+
+    # Two-CTA tiles wherever they take no more rounds than one-CTA ones and the products are long: a third less operand traffic per
+    # flop. One- / two-CTA, MLP block of rows x hidden x ffn, one B200, us: 1003 x 2048 x 5504 110 / 103, 300 x 2048 x 8192 107 / 101, 640 x 3072 x
+    # 8192 151 / 140, 4096 x 2048 x 8192 391 / 356; with K of 1024 and less the two halves of a tile wait for each other's epilogue:
+    # 2048 x 1024 x 2816 73.4 / 76.5, 8192 x 512 x 2048 137 / 144. Short products keep the older rule (tiles of 256 x 256 outputs
+    # cover every pair); few-row nodes keep the graph on one-CTA tiles.
+    cta_pair = mode == "static" and workers >= 4 and bool(gemm_nodes) and not any(_few_rows(n) for n in gemm_nodes)
+    if cta_pair:
+        long = all(_flat2d(n.inputs[0]).shape[0] > BM and _flat2d(n.inputs[0]).shape[1] >= 1536 for n in gemm_nodes)
+        cta_pair = ((long and sum(_waves(n, True) for n in gemm_nodes) <= sum(_waves(n, False) for n in gemm_nodes))
+                    or all(-(-_flat2d(n.inputs[0]).shape[0] // (2 * BM)) * -(-n.outputs[0].shape[-1] // 256) >= workers // 2 for n in gemm_nodes))
     from ..comm.process_group import get_world_size
     _COLL = (TaskType.ALLREDUCE, TaskType.BROADCAST, TaskType.ALL_TO_ALL, TaskType.ALLGATHER, TaskType.REDUCE_SCATTER)
     dist = get_world_size() > 1 and any(n.task_type in _COLL for n in graph._nodes)
@@ -1549,6 +1605,7 @@ def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None)
             if (len(cs) == 1 and cs[0].task_type == TaskType.REDUCE_SCATTER and len(cs[0].depends_on) == 1
                     and gc.fusable_linear_reduce_scatter(n, cs[0], heap.world) and not _few_rows(n)):
                 fused_rs[n._node_id] = cs[0]
+    fused_add = {} if dist else _residual_adds(graph, _few_rows, _static)       # linear node id -> (the add its epilogue does, the other operand)
     produced: Dict[int, Tuple[TaskNode, RowEvents]] = {}       # node id -> events of its output
     behind_collective: set = set()                             # nodes that (transitively) depend on a collective
 
@@ -1609,10 +1666,19 @@ def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None)
                                 and d.outputs[0].data_ptr() == node.inputs[0].data_ptr()), None)
                     if src is not None:
                         order = _fused.gathered_order(heap.rank, heap.world, x2.shape[0] // heap.world // BM, False)
-                ev = b.gemm(x2, w, out2, trans_b=(t == TaskType.MATMUL), epilogue=act, bias=bias,
-                            a_ready=aligned, extra_waits=extra, m_blocks=order)
+                if node._node_id in fused_add:
+                    add, res = fused_add[node._node_id]
+                    ev = b.gemm(x2, w, out2, trans_b=(t == TaskType.MATMUL), epilogue="residual_dual", aux=res.view(out2.shape),
+                                second=add.outputs[0].view(out2.shape), a_ready=aligned, extra_waits=extra)
+                    produced[add._node_id] = (add, ev)
+                    skip[add._node_id] = True
+                else:
+                    ev = b.gemm(x2, w, out2, trans_b=(t == TaskType.MATMUL), epilogue=act, bias=bias,
+                                a_ready=aligned, extra_waits=extra, m_blocks=order)
             produced[node._node_id] = (node, ev)
         elif t in _ELT_TYPES:
+            if skip.get(node._node_id):
+                continue
             x = node.inputs[0]
             cols = x.shape[-1]
             rows = x.numel() // cols

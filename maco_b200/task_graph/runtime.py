@@ -180,13 +180,40 @@ class StreamRuntime(_RuntimeBase):
         super().__init__(device, graph)
         from ..sync.stream_manager import StreamManager
         self._sm = StreamManager(self.device) if self.device.type == "cuda" else None
+        self._chain, self._chain_of = None, None
+
+    def _f32_chain(self, schedule: TaskSchedule):
+        """A graph of fp32 linears and matrix products alone runs as one native call; None for every other graph. What the nodes
+        hold is compared with what the chain was made for in each call."""
+        from ..config import config
+        if config.allow_tf32:
+            return None
+        nodes = [n for wave in schedule.waves for n in wave]
+        tensors = [t for n in nodes for t in n.inputs + n.outputs]
+        if self._chain_of is not schedule or (self._chain is not None and (len(tensors) != len(self._chain.tensors) or any(
+                a is not b for a, b in zip(tensors, self._chain.tensors)))):
+            from ..ops.gemm import F32Chain
+            self._chain, self._chain_of = None, schedule
+            if nodes and all(n.task_type in (TaskType.LINEAR, TaskType.MATMUL) and len(n.outputs) == 1 for n in nodes):
+                self._chain = F32Chain.make([(n.inputs[0], n.inputs[1], n.inputs[2] if n.attrs.get("has_bias") else None, n.outputs[0],
+                                              n.attrs.get("activation") if n.task_type == TaskType.LINEAR else None,
+                                              n.task_type == TaskType.MATMUL) for n in nodes])
+        return self._chain
 
     def execute(self, schedule: TaskSchedule, stream=None) -> None:
         if stream is not None and isinstance(stream, torch.cuda.Stream):
             with torch.cuda.stream(stream):
-                self._run(schedule)
+                self._execute(schedule)
         else:
-            self._run(schedule)
+            self._execute(schedule)
+
+    def _execute(self, schedule: TaskSchedule) -> None:
+        chain = self._f32_chain(schedule)
+        if chain is not None:
+            if chain.run():
+                return
+            self._chain_of = None            # a tensor has moved: this pass node by node, the next one with a new chain
+        self._run(schedule)
 
     def _run(self, schedule: TaskSchedule) -> None:
         main = torch.cuda.current_stream(self.device)
