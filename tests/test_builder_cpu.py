@@ -4,7 +4,7 @@ import collections
 
 import pytest
 
-from maco_b200.ops.megakernel import attention_pieces, pick_split_k
+from maco_b200.ops.megakernel import attention_pieces, pick_split_k, stream_pieces
 
 
 @pytest.mark.parametrize("groups,kv_len,workers", [(256, 4097, 148), (512, 4097, 148), (64, 4097, 148),
@@ -100,3 +100,16 @@ def test_switch_of_the_fused_finishing_pass_holds_for_few_rows(monkeypatch):
     assert mk.T_SPLITK_FIN in kinds and not any(few)
     assert all(types(1152)[1]) and all(types(1024, K=520)[1])
     assert all(types(1024, fused_finish=True)[1])                        # the argument goes before the switch
+
+
+@pytest.mark.parametrize("n_tiles,steps", [(1, 1), (1, 3), (16, 16), (20, 40), (24, 16), (40, 16), (96, 16), (100, 40), (148, 7), (149, 7), (224, 32), (60, 2)])
+def test_stream_pieces_cover_every_step_once(n_tiles, steps):
+    """A few-row GEMM's (tile, k-step) pairs: each in one part, and one part per worker where the tiles divide well over them."""
+    pieces = stream_pieces(n_tiles, steps, 148)
+    seen = sorted((t, s) for t, s0, n, _ in pieces for s in range(s0, s0 + n))
+    assert seen == [(t, s) for t in range(n_tiles) for s in range(steps)]
+    assert all(0 <= w < 148 and n > 0 for _, _, n, w in pieces)
+    if 90 <= n_tiles * (148 // n_tiles if n_tiles <= 148 else 0) and steps // 2 >= 148 // n_tiles:
+        workers = [w for _, _, _, w in pieces]
+        assert len(set(workers)) == len(workers)
+        assert max(n for _, _, n, _ in pieces) - min(n for _, _, n, _ in pieces) <= 1
