@@ -130,7 +130,7 @@ struct MacoGemmArgs {             /* one output tile */
   uint16_t epi;                   /* index into the epilogue table */
   uint8_t a_mn, b_mn;             /* operand majors (bit 0: MN-major). b_mn bit 1: B is stored tile by tile ([N/256][K/64][256][64]); count_base = its total k-blocks.
                                      b_mn bit 2: few-row task: tmap_a = weights, tmap_b = tokens, m0 = first feature, k_blocks in steps of 128, bn = padded tokens,
-                                     row_off = index of its arrival counter, count_base = arrivals that complete the tile */
+                                     row_off = index of its arrival counter, count_base = arrivals that complete the tile; bits 3 and 4: csrc/fewrow_gemm.cuh */
   int32_t m0, n0, k0, k_blocks;
   uint32_t idesc;
   int32_t peer;                   /* -1: store to the epilogue's out; >= 0: into that rank's heap at out_off; -2: into every rank's heap at out_off */

@@ -72,11 +72,15 @@ __device__ __noinline__ bool experts_produce(const Program& p, const MacoExpertA
       ok = gemm_produce_tile<256, STAGES, false, false>(smem, c, tmaps + a.tmap_x, tmaps + a.tmap_w1, m0, (el * tiles.tiles[0] + tiles.nb) * 256, 0,
                                                         a.hidden / kBK, it, p.budget_ns);
     } else {
-      // the first weights are on their way before the row block of activations is complete
+      // A row block that is complete (all but the first ones of a share) goes on without a pause: the look at its counter is over before
+      // the stages of the tile in front are free. Else the first weights are on their way while it is waited for.
       uint32_t ahead = 0;
       const int n0 = el * a.hidden + tiles.nb * 256;
-      ok = gemm_produce_b_ahead<256, STAGES>(smem, c, tmaps + a.tmap_w2, n0, 0, a.inter / kBK, it, p.budget_ns, -1, ahead);
-      if (!ok || !wait(a.ready + tiles.slab * (a.capacity / kBM) + tiles.mb, gate_done)) { it += ahead; return false; }
+      const uint32_t* ready = a.ready + tiles.slab * (a.capacity / kBM) + tiles.mb;
+      if (ld_acquire_gpu_u32(ready) < gate_done) {
+        ok = gemm_produce_b_ahead<256, STAGES>(smem, c, tmaps + a.tmap_w2, n0, 0, a.inter / kBK, it, p.budget_ns, -1, ahead);
+        if (!ok || !wait(ready, gate_done)) { it += ahead; return false; }
+      }
       fence_proxy_async_all();
       ok = gemm_produce_tile<256, STAGES, false, false>(smem, c, tmaps + a.tmap_act, tmaps + a.tmap_w2, m0, n0, 0, a.inter / kBK, it, p.budget_ns,
                                                         nullptr, kBK, -1, ahead);

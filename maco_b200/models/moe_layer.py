@@ -167,7 +167,8 @@ class MoEEPLayer:
             n_out += 1
         b.add_task(T_MOE_COUNTS, _pack_elt(0, 0, pp, N.ptr(self.ready), 0, 0, self.ready.numel() if grouped else 0, dt, 0, 0, i0=1),
                    waits=[(e_ret, n_ret, True, False)], signals=[e_out])
-        fused.epoch_fence_signal(b, [(e_out, n_out + 1, False, False)])
+        if W > 1:
+            fused.epoch_fence_signal(b, [(e_out, n_out + 1, False, False)])
         # (a CPU device plans only: the task list stays in ``self.builder`` for host-side schedule checks)
         self.builder = b
         self.program = b.build() if self.device.type == "cuda" else None

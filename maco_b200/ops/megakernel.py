@@ -833,21 +833,25 @@ class ProgramBuilder:
             pieces = [(t, 0, steps, t % self.num_workers) for t in range(n_tiles)]
         else:
             pieces = stream_pieces(n_tiles, steps, self.num_workers)
-        tiles_per_group = 2 if mode == 1 else 1
+        # A tile that is one part is finished from its accumulator (few_direct in csrc/fewrow_gemm.cuh); of a gate / up pair such a tile
+        # holds 64 features of each, so that no two workers have to meet.
+        direct = mode != 3 and all(n == steps for _, _, n, _ in pieces)
+        tiles_per_group = 2 if mode == 1 and not direct else 1
         n_groups = n_tiles // tiles_per_group
         arrivals = collections.Counter(tile // tiles_per_group for tile, _, _, _ in pieces)
         npad = -(-M // 16) * 16
-        ws = torch.zeros(M, Nn, device=a.device, dtype=torch.float32)
+        ws = torch.zeros(0 if direct else M, Nn, device=a.device, dtype=torch.float32)
         counters = torch.zeros(n_groups, device=a.device, dtype=torch.int32)
         self.launch_state += [ws, counters]
         par = self._rope_params(rope, M, Nn, a.device) if mode == 3 else aux
-        fin = _pack_elt(ws.data_ptr(), N.ptr(par), 0, N.ptr(out), 0, M, Nn // tiles_per_group, N.DTYPE_CODE[out_dtype], Nn, ld_o, i0=mode, i1=-1)
+        fin = _pack_elt(ws.data_ptr(), N.ptr(par), 0, N.ptr(out), 0, M, Nn // (2 if mode == 1 else 1), N.DTYPE_CODE[out_dtype], Nn, ld_o, i0=mode, i1=-1)
         fin_dev = torch.frombuffer(bytearray(fin), dtype=torch.uint8).to(a.device)
         self.epis.append(_pack_epilogue(ws.data_ptr(), counters.data_ptr(), fin_dev.data_ptr(), Nn, 0, EPI["fewrow"],
                                         N.DTYPE_CODE[torch.float32], 0, 0, Nn, M, 1.0))
         epi = len(self.epis) - 1
         self.keepalive += [t for t in (a, w, out, aux, ws, counters, fin_dev) if t is not None]
-        tw = self._tmap(w, Nn, K, w.stride(0), False, BM)
+        split = direct and mode == 1
+        tw = self._tmap(w, Nn, K, w.stride(0), False, 64 if split else BM)
         tx = self._tmap(a, M, K, a.stride(0), False, npad)
         idesc = make_idesc(1 if a.dtype == torch.bfloat16 else 0, BM, npad, 0, 0)
         node_id = self.new_node_id()
@@ -859,7 +863,8 @@ class ProgramBuilder:
         done = self.new_event()
         for tile, s0, n, wk in pieces:
             group = tile // tiles_per_group
-            raw = _pack_gemm(tw, tx, epi, 0, 4, tile * 128, 0, s0 * 128, n, idesc, -1, group, 0, npad, count_base=arrivals[group])
+            m0 = tile // 2 * 256 + tile % 2 * 64 if split else tile * 128
+            raw = _pack_gemm(tw, tx, epi, 0, 4 | (8 if direct else 0) | (16 if split else 0), m0, 0, s0 * 128, n, idesc, -1, group, 0, npad, count_base=arrivals[group])
             self.add_task(int(TaskType.LINEAR), raw, waits=waits, signals=[done], node_id=node_id, worker=wk, b_static=w_static)
         return RowEvents(rows=M, block=BM, row_events=[(done, n_groups)], all_event=(done, n_groups))
 
