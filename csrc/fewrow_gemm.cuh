@@ -8,12 +8,13 @@
 // are exchanged to keep every SM busy. A ring stage holds two k-blocks: 2 x 16 KB of weights and 2 x (tokens x 128) bytes
 // of x, so the four 48 KB stages keep 128 KB of weights in flight per SM.
 //
-// Work split: all (feature tile, 128-wide k-step) pairs of the GEMM in one line, cut into one equal piece per worker
-// (ProgramBuilder.gemm_stream). A worker's piece covers parts of one to three tiles; each part is a task that adds its fp32
-// sums into a [tokens, features] workspace. The accumulator has one feature per TMEM lane, so a warp's reduction
-// instruction covers 128 consecutive bytes of one token's row. Whoever arrives last at a tile's counter finds every
-// part summed and finishes the tile (operator, 16-bit store, workspace zeroed for the next launch) through shared
-// memory in short loops; only that task signals the tile's event.
+// Work split (ProgramBuilder.gemm_stream): equal parts of whole feature tiles, one part per worker; where the tiles do not divide well
+// over the workers, all (feature tile, 128-wide k-step) pairs in one line, cut into one equal piece per worker. A part is a
+// task that adds its fp32 sums into a [tokens, features] workspace. The accumulator has one feature per TMEM lane, so a
+// warp's reduction instruction covers 128 consecutive bytes of one token's row. Whoever arrives last at a tile's counter finds
+// every part summed and finishes the tile (operator, 16-bit store) through shared memory in short loops, signals the tile's
+// event and clears the tile's workspace for the next launch. A tile that is one part skips all that (few_direct).
+// One B200, decode layer of batch 64: 190 -> 162 us with one part per worker instead of the line alone, 159 with few_direct.
 #pragma once
 #include "gemm_tcgen05.cuh"
 #include "row_tasks.cuh"

@@ -134,9 +134,9 @@ def pick_split_k(n_tiles: int, k_blocks: int, workers: int) -> int:
 
 
 def stream_pieces(n_tiles: int, steps: int, workers: int) -> List[Tuple[int, int, int, int]]:
-    """Cuts the ``n_tiles * steps`` (tile, k-step) pairs of a few-row GEMM into one nearly equal piece per worker, at least
-    two steps (64 KB of weights) each. Returns (tile, first step, steps, worker): a worker's piece is split where it
-    crosses a tile. A cut that would leave less than an eighth of a piece on one side of a tile boundary moves to it
+    """Cuts the ``n_tiles * steps`` (tile, k-step) pairs of a few-row GEMM over the workers. Returns (tile, first step, steps, worker).
+    Where the tiles divide well, each is cut into equal parts of at least two steps (64 KB of weights), one per worker. Else all pairs
+    lie in one line with one nearly equal piece per worker, split where it crosses a tile; a cut that would leave less than an eighth of a piece on one side of a tile boundary moves to it
     (a part costs about a microsecond of reductions and arrival whatever its length)."""
     total = n_tiles * steps
     parts = min(workers // n_tiles, max(1, steps // 2)) if n_tiles else 0
@@ -810,7 +810,7 @@ class ProgramBuilder:
                     extra_waits: Sequence[Tuple[int, int, bool, bool]] = (), rope: Optional[dict] = None,
                     w_static: bool = False, whole_tiles: bool = False) -> RowEvents:
         """``out = op(a @ w.T)`` for at most 64 rows (csrc/fewrow_gemm.cuh): weights on the M side of the MMA, 128
-        features per tile, the whole GEMM cut into one equal piece of the weight stream per worker. Operators as in
+        features per tile, the weight stream cut over the workers (``stream_pieces``). Operators as in
         ``gemm_splitk``: None, "swiglu", "residual" (``aux``), "qk_rope" (``rope``, ``out=None``).
         The parts of a tile add up in the order in which they arrive, so the last bits of a result can differ from launch to
         launch; with ``whole_tiles`` a tile is one part and they do not."""
