@@ -1500,8 +1500,9 @@ def can_lower(graph) -> bool:
 
 def _residual_adds(graph, few_rows, static) -> Dict[int, Tuple[TaskNode, torch.Tensor]]:
     """Adds that the linear in front of them does in its epilogue (``residual_dual``): the add depends on that linear alone, its other
-    operand is written by no node of the graph, and all three tensors are contiguous 16-bit rows of 16-byte vectors. Both outputs are
-    written as before; what goes is a phase of the graph and a read of the product."""
+    operand is written by no node of the graph, its result lies in none of the product's operands (a tile would overwrite what other
+    tiles still load), and all three tensors are contiguous 16-bit rows of 16-byte vectors. Both outputs are written as before; what
+    goes is a phase of the graph and a read of the product."""
     found: Dict[int, Tuple[TaskNode, torch.Tensor]] = {}
     for add in graph._nodes:
         deps = list(dict.fromkeys(add.depends_on))
@@ -1512,13 +1513,16 @@ def _residual_adds(graph, few_rows, static) -> Dict[int, Tuple[TaskNode, torch.T
                 or lin.attrs.get("activation") not in (None, "none")):
             continue
         y, z = lin.outputs[0], add.outputs[0]
-        if any(n.outputs and n is not add and n.outputs[0].untyped_storage().data_ptr() == z.untyped_storage().data_ptr() for n in graph._nodes):
+        z_mem = z.untyped_storage().data_ptr()
+        if any(t.untyped_storage().data_ptr() == z_mem for t in lin.inputs):
+            continue
+        if any(n.outputs and n is not add and n.outputs[0].untyped_storage().data_ptr() == z_mem for n in graph._nodes):
             continue
         same = [t.data_ptr() == y.data_ptr() and t.shape == y.shape for t in add.inputs]
         if same.count(True) != 1:
             continue
         res = add.inputs[same.index(False)]
-        if (static(res) and _vector_rows(y, z, res) and res.untyped_storage().data_ptr() != z.untyped_storage().data_ptr()):
+        if static(res) and _vector_rows(y, z, res) and res.untyped_storage().data_ptr() != z_mem:
             found[lin._node_id] = (add, res)
     return found
 
