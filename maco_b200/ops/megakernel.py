@@ -1534,6 +1534,34 @@ def _vector_rows(*tensors: torch.Tensor) -> bool:
                and t.data_ptr() % 16 == 0 and (t.shape[-1] * 2) % 16 == 0 for t in tensors)
 
 
+def _row_by_row(node: TaskNode, dep: TaskNode) -> bool:
+    """Whether rows of ``node`` may follow the same rows of ``dep`` without the rest of it: of what ``dep`` writes ``node`` reads those rows
+    alone, and of what ``dep`` reads ``node`` overwrites those rows alone. A weight, a bias, a norm's scale or the right-hand side of a
+    matmul is read whole by every row."""
+    from ..task_graph.graph import _byte_range, _storage_key
+
+    def by_rows(n: TaskNode) -> int:
+        """How many inputs of ``n``, from the first on, are read row by row. (What a collective sends may leave in any order.)"""
+        if n.task_type in (TaskType.ADD, TaskType.SILU_GATE):
+            return 2
+        return 1 if n is node or n.task_type in (TaskType.LINEAR, TaskType.MATMUL) or n.task_type in _ELT_TYPES else 0
+
+    def same_rows(a: torch.Tensor, b: torch.Tensor) -> bool:
+        return (a.data_ptr() == b.data_ptr() and a.numel() == b.numel() and a.shape[-1:] == b.shape[-1:] and a.dtype == b.dtype
+                and a.is_contiguous() and b.is_contiguous())
+
+    def meet(a: torch.Tensor, b: torch.Tensor) -> bool:
+        (a0, a1), (b0, b1) = _byte_range(a), _byte_range(b)
+        return _storage_key(a) == _storage_key(b) and a0 < b1 and b0 < a1
+
+    for reader, writer in ((node, dep), (dep, node)):
+        for o in writer.outputs:
+            for i, t in enumerate(reader.inputs):
+                if meet(t, o) and not (i < by_rows(reader) and same_rows(t, o)):
+                    return False
+    return True
+
+
 def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None) -> Program:
     """Lowers a TaskGraph (dependencies already inferred) to a persistent-kernel program."""
     import os
@@ -1619,8 +1647,8 @@ def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None)
     behind_collective: set = set()                             # nodes that (transitively) depend on a collective
 
     def ready_of(node: TaskNode, t: torch.Tensor, rows: int) -> Tuple[Optional[RowEvents], List[tuple]]:
-        """Row-aligned events for tensor ``t`` if one dependency produced exactly this view; every other
-        dependency becomes a whole-node wait."""
+        """Row-aligned events for tensor ``t`` if one dependency produced exactly this view and its rows are all that matters
+        (``_row_by_row``); every other dependency becomes a whole-node wait."""
         aligned, extra = None, []
         for dep in node.depends_on:
             ent = produced.get(dep._node_id)
@@ -1629,7 +1657,7 @@ def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None)
             dnode, ev = ent
             o = dnode.outputs[0]
             if (aligned is None and t is not None and o.data_ptr() == t.data_ptr() and o.numel() == t.numel()
-                    and ev.rows == rows and o.numel() > 0):
+                    and ev.rows == rows and o.numel() > 0 and _row_by_row(node, dnode)):
                 aligned = ev
             else:
                 extra.append((ev.all_event[0], ev.all_event[1], ev.sys, False))
@@ -1708,7 +1736,8 @@ def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None)
                 # second operand: look for its own row-aligned producer among the remaining dependencies
                 for dep in node.depends_on:
                     ent = produced.get(dep._node_id)
-                    if ent and ent[0].outputs[0].data_ptr() == in1.data_ptr() and ent[1].rows == rows and ent[1] is not aligned:
+                    if (ent and ent[0].outputs[0].data_ptr() == in1.data_ptr() and ent[1].rows == rows and ent[1] is not aligned
+                            and _row_by_row(node, ent[0])):
                         readies.append(ent[1])
                         extra = [e for e in extra if e[0] != ent[1].all_event[0]]
                         break

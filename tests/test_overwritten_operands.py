@@ -40,6 +40,41 @@ def test_an_add_over_an_operand_of_its_product_is_a_task_of_its_own(form, folded
     assert (ADD not in kinds) == folded
 
 
+def _ran_without(tasks, withheld):
+    """Indices of the tasks that run when those in ``withheld`` never do: wait conditions alone, in any order of workers."""
+    done, events, again = set(), {}, True
+    while again:
+        again = False
+        for i, t in enumerate(tasks):
+            if i in done or i in withheld or any(e >= 0 and events.get(e, 0) < c for e, c in zip(t["wait_event"], t["wait_count"])):
+                continue
+            done.add(i)
+            again = True
+            for e in t["signal_event"]:
+                events[e] = events.get(e, 0) + 1
+    return done
+
+
+@pytest.mark.parametrize("form,whole", [("b", True), ("w", True), ("x", False)])
+def test_an_add_over_what_every_row_of_the_product_reads_waits_for_all_of_it(form, whole, monkeypatch):
+    """Over the weight or the right-hand side: behind every tile. Over the product's rows: behind the tiles of these rows."""
+    tasks = _lower(_graph("cpu", form, 512, 512)[0], monkeypatch).tasks
+    gemm, adds = [i for i, t in enumerate(tasks) if t["type"] in (100, 101)], [i for i, t in enumerate(tasks) if t["type"] == ADD]
+    assert len(gemm) >= 4 and adds
+    ran = [len(_ran_without(tasks, {g}) & set(adds)) for g in gemm]
+    assert all(n == 0 if whole else 0 < n < len(adds) for n in ran)
+
+
+def test_a_product_with_one_tensor_on_both_sides_waits_for_all_of_it(monkeypatch):
+    """``h @ h``: a tile reads every row of the right-hand side."""
+    g = maco.TaskGraph(num_workers=148, device="cpu")
+    h = g.gelu(torch.randn(512, 512).bfloat16())
+    g.matmul(h.output, h.output)
+    tasks = _lower(g, monkeypatch).tasks
+    gelu, gemm = [i for i, t in enumerate(tasks) if t["type"] not in (0, 100, 101)], {i for i, t in enumerate(tasks) if t["type"] in (100, 101)}
+    assert len(gelu) > 1 and all(not _ran_without(tasks, {i}) & gemm for i in gelu)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("rows", [130, 512, 1300])
 def test_residual_add_over_the_rows_of_its_product(rows):
@@ -55,3 +90,19 @@ def test_residual_add_over_the_rows_of_its_product(rows):
         # fp32 sums of 1024 terms in the tensor cores' order either way; one rounding each
         assert torch.allclose(y.output.float(), want.float(), rtol=2 ** -7, atol=1e-3)
         assert torch.equal(z.output, (y.output.float() + r.float()).to(x.dtype)) and torch.equal(w, w0)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["b", "w"])
+def test_add_over_what_every_row_of_the_product_reads(form):
+    g, y, z, args, r = _graph("cuda", form, 1024, 1024)
+    kept = [t.clone() for t in args]
+    want = kept[0].float() @ (kept[1].float() if form == "b" else kept[1].float().t())
+    g.compile()
+    assert g.runtime_kind == "persistent"
+    for _ in range(20):
+        for t, k in zip(args, kept):
+            t.copy_(k)
+        g.execute()
+        assert torch.allclose(y.output.float(), want, rtol=2 ** -7, atol=1e-3)      # fp32 sums in another order, one rounding
+        assert torch.equal(z.output, (y.output.float() + r.float()).to(r.dtype))
