@@ -276,7 +276,7 @@ static_assert(sizeof(MacoTaskDesc) == 128, "task descriptor must stay 128 bytes"
 
 /* ---- mixture-of-experts layer constants (one per layer, in device memory) --------------------- */
 struct MacoMoeParams {
-  const void* logits;             /* [tokens, experts] router output (16-bit) */
+  const void* logits;             /* [tokens, experts] router output (16-bit), rows of ld_logits elements: a multiple of 8 */
   const void* x;                  /* [tokens, hidden] */
   uint32_t* counts;               /* [experts] slots handed out by this rank, zero at launch start; then the dropped pairs of the last
                                      launch and of this one */
@@ -286,7 +286,7 @@ struct MacoMoeParams {
   unsigned long long cnt_off;     /* heap offset: received counts [world][experts_per_rank] (uint32) */
   unsigned long long comb_off;    /* heap offset of comb */
   const void* y;                  /* [experts_per_rank][world][capacity][hidden] expert outputs (local) */
-  int32_t hidden, experts, top_k, experts_per_rank, capacity, tokens, dtype, _pad;
+  int32_t hidden, experts, top_k, experts_per_rank, capacity, tokens, dtype, ld_logits;
 };
 
 /* The expert GEMMs of one layer (MACO_TASK_MOE_EXPERTS, csrc/moe_experts.cuh): slab (expert, source rank) holds `capacity` rows. */

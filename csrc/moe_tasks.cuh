@@ -60,7 +60,7 @@ MACO_DEVICE bool moe_topk_dispatch(const Program& p, const MacoEltArgs& ar, int 
 #pragma unroll
     for (int i = 0; i < kChunks; ++i) {
       const int e = 64 * i + 2 * lane;
-      if (e < E) v[i] = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(m.logits) + (size_t)t * E + e);
+      if (e < E) v[i] = *reinterpret_cast<const uint32_t*>(reinterpret_cast<const uint16_t*>(m.logits) + (size_t)t * m.ld_logits + e);
     }
   };
   bool ok = true;                                      // (after a wait that ran out a warp sends no more but meets the others at every barrier)

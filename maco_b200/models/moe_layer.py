@@ -90,7 +90,8 @@ class MoEEPLayer:
         self.w1 = torch.stack(w1)                                   # [EL, 2I, H], gate/up interleaved per 256 rows
         self.w2 = torch.stack(w2)                                   # [EL, H, I]
         self.x = torch.empty(T, H, device=dev, dtype=dtype)
-        self.logits = torch.empty(T, experts, device=dev, dtype=dtype)
+        # rows of whole 16-byte vectors: the router stores vectors and routing reads pairs of logits, whatever the number of experts
+        self.logits = torch.empty(T, -(-experts // 8) * 8, device=dev, dtype=dtype)[:, :experts]
         # per expert the slots handed out in this launch (cleared at its end); the pairs dropped by the last launch; by this one
         self.counts = torch.zeros(experts + 2, device=dev, dtype=torch.int32)
         self.recv = heap.alloc((EL, W, C, H), dtype)
@@ -103,7 +104,7 @@ class MoEEPLayer:
         params = struct.pack("<QQQQQQQQQiiiiiiii", self.logits.data_ptr(), self.x.data_ptr(), self.counts.data_ptr(),
                              self.comb.data_ptr(), heap.offset_of(self.recv), heap.offset_of(self.meta),
                              heap.offset_of(self.cnt), heap.offset_of(self.comb), self.y.data_ptr(), H, experts, K, EL, C, T,
-                             N.DTYPE_CODE[dtype], 0)
+                             N.DTYPE_CODE[dtype], self.logits.stride(0))
         self.d_params = torch.from_numpy(np.frombuffer(params, dtype=np.uint8).copy()).to(dev)
         # Dropped-pair count of the last step, delivered without a blocking read: every forward() copies the counter
         # into pinned host memory behind the launch, and the NEXT forward() (or dropped()) looks at it. A step that

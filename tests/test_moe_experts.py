@@ -1,0 +1,48 @@
+"""Expert layers at counts, types and routes where routing and the expert shares can go wrong."""
+import pytest
+import torch
+
+
+def _plan(**kw):
+    from maco_b200.models.moe_layer import MoEEPLayer
+    from maco_b200.parallel.symm_heap import PlanningHeap
+    return MoEEPLayer(device=torch.device("cpu"), heap=PlanningHeap(0, 1, 1 << 26), **kw)
+
+
+@pytest.mark.parametrize("experts", [1, 2, 3, 5, 7, 8, 9, 12, 20, 64, 255])
+def test_router_rows_are_whole_vectors(experts):
+    """The router's tail stores 16-byte vectors of 8 logits and routing reads two logits at a time, up to the last odd one: all of
+    them aligned, inside the allocation, and the kernel told the row length that the tensor has."""
+    import struct
+    layer = _plan(hidden=256, experts=experts, top_k=1, inter=128, tokens=128, capacity_factor=1.0)
+    ld = layer.logits.stride(0)
+    assert layer.logits.shape == (128, experts) and ld % 8 == 0 and layer.logits.data_ptr() % 16 == 0
+    assert layer.logits.storage_offset() == 0
+    last = layer.logits.untyped_storage().nbytes() // 2
+    for t in range(128):
+        for e in range(0, experts, 2):
+            assert (t * ld + e) % 2 == 0 and t * ld + e + 1 < last
+    words = struct.unpack("<QQQQQQQQQiiiiiiii", layer.d_params.numpy().tobytes())
+    assert words[0] == layer.logits.data_ptr() and words[-1] == ld
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode", ["static", "dynamic"])
+@pytest.mark.parametrize("experts,top_k", [(1, 1), (3, 2), (5, 5), (12, 4), (31, 8)])
+def test_any_number_of_experts(experts, top_k, mode):
+    from maco_b200 import _native
+    from maco_b200.models.moe_layer import MoEEPLayer
+    layer = MoEEPLayer(hidden=256, experts=experts, top_k=top_k, inter=128, tokens=256, capacity_factor=float(experts), seed=3, mode=mode,
+                       weight_std=0.05, router_std=0.5)
+    x = torch.randn(256, 256, device="cuda", dtype=torch.bfloat16)
+    ref = layer.reference(x)
+    for _ in range(2):
+        out = layer(x)
+        torch.cuda.synchronize()
+        assert layer.dropped() == 0
+        # the bound of the single-GPU layer test: bf16 activations, and a token whose logits tie may take another expert
+        assert (out.float() - ref).abs().max().item() < 4e-2 * max(1.0, ref.abs().max().item())
+    # the router's rows, the ragged last vector among them: fp32 sums of 256 terms, rounded once
+    logits = x.float() @ layer.w_router.float().t()
+    assert ((layer.logits.float() - logits).abs() <= 2.0 ** -8 * logits.abs() * 1.01 + 1e-3).all()
+    assert _native.status() == 0
