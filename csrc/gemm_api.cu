@@ -15,11 +15,11 @@ namespace {
 // Optional per-CTA cycle counters of the stand-alone GEMM kernels (8 x int64 per CTA), off unless set.
 long long* g_gemm_dbg = nullptr;
 
-template <int BN, int STAGES, bool A_MN, bool B_MN>
+template <int BN, int STAGES, bool A_MN, bool B_MN, bool BESIDE>
 int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmEpilogue& epi, int K, uint32_t idesc,
                 int max_ctas, uint64_t budget_ns, cudaStream_t stream) {
   using L = GemmSmemLayout<BN, STAGES>;
-  auto kern = gemm_tcgen05_kernel<BN, STAGES, A_MN, B_MN>;
+  auto kern = gemm_tcgen05_kernel<BN, STAGES, A_MN, B_MN, false, BESIDE>;
   static bool attr_set[64] = {};
   int dev = 0;
   MACO_CHECK_CUDA(cudaGetDevice(&dev));
@@ -39,20 +39,25 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmEpilog
   return 0;
 }
 
-template <int BN, int STAGES>
+// Products whose epilogue has a second tensor take the kernel instances that hold that epilogue.
+bool has_second(const GemmEpilogue& e) {
+  return e.mode == MACO_EPI_GELU_DUAL || (e.mode == MACO_EPI_GELU_BWD && e.out_type != MACO_DT_F32 && e.bias == nullptr);
+}
+
+template <int BN, int STAGES, bool BESIDE>
 int dispatch_major(bool a_mn, bool b_mn, const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmEpilogue& epi,
                    int K, uint32_t idesc, int max_ctas, uint64_t budget_ns, cudaStream_t stream) {
-  if (!a_mn && !b_mn) return launch_gemm<BN, STAGES, false, false>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
-  if (!a_mn && b_mn) return launch_gemm<BN, STAGES, false, true>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
-  if (a_mn && !b_mn) return launch_gemm<BN, STAGES, true, false>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
-  return launch_gemm<BN, STAGES, true, true>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
+  if (!a_mn && !b_mn) return launch_gemm<BN, STAGES, false, false, BESIDE>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
+  if (!a_mn && b_mn) return launch_gemm<BN, STAGES, false, true, BESIDE>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
+  if (a_mn && !b_mn) return launch_gemm<BN, STAGES, true, false, BESIDE>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
+  return launch_gemm<BN, STAGES, true, true, BESIDE>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
 }
 
 // fp32 operands on the tensor cores (kind::tf32): K-major operands only, 128 x 256 tiles.
 int launch_gemm_tf32(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmEpilogue& epi, int K, uint32_t idesc,
                      int max_ctas, uint64_t budget_ns, cudaStream_t stream) {
   using L = GemmSmemLayout<256, 4>;
-  auto kern = gemm_tcgen05_kernel<256, 4, false, false, true>;
+  auto kern = gemm_tcgen05_kernel<256, 4, false, false, true, false>;
   static bool attr_set[64] = {};
   int dev = 0;
   MACO_CHECK_CUDA(cudaGetDevice(&dev));
@@ -71,11 +76,11 @@ int launch_gemm_tf32(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmE
 }
 
 // Two-CTA tiles: clusters of two CTAs, 256 x BN per pair.
-template <int BN, bool A_MN, bool B_MN>
+template <int BN, bool A_MN, bool B_MN, bool BESIDE>
 int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmEpilogue& epi, int K, uint32_t idesc,
                      int max_ctas, uint64_t budget_ns, cudaStream_t stream) {
   using L = PairSmemLayout<kPairStages>;
-  auto kern = gemm_tcgen05_pair_kernel<BN, A_MN, B_MN>;
+  auto kern = gemm_tcgen05_pair_kernel<BN, A_MN, B_MN, BESIDE>;
   static bool attr_set[64] = {};
   int dev = 0;
   MACO_CHECK_CUDA(cudaGetDevice(&dev));
@@ -95,13 +100,13 @@ int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmE
   return 0;
 }
 
-template <int BN>
+template <int BN, bool BESIDE>
 int dispatch_major_pair(bool a_mn, bool b_mn, const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmEpilogue& epi,
                         int K, uint32_t idesc, int max_ctas, uint64_t budget_ns, cudaStream_t stream) {
-  if (!a_mn && !b_mn) return launch_gemm_pair<BN, false, false>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
-  if (!a_mn && b_mn) return launch_gemm_pair<BN, false, true>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
-  if (a_mn && !b_mn) return launch_gemm_pair<BN, true, false>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
-  return launch_gemm_pair<BN, true, true>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
+  if (!a_mn && !b_mn) return launch_gemm_pair<BN, false, false, BESIDE>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
+  if (!a_mn && b_mn) return launch_gemm_pair<BN, false, true, BESIDE>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
+  if (a_mn && !b_mn) return launch_gemm_pair<BN, true, false, BESIDE>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
+  return launch_gemm_pair<BN, true, true, BESIDE>(tmA, tmB, epi, K, idesc, max_ctas, budget_ns, stream);
 }
 
 // ---- CUDA-core GEMM for 16-bit operands without TMA alignment: 64x64 tile, 256 threads, 4x4 outputs per thread --------
@@ -273,14 +278,17 @@ int maco_gemm(const void* A, const void* B, void* D, int M, int N, int K, long l
   e.out = D; e.bias = bias; e.aux = aux; e.ld_out = ldd; e.ld_aux = ld_aux; e.mode = mode; e.out_type = out_type;
   e.bias_type = bias_type; e.aux_type = aux_type; e.M = M; e.N = N; e.alpha = alpha; e.aux_pack = 0;
   const uint64_t budget_ns = (uint64_t)((wait_budget_ms > 0 ? wait_budget_ms : 2000.0) * 1e6);
+  const bool second = has_second(e);
   if (pair) {
     const uint32_t idesc2 = make_idesc(ab_type == MACO_DT_BF16 ? 1u : 0u, 2 * kBM, bn, a_mn ? 1u : 0u, b_mn ? 1u : 0u);
-    if (bn == 256) return dispatch_major_pair<256>(a_mn, b_mn, tmA, tmB, e, K, idesc2, max_ctas, budget_ns, stream);
-    return dispatch_major_pair<128>(a_mn, b_mn, tmA, tmB, e, K, idesc2, max_ctas, budget_ns, stream);
+    auto run = bn == 256 ? (second ? dispatch_major_pair<256, true> : dispatch_major_pair<256, false>)
+                         : (second ? dispatch_major_pair<128, true> : dispatch_major_pair<128, false>);
+    return run(a_mn, b_mn, tmA, tmB, e, K, idesc2, max_ctas, budget_ns, stream);
   }
   const uint32_t idesc = make_idesc(ab_type == MACO_DT_BF16 ? 1u : 0u, kBM, bn, a_mn ? 1u : 0u, b_mn ? 1u : 0u);
-  if (bn == 256) return dispatch_major<256, 4>(a_mn, b_mn, tmA, tmB, e, K, idesc, max_ctas, budget_ns, stream);
-  return dispatch_major<128, 6>(a_mn, b_mn, tmA, tmB, e, K, idesc, max_ctas, budget_ns, stream);
+  auto run = bn == 256 ? (second ? dispatch_major<256, 4, true> : dispatch_major<256, 4, false>)
+                       : (second ? dispatch_major<128, 6, true> : dispatch_major<128, 6, false>);
+  return run(a_mn, b_mn, tmA, tmB, e, K, idesc, max_ctas, budget_ns, stream);
 }
 
 // fp32 inputs on the tensor cores as TF32 (10-bit mantissa: an opt-in, the default fp32 path is maco_gemm_simt).
