@@ -435,6 +435,7 @@ MACO_DEVICE bool gemm_epilogue_lean(int bn, const GemmCtrl& c, uint32_t tmem_bas
 // the general epilogue, whose element type and operator are asked for per element, its 32,768 derivatives took 50 us and the
 // backward pass of 8192 x 4096 layers ran at that rate. Here the operator is one branch per chunk of 32 columns and the
 // aux values of the next chunk are on their way while this one is computed.
+MACO_DEVICE bool epi_is_dual(const GemmEpilogue& e) { return e.mode == MACO_EPI_GELU_DUAL || e.mode == MACO_EPI_RESIDUAL_DUAL; }
 MACO_DEVICE bool epi_is_beside(const GemmEpilogue& e, int n0, int bn) {
   const bool res = e.mode == MACO_EPI_RESIDUAL_DUAL;
   const uintptr_t p = reinterpret_cast<uintptr_t>(e.aux) | (uintptr_t)(e.ld_aux * 2) | (res ? reinterpret_cast<uintptr_t>(e.bias) : 0);
@@ -516,7 +517,7 @@ __device__ __noinline__ bool gemm_epilogue_beside(int bn, const GemmCtrl& c, uin
 }
 
 // (DUAL: with the two modes that write a second tensor, for tiles of such a product that are ragged or not aligned)
-template <int BN, int SBN = BN, bool DUAL = true>
+template <int BN, int SBN, bool DUAL>
 MACO_DEVICE bool gemm_epilogue_tile(const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e_in,
                                     void* out_base, long long row_off, int m0, int n0,
                                     uint32_t tile_seq, uint64_t budget_ns, const EpiBroadcast* bc = nullptr,

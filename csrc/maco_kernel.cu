@@ -531,12 +531,15 @@ __device__ __noinline__ bool run_topk(const MacoProgram& p, const MacoEltArgs& a
   return moe_topk_dispatch(p, a, tid, bulk);
 }
 
-// The epilogue of a tile that is not a lean one (gemm_epilogue_lean), out of line.
+// The epilogue of a tile that is not a lean one (gemm_epilogue_lean), out of line. DUAL: ragged tiles with a second output, apart from the
+// others, whose spills those two modes triple (two-CTA form: 244 / 768 bytes stored / loaded without them, 760 / 1444 with them).
+template <bool DUAL>
 __device__ __noinline__ bool run_epilogue(const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e, void* out_base, const MacoGemmArgs& g,
                                           uint32_t seq, uint64_t budget_ns, const EpiBroadcast* bc, uint8_t* stage, uint32_t pair_empty_bar,
                                           int row_limit) {
-  if (g.bn == 128) return gemm_epilogue_tile<128, kMkBN>(c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, budget_ns, bc, stage, pair_empty_bar, row_limit);
-  return gemm_epilogue_tile<256, kMkBN>(c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, budget_ns, bc, stage, pair_empty_bar, row_limit);
+  if (g.bn == 128)
+    return gemm_epilogue_tile<128, kMkBN, DUAL>(c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, budget_ns, bc, stage, pair_empty_bar, row_limit);
+  return gemm_epilogue_tile<256, kMkBN, DUAL>(c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, budget_ns, bc, stage, pair_empty_bar, row_limit);
 }
 
 // Every task that is not a GEMM tile, behind one call: values of the task loop that live across a call cost a spill for each of
@@ -653,8 +656,10 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
         ok = gemm_epilogue_beside<kMkBN>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, pair_empty_bar);
       else if (g.peer == -1 && epi_is_lean(e, g.n0, (int)g.bn))
         ok = gemm_epilogue_lean<kMkBN>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, pair_empty_bar, row_limit);
+      else if (epi_is_dual(e))
+        ok = run_epilogue<true>(c, tmem_base, e, out_base, g, seq, p.budget_ns, bcp, stage, pair_empty_bar, row_limit);
       else
-        ok = run_epilogue(c, tmem_base, e, out_base, g, seq, p.budget_ns, bcp, stage, pair_empty_bar, row_limit);
+        ok = run_epilogue<false>(c, tmem_base, e, out_base, g, seq, p.budget_ns, bcp, stage, pair_empty_bar, row_limit);
       if (!ok) cur[2] = 1;
       ++seq;
       if (e.mode == MACO_EPI_SPLITK_FUSED) {
