@@ -1597,20 +1597,25 @@ def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None)
         return _storage_key(t) not in written                  # no node of the graph writes this tensor's storage
 
     gemm_nodes = [n for n in graph._nodes if n.task_type in (TaskType.LINEAR, TaskType.MATMUL) and n.outputs and n.outputs[0].numel()]
-    def _waves(n: TaskNode, pair: bool) -> int:
+    def _waves(n: TaskNode, pair: bool) -> float:
         """Rounds of tiles times their length, in k-blocks of 128 columns (``ProgramBuilder.gemm`` takes 128-column tiles where 256 leave
-        workers idle)."""
+        workers idle). A two-CTA tile of 256 columns takes about 5 % less than two one-CTA ones; one of 128 columns, or with a bias or an
+        activation in its epilogue, about 5 % more."""
         x2, w = _flat2d(n.inputs[0]), n.inputs[1]
         rows, (cols, k) = x2.shape[0], (w.shape if n.task_type == TaskType.LINEAR else w.shape[::-1])
         bn = 256 if n.attrs.get("activation") == "swiglu" or -(-rows // BM) * -(-cols // 256) >= workers else 128
         tiles = -(-rows // (2 * BM if pair else BM)) * -(-cols // bn)
-        return -(-tiles // (workers // 2 if pair else workers)) * -(-k // BK) * (bn // 128)
+        length = -(-k // BK) * (bn // 128)
+        if not pair:
+            return -(-tiles // workers) * length
+        return -(-tiles // (workers // 2)) * length * (0.95 if bn == 256 and (n.task_type == TaskType.MATMUL or _plain_linear(n)) else 1.05)
 
-    # Two-CTA tiles wherever they take no more rounds than one-CTA ones and the products are long: a third less operand traffic per
-    # flop. One- / two-CTA, MLP block of rows x hidden x ffn, one B200, us: 1003 x 2048 x 5504 110 / 103, 300 x 2048 x 8192 107 / 101, 640 x 3072 x
-    # 8192 151 / 140, 4096 x 2048 x 8192 391 / 356; with K of 1024 and less the two halves of a tile wait for each other's epilogue:
-    # 2048 x 1024 x 2816 73.4 / 76.5, 8192 x 512 x 2048 137 / 144. Short products keep the older rule (tiles of 256 x 256 outputs
-    # cover every pair); few-row nodes keep the graph on one-CTA tiles.
+    # Two-CTA tiles where they take less time by that count and the products are long: a third less operand traffic per flop.
+    # Two- / one-CTA, one B200, us: MLP blocks of rows x hidden x ffn 1003 x 2048 x 8192 109 / 119, 300 x 4096 x 8192 107 / 118, 640 x 2048 x
+    # 4096 64 / 63, with hidden of 1024 the two halves of a tile wait for each other's epilogue (2048 x 1024 x 2816 76.5 / 73.4);
+    # single products of rows x N x K, all in tiles of 128 columns, 200 x 8192 x 2048 25 / 24, 640 x 4096 x 2048 35 / 33, 2000 x 1024 x 4096 37 / 34
+    # (a K of 8192 at 200 or 300 rows gains 3 % and is not told apart), 1000 x 4096 x 4096 with a bias 73 / 68. Every graph keeps the older
+    # rule too, where tiles of 256 x 256 outputs cover every pair (4000 x 4096 x 4096 104 / 116); few-row nodes keep it on one-CTA tiles.
     cta_pair = mode == "static" and workers >= 4 and bool(gemm_nodes) and not any(_few_rows(n) for n in gemm_nodes)
     if cta_pair:
         long = all(_flat2d(n.inputs[0]).shape[0] > BM and _flat2d(n.inputs[0]).shape[1] >= 1536 for n in gemm_nodes)
