@@ -12,8 +12,10 @@
 // over the workers, all (feature tile, 128-wide k-step) pairs in one line, cut into one equal piece per worker. A part is a
 // task that adds its fp32 sums into a [tokens, features] workspace. The accumulator has one feature per TMEM lane, so a
 // warp's reduction instruction covers 128 consecutive bytes of one token's row. Whoever arrives last at a tile's counter finds
-// every part summed and finishes the tile (operator, 16-bit store) through shared memory in short loops, signals the tile's
-// event and clears the tile's workspace for the next launch. A tile that is one part skips all that (few_direct).
+// every part summed and finishes the tile (operator, 16-bit store, workspace zeroed for the next launch) through shared
+// memory in short loops; only that task signals the tile's event. (Zeroing in a pass of its own behind the signal cost 1 to 2 % where
+// a worker has a second part, and gained nothing in a decode layer: 158.5 / 157.9 us at batch 64, 71.3 / 70.6 at batch 3.) A tile that
+// is one part skips all that (few_direct).
 // One B200, decode layer of batch 64: 190 -> 162 us with one part per worker instead of the line alone, 159 with few_direct.
 #pragma once
 #include "gemm_tcgen05.cuh"
@@ -146,9 +148,13 @@ MACO_DEVICE void few_finish_rows(const MacoEltArgs& fa, int m0, int tid, uint8_t
       const uint32_t u = base + k * 128u + (uint32_t)tid;
       if (u >= units) break;
       const uint32_t t = u >> 4, col = (u & 15u) * 8u, s = s0 + k * V * 2048u;
+      float4* src = reinterpret_cast<float4*>(ws + (size_t)t * fa.ld_in + col);
+      const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+      src[0] = zero; src[1] = zero;
       const float4 a = few_lds_f4(s), b = few_lds_f4(s + 2048u);
       float v[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
       if (mode == 1) {
+        src[32] = zero; src[33] = zero;
         const float4 c = few_lds_f4(s + 4096u), d = few_lds_f4(s + 6144u);
         const float up[8] = {c.x, c.y, c.z, c.w, d.x, d.y, d.z, d.w};
 #pragma unroll
@@ -201,6 +207,7 @@ MACO_DEVICE void few_finish_qkrope(const MacoEltArgs& fa, int m0, int tid, uint8
     __syncwarp();
 #pragma unroll 1
     for (int j = 0; j < n; ++j) {
+      reinterpret_cast<float4*>(ws + (size_t)(t0 + j) * fa.ld_in)[lane] = make_float4(0.f, 0.f, 0.f, 0.f);
       const float2* x = reinterpret_cast<const float2*>(mine + j * 768);
       const uint32_t* c = reinterpret_cast<const uint32_t*>(mine + j * 768 + 512);
       // the projection's result in the layer's 16-bit type first (what a separate pass would have read)
@@ -219,16 +226,6 @@ MACO_DEVICE void few_finish_qkrope(const MacoEltArgs& fa, int m0, int tid, uint8
     }
     __syncwarp();
   }
-}
-
-// The workspace for the next launch, behind the tile's signal: nothing in this launch reads it again, and in front of the signal
-// its stores (64 KB for a gate / up pair of 64 tokens) were part of what the next phase waits for.
-MACO_DEVICE void few_clear(const MacoEltArgs& fa, int m0, int tid) {
-  const int tiles = fa.i0 == 1 ? 2 : 1, n0 = fa.i0 == 1 ? (m0 & ~255) : m0;
-  float4* ws = reinterpret_cast<float4*>(const_cast<float*>(reinterpret_cast<const float*>(fa.in0)) + n0);
-  const uint32_t vpr = 32u * tiles, total = (uint32_t)fa.rows * vpr;
-#pragma unroll 1
-  for (uint32_t i = tid; i < total; i += 128) ws[(size_t)(i / vpr) * (fa.ld_in / 4) + i % vpr] = make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
 // A tile that is one part goes from the accumulator to the result through shared memory, 32 tokens at a time. Gate and up features of
@@ -293,14 +290,12 @@ __device__ __noinline__ bool few_direct(const GemmCtrl& c, uint32_t tmem_base, c
 }
 
 // ---- general warps ----------------------------------------------------------------------------
-// Returns 0 on failure, 1 when all is done (the part that finishes its tile signals by itself: `signal`, one thread), 2 when the
-// caller signals.
+// Returns 0 on failure, 1 when other parts of the tile are still to come, 2 when this task finished the tile.
 // `word`: a shared control word; `bar`: the barrier of the 128 threads.
 // (out of line: inlined into the task loop it takes registers from the GEMM epilogue beside it)
-template <int ACC_COLS, typename BarFn, typename SignalFn>
+template <int ACC_COLS, typename BarFn>
 __device__ __noinline__ int few_epilogue(const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e, const MacoGemmArgs& g, int tid,
-                                         uint32_t tile_seq, uint64_t budget_ns, uint8_t* scratch, volatile uint32_t* word, BarFn bar,
-                                         SignalFn signal) {
+                                         uint32_t tile_seq, uint64_t budget_ns, uint8_t* scratch, volatile uint32_t* word, BarFn bar) {
   float* ws = reinterpret_cast<float*>(e.out);
   const long long ld = e.ld_out;
   const int M = e.N;                                 // tokens
@@ -342,10 +337,7 @@ __device__ __noinline__ int few_epilogue(const GemmCtrl& c, uint32_t tmem_base, 
   const MacoEltArgs fa = *fin;
   if (fa.i0 == 3) few_finish_qkrope(fa, g.m0, tid, scratch);
   else few_finish_rows(fa, g.m0, tid, scratch);
-  bar();
-  if (tid == 0) signal();
-  few_clear(fa, g.m0, tid);
-  return 1;
+  return 2;
 }
 
 }  // namespace maco

@@ -637,7 +637,7 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
       // counted tile without rows: nothing to compute (it still signals below)
     } else if (CG == 1 && is_gemm_type(d.type) && (d.u.gemm.b_mn & kFewFlag)) {
       const int r = few_epilogue<kMkBN>(c, tmem_base, p.epis[d.u.gemm.epi], d.u.gemm, tid, seq, p.budget_ns, scratch_smem, cur + 3,
-                                        [] { general_bar(); }, [&p, &d] { signal_done(p, d); });
+                                        [] { general_bar(); });
       if (r == 0) cur[2] = 1;
       signals = r == 2;                                // (the tile's event counts finished tiles, not parts)
       ++seq;
