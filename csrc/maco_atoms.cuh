@@ -453,8 +453,17 @@ MACO_DEVICE float gelu_tanh_grad_f32(float x) {
 static __device__ __noinline__ float gelu_tanh_f32_call(float x) { return gelu_tanh_f32(x); }
 static __device__ __noinline__ float gelu_tanh_grad_f32_call(float x) { return gelu_tanh_grad_f32(x); }
 MACO_DEVICE float silu(float x) { return x / (1.f + __expf(-x)); }
-// For results that are rounded to 16 bits: 2 ulp of fp32 instead of a division whose inlined form is most of an unrolled epilogue's
-// code (an SM that runs it for the first time in a launch fetches that code from L2).
-MACO_DEVICE float silu_16(float x) { return __fdividef(x, 1.f + __expf(-x)); }
+// The same quotient for unrolled epilogues, whose code would mostly be inlined divisions (an SM that runs them for the first time in a
+// launch fetches that code from L2): the product with the approximate reciprocal, corrected once by its residual (Markstein, 1990).
+// Both operands are quartered, so that the reciprocal stays normal up to the largest finite 1 + exp(-x). Over -130..130 these are the
+// bits of silu(); the product alone has an rms error of 1.40e-7 instead of 1.37e-7 and was 0 below -87.3. One B200, us, product alone /
+// corrected / division or a longer guard: SwiGLU block of 1003 rows 105.9 / 106.9 / 115, expert layer of 256 tokens 103 / 106 / 111.
+MACO_DEVICE float silu_16(float x) {
+  const float y4 = fmaf(__expf(-x), 0.25f, 0.25f), x4 = 0.25f * x;
+  float r;                                             // 4 / (1 + exp(-x))
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y4));
+  const float q = x4 * r, e = fmaf(-q, y4, x4);
+  return fabsf(e) > 0.f ? fmaf(e, r, q) : q;           // (no residual: the quotient is exact, or x or exp(-x) is infinite)
+}
 
 }  // namespace maco
