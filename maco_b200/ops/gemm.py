@@ -80,15 +80,18 @@ def gemm(
         out = torch.empty((M, n_out), device=a.device, dtype=od)
     if out.dim() != 2 or out.shape[0] != M or out.shape[1] != n_out or out.stride(1) != 1:
         raise ValueError(f"out must be a row-major [{M}, {n_out}] tensor, got {tuple(out.shape)}")
+    half = (torch.bfloat16, torch.float16)
+    if mode == EPI_GELU_DUAL and (aux is None or tuple(aux.shape) != (M, Nn) or aux.stride(1) != 1 or aux.dtype not in half or aux.device != a.device
+                                  or out.dtype not in half):
+        raise ValueError(f"the gelu_dual epilogue needs 16-bit outputs and aux, a row-major [{M}, {Nn}] tensor on the operands' device")
     if M == 0 or Nn == 0:
         return out
     if K == 0:
         if mode != EPI_F32_ACC:
             out.zero_()
+        if mode == EPI_GELU_DUAL:
+            aux.zero_()
         return out
-    if mode == EPI_GELU_DUAL and (aux is None or tuple(aux.shape) != (M, Nn) or aux.stride(1) != 1 or aux.dtype not in (torch.bfloat16, torch.float16)
-                                  or out.dtype not in (torch.bfloat16, torch.float16)):
-        raise ValueError(f"the gelu_dual epilogue needs 16-bit outputs and aux, a row-major [{M}, {Nn}] tensor")
     lib = N.lib()
     st = N.current_stream_ptr(stream)
     bias_t = N.DTYPE_CODE[bias.dtype] if bias is not None else 0
