@@ -33,15 +33,15 @@ class DPMLPStackBackward:
     def __init__(self, layers: int = 16, hidden: int = 4096, tokens: int = 8192, *, rank: int = 0, world: int = 1,
                  heap=None, device: Optional[torch.device] = None, dtype: torch.dtype = torch.bfloat16, seed: int = 0,
                  mode: str = "static", trace: bool = False, comm_workers: Optional[int] = None, weight_std: float = 0.02,
-                 cta_pair: bool = False):
-        # ``cta_pair``: two-CTA tiles whatever the size. Without it they are taken on one GPU where both GEMM kinds have about one
-        # 256 x 256 tile per worker or more (two per pair: below that the last wave costs more than the smaller operand traffic
-        # gains). Backward pass, one- / two-CTA, one B200: 4 layers of 4096 x 8192 tokens 1650 / 1535 us, 2 of 3072 x 6144 342 / 319,
+                 cta_pair: Optional[bool] = None):
+        # ``cta_pair``: two-CTA tiles (True) or one-CTA ones (False) whatever the size. None: two-CTA tiles on one GPU where both GEMM kinds
+        # have about one 256 x 256 tile per worker or more (two per pair: below that the last wave costs more than the smaller operand
+        # traffic gains). Backward pass, one- / two-CTA, one B200: 4 layers of 4096 x 8192 tokens 1650 / 1535 us, 2 of 3072 x 6144 342 / 319,
         # 4 of 2304 x 2304 271 / 297, 3 of 1024 x 8192 197 / 213. (More ranks: not measured, one-CTA.)
-        if not cta_pair and world == 1 and mode == "static":
+        if cta_pair is None:
             sms = torch.cuda.get_device_properties(device if device is not None else torch.cuda.current_device()).multi_processor_count \
                 if torch.cuda.is_available() and (device is None or torch.device(device).type == "cuda") else 148
-            cta_pair = 20 * min((hidden // 256) ** 2, (tokens // 256) * (hidden // 256)) >= 19 * sms
+            cta_pair = world == 1 and 20 * min((hidden // 256) ** 2, (tokens // 256) * (hidden // 256)) >= 19 * sms
         self.cta_pair = cta_pair and mode == "static"
         if tokens % BM or hidden % 256:
             raise ValueError("tokens must be a multiple of 128 and hidden of 256")
