@@ -144,11 +144,19 @@ MACO_DEVICE bool moe_topk_dispatch(const Program& p, const MacoEltArgs& ar, int 
   return ok;
 }
 
-// End of a launch, when every rank has returned its rows: counters for the next one.
+// End of a launch, when every rank has returned its rows: counters for the next one. in0: what this one counted per expert, for the
+// host; in1 (one rank, or null): the same as received counts.
 MACO_DEVICE void moe_reset_counts(const MacoEltArgs& a, int tid) {
   const MacoMoeParams m = *reinterpret_cast<const MacoMoeParams*>(a.in2);
   uint32_t* ready = reinterpret_cast<uint32_t*>(a.out);
-  for (int e = tid; e < m.experts; e += 128) m.counts[e] = 0;
+  uint32_t* routed = reinterpret_cast<uint32_t*>(const_cast<void*>(a.in0));
+  uint32_t* received = reinterpret_cast<uint32_t*>(const_cast<void*>(a.in1));
+  for (int e = tid; e < m.experts; e += 128) {
+    const uint32_t n = __ldcg(m.counts + e);           // (other SMs' atomics)
+    routed[e] = n;
+    if (received != nullptr) received[e] = min(n, (uint32_t)m.capacity);
+    m.counts[e] = 0;
+  }
   for (int i = tid; i < a.cols; i += 128) ready[i] = 0;
   if (tid == 0) {
     m.counts[m.experts] = m.counts[m.experts + 1];     // what the host reads: pairs dropped by this launch

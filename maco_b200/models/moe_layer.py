@@ -94,6 +94,8 @@ class MoEEPLayer:
         self.logits = torch.empty(T, -(-experts // 8) * 8, device=dev, dtype=dtype)[:, :experts]
         # per expert the slots handed out in this launch (cleared at its end); the pairs dropped by the last launch; by this one
         self.counts = torch.zeros(experts + 2, device=dev, dtype=torch.int32)
+        # per expert the pairs that this rank routed to it in the last step, those beyond a slab's capacity among them
+        self.routed = torch.zeros(experts, device=dev, dtype=torch.int32)
         self.recv = heap.alloc((EL, W, C, H), dtype)
         self.meta = heap.alloc((EL, W, C, 4), torch.int32)
         self.cnt = heap.alloc((W, EL), torch.int32)
@@ -166,7 +168,9 @@ class MoEEPLayer:
             b.add_task(T_MOE_COMBINE, _pack_elt(0, 0, pp, self.out.data_ptr(), t0, min(per, T - t0), H, dt, 0, 0),
                        waits=[(e_ret, n_ret, True, False)], signals=[e_out])
             n_out += 1
-        b.add_task(T_MOE_COUNTS, _pack_elt(0, 0, pp, N.ptr(self.ready), 0, 0, self.ready.numel() if grouped else 0, dt, 0, 0, i0=1),
+        # (one rank whose experts read the counts where dispatch made them: the received counts are written here)
+        b.add_task(T_MOE_COUNTS, _pack_elt(self.routed.data_ptr(), self.cnt.data_ptr() if W == 1 and grouped else 0, pp, N.ptr(self.ready), 0, 0,
+                                           self.ready.numel() if grouped else 0, dt, 0, 0, i0=1),
                    waits=[(e_ret, n_ret, True, False)], signals=[e_out])
         if W > 1:
             fused.epoch_fence_signal(b, [(e_out, n_out + 1, False, False)])

@@ -46,3 +46,20 @@ def test_any_number_of_experts(experts, top_k, mode):
     logits = x.float() @ layer.w_router.float().t()
     assert ((layer.logits.float() - logits).abs() <= 2.0 ** -8 * logits.abs() * 1.01 + 1e-3).all()
     assert _native.status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("mode,fused_return", [("static", True), ("static", False), ("dynamic", True)])
+def test_routed_and_received_counts_of_a_step(mode, fused_return):
+    """What a step routed to each expert, beyond a slab's capacity too, and what the slabs received, by a recount of the logits."""
+    from maco_b200.models.moe_layer import MoEEPLayer
+    layer = MoEEPLayer(hidden=256, experts=12, top_k=3, inter=128, tokens=1024, capacity_factor=0.5, seed=11, weight_std=0.05, router_std=2.0,
+                       mode=mode, fused_return=fused_return, on_drop="ignore")
+    for seed in (1, 2):
+        layer(torch.randn(1024, 256, generator=torch.Generator("cuda").manual_seed(seed), device="cuda", dtype=torch.bfloat16))
+        idx = torch.sort(layer.logits.float(), dim=-1, descending=True, stable=True)[1][:, :3]
+        load = torch.bincount(idx.flatten(), minlength=12)
+        assert (load > layer.capacity).any()
+        assert torch.equal(layer.routed.long(), load)
+        assert torch.equal(layer.cnt.view(-1).long(), load.clamp(max=layer.capacity))
+        assert layer.dropped() == int((load - layer.capacity).clamp(min=0).sum())
