@@ -545,7 +545,7 @@ __device__ __noinline__ bool run_epilogue(const GemmCtrl& c, uint32_t tmem_base,
 // Every task that is not a GEMM tile, behind one call: values of the task loop that live across a call cost a spill for each of
 // its sites, and they are paid for inside the GEMM epilogue (entry function 920 / 2144 bytes stored / loaded with the six calls
 // in the loop, 636 / 1284 with this one and the few-row epilogue out of line).
-enum : int { kTaskDone = 0, kTaskAborted = 1, kTaskBad = 2 };
+enum : int { kTaskDone = 0, kTaskAborted = 1, kTaskBad = 2, kTaskTimeout = 3 };      // (aborted: whoever gave up has reported it)
 template <int CG>
 __device__ __noinline__ int run_task(const MacoProgram& p, const MacoTaskDesc& d, int tid, uint8_t* scratch_smem, uint8_t* ring_smem,
                                      uint64_t* bulk_bars, uint64_t* attn_bars, volatile uint32_t* slots, volatile uint32_t* abort_word,
@@ -568,7 +568,7 @@ __device__ __noinline__ int run_task(const MacoProgram& p, const MacoTaskDesc& d
   } else if (d.type == MACO_TASK_TOPK) {
     // rows wait in the operand ring where nothing uses it before dispatch has ended, else in the scratch block
     if (!ring_free) { bulk.buf = scratch_smem; bulk.nbuf = 1; bulk.buf_bytes = kMkScratchSmem; }
-    return run_topk(p, d.u.elt, tid, &bulk) ? kTaskDone : kTaskAborted;
+    return run_topk(p, d.u.elt, tid, &bulk) ? kTaskDone : kTaskTimeout;
   } else if (d.type == MACO_TASK_MOE_COUNTS || d.type == MACO_TASK_MOE_RETURN ||
              d.type == MACO_TASK_SPLITK_FIN || d.type == MACO_TASK_MOE_COMBINE) {
     run_moe(p, d.type, d.u.elt, tid, scratch_smem, ring_free ? &bulk : nullptr);
@@ -701,13 +701,16 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
       const int r = run_task<CG>(p, d, tid, scratch_smem, ring_smem, bulk_bars, attn_bars, slots, c.abort_word, ait, cur + 3, ring_free);
       if (CG == 1 && d.type == MACO_TASK_ATTENTION && attn_pipelined(d.u.elt)) ait += attn_stage_uses(d.u.elt);
       if (r != kTaskDone) {
-        cur[2] = 1;
+        cur[2] = r == kTaskTimeout ? 2 : 1;
         if (leader && r == kTaskBad) report_failure(p, MACO_STATUS_BAD_TASK, task, d.type >= 200 && d.type < 300 ? (uint32_t)d.u.comm.op : d.type, c.abort_word);
       }
     }
     if (leader && *c.abort_word != 0) cur[2] = 1;
     general_bar();                              // every thread's stores are issued, failure word final
-    if (cur[2] != 0) break;
+    if (cur[2] != 0) {
+      if (leader && cur[2] == 2) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
+      break;
+    }
     if (leader) {
       // (A consumer that reads this output through TMA orders the two proxies itself, with a proxy fence behind its
       // acquire; one on this side as well was half a microsecond per task.)

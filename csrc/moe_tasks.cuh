@@ -44,6 +44,7 @@ MACO_DEVICE float moe_key_logit(uint32_t key, int dtype) {
 // atomics are in flight while the next token is routed.
 // Routing a token used to take 40 shuffles and its row went through registers into one buffer per warp, free again only when the
 // token's copies had read it: 76 us for 4096 tokens of 2048, top-8 of 64, most of it one warp's chain of 7 x 10 us.
+// False after a wait that ran out, in the threads whose wait it was.
 template <typename Program>
 MACO_DEVICE bool moe_topk_dispatch(const Program& p, const MacoEltArgs& ar, int tid, const BulkCtx* bc) {
   // private copies: descriptor and parameter block live in global memory; read in place every use inside the
@@ -71,7 +72,7 @@ MACO_DEVICE bool moe_topk_dispatch(const Program& p, const MacoEltArgs& ar, int 
       asm volatile("bar.sync 1, 128;" ::: "memory");   // (and the phase word is this batch's)
     }
     const uint32_t parity = *bc->phase & 1u;
-    if (tid == 0) {
+    if (tid == 0 && ok) {
       fence_proxy_async_all();
       mbar_arrive_expect_tx(&bc->bars[0], (uint32_t)n * row_bytes);
       const uint8_t* src = reinterpret_cast<const uint8_t*>(m.x) + (size_t)tok0 * row_bytes;
@@ -129,7 +130,11 @@ MACO_DEVICE bool moe_topk_dispatch(const Program& p, const MacoEltArgs& ar, int 
       if (lane < K) slot = atomicAdd(&m.counts[e], 1u);
       if (p_j < 0) {
         const uint64_t t0 = globaltimer_ns();
-        while (ok && !mbar_try_wait(&bc->bars[0], parity)) ok = globaltimer_ns() - t0 <= p.budget_ns;
+        while (ok && !mbar_try_wait(&bc->bars[0], parity)) {
+          if (globaltimer_ns() - t0 <= p.budget_ns) continue;
+          ok = false;                                  // (warp 0 has sent for the rows and gives them as long again to land)
+          if (warp == 0) while (!mbar_try_wait(&bc->bars[0], parity) && globaltimer_ns() - t0 <= 2 * p.budget_ns) {}
+        }
       } else if (ok) {
         send();
       }
