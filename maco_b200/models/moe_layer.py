@@ -192,9 +192,12 @@ class MoEEPLayer:
                            make_idesc(1 if self.dtype == torch.bfloat16 else 0, BM, 256, 0, 0), *tm, 0)
         self.d_experts = torch.from_numpy(np.frombuffer(blob, dtype=np.uint8).copy()).to(self.device)
         b.keepalive += [self.d_experts, self.ready, self.recv, self.w1, self.act, self.w2]
+        blocks = slabs * -(-self.tokens * self.top_k // (self.experts * BM))         # row blocks under even routing, for planning alone
+        per_share = blocks * ((I // 128) * (2.0 + 0.45 * (H // 64)) + (H // 256) * (2.0 + 0.45 * (I // 64))) / shares
         for w in range(shares):
             b.add_task(T_MOE_EXPERTS, _pack_elt(0, 0, self.d_experts.data_ptr(), 0, 0, 0, 0, 0, 0, 0, i0=w), waits=[arrived], signal_peer=-2,
                        signal_peer_event=e_ret, worker=w)
+            b.tasks[-1]["cost_us"] = per_share
         return W * shares
 
     def _expert_tiles(self, b: ProgramBuilder, arrived, e_ret: int, pp: int) -> int:

@@ -345,8 +345,11 @@ def simulate_static_queues(programs: Sequence[Tuple[Sequence[dict], List[List[in
 def default_task_cost(t: dict) -> float:
     """Rough duration of a task in microseconds for ``estimate_makespan``, from figures measured on B200 with this
     kernel: a 128 x 256 x 64 k-block of a GEMM tile 0.45 us (a pair half the same: two CTAs, twice the rows) plus 2 us
-    per tile; a 128-wide k-step of a few-row part (32 KB of weights) 1 us plus 2 us per part; a bulk push 43 us per MB; a staged reduction 0.06 us per KB of sources; everything else 5 us. Callers
-    with better numbers for their shapes pass their own function."""
+    per tile; a 128-wide k-step of a few-row part (32 KB of weights) 1 us plus 2 us per part; a bulk push 43 us per MB; a staged reduction
+    0.06 us per KB of sources; what the builder knows better (``cost_us``: a worker's share of an expert layer, by its tiles under even
+    routing); everything else 5 us. Callers with better numbers for their shapes pass their own function."""
+    if t.get("cost_us") is not None:
+        return float(t["cost_us"])
     ty = t["type"]
     raw = t["raw"]
     if ty in (100, 101, 102) and len(raw) >= 30:
@@ -371,7 +374,8 @@ def estimate_makespan(programs: Sequence[Tuple[Sequence[dict], List[List[int]]]]
     (microseconds) and ``hop_us`` between a signal and the waiter seeing it. Same rules as ``simulate_static_queues``
     (queue order, both wait conditions, pair halves together, peer signals, few-row tiles signalled by their last part). Returns the predicted length of the launch
     per rank, the busy fraction of the workers and the last finish time per task type: a planning aid for choosing the
-    number of communication workers, chunk sizes and tile orders before a GPU is involved, not a measurement."""
+    number of communication workers, chunk sizes and tile orders before a GPU is involved, not a measurement. (What a share of an expert
+    layer waits for inside, gate / up tiles of other shares, is not modelled, here or in ``simulate_static_queues``.)"""
     import heapq
     world = len(programs)
     counts = [collections.defaultdict(int) for _ in range(world)]

@@ -26,6 +26,23 @@ def test_router_rows_are_whole_vectors(experts):
     assert words[0] == layer.logits.data_ptr() and words[-1] == ld
 
 
+def test_makespan_of_an_expert_layer_follows_its_tiles():
+    """Twice the experts' width is about twice the tiles: the estimate of the launch grows by as much as a share does."""
+    from maco_b200.ops import megakernel as mk
+    spans, shares = [], []
+    for inter in (256, 512):
+        b = _plan(hidden=256, experts=8, top_k=2, inter=inter, tokens=1024, capacity_factor=2.0).builder
+        costs = {mk.default_task_cost(t) for t in b.tasks if t["type"] == mk.T_MOE_EXPERTS}
+        assert len(costs) == 1
+        # 8 slabs of 256 rows: 16 row blocks; inter / 128 gate tiles of 4 k-blocks and one down tile of inter / 64 each
+        want = 16 * (inter // 128 * (2 + 0.45 * 4) + 1 * (2 + 0.45 * (inter // 64))) / b.num_workers
+        assert costs.pop() == pytest.approx(want)
+        shares.append(want)
+        r = mk.estimate_makespan([(b.tasks, mk.assign_static_queues(b.tasks, b.num_workers, b.num_comm_workers))])
+        spans.append(r["span_us"][0])
+    assert spans[1] - spans[0] == pytest.approx(shares[1] - shares[0])
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("mode", ["static", "dynamic"])
 @pytest.mark.parametrize("experts,top_k", [(1, 1), (3, 2), (5, 5), (12, 4), (31, 8)])
