@@ -78,9 +78,13 @@ def test_residual_add_in_the_epilogue_is_the_add(rows, hidden, ffn):
     for _ in range(2):
         g.execute()
     torch.cuda.synchronize()
-    if g.runtime_kind == "persistent":
-        kinds = g._runtime._program.task_types
-        assert (kinds == 113).any()                   # the second add
+    # one add in the product's epilogue and one as tasks of its own: as many as a graph with that add alone has
+    alone = maco.TaskGraph()
+    alone.add(x, torch.empty_like(x))
+    alone.compile()
+    assert g.runtime_kind == alone.runtime_kind == "persistent"
+    kinds = g._runtime._program.task_types
+    assert (kinds == 113).sum() == (alone._runtime._program.task_types == 113).sum() > 0
     h = (x.float() @ w.float().t()).to(dt).float()
     assert (y.output.float() - h @ w2.float().t()).abs().max() < 2e-2 * h.abs().max()
     assert torch.equal(s.output, (y.output.float() + x.float()).to(dt))

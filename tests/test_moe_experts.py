@@ -80,3 +80,37 @@ def test_routed_and_received_counts_of_a_step(mode, fused_return):
         assert torch.equal(layer.routed.long(), load)
         assert torch.equal(layer.cnt.view(-1).long(), load.clamp(max=layer.capacity))
         assert layer.dropped() == int((load - layer.capacity).clamp(min=0).sum())
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+@pytest.mark.parametrize("mode,fused_return", [("static", True), ("static", False), ("dynamic", True)])
+def test_expert_layer_in_both_types_against_its_own_logits(dtype, mode, fused_return):
+    """fp16 and bf16 on all three routes, positive, negative, tied and zero logits among them, against routing and experts in plain torch
+    from the logits that the router wrote: no token may take another expert."""
+    from maco_b200 import _native
+    from maco_b200.models.moe_layer import MoEEPLayer
+    E, K, H, I, T = 16, 4, 256, 128, 256
+    layer = MoEEPLayer(hidden=H, experts=E, top_k=K, inter=I, tokens=T, capacity_factor=4.0, seed=3, mode=mode, dtype=dtype, weight_std=0.05,
+                       router_std=0.3, fused_return=fused_return)
+    layer.w_router[5].copy_(layer.w_router[2])       # equal logits: the lower expert goes first
+    layer.w_router[7].zero_()
+    x = torch.randn(T, H, device="cuda", dtype=dtype)
+    out = layer(x)
+    assert layer.dropped() == 0
+    val, idx = torch.sort(layer.logits.float(), dim=-1, descending=True, stable=True)
+    weight, idx = torch.softmax(val[:, :K].double(), dim=-1), idx[:, :K]
+    rnd = lambda t: t.to(dtype).double()
+    ref = torch.zeros(T, H, device="cuda", dtype=torch.float64)
+    for e in range(E):
+        tok, k = (idx == e).nonzero(as_tuple=True)
+        wg, wu, wd = (w.double() for w in layer.expert_weights(e))
+        xe = x[tok].double()
+        h = rnd(torch.nn.functional.silu(xe @ wg.t()) * (xe @ wu.t()))
+        ref.index_add_(0, tok, rnd(rnd(h @ wd.t()) * weight[tok, k].unsqueeze(1)))
+    # what is rounded, activations, expert outputs, weighted rows and the sum, is rounded alike on both sides but for fp32 sums near a
+    # tie: a few units of the type's half ulp in norm, where another expert would show as a difference of the size of the output
+    half = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    assert (out.double() - ref).norm() <= 2 * half * ref.norm()
+    assert ((out.double() - ref).norm(dim=1) <= 8 * half * ref.norm(dim=1) + half).all()
+    assert _native.status() == 0
