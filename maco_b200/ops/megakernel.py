@@ -133,18 +133,22 @@ def pick_split_k(n_tiles: int, k_blocks: int, workers: int) -> int:
     return min(range(1, max(1, min(16, k_blocks // 2)) + 1), key=cost)
 
 
-def stream_pieces(n_tiles: int, steps: int, workers: int) -> List[Tuple[int, int, int, int]]:
+def stream_pieces(n_tiles: int, steps: int, workers: int, rows: int = 64) -> List[Tuple[int, int, int, int]]:
     """Cuts the ``n_tiles * steps`` (tile, k-step) pairs of a few-row GEMM over the workers. Returns (tile, first step, steps, worker).
     Where the tiles divide well, each is cut into equal parts of at least two steps (64 KB of weights), one per worker. Else all pairs
     lie in one line with one nearly equal piece per worker, split where it crosses a tile; a cut that would leave less than an eighth of a piece on one side of a tile boundary moves to it
     (a part costs about a microsecond of reductions and arrival whatever its length)."""
     total = n_tiles * steps
     parts = min(workers // n_tiles, max(1, steps // 2)) if n_tiles else 0
-    if 5 * parts * n_tiles >= 3 * workers or 0 < parts == steps // 2:
+    few = rows <= 8 and parts > 0 and steps // parts - total // workers > 7
+    if (5 * parts * n_tiles >= 3 * workers and not few) or 0 < parts == steps // 2:
         # One part per worker. A second one on a worker costs its own reductions and arrival, 4 us, and stands behind the finishing
         # pass of the first, 3-7 us, so that the tiles of a phase completed one after the other; and 90 SMs with a full ring each keep
         # enough of the stream in flight. (64 tokens: a QKV projection of 20 tiles ended 20 us after its last MMA, an output
-        # projection of 40 tiles 16 us.)
+        # projection of 40 tiles 16 us.) Line / equal parts, one B200, us, weights from memory, 8 k-steps: 90 tiles, 64 rows 34 / 24, 1 row
+        # 25 / 21; 32 k-steps: 90 tiles, 64 rows 41 / 36, 16 rows 35.6 / 33.9. With few rows that pass is short, and parts of many steps on fewer
+        # workers take as long or longer: 100 tiles of 32 steps, 1 row, 35 / 36 from memory, 27 / 31 where the weights lie in L2.
+        # (Below 60 % of the workers the line stays: 76 tiles of 32 steps, 1 row, 24 / 27; of 8 steps, 20 / 17, not told apart.)
         return [(t, i * steps // parts, (i + 1) * steps // parts - i * steps // parts, t * parts + i) for t in range(n_tiles) for i in range(parts)]
     workers = max(1, min(workers, total // 2))
     slack = total // workers // 8
@@ -836,7 +840,7 @@ class ProgramBuilder:
         if whole_tiles:
             pieces = [(t, 0, steps, t % self.num_workers) for t in range(n_tiles)]
         else:
-            pieces = stream_pieces(n_tiles, steps, self.num_workers)
+            pieces = stream_pieces(n_tiles, steps, self.num_workers, M)
         # A tile that is one part is finished from its accumulator (few_direct in csrc/fewrow_gemm.cuh); of a gate / up pair such a tile
         # holds 64 features of each, so that no two workers have to meet.
         direct = mode != 3 and all(n == steps for _, _, n, _ in pieces)

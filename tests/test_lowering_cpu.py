@@ -37,3 +37,13 @@ def test_mlp_blocks_take_two_cta_tiles_where_their_products_are_long(rows, hidde
     y = g.linear(_bf(rows, hidden), _bf(2 * ffn, hidden), activation="swiglu")
     g.linear(y.output, _bf(hidden, ffn))
     assert _lower(g, monkeypatch).cta_pair == pair
+
+
+@pytest.mark.parametrize("n_tiles,steps,rows,parts", [(100, 32, 1, False), (100, 32, 8, False), (100, 32, 16, True), (100, 32, 64, True), (100, 8, 1, True),
+                                                      (96, 16, 3, True), (24, 16, 1, True), (124, 32, 1, True), (76, 32, 64, False)])
+def test_few_rows_keep_long_parts_in_one_line(n_tiles, steps, rows, parts):
+    """Whole tiles or equal parts of them, against one line that every worker has a piece of."""
+    pieces = mk.stream_pieces(n_tiles, steps, 148, rows)
+    per_tile = {t: sum(1 for p in pieces if p[0] == t) for t in range(n_tiles)}
+    assert (len(set(per_tile.values())) == 1 and len({w for *_, w in pieces}) == len(pieces)) == parts
+    assert sorted((t, s) for t, s0, n, _ in pieces for s in range(s0, s0 + n)) == [(t, s) for t in range(n_tiles) for s in range(steps)]
