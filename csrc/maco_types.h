@@ -289,17 +289,16 @@ struct MacoMoeParams {
   int32_t hidden, experts, top_k, experts_per_rank, capacity, tokens, dtype, ld_logits;
 };
 
-/* The expert GEMMs of one layer (MACO_TASK_MOE_EXPERTS, csrc/moe_experts.cuh): slab (expert, source rank) holds `capacity` rows. */
+/* The expert GEMMs of one layer on one rank (MACO_TASK_MOE_EXPERTS, csrc/moe_experts.cuh): an expert's slab holds `capacity` rows. */
 struct MacoExpertArgs {
-  const uint32_t* counts;         /* [world][experts] rows received per slab */
-  uint32_t* ready;                /* [experts][world][capacity / 128] epilogue warps that have finished a gate / up tile; zero at launch start */
-  const void* meta;               /* [experts][world][capacity] {token, k, weight, -} */
-  void* act;                      /* [experts][world][capacity][inter] */
-  unsigned long long comb_off;    /* heap offset of the combine buffer */
-  int32_t experts, world, capacity, hidden, inter, top_k, shares, dtype;   /* local experts; workers that share the tiles */
+  const uint32_t* counts;         /* [experts] pairs routed to the expert */
+  uint32_t* ready;                /* [experts][capacity / 128] epilogue warps that have finished a gate / up tile; zero at launch start */
+  const void* meta;               /* [experts][capacity] {token, k, weight, -} */
+  void* act;                      /* [experts][capacity][inter] */
+  void* comb;                     /* [tokens][top_k][hidden] combine buffer */
+  int32_t experts, capacity, hidden, inter, top_k, shares, dtype;          /* shares: workers that share the tiles */
   uint32_t idesc;
   uint16_t tmap_x, tmap_w1, tmap_act, tmap_w2;
-  int32_t _pad;
 };
 
 /* ---- device trace ring ----------------------------------------------------------------------- */

@@ -1,7 +1,7 @@
-// The expert GEMMs of a mixture-of-experts layer as one task per worker.
+// The expert GEMMs of a mixture-of-experts layer on one rank as one task per worker.
 //
 // How many 128-row tiles an expert has is known only when dispatch has ended. With a task per tile of every slab's capacity
-// (MACO_TF_COUNTED, still the form of the dynamic scheduler and of separate return tasks) half of 7,168 tasks were empty at 2-5 us each on three
+// (MACO_TF_COUNTED, still the form of several ranks, of the dynamic scheduler and of separate return tasks) half of 7,168 tasks were empty at 2-5 us each on three
 // roles, and a tile of the down projection, 12 k-blocks or 4.5 us of MMA, took 15-20 us of waits, count reads, fences and
 // signals. Here every role of a worker walks over the tiles that exist: tile t of the line
 //   [gate / up tiles of slab 0, slab 1, ...][down tiles of slab 0, slab 1, ...]
@@ -9,23 +9,21 @@
 // row blocks of one 256-column weight tile, so a weight tile is read by its workers at the same time. A down tile waits
 // for the gate / up tiles of its row block (a counter per block, bumped by each of the four epilogue warps); these lie in front of
 // every down tile in each worker's share, so the workers cannot wait for one another in a circle. Rows leave, scaled by their routing
-// weight, for their source rank's combine buffer; one signal per worker says that all of its rows have.
+// weight, for the combine buffer; one signal per worker says that all of its rows have.
 #pragma once
 #include "gemm_tcgen05.cuh"
 #include "moe_tasks.cuh"
 
 namespace maco {
 
-constexpr int kMaxSlabs = 256;                // local experts x ranks = experts of the layer
+constexpr int kMaxSlabs = 256;                // experts of the layer, a slab each
 
 // Row blocks per slab, in shared memory: counts read from global memory again for every tile were an L2 round trip per slab passed
 // (each acquire of the SM empties its L1), 2-5 us between two tiles. `first`, `step`: the threads that fill the table.
 MACO_DEVICE void expert_blocks(uint16_t* table, const MacoExpertArgs& a, int first, int step) {
 #pragma unroll 4
-  for (int i = first; i < a.experts * a.world; i += step) {
-    const int el = a.world == 1 ? i : i / a.world, src = i - el * a.world;
-    table[i] = (uint16_t)((min((int)__ldcg(a.counts + src * a.experts + el), a.capacity) + kBM - 1) / kBM);   // (final: dispatch has ended everywhere)
-  }
+  for (int i = first; i < a.experts; i += step)
+    table[i] = (uint16_t)((min((int)__ldcg(a.counts + i), a.capacity) + kBM - 1) / kBM);      // (final: dispatch has ended)
 }
 
 struct ExpertTiles {
@@ -35,7 +33,7 @@ struct ExpertTiles {
   int phase, slab, mb, nb;                    // the current tile: projection, slab, row block, column tile
 
   MACO_DEVICE ExpertTiles(const MacoExpertArgs& a, const uint16_t* table, int share)
-      : blocks(table), slabs(a.experts * a.world), tiles{a.inter / 128, a.hidden / 256}, t(share), step(a.shares), base(0), phase(0), slab(0),
+      : blocks(table), slabs(a.experts), tiles{a.inter / 128, a.hidden / 256}, t(share), step(a.shares), base(0), phase(0), slab(0),
         mb(0), nb(0) {}
 
   MACO_DEVICE bool next() {
@@ -66,7 +64,7 @@ __device__ __noinline__ bool experts_produce(const Program& p, const MacoExpertA
   ExpertTiles tiles(a, table, share);
   const uint32_t gate_done = 4u * (uint32_t)tiles.tiles[0];
   while (tiles.next()) {
-    const int m0 = tiles.slab * a.capacity + tiles.mb * kBM, el = a.world == 1 ? tiles.slab : tiles.slab / a.world;
+    const int m0 = tiles.slab * a.capacity + tiles.mb * kBM, el = tiles.slab;
     bool ok;
     if (tiles.phase == 0) {
       ok = gemm_produce_tile<256, STAGES, false, false>(smem, c, tmaps + a.tmap_x, tmaps + a.tmap_w1, m0, (el * tiles.tiles[0] + tiles.nb) * 256, 0,
@@ -120,14 +118,14 @@ __device__ __noinline__ int experts_epilogue(const Program& p, const MacoExpertA
   while (tiles.next()) {
     const uint32_t acc = seq & 1;
     const bool down = tiles.phase != 0;
-    const int row = tiles.mb * kBM + (int)(q * 32 + lane), el = a.world == 1 ? tiles.slab : tiles.slab / a.world, src = tiles.slab - el * a.world;
+    const int row = tiles.mb * kBM + (int)(q * 32 + lane);
     const long long cell = (long long)tiles.slab * a.capacity + row;
     // both loads are back before the accumulator is complete
-    const int rows = min((int)__ldcg(a.counts + src * a.experts + el), a.capacity);
+    const int rows = min((int)__ldcg(a.counts + tiles.slab), a.capacity);
     int4 rec = make_int4(0, 0, 0, 0);
     if (down) rec = reinterpret_cast<const int4*>(a.meta)[cell];        // (rows beyond the count hold old records, and are not written)
     const bool row_ok = row < rows;
-    uint8_t* dst = down ? p.peer_heap[src] + a.comb_off + (((long long)rec.x * a.top_k + rec.y) * a.hidden + tiles.nb * 256) * 2
+    uint8_t* dst = down ? reinterpret_cast<uint8_t*>(a.comb) + (((long long)rec.x * a.top_k + rec.y) * a.hidden + tiles.nb * 256) * 2
                         : reinterpret_cast<uint8_t*>(a.act) + (cell * a.inter + tiles.nb * 128) * 2;
     const float weight = __int_as_float(rec.z);
     uint32_t ok = 1;

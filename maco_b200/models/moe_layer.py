@@ -9,11 +9,12 @@ Per rank, inside the persistent kernel:
    fused with the router permute), with a {token, k, weight} record beside it
 3. the per-expert counts are published to the expert owners
    (one rank: the experts read them where dispatch counted)
-4. grouped expert GEMMs over the slabs: gate/up with SwiGLU in the epilogue, then down; every worker takes its share of
-   the tiles that the received counts leave (csrc/moe_experts.cuh)
+4. grouped expert GEMMs over the slabs: gate/up with SwiGLU in the epilogue, then down. One rank: every worker takes its
+   share of the tiles that the received counts leave (csrc/moe_experts.cuh); else a task per tile of every slab, skipped at
+   run time where no tokens are
 5. the down projection's epilogue scales every valid output row by its routing weight and sends it back into the
    source rank's combine buffer at [token, k] (combine all-to-all fused into the GEMM; ``fused_return=False``: separate
-   MOE_RETURN tasks do it from a slab of outputs, and a task per tile of every slab, skipped at run time where no tokens are)
+   MOE_RETURN tasks do it from a slab of outputs)
 6. the source sums the k rows of every token.
 
 Receive slabs have a fixed capacity per (source rank, expert); routed pairs that do not fit are
@@ -147,10 +148,12 @@ class MoEEPLayer:
             b.add_task(T_TOPK, _pack_elt(0, 0, pp, 0, t0, nt, H, dt, 0, 0), waits=[(ev, cnt, False, False)] + ([fence] if W > 1 else []),
                        signals=[e_disp_local], ring_free=static)
             n_disp += 1
-        grouped = self.fused_return and static
+        # Expert shares store their rows from registers, 16 bytes a thread. To another GPU that reaches a fraction of what the bulk engine
+        # does, which the tiles of the other form go through: more than one rank keeps a task per tile.
+        grouped = self.fused_return and static and W == 1
         # 3. counts to the expert owners; every rank learns that every rank has dispatched
         arrived = (e_disp_local, n_disp, False, False)
-        if W > 1 or not grouped:
+        if not grouped:
             e_disp = b.new_event()
             b.add_task(T_MOE_COUNTS, _pack_elt(0, 0, pp, 0, 0, 0, 0, dt, 0, 0), waits=[arrived], signal_peer=-2, signal_peer_event=e_disp)
             arrived = (e_disp, W, True, False)
@@ -168,8 +171,8 @@ class MoEEPLayer:
             b.add_task(T_MOE_COMBINE, _pack_elt(0, 0, pp, self.out.data_ptr(), t0, min(per, T - t0), H, dt, 0, 0),
                        waits=[(e_ret, n_ret, True, False)], signals=[e_out])
             n_out += 1
-        # (one rank whose experts read the counts where dispatch made them: the received counts are written here)
-        b.add_task(T_MOE_COUNTS, _pack_elt(self.routed.data_ptr(), self.cnt.data_ptr() if W == 1 and grouped else 0, pp, N.ptr(self.ready), 0, 0,
+        # (expert shares read the counts where dispatch made them: the received counts are written here)
+        b.add_task(T_MOE_COUNTS, _pack_elt(self.routed.data_ptr(), self.cnt.data_ptr() if grouped else 0, pp, N.ptr(self.ready), 0, 0,
                                            self.ready.numel() if grouped else 0, dt, 0, 0, i0=1),
                    waits=[(e_ret, n_ret, True, False)], signals=[e_out])
         if W > 1:
@@ -179,30 +182,29 @@ class MoEEPLayer:
         self.program = b.build() if self.device.type == "cuda" else None
 
     def _expert_shares(self, b: ProgramBuilder, arrived, e_ret: int) -> int:
-        """The expert GEMMs and the weighted return as one task per worker. Returns the signals of ``e_ret`` on every rank."""
-        EL, W, C, H, I = self.el, self.world, self.capacity, self.hidden, self.inter
-        slabs, shares = EL * W, b.num_workers
-        self.ready = torch.zeros(slabs * (C // BM), device=self.device, dtype=torch.int32)
+        """One rank: the expert GEMMs and the weighted return as one task per worker. Returns the signals of ``e_ret``."""
+        E, C, H, I = self.experts, self.capacity, self.hidden, self.inter
+        shares = b.num_workers
+        self.ready = torch.zeros(E * (C // BM), device=self.device, dtype=torch.int32)
         b.launch_state.append(self.ready)
         tm = [b._tmap(t.view(-1, cols), rows, cols, cols, False, box) for t, rows, cols, box in
-              ((self.recv, slabs * C, H, BM), (self.w1, EL * 2 * I, H, 256), (self.act, slabs * C, I, BM), (self.w2, EL * H, I, 256))]
-        counts = self.cnt if W > 1 else self.counts
-        blob = struct.pack("<QQQQQiiiiiiiiIHHHHi", counts.data_ptr(), self.ready.data_ptr(), self.meta.data_ptr(), self.act.data_ptr(),
-                           self.heap.offset_of(self.comb), EL, W, C, H, I, self.top_k, shares, N.DTYPE_CODE[self.dtype],
-                           make_idesc(1 if self.dtype == torch.bfloat16 else 0, BM, 256, 0, 0), *tm, 0)
+              ((self.recv, E * C, H, BM), (self.w1, E * 2 * I, H, 256), (self.act, E * C, I, BM), (self.w2, E * H, I, 256))]
+        blob = struct.pack("<QQQQQiiiiiiiIHHHH", self.counts.data_ptr(), self.ready.data_ptr(), self.meta.data_ptr(), self.act.data_ptr(),
+                           self.comb.data_ptr(), E, C, H, I, self.top_k, shares, N.DTYPE_CODE[self.dtype],
+                           make_idesc(1 if self.dtype == torch.bfloat16 else 0, BM, 256, 0, 0), *tm)
         self.d_experts = torch.from_numpy(np.frombuffer(blob, dtype=np.uint8).copy()).to(self.device)
         b.keepalive += [self.d_experts, self.ready, self.recv, self.w1, self.act, self.w2]
-        blocks = slabs * -(-self.tokens * self.top_k // (self.experts * BM))         # row blocks under even routing, for planning alone
+        blocks = E * -(-self.tokens * self.top_k // (E * BM))         # row blocks under even routing, for planning alone
         per_share = blocks * ((I // 128) * (2.0 + 0.45 * (H // 64)) + (H // 256) * (2.0 + 0.45 * (I // 64))) / shares
         for w in range(shares):
             b.add_task(T_MOE_EXPERTS, _pack_elt(0, 0, self.d_experts.data_ptr(), 0, 0, 0, 0, 0, 0, 0, i0=w), waits=[arrived], signal_peer=-2,
                        signal_peer_event=e_ret, worker=w)
             b.tasks[-1]["cost_us"] = per_share
-        return W * shares
+        return shares
 
     def _expert_tiles(self, b: ProgramBuilder, arrived, e_ret: int, pp: int) -> int:
-        """A task per tile of every slab, skipped at run time where the slab holds no rows (dynamic scheduler, or a slab of outputs
-        with separate return tasks)."""
+        """A task per tile of every slab, skipped at run time where the slab holds no rows (more than one rank, the dynamic scheduler, or a
+        slab of outputs with separate return tasks)."""
         EL, W, C, H, K = self.el, self.world, self.capacity, self.hidden, self.top_k
         dt = N.DTYPE_CODE[self.dtype]
         cnt_base = self.cnt.data_ptr()

@@ -26,6 +26,22 @@ def test_router_rows_are_whole_vectors(experts):
     assert words[0] == layer.logits.data_ptr() and words[-1] == ld
 
 
+@pytest.mark.parametrize("world", [1, 2])
+def test_rows_for_other_ranks_leave_through_the_bulk_engine(world):
+    """Expert shares store their rows from registers, which is for this GPU's memory alone: with more ranks the down projection is tiles
+    with a destination rank, whose epilogue stages its rows, and each of them signals that rank."""
+    from maco_b200.models.moe_layer import MoEEPLayer
+    from maco_b200.ops import megakernel as mk
+    from maco_b200.parallel.symm_heap import PlanningHeap
+    layer = MoEEPLayer(hidden=256, experts=8, top_k=2, inter=128, tokens=256, rank=0, world=world, heap=PlanningHeap(0, world, 1 << 26),
+                       device=torch.device("cpu"), capacity_factor=4.0)
+    shares = [t for t in layer.builder.tasks if t["type"] == mk.T_MOE_EXPERTS]
+    assert (len(shares) > 0) == (world == 1)
+    if world > 1:
+        to = {t["signal_peer"] for t in layer.builder.tasks if t["type"] in (100, 101, 102) and t["signal_peer_event"] >= 0}
+        assert to == set(range(world))
+
+
 def test_makespan_of_an_expert_layer_follows_its_tiles():
     """Twice the experts' width is about twice the tiles: the estimate of the launch grows by as much as a share does."""
     from maco_b200.ops import megakernel as mk
