@@ -173,7 +173,7 @@ int launch_gemm_f32(const F32Operand& A, const F32Operand& B, const GemmEpilogue
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim = {(unsigned)split, 1, 1};
-  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // set up while the launch in front of it ends
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;      // begins when the blocks in front of it have ended
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = chained ? 2 : 1;
@@ -216,8 +216,9 @@ struct MacoF32Gemm {
   int M, N, K, mode, bias_type, out_type;
 };
 
-// The fp32 GEMMs of a graph in order on one stream, each behind the one in front of it: one call for the host, and the set-up of a
-// launch under the end of the previous one. (Two layers of 32 rows through one Python call each: 41 us, 17 us of host time a launch.)
+// The fp32 GEMMs of a graph in order on one stream, each behind the one in front of it: one call for the host, and launches that follow
+// each other as soon as the previous one's blocks have ended (no kernel here starts its successor earlier). Two layers of 32 rows: 41 us
+// through one Python call each, of which 17 us a launch on the host; 14 us now.
 int maco_gemm_f32_chain(const MacoF32Gemm* g, int n, void* stream_) {
   cudaStream_t stream = reinterpret_cast<cudaStream_t>(stream_);
   for (int i = 0; i < n; ++i) {
