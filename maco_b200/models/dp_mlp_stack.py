@@ -78,8 +78,8 @@ class DPMLPStackBackward:
     def forward(self) -> torch.Tensor:
         cur = self.x
         for l in range(self.layers):
-            # two launches: the product with the GELU in its epilogue (gelu_dual) is slower at every size, 3 layers, one B200, us: 1024 x 8192
-            # tokens 132 / 100, 2048 x 4096 156 / 132, 3072 x 8192 430 / 428, 4096 x 8192 701 / 665
+            # two launches: the product with the GELU in its epilogue (gelu_dual) gains 1 % at 2816 x 8192 tokens and loses elsewhere. It / these,
+            # 3 layers, one B200, us: 1024 x 8192 tokens 132 / 100, 2048 x 4096 156 / 132, 3072 x 8192 430 / 428, 4096 x 8192 701 / 665
             ops.gemm(cur, self.weights[l], out=self.z[l])
             ops.gelu(self.z[l], out=self.a[l])
             cur = self.a[l]
