@@ -91,19 +91,17 @@ attn_stream_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   constexpr uint64_t kBudgetNs = 2000000000ull;
   const long long begin = share_begin(p, blockIdx.x, gridDim.x), end = share_begin(p, blockIdx.x + 1, gridDim.x);
   uint32_t ait = 0;
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
   bool ok = true;
   for (long long pos = begin; pos < end && ok;) {
     const int group = (int)(pos / p.chunks_per_head), c0 = (int)(pos - (long long)group * p.chunks_per_head);
     const int n = (int)min((long long)(p.chunks_per_head - c0), end - pos);
     const int key0 = c0 * 128, rows = min(p.S - key0, n * 128);
-    if (tid >= 128) {
-      if (tid == 128) {
-        const uint64_t pol = attn_evict_first();
-        const int b = group / p.Hkv, h = group - b * p.Hkv;
-        for (int i = 0; i < n && ok; ++i)
-          ok = attn_load_chunk(ring, full, empty, &tmK, &tmV, key0 + i * 128, h, b, ait, pol, kBudgetNs, abort_word);
-      }
+    if (warp == 4) {
+      const uint64_t pol = attn_evict_first();
+      const int b = group / p.Hkv, h = group - b * p.Hkv;
+      for (int i = 0; i < n && ok; ++i)
+        ok = attn_load_chunk(ring, full, empty, &tmK, &tmV, key0 + i * 128, h, b, ait, pol, kBudgetNs, abort_word);
     } else {
       float o[kAttnMaxG], M[kAttnMaxG], L[kAttnMaxG];
       auto bar = [] { attn_bar(); };
@@ -121,7 +119,7 @@ attn_stream_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
     }
     pos += n;
   }
-  if (!ok && tid == 128) {                           // loads in flight land in this CTA's memory
+  if (!ok && warp == 4) {                            // loads in flight land in this CTA's memory
     const AttnPipe pp{ring, full, empty, kBudgetNs, abort_word};
     attn_drain_loads(pp, ait);
   }

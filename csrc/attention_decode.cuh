@@ -161,7 +161,7 @@ __device__ __noinline__ void attn_decode_task_t(const MacoEltArgs& ar, int tid, 
 }
 
 // ---- streaming form -----------------------------------------------------------------------------
-// Decode attention of one key range of one (sequence, kv head), bound by streaming K and V out of HBM. A TMA thread
+// Decode attention of one key range of one (sequence, kv head), bound by streaming K and V out of HBM. A TMA warp
 // brings 128-key chunks of K and V (two boxes of 64 dims x 128 keys each, 128-byte swizzle) through a ring of six 32 KB
 // stages (192 KB in flight per SM); four warps consume it. Warp w owns keys [32 w, 32 w + 32) of every chunk and
 // keeps its own softmax state, so there is no barrier among the warps before the range is done:
@@ -193,18 +193,20 @@ MACO_DEVICE uint64_t attn_evict_first() {            // every K / V row is read 
   asm volatile("createpolicy.fractional.L2::evict_first.b64 %0, 1.0;" : "=l"(pol));
   return pol;
 }
-// Both stages of one chunk (K, then V); one thread. `ait` counts stage uses.
+// Both stages of one chunk (K, then V); a whole, converged warp. `ait` counts stage uses.
 MACO_DEVICE bool attn_load_chunk(uint8_t* ring, uint64_t* full, uint64_t* empty, const void* tmK, const void* tmV, int key, int head, int batch,
                                  uint32_t& ait, uint64_t pol, uint64_t budget_ns, volatile uint32_t* abort_word) {
 #pragma unroll
   for (int kv = 0; kv < 2; ++kv, ++ait) {
     const uint32_t s = ait % kAttnStages;
-    if (!mbar_wait(&empty[s], ((ait / kAttnStages) & 1) ^ 1, budget_ns, abort_word)) return false;
-    mbar_arrive_expect_tx(&full[s], kAttnStageBytes);
-    uint8_t* dst = ring + (size_t)s * kAttnStageBytes;
-    const void* tm = kv == 0 ? tmK : tmV;
-    attn_load_box(dst, tm, &full[s], 0, key, head, batch, pol);
-    attn_load_box(dst + kAttnHalfBytes, tm, &full[s], 64, key, head, batch, pol);
+    if (!mbar_wait_warp(&empty[s], ((ait / kAttnStages) & 1) ^ 1, budget_ns, abort_word)) return false;
+    if (elect_one()) {
+      mbar_arrive_expect_tx(&full[s], kAttnStageBytes);
+      uint8_t* dst = ring + (size_t)s * kAttnStageBytes;
+      const void* tm = kv == 0 ? tmK : tmV;
+      attn_load_box(dst, tm, &full[s], 0, key, head, batch, pol);
+      attn_load_box(dst + kAttnHalfBytes, tm, &full[s], 64, key, head, batch, pol);
+    }
   }
   return true;
 }
@@ -477,10 +479,10 @@ MACO_DEVICE bool attn_pipelined(const MacoEltArgs& a) { return a.ld_in == kAttnD
 MACO_DEVICE uint32_t attn_stage_uses(const MacoEltArgs& a) { return 2u * (uint32_t)((a.rows + 127) / 128); }
 
 // Waits (bounded) until the last uses of the attention ring have been released by the consumer: the
-// operand memory may then be handed to another pipeline.
+// operand memory may then be handed to another pipeline. A whole, converged warp.
 MACO_DEVICE bool attn_ring_drained(const AttnPipe& pp, uint32_t ait) {
   for (uint32_t u = ait > (uint32_t)kAttnStages ? ait - kAttnStages : 0; u < ait; ++u)
-    if (!mbar_wait(&pp.empty[u % kAttnStages], (u / kAttnStages) & 1, pp.budget_ns, pp.abort_word)) return false;
+    if (!mbar_wait_warp(&pp.empty[u % kAttnStages], (u / kAttnStages) & 1, pp.budget_ns, pp.abort_word)) return false;
   return true;
 }
 

@@ -41,64 +41,69 @@ MACO_DEVICE void tma_load_2d_hint(void* smem_dst, const void* tmap, uint64_t* ba
       :: "r"(smem_u32(smem_dst)), "l"(tmap), "r"(smem_u32(bar)), "r"(x), "r"(y), "l"(pol) : "memory");
 }
 
-// ---- TMA thread -------------------------------------------------------------------------------
+// ---- TMA warp (converged) ----------------------------------------------------------------------
 template <int STAGES, int STAGE_BYTES>
 MACO_DEVICE bool few_load_weights(uint8_t* smem, const GemmCtrl& c, const CUtensorMap* tmW, const MacoGemmArgs& g, uint32_t u,
                                   uint32_t step, uint64_t pol, uint64_t budget_ns) {
   const uint32_t s = u % STAGES, ph = (u / STAGES) & 1;
-  if (!mbar_wait(&c.empty[s], ph ^ 1, budget_ns, c.abort_word)) return false;
-  mbar_arrive_expect_tx(&c.full[s], kFewWBytes + g.bn * (kFewK * 2u));
-  uint8_t* sw = smem + s * STAGE_BYTES;
-  const int k = g.k0 + (int)step * kFewK;
-  if (g.b_mn & kFewSplit) {                          // boxes of 64 rows (gate and up alternate in blocks of 128)
+  if (!mbar_wait_warp(&c.empty[s], ph ^ 1, budget_ns, c.abort_word)) return false;
+  const int k = warp_uniform(g.k0) + (int)step * kFewK, m0 = warp_uniform(g.m0);
+  const bool split = warp_uniform((int)g.b_mn & kFewSplit) != 0;
+  if (elect_one()) {
+    mbar_arrive_expect_tx(&c.full[s], kFewWBytes + g.bn * (kFewK * 2u));
+    uint8_t* sw = smem + s * STAGE_BYTES;
+    if (split) {                                     // boxes of 64 rows (gate and up alternate in blocks of 128)
 #pragma unroll 1
-    for (int i = 0; i < 4; ++i) tma_load_2d_hint(sw + i * (kFewWBytes / 4), tmW, &c.full[s], k + (i >> 1) * kBK, g.m0 + (i & 1) * 128, pol);
-    return true;
+      for (int i = 0; i < 4; ++i) tma_load_2d_hint(sw + i * (kFewWBytes / 4), tmW, &c.full[s], k + (i >> 1) * kBK, m0 + (i & 1) * 128, pol);
+    } else {
+      tma_load_2d_hint(sw, tmW, &c.full[s], k, m0, pol);
+      tma_load_2d_hint(sw + kFewWBytes / 2, tmW, &c.full[s], k + kBK, m0, pol);
+    }
   }
-  tma_load_2d_hint(sw, tmW, &c.full[s], k, g.m0, pol);
-  tma_load_2d_hint(sw + kFewWBytes / 2, tmW, &c.full[s], k + kBK, g.m0, pol);
   return true;
 }
 template <int STAGES, int STAGE_BYTES>
 MACO_DEVICE void few_load_tokens(uint8_t* smem, const GemmCtrl& c, const CUtensorMap* tmX, const MacoGemmArgs& g, uint32_t u, uint32_t step) {
   const uint32_t s = u % STAGES;
   uint8_t* sx = smem + s * STAGE_BYTES + kFewWBytes;
-  const int k = g.k0 + (int)step * kFewK;
-  tma_load_2d(sx, tmX, &c.full[s], k, 0);
-  tma_load_2d(sx + g.bn * (kBK * 2u), tmX, &c.full[s], k + kBK, 0);
+  const int k = warp_uniform(g.k0) + (int)step * kFewK;
+  const uint32_t half = warp_uniform(g.bn) * (kBK * 2u);
+  if (elect_one()) {
+    tma_load_2d(sx, tmX, &c.full[s], k, 0);
+    tma_load_2d(sx + half, tmX, &c.full[s], k + kBK, 0);
+  }
 }
 
-// ---- MMA thread -------------------------------------------------------------------------------
+// ---- MMA warp (converged) ----------------------------------------------------------------------
 template <int STAGES, int STAGE_BYTES, int ACC_COLS>
 MACO_DEVICE bool few_mma_tile(uint8_t* smem, const GemmCtrl& c, uint32_t tmem_base, const MacoGemmArgs& g, uint32_t& it, uint32_t tile_seq,
                               uint64_t budget_ns) {
-  const uint32_t acc = tile_seq & 1, acc_ph = (tile_seq >> 1) & 1, idesc = g.idesc;
-  const int steps = g.k_blocks;
-  if (!mbar_wait(&c.tmem_empty[acc], acc_ph ^ 1, budget_ns, c.abort_word)) return false;
+  const uint32_t acc = tile_seq & 1, acc_ph = (tile_seq >> 1) & 1, idesc = warp_uniform(g.idesc);
+  const int steps = warp_uniform(g.k_blocks);
+  if (!mbar_wait_warp(&c.tmem_empty[acc], acc_ph ^ 1, budget_ns, c.abort_word)) return false;
   tc_fence_after();
-  const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
+  const uint32_t d_tmem = warp_uniform(tmem_base) + acc * ACC_COLS;
   const uint64_t d0 = make_smem_desc(0, 16, 1024, 2);
   const uint32_t hi = (uint32_t)(d0 >> 32), lbo = (uint32_t)d0;
-  const uint32_t base_lo = (smem_u32(smem) & 0x3FFFFu) >> 4, x_half = g.bn * (kBK * 2u) >> 4;
-  uint32_t accum = 0;
+  const uint32_t base_lo = (smem_u32(smem) & 0x3FFFFu) >> 4, x_half = warp_uniform(g.bn) * (kBK * 2u) >> 4;
   for (int st = 0; st < steps; ++st) {
     const uint32_t u = it + (uint32_t)st, s = u % STAGES;
-    if (!mbar_wait(&c.full[s], (u / STAGES) & 1, budget_ns, c.abort_word)) { it = u; return false; }
-    uint32_t w_lo = base_lo + s * (STAGE_BYTES >> 4), x_lo = w_lo + (kFewWBytes >> 4);
-#pragma unroll 1
-    for (int half = 0; half < 2; ++half) {
+    if (!mbar_wait_warp(&c.full[s], (u / STAGES) & 1, budget_ns, c.abort_word)) { it = u; return false; }
+    if (elect_one()) {
+      uint32_t w_lo = base_lo + s * (STAGE_BYTES >> 4), x_lo = w_lo + (kFewWBytes >> 4);
 #pragma unroll
-      for (int k = 0; k < kBK / kUmmaK; ++k) {
-        tc_mma_f16_lo(d_tmem, (w_lo + k * 2) | lbo, hi, (x_lo + k * 2) | lbo, hi, idesc, accum);
-        accum = 1;
+      for (int half = 0; half < 2; ++half) {
+#pragma unroll
+        for (int k = 0; k < kBK / kUmmaK; ++k)
+          tc_mma_f16_lo(d_tmem, (w_lo + k * 2) | lbo, hi, (x_lo + k * 2) | lbo, hi, idesc, half + k == 0 ? (st != 0 ? 1u : 0u) : 1u);
+        w_lo += kFewWBytes >> 5;
+        x_lo += x_half;
       }
-      w_lo += kFewWBytes >> 5;
-      x_lo += x_half;
+      tc_commit(&c.empty[s]);
     }
-    tc_commit(&c.empty[s]);
   }
   it += (uint32_t)steps;
-  tc_commit(&c.tmem_full[acc]);
+  if (elect_one()) tc_commit(&c.tmem_full[acc]);
   return true;
 }
 

@@ -8,13 +8,19 @@
 //
 // One CTA = 6 warps:
 //   warp 0      TMA producer   cp.async.bulk.tensor tiles -> 128B-swizzled smem ring
-//   warp 1      MMA issuer     one lane issues tcgen05.mma (128 x BN x 16) into a TMEM accumulator
+//   warp 1      MMA issuer     one elected lane issues tcgen05.mma (128 x BN x 16) into a TMEM accumulator
 //   warps 2..5  epilogue       tcgen05.ld the accumulator (one TMEM lane quarter per warp),
 //                              apply the fused epilogue, store to global (local or peer memory)
 // The accumulator is double buffered in TMEM (2 x BN columns) so the epilogue of tile i runs
 // under the main loop of tile i+1. All hand-offs are mbarriers; every wait is bounded and a
 // wait that runs out sets a CTA-wide abort word, after which all roles drain and the CTA frees
 // its TMEM and returns.
+//
+// Warps 0 and 1 run converged and elect the lane that issues (elect.sync) in each k-block. tcgen05.mma, cp.async.bulk.tensor and their
+// operands live on the warp-uniform datapath: in code that one lane runs under `lane == 0` the compiler cannot know that, and serialises
+// every such instruction over the lanes that may be active, about 100 cycles apiece. A k-block then took 0.32 us to issue whatever its size,
+// more than its products (0.13 us for 128 x 128) and more than the loads. One B200, lane 0 / elected lane, us: 1024 x 2048 x 8192 in
+// 256 x 128 tiles 58 / 34, 8192 x 4096 x 4096 in 256 x 256 tiles 205 / 185 (one-CTA tiles 205 / 195).
 //
 // Operands may be K-major (row-major [rows, K]) or MN-major (row-major [K, rows]); the latter is
 // what the backward GEMMs need (wgrad = dY^T · X contracts over the token dimension).
@@ -81,7 +87,7 @@ MACO_DEVICE void gemm_tile_coords(int tile, int m_tiles, int n_tiles, int& m_blk
   n_blk = r / gsize;
 }
 
-// ---- producer ------------------------------------------------------------------------------
+// ---- producer: a whole, converged warp -------------------------------------------------------
 // Loads one (128 x 64) A block and one (BN x 64) B block per k-step. K-major operands take one
 // box; MN-major operands take one 64-wide box per 64 rows (each box is a 64x64 swizzle panel).
 template <int BN, int STAGES, bool A_MN, bool B_MN, int SBN = BN>
@@ -96,7 +102,9 @@ MACO_DEVICE bool gemm_produce_tile(uint8_t* smem, const GemmCtrl& c, const CUten
   // page; the blocked form streams at the rate of a plain copy.)
   // k_step: elements per 128-byte k-block (64 for 16-bit operands, 32 for fp32 operands run as TF32)
   using L = GemmSmemLayout<BN, STAGES, SBN>;
-  // stage index and phase advance incrementally: the loop is one thread's instruction stream, and a division
+  m0 = warp_uniform(m0); n0 = warp_uniform(n0); k0 = warp_uniform(k0); k_blocks = warp_uniform(k_blocks);
+  b_blocked_row0 = warp_uniform(b_blocked_row0); b_ahead = warp_uniform(b_ahead);
+  // stage index and phase advance incrementally: the loop is one instruction stream, and a division
   // per k-block is a measurable part of it
   uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
   uint8_t* sa = smem + s * L::kStageBytes;
@@ -104,25 +112,25 @@ MACO_DEVICE bool gemm_produce_tile(uint8_t* smem, const GemmCtrl& c, const CUten
   for (int kb = 0; kb < k_blocks; ++kb, k += k_step) {
     const long long t0 = prof ? clock64() : 0;
     const bool b_done = (uint32_t)kb < b_ahead;
-    if (!b_done) {
-      if (!mbar_wait(&c.empty[s], ph ^ 1, budget_ns, c.abort_word)) { it += kb; return false; }
-      mbar_arrive_expect_tx(&c.full[s], L::kLoadBytes);
-    }
+    if (!b_done && !mbar_wait_warp(&c.empty[s], ph ^ 1, budget_ns, c.abort_word)) { it += kb; return false; }
     if (prof) prof[0] += clock64() - t0;
-    uint8_t* sb = sa + L::kABytes;
-    if constexpr (!A_MN) {
-      tma_load_2d(sa, tmA, &c.full[s], k, m0);
-    } else {
+    if (elect_one()) {
+      if (!b_done) mbar_arrive_expect_tx(&c.full[s], L::kLoadBytes);
+      uint8_t* sb = sa + L::kABytes;
+      if constexpr (!A_MN) {
+        tma_load_2d(sa, tmA, &c.full[s], k, m0);
+      } else {
 #pragma unroll
-      for (int j = 0; j < kBM / 64; ++j) tma_load_2d(sa + j * 8192, tmA, &c.full[s], m0 + j * 64, k);
-    }
-    if constexpr (!B_MN) {
-      if (b_done) {}
-      else if (b_blocked_row0 >= 0) tma_load_2d(sb, tmB, &c.full[s], 0, b_blocked_row0 + kb * BN);
-      else tma_load_2d(sb, tmB, &c.full[s], k, n0);
-    } else {
+        for (int j = 0; j < kBM / 64; ++j) tma_load_2d(sa + j * 8192, tmA, &c.full[s], m0 + j * 64, k);
+      }
+      if constexpr (!B_MN) {
+        if (b_done) {}
+        else if (b_blocked_row0 >= 0) tma_load_2d(sb, tmB, &c.full[s], 0, b_blocked_row0 + kb * BN);
+        else tma_load_2d(sb, tmB, &c.full[s], k, n0);
+      } else {
 #pragma unroll
-      for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * 8192, tmB, &c.full[s], n0 + j * 64, k);
+        for (int j = 0; j < BN / 64; ++j) tma_load_2d(sb + j * 8192, tmB, &c.full[s], n0 + j * 64, k);
+      }
     }
     if (++s == STAGES) { s = 0; ph ^= 1; sa = smem; } else { sa += L::kStageBytes; }
   }
@@ -136,14 +144,17 @@ template <int BN, int STAGES, int SBN = BN>
 MACO_DEVICE bool gemm_produce_b_ahead(uint8_t* smem, const GemmCtrl& c, const CUtensorMap* tmB, int n0, int k0, int k_blocks,
                                       uint32_t it, uint64_t budget_ns, int b_blocked_row0, uint32_t& ahead) {
   using L = GemmSmemLayout<BN, STAGES, SBN>;
+  n0 = warp_uniform(n0); k0 = warp_uniform(k0); k_blocks = warp_uniform(k_blocks); b_blocked_row0 = warp_uniform(b_blocked_row0);
   const uint32_t most = k_blocks < STAGES ? (uint32_t)k_blocks : (uint32_t)STAGES;
   for (ahead = 0; ahead < most; ++ahead) {
     const uint32_t u = it + ahead, s = u % STAGES, ph = (u / STAGES) & 1;
-    if (!mbar_wait(&c.empty[s], ph ^ 1, budget_ns, c.abort_word)) return false;
-    mbar_arrive_expect_tx(&c.full[s], L::kLoadBytes);
-    uint8_t* sb = smem + s * L::kStageBytes + L::kABytes;
-    if (b_blocked_row0 >= 0) tma_load_2d(sb, tmB, &c.full[s], 0, b_blocked_row0 + (int)ahead * BN);
-    else tma_load_2d(sb, tmB, &c.full[s], k0 + (int)ahead * kBK, n0);
+    if (!mbar_wait_warp(&c.empty[s], ph ^ 1, budget_ns, c.abort_word)) return false;
+    if (elect_one()) {
+      mbar_arrive_expect_tx(&c.full[s], L::kLoadBytes);
+      uint8_t* sb = smem + s * L::kStageBytes + L::kABytes;
+      if (b_blocked_row0 >= 0) tma_load_2d(sb, tmB, &c.full[s], 0, b_blocked_row0 + (int)ahead * BN);
+      else tma_load_2d(sb, tmB, &c.full[s], k0 + (int)ahead * kBK, n0);
+    }
   }
   return true;
 }
@@ -161,18 +172,19 @@ MACO_DEVICE void gemm_drain_loads(const GemmCtrl& c, uint32_t issued) {
   }
 }
 
-// ---- MMA issuer ----------------------------------------------------------------------------
+// ---- MMA issuer: a whole, converged warp (the elected lane is the same one each time, so its commits cover its products) -----
 template <int BN, int STAGES, bool A_MN, bool B_MN, int SBN = BN, bool TF32 = false>
 MACO_DEVICE bool gemm_mma_tile(uint8_t* smem, const GemmCtrl& c, uint32_t tmem_base, uint32_t idesc,
                                int k_blocks, uint32_t& it, uint32_t tile_seq, uint64_t budget_ns,
                                long long* prof = nullptr) {
   using L = GemmSmemLayout<BN, STAGES, SBN>;
   const uint32_t acc = tile_seq & 1, acc_ph = (tile_seq >> 1) & 1;
+  k_blocks = warp_uniform(k_blocks); idesc = warp_uniform(idesc);
   long long t0 = prof ? clock64() : 0;
-  if (!mbar_wait(&c.tmem_empty[acc], acc_ph ^ 1, budget_ns, c.abort_word)) return false;
+  if (!mbar_wait_warp(&c.tmem_empty[acc], acc_ph ^ 1, budget_ns, c.abort_word)) return false;
   if (prof) prof[1] += clock64() - t0;
   tc_fence_after();
-  const uint32_t d_tmem = tmem_base + acc * SBN;
+  const uint32_t d_tmem = warp_uniform(tmem_base) + acc * SBN;
   // K-major: 8-row groups are 1024 B apart (SBO); a K step of 16 elements is 32 B inside the swizzled row.
   // MN-major: 64-row panels are 8192 B apart (LBO), 8-k groups 1024 B apart (SBO); a K step of 16 is two groups
   // = 2048 B. The descriptors' high words are constant; the low word is the start address in 16-byte units.
@@ -185,25 +197,26 @@ MACO_DEVICE bool gemm_mma_tile(uint8_t* smem, const GemmCtrl& c, uint32_t tmem_b
   const uint32_t base_lo = (smem_u32(smem) & 0x3FFFFu) >> 4;
   uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
   uint32_t a_lo = base_lo + s * kStage16;
-  uint32_t accum = 0;
   for (int kb = 0; kb < k_blocks; ++kb) {
     if (prof) t0 = clock64();
-    if (!mbar_wait(&c.full[s], ph, budget_ns, c.abort_word)) { it += kb; return false; }
+    if (!mbar_wait_warp(&c.full[s], ph, budget_ns, c.abort_word)) { it += kb; return false; }
     if (prof) prof[2] += clock64() - t0;
-    const uint32_t b_lo = a_lo + kAB16;
+    if (elect_one()) {
+      const uint32_t b_lo = a_lo + kAB16;
 #pragma unroll
-    for (int k = 0; k < kBK / kUmmaK; ++k) {
-      // low descriptor words: start address (bits 0-13, never carries: shared memory is below 256 KB) | leading offset
-      // fp32 operands (TF32): 8 elements of 4 bytes per MMA, the same 32-byte step inside the swizzled row
-      if constexpr (TF32) tc_mma_tf32_lo(d_tmem, (a_lo + k * kStepA) | a_lbo, a_hi, (b_lo + k * kStepB) | b_lbo, b_hi, idesc, accum);
-      else tc_mma_f16_lo(d_tmem, (a_lo + k * kStepA) | a_lbo, a_hi, (b_lo + k * kStepB) | b_lbo, b_hi, idesc, accum);
-      accum = 1;
+      for (int k = 0; k < kBK / kUmmaK; ++k) {
+        // low descriptor words: start address (bits 0-13, never carries: shared memory is below 256 KB) | leading offset
+        // fp32 operands (TF32): 8 elements of 4 bytes per MMA, the same 32-byte step inside the swizzled row
+        const uint32_t add = k == 0 ? (kb != 0 ? 1u : 0u) : 1u;
+        if constexpr (TF32) tc_mma_tf32_lo(d_tmem, (a_lo + k * kStepA) | a_lbo, a_hi, (b_lo + k * kStepB) | b_lbo, b_hi, idesc, add);
+        else tc_mma_f16_lo(d_tmem, (a_lo + k * kStepA) | a_lbo, a_hi, (b_lo + k * kStepB) | b_lbo, b_hi, idesc, add);
+      }
+      tc_commit(&c.empty[s]);        // frees the smem stage once these MMAs have read it
     }
-    tc_commit(&c.empty[s]);          // frees the smem stage once these MMAs have read it
     if (++s == STAGES) { s = 0; ph ^= 1; a_lo = base_lo; } else { a_lo += kStage16; }
   }
   it += k_blocks;
-  tc_commit(&c.tmem_full[acc]);      // accumulator complete -> epilogue
+  if (elect_one()) tc_commit(&c.tmem_full[acc]);      // accumulator complete -> epilogue
   return true;
 }
 
@@ -778,29 +791,32 @@ MACO_DEVICE bool pair_produce_tile(uint8_t* smem, const GemmCtrl& c, uint32_t ra
   constexpr int kBHalf = BN / 2;
   constexpr uint32_t kPairBytes = 2u * (L::kABytes + kBHalf * kBK * 2);
   const uint32_t full0 = mapa_u32(smem_u32(&c.full[0]), 0);
+  m0 = warp_uniform(m0); n0 = warp_uniform(n0); k0 = warp_uniform(k0); k_blocks = warp_uniform(k_blocks);
   const int nb0 = n0 + (int)rank * kBHalf;
   uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
   uint8_t* sa = smem + s * L::kStageBytes;
   int k = k0;
   for (int kb = 0; kb < k_blocks; ++kb, k += kBK) {
     const long long t0 = prof ? clock64() : 0;
-    if (!mbar_wait(&c.empty[s], ph ^ 1, budget_ns, c.abort_word)) { it += kb; return false; }
+    if (!mbar_wait_warp(&c.empty[s], ph ^ 1, budget_ns, c.abort_word)) { it += kb; return false; }
     if (prof) prof[0] += clock64() - t0;
     if (prof && prof[4] && prof[5] < 512) reinterpret_cast<uint64_t*>(prof[4])[2 * prof[5]] = globaltimer_ns();
-    uint8_t* sb = sa + L::kABytes;
-    if (rank == 0) mbar_arrive_expect_tx(&c.full[s], kPairBytes);
-    const uint32_t bar = full0 + s * 8;
-    if constexpr (!A_MN) {
-      tma_load_2d_pair(sa, tmA, bar, k, m0);
-    } else {
+    if (elect_one()) {
+      uint8_t* sb = sa + L::kABytes;
+      if (rank == 0) mbar_arrive_expect_tx(&c.full[s], kPairBytes);
+      const uint32_t bar = full0 + s * 8;
+      if constexpr (!A_MN) {
+        tma_load_2d_pair(sa, tmA, bar, k, m0);
+      } else {
 #pragma unroll
-      for (int j = 0; j < kBM / 64; ++j) tma_load_2d_pair(sa + j * 8192, tmA, bar, m0 + j * 64, k);
-    }
-    if constexpr (!B_MN) {
-      tma_load_2d_pair(sb, tmB, bar, k, nb0);
-    } else {
+        for (int j = 0; j < kBM / 64; ++j) tma_load_2d_pair(sa + j * 8192, tmA, bar, m0 + j * 64, k);
+      }
+      if constexpr (!B_MN) {
+        tma_load_2d_pair(sb, tmB, bar, k, nb0);
+      } else {
 #pragma unroll
-      for (int j = 0; j < kBHalf / 64; ++j) tma_load_2d_pair(sb + j * 8192, tmB, bar, nb0 + j * 64, k);
+        for (int j = 0; j < kBHalf / 64; ++j) tma_load_2d_pair(sb + j * 8192, tmB, bar, nb0 + j * 64, k);
+      }
     }
     if (prof && prof[4] && prof[5] < 512) { reinterpret_cast<uint64_t*>(prof[4])[2 * prof[5] + 1] = globaltimer_ns(); ++prof[5]; }
     if (++s == STAGES) { s = 0; ph ^= 1; sa = smem; } else { sa += L::kStageBytes; }
@@ -816,11 +832,12 @@ MACO_DEVICE bool pair_mma_tile(uint8_t* smem, const GemmCtrl& c, uint32_t tmem_b
   using L = PairSmemLayout<STAGES>;
   const uint32_t acc = tile_seq & 1, acc_ph = (tile_seq >> 1) & 1;
   const uint32_t empty0 = smem_u32(&c.empty[0]), tfull0 = smem_u32(&c.tmem_full[0]);
+  k_blocks = warp_uniform(k_blocks); idesc = warp_uniform(idesc);
   long long t0 = prof ? clock64() : 0;
-  if (!mbar_wait(&c.tmem_empty[acc], acc_ph ^ 1, budget_ns, c.abort_word)) return false;
+  if (!mbar_wait_warp(&c.tmem_empty[acc], acc_ph ^ 1, budget_ns, c.abort_word)) return false;
   if (prof) prof[1] += clock64() - t0;
   tc_fence_after();
-  const uint32_t d_tmem = tmem_base + acc * 256;
+  const uint32_t d_tmem = warp_uniform(tmem_base) + acc * 256;
   const uint64_t da0 = A_MN ? make_smem_desc(0, 8192, 1024, 2) : make_smem_desc(0, 16, 1024, 2);
   const uint64_t db0 = B_MN ? make_smem_desc(0, 8192, 1024, 2) : make_smem_desc(0, 16, 1024, 2);
   const uint32_t a_hi = (uint32_t)(da0 >> 32), b_hi = (uint32_t)(db0 >> 32);
@@ -830,24 +847,23 @@ MACO_DEVICE bool pair_mma_tile(uint8_t* smem, const GemmCtrl& c, uint32_t tmem_b
   const uint32_t base_lo = (smem_u32(smem) & 0x3FFFFu) >> 4;
   uint32_t s = it % STAGES, ph = (it / STAGES) & 1;
   uint32_t a_lo = base_lo + s * kStage16;
-  uint32_t accum = 0;
   for (int kb = 0; kb < k_blocks; ++kb) {
     if (prof) t0 = clock64();
-    if (!mbar_wait(&c.full[s], ph, budget_ns, c.abort_word)) { it += kb; return false; }
+    if (!mbar_wait_warp(&c.full[s], ph, budget_ns, c.abort_word)) { it += kb; return false; }
     if (prof) prof[2] += clock64() - t0;
     if (prof && prof[4] && prof[5] < 512) reinterpret_cast<uint64_t*>(prof[4])[2 * prof[5]] = globaltimer_ns();
-    const uint32_t b_lo = a_lo + kAB16;
+    if (elect_one()) {
+      const uint32_t b_lo = a_lo + kAB16;
 #pragma unroll
-    for (int k = 0; k < kBK / kUmmaK; ++k) {
-      tc_mma2_f16_lo(d_tmem, (a_lo + k * kStepA) | a_lbo, a_hi, (b_lo + k * kStepB) | b_lbo, b_hi, idesc, accum);
-      accum = 1;
+      for (int k = 0; k < kBK / kUmmaK; ++k)
+        tc_mma2_f16_lo(d_tmem, (a_lo + k * kStepA) | a_lbo, a_hi, (b_lo + k * kStepB) | b_lbo, b_hi, idesc, k == 0 ? (kb != 0 ? 1u : 0u) : 1u);
+      tc_commit2_both(empty0 + s * 8); // both CTAs may refill the stage once these MMAs have read it
     }
-    tc_commit2_both(empty0 + s * 8);   // both CTAs may refill the stage once these MMAs have read it
     if (prof && prof[4] && prof[5] < 512) { reinterpret_cast<uint64_t*>(prof[4])[2 * prof[5] + 1] = globaltimer_ns(); ++prof[5]; }
     if (++s == STAGES) { s = 0; ph ^= 1; a_lo = base_lo; } else { a_lo += kStage16; }
   }
   it += k_blocks;
-  tc_commit2_both(tfull0 + acc * 8);   // accumulator complete -> both CTAs' epilogues
+  if (elect_one()) tc_commit2_both(tfull0 + acc * 8);   // accumulator complete -> both CTAs' epilogues
   return true;
 }
 
@@ -918,13 +934,13 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   const int num_tiles = m_pairs * n_tiles;
   const int k_blocks = (K + kBK - 1) / kBK;
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const uint32_t tempty_leader = mapa_u32(smem_u32(&c.tmem_empty[0]), 0);
 
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
+    if (lane == 0) { tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); }
+    __syncwarp();
+    {
       uint32_t it = 0;
       bool ok = true;
       for (int tile = pair; ok && tile < num_tiles; tile += num_pairs) {
@@ -936,16 +952,16 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
       // after an abort the leader's barriers count both CTAs' bytes; the other CTA stays until the leader
       // reaches the teardown (cluster barrier)
       if (!ok && rank == 0) gemm_drain_loads<kPairStages>(c, it);
-      if (dbg != nullptr) { dbg[blockIdx.x * 8 + 0] = prof[0]; dbg[blockIdx.x * 8 + 4] = clock64() - t_begin; }
+      if (dbg != nullptr && lane == 0) { dbg[blockIdx.x * 8 + 0] = prof[0]; dbg[blockIdx.x * 8 + 4] = clock64() - t_begin; }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0 && rank == 0) {
+    if (rank == 0) {
       uint32_t it = 0, seq = 0;
       bool ok = true;
       for (int tile = pair; ok && tile < num_tiles; tile += num_pairs, ++seq)
         ok = pair_mma_tile<BN, kPairStages, A_MN, B_MN>(smem, c, tmem_base, idesc, k_blocks, it, seq, budget_ns, pp);
-      if (dbg != nullptr) { dbg[blockIdx.x * 8 + 1] = prof[1]; dbg[blockIdx.x * 8 + 2] = prof[2]; dbg[blockIdx.x * 8 + 3] = clock64() - t_begin; }
+      if (dbg != nullptr && lane == 0) { dbg[blockIdx.x * 8 + 1] = prof[1]; dbg[blockIdx.x * 8 + 2] = prof[2]; dbg[blockIdx.x * 8 + 3] = clock64() - t_begin; }
     }
     __syncwarp();
   } else {
@@ -989,12 +1005,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   const int num_tiles = m_tiles * n_tiles;
   constexpr int kStepElems = TF32 ? kBK / 2 : kBK;
   const int k_blocks = (K + kStepElems - 1) / kStepElems;
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
 
   if (warp == 0) {
-    if (lane == 0) {
-      tma_prefetch_desc(&tmA);
-      tma_prefetch_desc(&tmB);
+    if (lane == 0) { tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); }
+    __syncwarp();
+    {
       uint32_t it = 0;
       bool ok = true;
       for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x) {
@@ -1003,16 +1019,16 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         ok = gemm_produce_tile<BN, STAGES, A_MN, B_MN>(smem, c, &tmA, &tmB, mb * kBM, nb * BN, 0, k_blocks, it, budget_ns, pp, kStepElems);
       }
       if (!ok) gemm_drain_loads<STAGES>(c, it);
-      if (dbg != nullptr) { dbg[blockIdx.x * 8 + 0] = prof[0]; dbg[blockIdx.x * 8 + 4] = clock64() - t_begin; }
+      if (dbg != nullptr && lane == 0) { dbg[blockIdx.x * 8 + 0] = prof[0]; dbg[blockIdx.x * 8 + 4] = clock64() - t_begin; }
     }
     __syncwarp();
   } else if (warp == 1) {
-    if (lane == 0) {
+    {
       uint32_t it = 0, seq = 0;
       bool ok = true;
       for (int tile = blockIdx.x; ok && tile < num_tiles; tile += gridDim.x, ++seq)
         ok = gemm_mma_tile<BN, STAGES, A_MN, B_MN, BN, TF32>(smem, c, tmem_base, idesc, k_blocks, it, seq, budget_ns, pp);
-      if (dbg != nullptr) { dbg[blockIdx.x * 8 + 1] = prof[1]; dbg[blockIdx.x * 8 + 2] = prof[2]; dbg[blockIdx.x * 8 + 3] = clock64() - t_begin; }
+      if (dbg != nullptr && lane == 0) { dbg[blockIdx.x * 8 + 1] = prof[1]; dbg[blockIdx.x * 8 + 2] = prof[2]; dbg[blockIdx.x * 8 + 3] = clock64() - t_begin; }
     }
     __syncwarp();
   } else {

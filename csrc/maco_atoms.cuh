@@ -125,6 +125,8 @@ MACO_DEVICE bool elect_one() {
   asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.b32 %0, 1, 0, p;\n}" : "=r"(pred));
   return pred != 0;
 }
+// Lane 0's value in every lane: values read from memory become ones the compiler knows to be uniform.
+template <typename T> MACO_DEVICE T warp_uniform(T v) { return __shfl_sync(0xffffffffu, v, 0); }
 MACO_DEVICE uint32_t elect_warp_leader() { return __ffs(__activemask()) - 1; }
 MACO_DEVICE bool is_warp_leader() { return lane_id() == elect_warp_leader(); }
 
@@ -184,6 +186,22 @@ MACO_DEVICE bool mbar_wait(uint64_t* bar, uint32_t parity, uint64_t budget_ns, v
     if ((++spins & 255u) == 0) {
       if (*abort_smem != 0) return false;
       if (globaltimer_ns() - t0 > budget_ns) { *abort_smem = 1; return false; }
+    }
+  }
+  return true;
+}
+
+// The same for a whole, converged warp, with one verdict for all lanes: a lane that gave up while another saw the phase complete would
+// leave that one alone at the next elect.sync.
+MACO_DEVICE bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint64_t budget_ns, volatile uint32_t* abort_smem) {
+  if (__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) return true;
+  const uint64_t t0 = globaltimer_ns();
+  uint32_t spins = 0;
+  while (!__all_sync(0xffffffffu, mbar_try_wait(bar, parity))) {
+    if ((++spins & 255u) == 0) {
+      const bool late = globaltimer_ns() - t0 > budget_ns;
+      if (late) *abort_smem = 1;
+      if (__any_sync(0xffffffffu, late || *abort_smem != 0)) return false;
     }
   }
   return true;

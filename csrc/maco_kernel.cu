@@ -247,19 +247,49 @@ struct TaskStream {
   }
 };
 
+// The producer's and the MMA issuer's view: a whole, converged warp. Lane 0 fetches and waits, all lanes get the answer.
+__device__ __forceinline__ const MacoTaskDesc* next_warp(const MacoProgram& p, TaskStream& ts, uint32_t& task, bool& failed,
+                                                         volatile uint32_t* cta_abort) {
+  __syncwarp();                                         // every lane is done with the slot that is refilled here
+  int state = -1;                                       // index of the slot; -1: end of the queue, -2: aborted
+  task = 0;
+  if (lane_id() == 0) {
+    bool gave_up = false;
+    const MacoTaskDesc* d = ts.next(p, task, gave_up, cta_abort);
+    state = d != nullptr ? (int)(d - ts.slots) : (gave_up ? -2 : -1);
+  }
+  state = warp_uniform(state);
+  task = warp_uniform(task);
+  __syncwarp();
+  failed = state == -2;
+  return state < 0 ? nullptr : ts.slots + state;
+}
+__device__ __forceinline__ bool wait_deps_warp(const MacoProgram& p, const MacoTaskDesc& d, uint32_t task, volatile uint32_t* cta_abort) {
+  int ok = 1;
+  if (lane_id() == 0) ok = wait_deps(p, d, task, cta_abort, nullptr) ? 1 : 0;
+  ok = warp_uniform(ok);
+  __syncwarp();                                         // what lane 0 acquired holds for all lanes
+  return ok != 0;
+}
+__device__ __forceinline__ void report_failure_warp(const MacoProgram& p, uint32_t status, uint32_t task, uint32_t event, volatile uint32_t* cta_abort) {
+  if (lane_id() == 0) report_failure(p, status, task, event, cta_abort);
+  __syncwarp();
+}
+
 // A role's table of row blocks per slab, behind the descriptor slots of all three (`desc_slots`: this role's).
 __device__ __forceinline__ uint16_t* expert_table(MacoTaskDesc* desc_slots, int role) {
   return reinterpret_cast<uint16_t*>(desc_slots + (3 - role) * kStreamSlots) + role * kMaxSlabs;
 }
 
-// ---- producer warp (lane 0), two-CTA programs ----------------------------------------------------
+// ---- producer warp, two-CTA programs (this and the three below: a whole, converged warp) -----------
 // Every GEMM task of such a program is one half (128 rows) of a 256 x BN tile; the two halves sit at the same
 // position of the GEMM sequences of workers 2j and 2j+1 (one cluster). Each CTA waits for ITS half's
 // conditions and loads its rows of A and its half of B; the leader's MMA warp starts when both have landed.
 __device__ void producer_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_base, uint8_t* smem, const GemmCtrl& c,
                                    MacoTaskDesc* desc_slots) {
   TaskStream ts;
-  ts.start(p, desc_slots, w, q_base);
+  if (lane_id() == 0) ts.start(p, desc_slots, w, q_base);
+  ts.slots = desc_slots;
   uint32_t it = 0;
   bool ok = true;
   const uint32_t rank = cluster_ctarank();
@@ -267,16 +297,16 @@ __device__ void producer_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_
   while (ok) {
     uint32_t task;
     bool failed = false;
-    const MacoTaskDesc* dp = ts.next(p, task, failed, c.abort_word);
+    const MacoTaskDesc* dp = next_warp(p, ts, task, failed, c.abort_word);
     if (dp == nullptr) { ok = !failed; break; }
     const MacoTaskDesc& d = *dp;
     if (!is_gemm_type(d.type)) continue;
-    if (p.debug != 0 && !desc_ok(p, d)) { report_failure(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word); ok = false; break; }
-    if (!wait_deps(p, d, task, c.abort_word, nullptr)) { ok = false; break; }
+    if (p.debug != 0 && !desc_ok(p, d)) { report_failure_warp(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word); ok = false; break; }
+    if (!wait_deps_warp(p, d, task, c.abort_word)) { ok = false; break; }
     const MacoGemmArgs& g = d.u.gemm;
     fence_proxy_async_all();           // operands were written by generic-proxy stores of other CTAs
-    const CUtensorMap* ta = tmaps + g.tmap_a;
-    const CUtensorMap* tb = tmaps + g.tmap_b;
+    const CUtensorMap* ta = tmaps + warp_uniform((uint32_t)g.tmap_a);
+    const CUtensorMap* tb = tmaps + warp_uniform((uint32_t)g.tmap_b);
     const int sel = (g.bn == 128 ? 4 : 0) | (g.a_mn ? 2 : 0) | ((g.b_mn & 1) ? 1 : 0);
     switch (sel) {
       case 0: ok = pair_produce_tile<256, kPairStages, false, false>(smem, c, rank, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
@@ -288,7 +318,7 @@ __device__ void producer_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_
       case 6: ok = pair_produce_tile<128, kPairStages, true, false>(smem, c, rank, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
       default: ok = pair_produce_tile<128, kPairStages, true, true>(smem, c, rank, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
     }
-    if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
+    if (!ok) report_failure_warp(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
   }
   if (!ok) {
     // loads in flight land in this CTA's memory: the leader's barriers count both CTAs' bytes, the other CTA
@@ -298,17 +328,18 @@ __device__ void producer_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_
   }
 }
 
-// ---- MMA warp (lane 0) of the pair's leader ------------------------------------------------------
+// ---- MMA warp of the pair's leader ---------------------------------------------------------------
 __device__ void mma_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_base, uint8_t* smem, const GemmCtrl& c,
                               uint32_t tmem_base, MacoTaskDesc* desc_slots) {
   TaskStream ts;
-  ts.start(p, desc_slots, w, q_base);
+  if (lane_id() == 0) ts.start(p, desc_slots, w, q_base);
+  ts.slots = desc_slots;
   uint32_t it = 0, seq = 0;
   bool ok = true;
   while (ok) {
     uint32_t task;
     bool failed = false;
-    const MacoTaskDesc* dp = ts.next(p, task, failed, c.abort_word);
+    const MacoTaskDesc* dp = next_warp(p, ts, task, failed, c.abort_word);
     if (dp == nullptr) break;
     const MacoTaskDesc& d = *dp;
     if (!is_gemm_type(d.type)) continue;
@@ -328,8 +359,8 @@ __device__ void mma_role_pair(const MacoProgram& p, uint32_t w, uint32_t q_base,
   }
 }
 
-// ---- producer warp (lane 0) ---------------------------------------------------------------------
-// A few-row GEMM task on lane 0: the weights (operand A here) of up to a whole ring go out before the task waits for its
+// ---- producer warp ------------------------------------------------------------------------------
+// A few-row GEMM task: the weights (operand A here) of up to a whole ring go out before the task waits for its
 // tokens, unless a task of the program writes them.
 __device__ int producer_few_task(const MacoProgram& p, const MacoTaskDesc& d, uint32_t task, uint8_t* smem, const GemmCtrl& c,
                                  const CUtensorMap* tmW, const CUtensorMap* tmX, uint32_t& it) {
@@ -344,27 +375,27 @@ __device__ int producer_few_task(const MacoProgram& p, const MacoTaskDesc& d, ui
   };
   if (d.flags & MACO_TF_B_STATIC)
     while (ok && armed < steps && armed < (uint32_t)kMkStages) weights();
-  if (ok && !wait_deps(p, d, task, c.abort_word, nullptr)) { it += armed; return 0; }
+  if (ok && !wait_deps_warp(p, d, task, c.abort_word)) { it += armed; return 0; }
   fence_proxy_async_all();           // the tokens were written by generic-proxy stores of other CTAs
   for (uint32_t st = 0; ok && st < steps; ++st) {
     if (st >= armed) weights();
     if (ok) few_load_tokens<kMkStages, MkLayout::kStageBytes>(smem, c, tmX, g, it + st, st);
   }
   it += armed;
-  if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
+  if (!ok) report_failure_warp(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
   return ok ? 1 : 0;
 }
 
-// One GEMM task on lane 0: 1 = carry on, 0 = stop (failure already reported where it has a reporter).
+// One GEMM task: 1 = carry on, 0 = stop (failure already reported where it has a reporter).
 __device__ int producer_gemm_task(const MacoProgram& p, const MacoTaskDesc& d, uint32_t task, uint8_t* smem, const GemmCtrl& c,
                                   const CUtensorMap* tmaps, const AttnPipe& apipe, uint32_t ait, uint32_t& it, int& owner) {
-  if (p.debug != 0 && !desc_ok(p, d)) { report_failure(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word); return 0; }
+  if (p.debug != 0 && !desc_ok(p, d)) { report_failure_warp(p, MACO_STATUS_BAD_TASK, task, d.type, c.abort_word); return 0; }
   const MacoGemmArgs& g = d.u.gemm;
-  const CUtensorMap* ta = tmaps + g.tmap_a;
-  const CUtensorMap* tb = tmaps + g.tmap_b;
+  const CUtensorMap* ta = tmaps + warp_uniform((uint32_t)g.tmap_a);
+  const CUtensorMap* tb = tmaps + warp_uniform((uint32_t)g.tmap_b);
   const int sel = (g.bn == 128 ? 4 : 0) | (g.a_mn ? 2 : 0) | ((g.b_mn & 1) ? 1 : 0);
   if (d.flags & MACO_TF_COUNTED) {
-    if (!wait_deps(p, d, task, c.abort_word, nullptr)) return 0;
+    if (!wait_deps_warp(p, d, task, c.abort_word)) return 0;
     // run-time guarded tile: every role reads the same (final) count after the task's conditions hold
     if (ld_relaxed_gpu_u32(g.count_ptr) <= g.count_base) return 1;
   }
@@ -380,11 +411,11 @@ __device__ int producer_gemm_task(const MacoProgram& p, const MacoTaskDesc& d, u
     const bool ok_b = gemm_produce_b_ahead<256, kMkStages, kMkBN>(smem, c, tb, g.n0, g.k0, g.k_blocks, it, p.budget_ns, b_row, ahead);
     if (!ok_b) {
       it += ahead;
-      report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
+      report_failure_warp(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
       return 0;
     }
   }
-  if (!(d.flags & MACO_TF_COUNTED) && !wait_deps(p, d, task, c.abort_word, nullptr)) { it += ahead; return 0; }
+  if (!(d.flags & MACO_TF_COUNTED) && !wait_deps_warp(p, d, task, c.abort_word)) { it += ahead; return 0; }
   fence_proxy_async_all();           // operands were written by generic-proxy stores of other CTAs
   bool ok;
   // b_mn bit 1: blocked B (256-column tiles only); count_base then holds the weight's total number of k-blocks
@@ -399,7 +430,7 @@ __device__ int producer_gemm_task(const MacoProgram& p, const MacoTaskDesc& d, u
     case 6: ok = gemm_produce_tile<128, kMkStages, true, false, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
     default: ok = gemm_produce_tile<128, kMkStages, true, true, kMkBN>(smem, c, ta, tb, g.m0, g.n0, g.k0, g.k_blocks, it, p.budget_ns); break;
   }
-  if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
+  if (!ok) report_failure_warp(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
   return ok ? 1 : 0;
 }
 
@@ -410,27 +441,28 @@ __device__ int producer_gemm_task(const MacoProgram& p, const MacoTaskDesc& d, u
 __device__ int producer_attn_task(const MacoProgram& p, const MacoTaskDesc& d, uint32_t task, const CUtensorMap* tmaps, const AttnPipe& pp,
                                   uint32_t& ait) {
   const MacoEltArgs& a = d.u.elt;
-  const CUtensorMap* tmK = tmaps + ((a.ld_out & 0xffff) - 1);
-  const CUtensorMap* tmV = tmaps + (((uint32_t)a.ld_out >> 16) - 1);
+  const CUtensorMap* tmK = tmaps + (warp_uniform(a.ld_out & 0xffff) - 1);
+  const CUtensorMap* tmV = tmaps + (warp_uniform((uint32_t)a.ld_out >> 16) - 1);
   const uint64_t pol = attn_evict_first();
-  const int fixed = a.i0 >> 8, row0 = a.row0, rows = a.rows, bh = a.cols;
+  const int fixed = warp_uniform(a.i0 >> 8), row0 = warp_uniform(a.row0), rows = warp_uniform(a.rows), bh = warp_uniform(a.cols);
   bool waited = false, ok = true;
   for (int base = 0; ok && base < rows; base += 128) {
     if (!waited && row0 + base + 128 > fixed) {
-      if (!wait_deps(p, d, task, pp.abort_word, nullptr)) return 0;
+      if (!wait_deps_warp(p, d, task, pp.abort_word)) return 0;
       fence_proxy_async_all();
       waited = true;
     }
     ok = attn_load_chunk(pp.ring, pp.full, pp.empty, tmK, tmV, row0 + base, bh, 0, ait, pol, pp.budget_ns, pp.abort_word);
   }
-  if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, pp.abort_word);
+  if (!ok) report_failure_warp(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, pp.abort_word);
   return ok ? 1 : 0;
 }
 
 __device__ void producer_role(const MacoProgram& p, uint32_t w, uint32_t q_base, uint8_t* smem, const GemmCtrl& c,
                               uint64_t* attn_ring_bars, MacoTaskDesc* desc_slots) {
   TaskStream ts;
-  ts.start(p, desc_slots, w, q_base);
+  if (lane_id() == 0) ts.start(p, desc_slots, w, q_base);
+  ts.slots = desc_slots;
   uint32_t it = 0;                   // stage uses of the GEMM ring
   uint32_t ait = 0;                  // stage uses of the attention ring (same memory)
   int owner = 0;                     // which pipeline used the operand memory last: 1 GEMM, 2 attention
@@ -440,55 +472,58 @@ __device__ void producer_role(const MacoProgram& p, uint32_t w, uint32_t q_base,
   while (ok) {
     uint32_t task;
     bool failed = false;
-    const MacoTaskDesc* dp = ts.next(p, task, failed, c.abort_word);
+    const MacoTaskDesc* dp = next_warp(p, ts, task, failed, c.abort_word);
     if (dp == nullptr) { ok = !failed; break; }
     const MacoTaskDesc& d = *dp;
     if (d.type == MACO_TASK_ATTENTION && attn_pipelined(d.u.elt)) {
       if (owner == 1) {              // the MMA warp may still be reading the last GEMM stages out of this memory
         for (uint32_t u = it > (uint32_t)kMkStages ? it - kMkStages : 0; u < it && ok; ++u)
-          ok = mbar_wait(&c.empty[u % kMkStages], (u / kMkStages) & 1, p.budget_ns, c.abort_word);
-        if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
+          ok = mbar_wait_warp(&c.empty[u % kMkStages], (u / kMkStages) & 1, p.budget_ns, c.abort_word);
+        if (!ok) report_failure_warp(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
       }
       owner = 2;
       ok = ok && producer_attn_task(p, d, task, tmaps, apipe, ait) != 0;
     } else if (is_gemm_type(d.type)) {
       ok = producer_gemm_task(p, d, task, smem, c, tmaps, apipe, ait, it, owner) != 0;
     } else if (d.type == MACO_TASK_MOE_EXPERTS) {
-      ok = wait_deps(p, d, task, c.abort_word, nullptr) && (owner != 2 || attn_ring_drained(apipe, ait));
+      ok = wait_deps_warp(p, d, task, c.abort_word) && (owner != 2 || attn_ring_drained(apipe, ait));
       owner = 1;
       if (ok) {
         fence_proxy_async_all();       // rows and activations are written by other CTAs (bulk copies and generic stores)
         ok = experts_produce<kMkStages>(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, expert_table(desc_slots, 0), smem, c, tmaps, it,
-                                        [&p](const uint32_t* flag, uint32_t expect) { return mk_wait(p, flag, expect, false); });
-        if (!ok) report_failure(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
+                                        [&p](const uint32_t* flag, uint32_t expect) {
+                                          return warp_uniform(lane_id() == 0 && mk_wait(p, flag, expect, false) ? 1 : 0) != 0;
+                                        });
+        if (!ok) report_failure_warp(p, MACO_STATUS_TIMEOUT, task, 0xffffffffu, c.abort_word);
       }
     }
   }
   if (!ok) { gemm_drain_loads<kMkStages>(c, it); attn_drain_loads(apipe, ait); }
 }
 
-// ---- MMA warp (lane 0) --------------------------------------------------------------------------
+// ---- MMA warp -----------------------------------------------------------------------------------
 __device__ void mma_role(const MacoProgram& p, uint32_t w, uint32_t q_base, uint8_t* smem, const GemmCtrl& c,
                          uint32_t tmem_base, MacoTaskDesc* desc_slots) {
   TaskStream ts;
-  ts.start(p, desc_slots, w, q_base);
+  if (lane_id() == 0) ts.start(p, desc_slots, w, q_base);
+  ts.slots = desc_slots;
   uint32_t it = 0, seq = 0;
   bool ok = true;
   while (ok) {
     uint32_t task;
     bool failed = false;
-    const MacoTaskDesc* dp = ts.next(p, task, failed, c.abort_word);
+    const MacoTaskDesc* dp = next_warp(p, ts, task, failed, c.abort_word);
     if (dp == nullptr) break;
     const MacoTaskDesc& d = *dp;
     if (d.type == MACO_TASK_MOE_EXPERTS) {
-      ok = wait_deps(p, d, task, c.abort_word, nullptr) &&
+      ok = wait_deps_warp(p, d, task, c.abort_word) &&
            experts_mma<kMkStages>(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, expert_table(desc_slots, 1), smem, c, tmem_base, it, seq);
       continue;
     }
     if (!is_gemm_type(d.type)) continue;
     const MacoGemmArgs& g = d.u.gemm;
     if (d.flags & MACO_TF_COUNTED) {
-      if (!wait_deps(p, d, task, c.abort_word, nullptr)) break;
+      if (!wait_deps_warp(p, d, task, c.abort_word)) break;
       if (ld_relaxed_gpu_u32(g.count_ptr) <= g.count_base) continue;
     }
     if (g.b_mn & kFewFlag) {
@@ -816,7 +851,7 @@ __device__ void scheduler_role(const MacoProgram& p, uint32_t* heads_sm) {
 template <int CG>
 __device__ __forceinline__ void persistent_body(const MacoProgram& p) {
   extern __shared__ uint8_t dyn_smem[];
-  const uint32_t warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t warp = warp_uniform(threadIdx.x >> 5);
   const bool is_worker = blockIdx.x < p.num_workers;
   GemmCtrl c;
   uint32_t tmem_base;
@@ -841,16 +876,14 @@ __device__ __forceinline__ void persistent_body(const MacoProgram& p) {
     MacoTaskDesc* desc_slots = reinterpret_cast<MacoTaskDesc*>(reinterpret_cast<uint8_t*>(extra) + kStreamOffset);
     if (warp == 0) {
       if constexpr (CG == 2) {
-        if (lane == 0) producer_role_pair(p, w, q_base, smem, c, desc_slots);
+        producer_role_pair(p, w, q_base, smem, c, desc_slots);
       } else {
-        if (lane == 0) producer_role(p, w, q_base, smem, c, attn_bars, desc_slots);
+        producer_role(p, w, q_base, smem, c, attn_bars, desc_slots);
       }
       __syncwarp();
     } else if (warp == 1) {
-      if (lane == 0) {
-        if constexpr (CG == 2) { if (cluster_ctarank() == 0) mma_role_pair(p, w, q_base, smem, c, tmem_base, desc_slots + kStreamSlots); }
-        else mma_role(p, w, q_base, smem, c, tmem_base, desc_slots + kStreamSlots);
-      }
+      if constexpr (CG == 2) { if (cluster_ctarank() == 0) mma_role_pair(p, w, q_base, smem, c, tmem_base, desc_slots + kStreamSlots); }
+      else mma_role(p, w, q_base, smem, c, tmem_base, desc_slots + kStreamSlots);
       __syncwarp();
     } else {
       general_role<CG>(p, w, q_base, c, tmem_base, extra, reinterpret_cast<uint8_t*>(extra) + kMkExtraSmem, smem, bulk_bars, attn_bars,

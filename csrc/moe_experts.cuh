@@ -55,12 +55,13 @@ struct ExpertTiles {
   }
 };
 
-// ---- TMA thread -------------------------------------------------------------------------------
+// ---- TMA warp (converged) ----------------------------------------------------------------------
 template <int STAGES, typename Program, typename WaitFn>
 __device__ __noinline__ bool experts_produce(const Program& p, const MacoExpertArgs& args, int share, uint16_t* table, uint8_t* smem, const GemmCtrl& c,
                                              const CUtensorMap* tmaps, uint32_t& it, WaitFn wait) {
   const MacoExpertArgs a = args;
-  expert_blocks(table, a, 0, 1);
+  expert_blocks(table, a, threadIdx.x & 31, 32);
+  __syncwarp();
   ExpertTiles tiles(a, table, share);
   const uint32_t gate_done = 4u * (uint32_t)tiles.tiles[0];
   while (tiles.next()) {
@@ -75,10 +76,12 @@ __device__ __noinline__ bool experts_produce(const Program& p, const MacoExpertA
       uint32_t ahead = 0;
       const int n0 = el * a.hidden + tiles.nb * 256;
       const uint32_t* ready = a.ready + tiles.slab * (a.capacity / kBM) + tiles.mb;
-      if (ld_acquire_gpu_u32(ready) < gate_done) {
+      // (one lane looks, for all)
+      if (warp_uniform((threadIdx.x & 31) == 0 ? ld_acquire_gpu_u32(ready) : 0u) < gate_done) {
         ok = gemm_produce_b_ahead<256, STAGES>(smem, c, tmaps + a.tmap_w2, n0, 0, a.inter / kBK, it, p.budget_ns, -1, ahead);
         if (!ok || !wait(ready, gate_done)) { it += ahead; return false; }
       }
+      __syncwarp();
       fence_proxy_async_all();
       ok = gemm_produce_tile<256, STAGES, false, false>(smem, c, tmaps + a.tmap_act, tmaps + a.tmap_w2, m0, n0, 0, a.inter / kBK, it, p.budget_ns,
                                                         nullptr, kBK, -1, ahead);
@@ -88,12 +91,13 @@ __device__ __noinline__ bool experts_produce(const Program& p, const MacoExpertA
   return true;
 }
 
-// ---- MMA thread -------------------------------------------------------------------------------
+// ---- MMA warp (converged) ----------------------------------------------------------------------
 template <int STAGES, typename Program>
 __device__ __noinline__ bool experts_mma(const Program& p, const MacoExpertArgs& args, int share, uint16_t* table, uint8_t* smem, const GemmCtrl& c,
                                          uint32_t tmem_base, uint32_t& it, uint32_t& seq) {
   const MacoExpertArgs a = args;
-  expert_blocks(table, a, 0, 1);
+  expert_blocks(table, a, threadIdx.x & 31, 32);
+  __syncwarp();
   ExpertTiles tiles(a, table, share);
   while (tiles.next()) {
     if (!gemm_mma_tile<256, STAGES, false, false>(smem, c, tmem_base, a.idesc, (tiles.phase == 0 ? a.hidden : a.inter) / kBK, it, seq, p.budget_ns))
