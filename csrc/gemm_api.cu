@@ -24,7 +24,7 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmEpilog
   int dev = 0;
   MACO_CHECK_CUDA(cudaGetDevice(&dev));
   if (!attr_set[dev]) {
-    MACO_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotalBytes));
+    MACO_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotalBytes + kEpiBlockBytes));
     attr_set[dev] = true;
   }
   const int m_tiles = (epi.M + kBM - 1) / kBM, n_tiles = (epi.N + BN - 1) / BN;
@@ -34,7 +34,7 @@ int launch_gemm(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmEpilog
   if (grid > sms) grid = sms;
   if (grid <= 0) return 0;
   uint32_t* status = maco_host::status_device_ptr();
-  kern<<<grid, kGemmThreads, L::kTotalBytes, stream>>>(tmA, tmB, epi, K, idesc, budget_ns, status, g_gemm_dbg);
+  kern<<<grid, kGemmThreads, L::kTotalBytes + kEpiBlockBytes, stream>>>(tmA, tmB, epi, K, idesc, budget_ns, status, g_gemm_dbg);
   MACO_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
@@ -62,7 +62,7 @@ int launch_gemm_tf32(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmE
   int dev = 0;
   MACO_CHECK_CUDA(cudaGetDevice(&dev));
   if (!attr_set[dev]) {
-    MACO_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotalBytes));
+    MACO_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotalBytes + kEpiBlockBytes));
     attr_set[dev] = true;
   }
   int grid = ((epi.M + kBM - 1) / kBM) * ((epi.N + 255) / 256);
@@ -70,7 +70,7 @@ int launch_gemm_tf32(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmE
   if (max_ctas > 0 && max_ctas < sms) sms = max_ctas;
   if (grid > sms) grid = sms;
   if (grid <= 0) return 0;
-  kern<<<grid, kGemmThreads, L::kTotalBytes, stream>>>(tmA, tmB, epi, K, idesc, budget_ns, maco_host::status_device_ptr(), g_gemm_dbg);
+  kern<<<grid, kGemmThreads, L::kTotalBytes + kEpiBlockBytes, stream>>>(tmA, tmB, epi, K, idesc, budget_ns, maco_host::status_device_ptr(), g_gemm_dbg);
   MACO_CHECK_CUDA(cudaGetLastError());
   return 0;
 }
@@ -85,7 +85,7 @@ int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmE
   int dev = 0;
   MACO_CHECK_CUDA(cudaGetDevice(&dev));
   if (!attr_set[dev]) {
-    MACO_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotalBytes));
+    MACO_CHECK_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::kTotalBytes + kEpiBlockBytes));
     attr_set[dev] = true;
   }
   const int m_pairs = (epi.M + 2 * kBM - 1) / (2 * kBM), n_tiles = (epi.N + BN - 1) / BN;
@@ -95,7 +95,7 @@ int launch_gemm_pair(const CUtensorMap& tmA, const CUtensorMap& tmB, const GemmE
   if (pairs > sms / 2) pairs = sms / 2;
   if (pairs <= 0) return 0;
   uint32_t* status = maco_host::status_device_ptr();
-  kern<<<2 * pairs, kGemmThreads, L::kTotalBytes, stream>>>(tmA, tmB, epi, K, idesc, budget_ns, status, g_gemm_dbg);
+  kern<<<2 * pairs, kGemmThreads, L::kTotalBytes + kEpiBlockBytes, stream>>>(tmA, tmB, epi, K, idesc, budget_ns, status, g_gemm_dbg);
   MACO_CHECK_CUDA(cudaGetLastError());
   return 0;
 }

@@ -359,14 +359,13 @@ struct EpiBroadcast {
   unsigned long long off;
 };
 
-// The common tiles of the persistent kernel: whole columns into this GPU's memory and no bias (plain 16-bit or fp32 store, SwiGLU,
+// The common tiles of the persistent kernel: whole columns into this GPU's memory and no bias (plain 16-bit store, SwiGLU,
 // rows scattered by record). Same arithmetic as gemm_epilogue_tile below without its other modes around it, which cost a few
 // hundred bytes of spills per thread and tile with a 28 KB L1 to hold them: the entry function goes from 636 / 1284 bytes
 // stored / loaded to 308 / 404 with this form inlined and the general one behind a call.
 MACO_DEVICE bool epi_is_lean(const GemmEpilogue& e, int n0, int bn) {
   const bool plain = e.mode == MACO_EPI_STORE || e.mode == MACO_EPI_F32_STORE;
-  const bool half = e.out_type != MACO_DT_F32;
-  return e.bias == nullptr && n0 + bn <= e.N && (plain || (half && (e.mode == MACO_EPI_SWIGLU || e.mode == MACO_EPI_SCATTER_ROWS)));
+  return e.out_type != MACO_DT_F32 && e.bias == nullptr && n0 + bn <= e.N && (plain || e.mode == MACO_EPI_SWIGLU || e.mode == MACO_EPI_SCATTER_ROWS);
 }
 template <int SBN>
 MACO_DEVICE bool gemm_epilogue_lean(int bn, const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e, void* out_base, long long row_off,
@@ -389,7 +388,7 @@ MACO_DEVICE bool gemm_epilogue_lean(int bn, const GemmCtrl& c, uint32_t tmem_bas
     row_weight = __int_as_float(rec.z);
   }
   const float alpha = e.alpha;
-  uint8_t* dst = reinterpret_cast<uint8_t*>(out_base) + (out_row * e.ld_out + (swiglu ? n0 / 2 : n0)) * (dt == MACO_DT_F32 ? 4 : 2);
+  uint8_t* dst = reinterpret_cast<uint8_t*>(out_base) + (out_row * e.ld_out + (swiglu ? n0 / 2 : n0)) * 2;
   const uint32_t t_row = tmem_base + ((q * 32u) << 16) + acc * SBN;
   const int cols = swiglu ? bn / 2 : bn;
 #pragma unroll 1
@@ -407,30 +406,135 @@ MACO_DEVICE bool gemm_epilogue_lean(int bn, const GemmCtrl& c, uint32_t tmem_bas
 #pragma unroll
       for (int j = 0; j < 32; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
     }
-    if (dt == MACO_DT_F32) {
-      if (row_ok) {
+    uint32_t w[16];
 #pragma unroll
-        for (int j = 0; j < 32; j += 4) reinterpret_cast<uint4*>(dst)[j >> 2] = make_uint4(r[j], r[j + 1], r[j + 2], r[j + 3]);
+    for (int j = 0; j < 16; ++j) w[j] = epi_pack(dt, __uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+    if (scatter) {
+      // the expert's output row is rounded to the output type first (what a separate return pass would read)
+#pragma unroll
+      for (int j = 0; j < 16; ++j) {
+        const float2 f = dt == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[j])) : unpack_bf16x2(w[j]);
+        w[j] = epi_pack(dt, f.x * row_weight, f.y * row_weight);
       }
-      dst += 128;
-    } else {
-      uint32_t w[16];
-#pragma unroll
-      for (int j = 0; j < 16; ++j) w[j] = epi_pack(dt, __uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-      if (scatter) {
-        // the expert's output row is rounded to the output type first (what a separate return pass would read)
-#pragma unroll
-        for (int j = 0; j < 16; ++j) {
-          const float2 f = dt == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[j])) : unpack_bf16x2(w[j]);
-          w[j] = epi_pack(dt, f.x * row_weight, f.y * row_weight);
-        }
-      }
-      if (row_ok) {
-#pragma unroll
-        for (int j = 0; j < 16; j += 4) reinterpret_cast<uint4*>(dst)[j >> 2] = make_uint4(w[j], w[j + 1], w[j + 2], w[j + 3]);
-      }
-      dst += 64;
     }
+    if (row_ok) {
+#pragma unroll
+      for (int j = 0; j < 16; j += 4) reinterpret_cast<uint4*>(dst)[j >> 2] = make_uint4(w[j], w[j + 1], w[j + 2], w[j + 3]);
+    }
+    dst += 64;
+    __syncwarp();
+  }
+  tc_fence_before();
+  if (pair_empty_bar == 0) {
+    mbar_arrive(&c.tmem_empty[acc]);
+  } else {
+    __syncwarp();
+    if (lane == 0) mbar_arrive_cluster(pair_empty_bar + acc * 8);
+  }
+  return true;
+}
+
+// Rows of a warp's 32 accumulator rows on their way to global memory. A thread holds one row (its TMEM lane), so a vector store straight
+// from its registers touches 32 lines with half a sector each (L2 counted 3.3 sectors written per sector of output); through a block of
+// shared memory every instruction moves whole sectors of a few rows. PIECES 16-byte pieces a row (8 or 4), swizzled by the row: free of
+// bank conflicts in both directions. The block is the calling warp's own. `row_ptr(r)`: where row r of the 32 starts in this column
+// group, null for a row that does not exist.
+constexpr int kEpiRowsBytes = 4096;                    // 32 rows of 128 bytes
+constexpr int kEpiWarpBytes = 6144;                    // ... and of a warp in all: three blocks of 32 rows of 64 bytes (gemm_epilogue_beside)
+constexpr int kEpiBlockBytes = 4 * kEpiWarpBytes;
+template <int PIECES>
+MACO_DEVICE uint32_t epi_piece(uint32_t block, uint32_t row, uint32_t piece) {
+  return PIECES == 8 ? block + row * 128u + ((piece ^ (row & 7u)) << 4) : block + row * 64u + ((piece ^ ((row >> 1) & 3u)) << 4);
+}
+MACO_DEVICE void epi_sts(uint32_t saddr, uint4 v) {
+  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" :: "r"(saddr), "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w) : "memory");
+}
+MACO_DEVICE uint4 epi_lds(uint32_t saddr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(saddr) : "memory");
+  return v;
+}
+// Block to global memory; a barrier of the warp in front and behind.
+template <int PIECES, typename RowFn>
+MACO_DEVICE void epi_flush_rows(uint32_t block, uint32_t lane, RowFn row_ptr) {
+  __syncwarp();
+#pragma unroll 4
+  for (uint32_t i = 0; i < PIECES; ++i) {
+    const uint32_t r = i * (32 / PIECES) + lane / PIECES;
+    const uint4 v = epi_lds(epi_piece<PIECES>(block, r, lane % PIECES));
+    uint8_t* dst = row_ptr(r);
+    if (dst != nullptr) reinterpret_cast<uint4*>(dst)[lane % PIECES] = v;
+  }
+  __syncwarp();
+}
+MACO_DEVICE float2 epi_unpack(int type, uint32_t w) { return type == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w)) : unpack_bf16x2(w); }
+
+// Whole columns into this GPU's memory: fp32 rows, and 16-bit ones with a bias, GELU or SiLU. Same arithmetic as gemm_epilogue_tile below,
+// in steps of 16 columns so that nothing lives in local memory: the persistent kernel leaves its L1 28 KB, a spilled value of the
+// column loop is a miss to L2 two times in three, and one warp per scheduler has nothing to cover it with (32 columns at a time,
+// with GELU: 20 local loads per 32 columns). fp32 rows go through `block`; 16-bit rows do not (a short chain per step counts for more there: through
+// the block, products of K = 256 without a term took 79 us instead of 65). One B200, graph linears
+// with GELU, us, before / now: 2048 x 4096 x 4096 76 / 58, 4096 x 8192 x 1024 170 / 99, 8192 x 4096 x 256 159 / 90.
+MACO_DEVICE bool epi_is_stepped(const GemmEpilogue& e, int n0, int bn) {
+  if (n0 + bn > e.N) return false;
+  const bool f32 = e.out_type == MACO_DT_F32, plain = e.mode == MACO_EPI_STORE || e.mode == MACO_EPI_F32_STORE;
+  return f32 ? plain : (e.mode == MACO_EPI_GELU || e.mode == MACO_EPI_SILU || (plain && e.bias != nullptr));
+}
+template <int SBN>
+MACO_DEVICE bool gemm_epilogue_stepped(int bn, const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e, void* out_base, long long row_off,
+                                       int m0, int n0, uint32_t tile_seq, uint64_t budget_ns, uint32_t pair_empty_bar, uint8_t* block) {
+  const uint32_t q = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  const uint32_t acc = tile_seq & 1;
+  uint32_t ok = 1;
+  if (lane == 0) ok = mbar_wait(&c.tmem_full[acc], (tile_seq >> 1) & 1, budget_ns, c.abort_word) ? 1u : 0u;
+  ok = __shfl_sync(0xffffffffu, ok, 0);
+  if (!ok) return false;
+  tc_fence_after();
+  const int row0 = m0 + (int)(q * 32), dt = e.out_type, mode = e.mode;
+  const bool f32 = dt == MACO_DT_F32, bias = e.bias != nullptr;
+  const int rows = min(32, e.M - row0);                                // of this warp (may be <= 0)
+  const float alpha = e.alpha;
+  const long long pitch = e.ld_out * (f32 ? 4 : 2);
+  uint8_t* dst = reinterpret_cast<uint8_t*>(out_base) + (row0 + row_off + (f32 ? 0 : (int)lane)) * pitch + (long long)n0 * (f32 ? 4 : 2);
+  const uint32_t t_row = tmem_base + ((q * 32u) << 16) + acc * SBN;
+  const uint32_t mine = smem_u32(block) + q * kEpiWarpBytes;
+#pragma unroll 1
+  for (int col = rows > 0 ? 0 : bn; col < bn; col += 16) {
+    uint32_t r[16];
+    tmem_ld_32x16(t_row + col, r);
+    tmem_ld_wait();
+#pragma unroll
+    for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) * alpha);
+    if (bias) {
+      const float b = epi_bias(e, n0 + col + (int)(lane & 15));
+#pragma unroll
+      for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(__uint_as_float(r[j]) + __shfl_sync(0xffffffffu, b, j));
+    }
+    if (f32) {
+#pragma unroll
+      for (uint32_t j = 0; j < 4; ++j)
+        epi_sts(epi_piece<8>(mine, lane, (col & 16) / 4 + j), make_uint4(r[4 * j], r[4 * j + 1], r[4 * j + 2], r[4 * j + 3]));
+      if (col & 16) {
+        epi_flush_rows<8>(mine, lane, [&](uint32_t k) -> uint8_t* { return (int)k < rows ? dst + k * pitch : nullptr; });
+        dst += 128;
+      }
+      continue;
+    }
+    if (mode == MACO_EPI_GELU) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(gelu_tanh(__uint_as_float(r[j])));
+    } else if (mode == MACO_EPI_SILU) {
+#pragma unroll
+      for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(silu_16(__uint_as_float(r[j])));
+    }
+    uint32_t w[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) w[j] = epi_pack(dt, __uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+    if ((int)lane < rows) {
+      reinterpret_cast<uint4*>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+      reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
+    }
+    dst += 32;
     __syncwarp();
   }
   tc_fence_before();
@@ -444,10 +548,10 @@ MACO_DEVICE bool gemm_epilogue_lean(int bn, const GemmCtrl& c, uint32_t tmem_bas
 }
 
 // Tiles with a second tensor beside the result, 16-bit, whole columns, no bias, 16-byte rows: the result times gelu'(aux)
-// (MACO_EPI_GELU_BWD), the result and its GELU (MACO_EPI_GELU_DUAL), the result and its sum with aux (MACO_EPI_RESIDUAL_DUAL). A tile of 64 k-blocks leaves the tensor cores after about 24 us; in
-// the general epilogue, whose element type and operator are asked for per element, its 32,768 derivatives took 50 us and the
-// backward pass of 8192 x 4096 layers ran at that rate. Here the operator is one branch per chunk of 32 columns and the
-// aux values of the next chunk are on their way while this one is computed.
+// (MACO_EPI_GELU_BWD), the result and its GELU (MACO_EPI_GELU_DUAL), the result and its sum with aux (MACO_EPI_RESIDUAL_DUAL). In
+// steps of 16 columns as above; aux comes in by cp.async, whole sectors of eight rows an instruction, up to three groups of 32 columns ahead
+// without a register held for it. One B200, us, before (32 columns at a time, aux in registers, the operators in one function with 12 local loads per step)
+// / now: linear + add of 8192 x 4096 x 256 180 / 110, 2048 x 4096 x 4096 84 / 66; training stack of four 4096 x 4096 layers 2788 / 2595.
 MACO_DEVICE bool epi_is_dual(const GemmEpilogue& e) { return e.mode == MACO_EPI_GELU_DUAL || e.mode == MACO_EPI_RESIDUAL_DUAL; }
 MACO_DEVICE bool epi_is_beside(const GemmEpilogue& e, int n0, int bn) {
   const bool res = e.mode == MACO_EPI_RESIDUAL_DUAL;
@@ -455,70 +559,92 @@ MACO_DEVICE bool epi_is_beside(const GemmEpilogue& e, int n0, int bn) {
   return (e.mode == MACO_EPI_GELU_BWD || e.mode == MACO_EPI_GELU_DUAL || res) && (res || e.bias == nullptr) && n0 + bn <= e.N &&
          e.out_type != MACO_DT_F32 && (p & 15) == 0;
 }
-template <int SBN>
-__device__ __noinline__ bool gemm_epilogue_beside(int bn, const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e_in, void* out_base,
+template <int SBN, int MODE>
+__device__ __noinline__ bool gemm_epilogue_beside_as(int bn, const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e_in, void* out_base,
                                                 long long row_off, int m0, int n0, uint32_t tile_seq, uint64_t budget_ns,
-                                                uint32_t pair_empty_bar) {
+                                                uint32_t pair_empty_bar, uint8_t* block) {
   const uint32_t q = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31, acc = tile_seq & 1;
-  const int row = m0 + (int)(q * 32 + lane), dt = e_in.out_type, at = e_in.aux_type;
-  const bool row_ok = row < e_in.M, dual = e_in.mode == MACO_EPI_GELU_DUAL, res = e_in.mode == MACO_EPI_RESIDUAL_DUAL;
+  const int row0 = m0 + (int)(q * 32), dt = e_in.out_type, at = e_in.aux_type;
+  const int rows = min(32, e_in.M - row0);                             // of this warp (may be <= 0)
+  constexpr bool dual = MODE == MACO_EPI_GELU_DUAL, res = MODE == MACO_EPI_RESIDUAL_DUAL;
   const float alpha = e_in.alpha;
-  uint16_t* dst = reinterpret_cast<uint16_t*>(out_base) + (row + row_off) * e_in.ld_out + n0;
-  uint16_t* aux = reinterpret_cast<uint16_t*>(const_cast<void*>(e_in.aux)) + (long long)row * e_in.ld_aux + n0;
-  uint16_t* second = dual ? aux : reinterpret_cast<uint16_t*>(const_cast<void*>(e_in.bias)) + (row + row_off) * e_in.ld_out + n0;
-  uint4 ax[4];
-  auto fetch = [&](int col) {
-    if (row_ok && !dual) {
+  const long long pitch = e_in.ld_out * 2, aux_pitch = e_in.ld_aux * 2;
+  uint8_t* dst = reinterpret_cast<uint8_t*>(out_base) + (row0 + row_off + (int)lane) * pitch + n0 * 2;
+  uint8_t* aux = reinterpret_cast<uint8_t*>(const_cast<void*>(e_in.aux)) + (long long)row0 * aux_pitch + n0 * 2;
+  uint8_t* second = dual ? aux + lane * aux_pitch : reinterpret_cast<uint8_t*>(const_cast<void*>(e_in.bias)) + (row0 + row_off + (int)lane) * pitch + n0 * 2;
+  const uint32_t mine = smem_u32(block) + q * kEpiWarpBytes;
+  uint32_t in = 0;                                     // which of the three 2 KB blocks is filled next
+  int fetched = dual ? bn : 0;
+  auto fetch = [&] {                                   // 32 columns of aux, and always a group for the waits to count
+    if (fetched < bn) {
 #pragma unroll
-      for (int i = 0; i < 4; ++i) ax[i] = reinterpret_cast<const uint4*>(aux + col)[i];
+      for (uint32_t i = 0; i < 4; ++i) {
+        const uint32_t r = i * 8 + (lane >> 2);
+        if ((int)r < rows) cp_async16(epi_piece<4>(mine + in, r, lane & 3), aux + r * aux_pitch + fetched * 2 + (lane & 3) * 16);
+      }
+      fetched += 32;
+      in = in + 2048u == kEpiWarpBytes ? 0u : in + 2048u;
     }
+    cp_async_commit();
   };
-#pragma unroll
-  for (int i = 0; i < 4; ++i) ax[i] = make_uint4(0, 0, 0, 0);
   uint32_t ok = 1;
   if (lane == 0) ok = mbar_wait(&c.tmem_full[acc], (tile_seq >> 1) & 1, budget_ns, c.abort_word) ? 1u : 0u;
   ok = __shfl_sync(0xffffffffu, ok, 0);
   if (!ok) return false;
   tc_fence_after();
-  fetch(0);                                            // (behind the accumulator's barrier: what the tile depends on has happened)
+  fetch();                                             // (behind the accumulator's barrier: what the tile depends on has happened)
+  fetch();
+  fetch();
   const uint32_t t_row = tmem_base + ((q * 32u) << 16) + acc * SBN;
+  uint32_t cur = mine;
 #pragma unroll 1
-  for (int col = 0; col < bn; col += 32) {
-    uint32_t r[32], w[16], g[16];
-    tmem_ld_32x32(t_row + col, r);
+  for (int col = rows > 0 ? 0 : bn; col < bn;) {
+    cp_async_wait<2>();
+    __syncwarp();
+#pragma unroll 1
+    for (uint32_t piece = 0; piece < 4; piece += 2, col += 16) {
+      uint32_t r[16], w[8], g[8];
+      tmem_ld_32x16(t_row + col, r);
+      if (!dual) {
+        const uint4 a = epi_lds(epi_piece<4>(cur, lane, piece)), b = epi_lds(epi_piece<4>(cur, lane, piece + 1));
+        g[0] = a.x; g[1] = a.y; g[2] = a.z; g[3] = a.w; g[4] = b.x; g[5] = b.y; g[6] = b.z; g[7] = b.w;
+      }
+      tmem_ld_wait();
+      if (dual || res) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) { g[4 * i] = ax[i].x; g[4 * i + 1] = ax[i].y; g[4 * i + 2] = ax[i].z; g[4 * i + 3] = ax[i].w; }
-    if (col + 32 < bn) fetch(col + 32);
-    tmem_ld_wait();
-    if (dual || res) {
+        for (int j = 0; j < 8; ++j) {
+          w[j] = epi_pack(dt, __uint_as_float(r[2 * j]) * alpha, __uint_as_float(r[2 * j + 1]) * alpha);
+          const float2 z = epi_unpack(dt, w[j]);
+          if (dual) {
+            g[j] = epi_pack(at, gelu_tanh(z.x), gelu_tanh(z.y));
+          } else {
+            const float2 x = epi_unpack(at, g[j]);
+            g[j] = epi_pack(dt, z.x + x.x, z.y + x.y);
+          }
+        }
+        if ((int)lane < rows) {
+          reinterpret_cast<uint4*>(second)[0] = make_uint4(g[0], g[1], g[2], g[3]);
+          reinterpret_cast<uint4*>(second)[1] = make_uint4(g[4], g[5], g[6], g[7]);
+        }
+        second += 32;
+      } else {
 #pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        w[j] = epi_pack(dt, __uint_as_float(r[2 * j]) * alpha, __uint_as_float(r[2 * j + 1]) * alpha);
-        const float2 z = dt == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[j])) : unpack_bf16x2(w[j]);
-        if (dual) {
-          g[j] = epi_pack(at, gelu_tanh(z.x), gelu_tanh(z.y));
-        } else {
-          const float2 x = at == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&g[j])) : unpack_bf16x2(g[j]);
-          g[j] = epi_pack(dt, z.x + x.x, z.y + x.y);
+        for (int j = 0; j < 8; ++j) {
+          const float2 z = epi_unpack(at, g[j]);
+          w[j] = epi_pack(dt, __uint_as_float(r[2 * j]) * alpha * gelu_tanh_grad(z.x), __uint_as_float(r[2 * j + 1]) * alpha * gelu_tanh_grad(z.y));
         }
       }
-      if (row_ok) {
-#pragma unroll
-        for (int j = 0; j < 16; j += 4) reinterpret_cast<uint4*>(second + col)[j >> 2] = make_uint4(g[j], g[j + 1], g[j + 2], g[j + 3]);
+      if ((int)lane < rows) {
+        reinterpret_cast<uint4*>(dst)[0] = make_uint4(w[0], w[1], w[2], w[3]);
+        reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
       }
-    } else {
-#pragma unroll
-      for (int j = 0; j < 16; ++j) {
-        const float2 z = at == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&g[j])) : unpack_bf16x2(g[j]);
-        w[j] = epi_pack(dt, __uint_as_float(r[2 * j]) * alpha * gelu_tanh_grad(z.x), __uint_as_float(r[2 * j + 1]) * alpha * gelu_tanh_grad(z.y));
-      }
+      dst += 32;
     }
-    if (row_ok) {
-#pragma unroll
-      for (int j = 0; j < 16; j += 4) reinterpret_cast<uint4*>(dst + col)[j >> 2] = make_uint4(w[j], w[j + 1], w[j + 2], w[j + 3]);
-    }
-    __syncwarp();
+    __syncwarp();                                      // every lane has read its row of the block that is filled next
+    cur = cur + 2048u == mine + kEpiWarpBytes ? mine : cur + 2048u;
+    fetch();
   }
+  cp_async_wait<0>();
   tc_fence_before();
   if (pair_empty_bar == 0) {
     mbar_arrive(&c.tmem_empty[acc]);
@@ -527,6 +653,17 @@ __device__ __noinline__ bool gemm_epilogue_beside(int bn, const GemmCtrl& c, uin
     if (lane == 0) mbar_arrive_cluster(pair_empty_bar + acc * 8);
   }
   return true;
+}
+
+// (a function per operator: together they keep more values than a callee of the persistent kernel has registers for)
+template <int SBN>
+MACO_DEVICE bool gemm_epilogue_beside(int bn, const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e, void* out_base, long long row_off,
+                                      int m0, int n0, uint32_t tile_seq, uint64_t budget_ns, uint32_t pair_empty_bar, uint8_t* block) {
+  if (e.mode == MACO_EPI_GELU_BWD)
+    return gemm_epilogue_beside_as<SBN, MACO_EPI_GELU_BWD>(bn, c, tmem_base, e, out_base, row_off, m0, n0, tile_seq, budget_ns, pair_empty_bar, block);
+  if (e.mode == MACO_EPI_GELU_DUAL)
+    return gemm_epilogue_beside_as<SBN, MACO_EPI_GELU_DUAL>(bn, c, tmem_base, e, out_base, row_off, m0, n0, tile_seq, budget_ns, pair_empty_bar, block);
+  return gemm_epilogue_beside_as<SBN, MACO_EPI_RESIDUAL_DUAL>(bn, c, tmem_base, e, out_base, row_off, m0, n0, tile_seq, budget_ns, pair_empty_bar, block);
 }
 
 // (DUAL: with the two modes that write a second tensor, for tiles of such a product that are ragged or not aligned)
@@ -936,6 +1073,7 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
   const int pair = blockIdx.x >> 1, num_pairs = gridDim.x >> 1;
   const uint32_t warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
   const uint32_t tempty_leader = mapa_u32(smem_u32(&c.tmem_empty[0]), 0);
+  uint8_t* block = smem + PairSmemLayout<kPairStages>::kRingBytes + PairSmemLayout<kPairStages>::kCtrlBytes;
 
   if (warp == 0) {
     if (lane == 0) { tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); }
@@ -978,7 +1116,9 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         continue;
       }
       if (BESIDE && epi_is_beside(epi, nb * BN, BN))
-        ok = gemm_epilogue_beside<256>(BN, c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns, tempty_leader);
+        ok = gemm_epilogue_beside<256>(BN, c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns, tempty_leader, block);
+      else if (!BESIDE && epi_is_stepped(epi, nb * BN, BN))
+        ok = gemm_epilogue_stepped<256>(BN, c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns, tempty_leader, block);
       else
         ok = gemm_epilogue_tile<BN, 256, BESIDE>(c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns,
                                                  nullptr, nullptr, tempty_leader);
@@ -1006,6 +1146,7 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
   constexpr int kStepElems = TF32 ? kBK / 2 : kBK;
   const int k_blocks = (K + kStepElems - 1) / kStepElems;
   const uint32_t warp = warp_uniform(threadIdx.x >> 5), lane = threadIdx.x & 31;
+  uint8_t* block = smem + GemmSmemLayout<BN, STAGES>::kRingBytes + GemmSmemLayout<BN, STAGES>::kCtrlBytes;
 
   if (warp == 0) {
     if (lane == 0) { tma_prefetch_desc(&tmA); tma_prefetch_desc(&tmB); }
@@ -1044,7 +1185,9 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         continue;
       }
       if (BESIDE && epi_is_beside(epi, nb * BN, BN))
-        ok = gemm_epilogue_beside<BN>(BN, c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns, 0);
+        ok = gemm_epilogue_beside<BN>(BN, c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns, 0, block);
+      else if (!BESIDE && epi_is_stepped(epi, nb * BN, BN))
+        ok = gemm_epilogue_stepped<BN>(BN, c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns, 0, block);
       else
         ok = gemm_epilogue_tile<BN, BN, BESIDE>(c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns);
     }

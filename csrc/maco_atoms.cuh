@@ -207,6 +207,12 @@ MACO_DEVICE bool mbar_wait_warp(uint64_t* bar, uint32_t parity, uint64_t budget_
   return true;
 }
 
+MACO_DEVICE void cp_async16(uint32_t sdst, const void* gsrc) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" :: "r"(sdst), "l"(gsrc) : "memory");
+}
+MACO_DEVICE void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> MACO_DEVICE void cp_async_wait() { asm volatile("cp.async.wait_group %0;" :: "n"(N) : "memory"); }
+
 // ---------------------------------------------------------------------------------------------
 // TMA (tile mode, no cluster qualifier: every CTA fetches its own tiles)
 // ---------------------------------------------------------------------------------------------

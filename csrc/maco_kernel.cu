@@ -56,6 +56,7 @@ static_assert(kFewWBytes + 64 * kFewK * 2 <= (uint32_t)MkLayout::kStageBytes, "a
 constexpr int kExpertOffset = kStreamOffset + 3 * kStreamSlots * sizeof(MacoTaskDesc);   // ... of the expert tables, one per role
 static_assert(kExpertOffset + 3 * kMaxSlabs * 2 <= kMkExtraSmem, "descriptor slots and expert tables");
 static_assert(kMkScratchSmem >= (int)kRowScratch, "staged row tasks must fit the scratch block");
+static_assert(kMkScratchSmem >= kEpiBlockBytes, "epilogue rows must fit the scratch block");
 static_assert(kMkScratchSmem >= kEpiStageBytes, "epilogue staging must fit the scratch block");
 static_assert(kMkScratchSmem >= kAttnScratchBytes && kMkScratchSmem >= kAttnTcScratchBytes, "attention scratch must fit the scratch block");
 static_assert(kMkSmemBytes <= 227 * 1024, "persistent kernel exceeds the shared memory of an SM");
@@ -577,6 +578,12 @@ __device__ __noinline__ bool run_epilogue(const GemmCtrl& c, uint32_t tmem_base,
   return gemm_epilogue_tile<256, kMkBN, DUAL>(c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, budget_ns, bc, stage, pair_empty_bar, row_limit);
 }
 
+__device__ __noinline__ bool run_epilogue_stepped(const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e_in, void* out_base, const MacoGemmArgs& g,
+                                                  uint32_t seq, uint64_t budget_ns, uint32_t pair_empty_bar, uint8_t* block) {
+  const GemmEpilogue e = e_in;           // private copy: the stores of the tile could alias the record
+  return gemm_epilogue_stepped<kMkBN>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, budget_ns, pair_empty_bar, block);
+}
+
 // Every task that is not a GEMM tile, behind one call: values of the task loop that live across a call cost a spill for each of
 // its sites, and they are paid for inside the GEMM epilogue (entry function 920 / 2144 bytes stored / loaded with the six calls
 // in the loop, 636 / 1284 with this one and the few-row epilogue out of line).
@@ -688,9 +695,11 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
       // run-time row count of a counted tile's operand block (rows at or beyond it hold no tokens)
       const int row_limit = (d.flags & MACO_TF_COUNTED) ? (int)ld_relaxed_gpu_u32(g.count_ptr) : 0x7fffffff;
       if (g.peer == -1 && epi_is_beside(e, g.n0, (int)g.bn))
-        ok = gemm_epilogue_beside<kMkBN>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, pair_empty_bar);
+        ok = gemm_epilogue_beside<kMkBN>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, pair_empty_bar, scratch_smem);
       else if (g.peer == -1 && epi_is_lean(e, g.n0, (int)g.bn))
         ok = gemm_epilogue_lean<kMkBN>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, pair_empty_bar, row_limit);
+      else if (g.peer == -1 && epi_is_stepped(e, g.n0, (int)g.bn))
+        ok = run_epilogue_stepped(c, tmem_base, e, out_base, g, seq, p.budget_ns, pair_empty_bar, scratch_smem);
       else if (epi_is_dual(e))
         ok = run_epilogue<true>(c, tmem_base, e, out_base, g, seq, p.budget_ns, bcp, stage, pair_empty_bar, row_limit);
       else

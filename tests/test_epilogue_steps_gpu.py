@@ -1,0 +1,69 @@
+"""GEMM epilogues that walk over a tile in steps of 16 columns: ragged last rows, both tile widths and forms, every operator, stand-alone and
+in a graph, against fp64."""
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+F = torch.nn.functional
+
+
+def _operands(M, N, K, dtype, seed):
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    x = torch.randn(M, K, device="cuda", generator=g).to(dtype)
+    w = (torch.randn(N, K, device="cuda", generator=g) * K ** -0.5).to(dtype)
+    return x, w, g, x.double() @ w.double().t()
+
+
+def _close(got, want, dtype, slack=0.0):
+    # one rounding to the output type, and a fast exponential or sums of K products in fp32 (a few 2^-20) in front of it
+    eps = {torch.bfloat16: 2.0 ** -8, torch.float16: 2.0 ** -10, torch.float32: 2.0 ** -18}[dtype]
+    assert ((got.double() - want).abs() <= eps * want.abs() + 2.0 ** -16 + slack).all()
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M", [1, 32, 97, 129, 300])
+@pytest.mark.parametrize("bn", [128, 256])
+@pytest.mark.parametrize("pair", [False, True])
+def test_standalone(dtype, M, bn, pair):
+    from maco_b200 import ops
+    N, K = 512, 192
+    x, w, g, z = _operands(M, N, K, dtype, M)
+    bias = torch.randn(N, device="cuda", generator=g)
+    kw = dict(bn=bn, cta_pair=pair)
+    _close(ops.gemm(x, w, bias=bias, **kw), z + bias.double(), dtype)
+    _close(ops.gemm(x, w, bias=bias.to(dtype), epilogue="gelu", **kw), F.gelu(z + bias.to(dtype).double(), approximate="tanh"), dtype)
+    _close(ops.gemm(x, w, epilogue="silu", **kw), F.silu(z), dtype)
+    _close(ops.gemm(x, w, epilogue="f32", **kw), z, torch.float32)
+    _close(ops.gemm(x, w, bias=bias, epilogue="f32", alpha=0.5, **kw), 0.5 * z + bias.double(), torch.float32)
+    aux = torch.randn(M, N, device="cuda", generator=g).to(dtype)
+    a = aux.double().requires_grad_(True)
+    F.gelu(a, approximate="tanh").sum().backward()
+    _close(ops.gemm(x, w, epilogue="gelu_bwd", aux=aux, **kw), z * a.grad, dtype, slack=2.0 ** -14)
+    act = torch.empty(M, N, device="cuda", dtype=dtype)
+    out = ops.gemm(x, w, epilogue="gelu_dual", aux=act, **kw)
+    _close(out, z, dtype)
+    _close(act, F.gelu(out.double(), approximate="tanh"), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("M,N", [(97, 1024), (300, 512), (1000, 4096), (2049, 2048)])
+def test_graph(dtype, M, N):
+    import maco_b200 as maco
+    x, w, g, z = _operands(M, N, 320, dtype, N)
+    bias = torch.randn(N, device="cuda", generator=g).to(dtype)
+    r = torch.randn(M, N, device="cuda", generator=g).to(dtype)
+    for bias_, act in ((bias, None), (None, "gelu"), (bias, "silu")):
+        graph = maco.TaskGraph()
+        y = graph.linear(x, w, bias=bias_, activation=act) if act else graph.linear(x, w, bias=bias_)
+        graph.compile()
+        graph.execute()
+        v = z if bias_ is None else z + bias_.double()
+        _close(y.output, F.gelu(v, approximate="tanh") if act == "gelu" else F.silu(v) if act == "silu" else v, dtype)
+    graph = maco.TaskGraph()
+    y = graph.linear(x, w)
+    s = graph.add(y.output, r)
+    graph.compile()
+    for _ in range(2):
+        graph.execute()
+    _close(y.output, z, dtype)
+    _close(s.output, y.output.double() + r.double(), dtype)
