@@ -737,7 +737,7 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
         }
       }
     } else if (CG == 1 && d.type == MACO_TASK_MOE_EXPERTS) {
-      const int r = experts_epilogue(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, expert_table(desc_slots, 2), tid, c, tmem_base, seq,
+      const int r = experts_epilogue(p, *reinterpret_cast<const MacoExpertArgs*>(d.u.elt.in2), d.u.elt.i0, expert_table(desc_slots, 2), tid, c, tmem_base, seq, scratch_smem,
                                      [] { general_bar(); });
       if (r < 0) cur[2] = 1;
       else seq += (uint32_t)r;

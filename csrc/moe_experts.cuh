@@ -111,12 +111,13 @@ __device__ __noinline__ bool experts_mma(const Program& p, const MacoExpertArgs&
 // Returns the number of tiles, or -1 after a wait that ran out.
 template <typename Program, typename BarFn>
 __device__ __noinline__ int experts_epilogue(const Program& p, const MacoExpertArgs& args, int share, uint16_t* table, int tid, const GemmCtrl& c,
-                                             uint32_t tmem_base, uint32_t seq0, BarFn bar) {
+                                             uint32_t tmem_base, uint32_t seq0, uint8_t* block, BarFn bar) {
   const MacoExpertArgs a = args;
   expert_blocks(table, a, tid, 128);
   bar();
   ExpertTiles tiles(a, table, share);
   const uint32_t q = (threadIdx.x >> 5) & 3, lane = threadIdx.x & 31;
+  const uint32_t mine = smem_u32(block) + q * kEpiWarpBytes;
   const int dt = a.dtype;
   uint32_t seq = seq0;
   while (tiles.next()) {
@@ -128,10 +129,14 @@ __device__ __noinline__ int experts_epilogue(const Program& p, const MacoExpertA
     const int rows = min((int)__ldcg(a.counts + tiles.slab), a.capacity);
     int4 rec = make_int4(0, 0, 0, 0);
     if (down) rec = reinterpret_cast<const int4*>(a.meta)[cell];        // (rows beyond the count hold old records, and are not written)
-    const bool row_ok = row < rows;
-    uint8_t* dst = down ? reinterpret_cast<uint8_t*>(a.comb) + (((long long)rec.x * a.top_k + rec.y) * a.hidden + tiles.nb * 256) * 2
-                        : reinterpret_cast<uint8_t*>(a.act) + (cell * a.inter + tiles.nb * 128) * 2;
+    const int valid = rows - (tiles.mb * kBM + (int)(q * 32));          // rows of this warp's 32 that hold a token (may be <= 0 or more)
+    uint8_t* dst = down ? reinterpret_cast<uint8_t*>(a.comb) + tiles.nb * 512
+                        : reinterpret_cast<uint8_t*>(a.act) + ((cell - lane) * a.inter + tiles.nb * 128) * 2;
+    const int out_row = down ? rec.x * a.top_k + rec.y : (int)lane, pitch = (down ? a.hidden : a.inter) * 2;
     const float weight = __int_as_float(rec.z);
+    // Rows leave in whole lines through shared memory where there are many of them (4096 tokens, 64 experts: 547 -> 515 us); a slab of less than
+    // one row block has few, and the way through the block is only longer (256 tokens, 32 experts: 102.5 instead of 100.8).
+    const bool lines = rows >= kBM;
     uint32_t ok = 1;
     if (lane == 0) ok = mbar_wait(&c.tmem_full[acc], (seq >> 1) & 1, p.budget_ns, c.abort_word) ? 1u : 0u;
     ok = __shfl_sync(0xffffffffu, ok, 0);
@@ -140,33 +145,44 @@ __device__ __noinline__ int experts_epilogue(const Program& p, const MacoExpertA
     const uint32_t t_row = tmem_base + ((q * 32u) << 16) + acc * 256;
     const int cols = down ? 256 : 128;
 #pragma unroll 1
-    for (int col = 0; col < cols; col += 16) {
-      uint32_t r[16], w[8];
-      tmem_ld_32x16(t_row + col, r);
-      if (!down) {
-        uint32_t u[16];
-        tmem_ld_32x16(t_row + 128 + col, u);
-        tmem_ld_wait();
+    for (int col = valid > 0 ? 0 : cols; col < cols; dst += 128) {      // (a warp without tokens has nothing to compute)
+#pragma unroll 1
+      for (uint32_t piece = 0; piece < 8; piece += 2, col += 16) {
+        uint32_t r[16], w[8];
+        tmem_ld_32x16(t_row + col, r);
+        if (!down) {
+          uint32_t u[16];
+          tmem_ld_32x16(t_row + 128 + col, u);
+          tmem_ld_wait();
 #pragma unroll
-        for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(silu_16(__uint_as_float(r[j])) * __uint_as_float(u[j]));
-      } else {
-        tmem_ld_wait();
-      }
+          for (int j = 0; j < 16; ++j) r[j] = __float_as_uint(silu_16(__uint_as_float(r[j])) * __uint_as_float(u[j]));
+        } else {
+          tmem_ld_wait();
+        }
 #pragma unroll
-      for (int j = 0; j < 8; ++j) w[j] = epi_pack(dt, __uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
-      if (down) {
-        // the expert's output row is rounded to the output type first (what a separate return pass would read)
+        for (int j = 0; j < 8; ++j) w[j] = epi_pack(dt, __uint_as_float(r[2 * j]), __uint_as_float(r[2 * j + 1]));
+        if (down) {
+          // the expert's output row is rounded to the output type first (what a separate return pass would read)
 #pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          const float2 f = dt == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w[j])) : unpack_bf16x2(w[j]);
-          w[j] = epi_pack(dt, f.x * weight, f.y * weight);
+          for (int j = 0; j < 8; ++j) {
+            const float2 f = epi_unpack(dt, w[j]);
+            w[j] = epi_pack(dt, f.x * weight, f.y * weight);
+          }
+        }
+        if (lines) {
+          epi_sts(epi_piece<8>(mine, lane, piece), make_uint4(w[0], w[1], w[2], w[3]));
+          epi_sts(epi_piece<8>(mine, lane, piece + 1), make_uint4(w[4], w[5], w[6], w[7]));
+        } else if ((int)lane < valid) {
+          uint4* to = reinterpret_cast<uint4*>(dst + (long long)out_row * pitch) + piece;
+          to[0] = make_uint4(w[0], w[1], w[2], w[3]);
+          to[1] = make_uint4(w[4], w[5], w[6], w[7]);
         }
       }
-      if (row_ok) {
-        reinterpret_cast<uint4*>(dst + col * 2)[0] = make_uint4(w[0], w[1], w[2], w[3]);
-        reinterpret_cast<uint4*>(dst + col * 2)[1] = make_uint4(w[4], w[5], w[6], w[7]);
-      }
-      __syncwarp();
+      if (lines)
+        epi_flush_rows<8>(mine, lane, [&](uint32_t r) -> uint8_t* {
+          const int o = __shfl_sync(0xffffffffu, out_row, r);
+          return (int)r < valid ? dst + (long long)o * pitch : nullptr;
+        });
     }
     tc_fence_before();
     mbar_arrive(&c.tmem_empty[acc]);
