@@ -12,6 +12,7 @@ import os
 import shutil
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -21,6 +22,8 @@ CSRC_DIR = REPO_DIR / "csrc"
 LIB_DIR = PKG_DIR / "_lib"
 LIB_PATH = LIB_DIR / "libmaco_b200.so"
 OBJ_DIR = REPO_DIR / "build" / "obj"
+FASTCALL_SRC = CSRC_DIR / "py" / "fastcall.c"
+FASTCALL_PATH = LIB_DIR / "maco_fastcall.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -67,6 +70,28 @@ def _compile_one(src: Path, verbose: bool) -> Path:
     return obj
 
 
+def build_fastcall() -> "Path | None":
+    """The C extension behind the smallest calls (csrc/py/fastcall.c), for this interpreter. None where there is no compiler or no Python
+    header: those calls then take their general path."""
+    include = sysconfig.get_paths()["include"]
+    cc = os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc")
+    if cc is None or not os.path.exists(os.path.join(include, "Python.h")):
+        return None
+    digest = hashlib.sha256(FASTCALL_SRC.read_bytes() + sys.version.encode()).hexdigest()
+    stamp = OBJ_DIR / "fastcall.sha"
+    if FASTCALL_PATH.exists() and stamp.exists() and stamp.read_text() == digest:
+        return FASTCALL_PATH
+    LIB_DIR.mkdir(parents=True, exist_ok=True)
+    OBJ_DIR.mkdir(parents=True, exist_ok=True)
+    tmp = FASTCALL_PATH.with_suffix(f".{os.getpid()}.tmp")
+    res = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, str(FASTCALL_SRC), "-o", str(tmp)], capture_output=True, text=True)
+    if res.returncode != 0:
+        raise RuntimeError(f"{cc} failed for {FASTCALL_SRC.name}:\n{res.stdout}\n{res.stderr}")
+    os.replace(tmp, FASTCALL_PATH)
+    stamp.write_text(digest)
+    return FASTCALL_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> Path:
     """Compiles every ``csrc/*.cu`` for sm_100a and links ``maco_b200/_lib/libmaco_b200.so``."""
     srcs = sources()
@@ -85,6 +110,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
+    build_fastcall()
     return LIB_PATH
 
 

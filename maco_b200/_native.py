@@ -87,6 +87,42 @@ def lib() -> ctypes.CDLL:
         return _lib
 
 
+_FASTCALL_PATH = _LIB_PATH.parent / "maco_fastcall.so"
+_fastcall = None
+
+
+def fastcall(name: str):
+    """A function of the C extension (csrc/py/fastcall.c). Where that cannot be loaded or built, one that answers every call with None,
+    "take the general path"."""
+    global _fastcall
+    if _fastcall is None:
+        handle = lib()
+        with _lock:
+            if _fastcall is None:
+                _fastcall = _load_fastcall(handle) or False
+    return getattr(_fastcall, name) if _fastcall else (lambda *a: None)
+
+
+def _load_fastcall(handle):
+    import importlib.machinery
+    import importlib.util
+    try:
+        if not _FASTCALL_PATH.exists():
+            from . import _build
+            if _build.build_fastcall() is None:
+                return None
+        loader = importlib.machinery.ExtensionFileLoader("maco_fastcall", str(_FASTCALL_PATH))
+        mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("maco_fastcall", loader))
+        loader.exec_module(mod)
+    except (ImportError, OSError, RuntimeError):             # (another interpreter's build, a read-only tree without one)
+        return None
+    address = lambda fn: ctypes.cast(fn, ctypes.c_void_p).value
+    mod.setup(torch.Tensor, torch.nn.Parameter, DTYPE_CODE, torch.empty_like, torch.empty, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream,
+              torch.float32, address(handle.maco_elementwise), address(handle.maco_attention_decode_stream),
+              address(handle.maco_attention_stream_scratch_bytes))
+    return mod
+
+
 def last_error() -> str:
     return lib().maco_last_error().decode(errors="replace")
 

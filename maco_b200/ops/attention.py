@@ -84,6 +84,18 @@ def attention_decode_tensor_core(q: torch.Tensor, k: torch.Tensor, v: torch.Tens
     return out
 
 
+def _load_quick(q, *rest):
+    global _quick
+    if not q.is_cuda:
+        return None
+    _lib()
+    _quick = N.fastcall("attention")
+    return _quick(q, *rest)
+
+
+_quick = _load_quick       # the ordinary call as one call into C (csrc/py/fastcall.c); None: not an ordinary one
+
+
 def attention_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale: Optional[float] = None,
                      splits: Optional[int] = None, out: Optional[torch.Tensor] = None,
                      scratch: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -91,6 +103,12 @@ def attention_decode(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, *, scale
     Without an explicit ``splits`` / ``scratch`` the call streams K and V through the tensor cores, one equal share per
     SM; with one of them it runs the CUDA-core kernel with that many splits (into that scratch). Scores, softmax and sums are
     fp32 in both, and so are the probabilities (on the tensor cores each is the sum of two values of the operand type)."""
+    if splits is None and scratch is None:
+        res = _quick(q, k, v, out, 128 ** -0.5 if scale is None else scale)
+        if res.__class__ is int:
+            N.check(res, "maco_attention_decode_stream")
+        if res is not None:
+            return res
     B, Hq, D = q.shape
     _, Hkv, S, _ = k.shape
     strides = _kv_strides(k)

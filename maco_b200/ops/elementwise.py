@@ -60,17 +60,39 @@ def _launch(kind: int, x: torch.Tensor, in1=None, in2=None, out: Optional[torch.
     return out
 
 
-def gelu(x, out=None): return _launch(T_GELU, x, out=out)
-def silu(x, out=None): return _launch(T_SILU, x, out=out)
-def softmax(x, out=None): return _launch(T_SOFTMAX, x, out=out)
-def scale(x, factor: float, out=None): return _launch(T_SCALE, x, out=out, f0=factor)
-def add(a, b, out=None): return _launch(T_ADD, a, in1=b, out=out)
-def silu_gate(gate, up, out=None): return _launch(T_SILU_GATE, gate, in1=up, out=out)
-def gelu_bwd(dy, pre, out=None): return _launch(T_GELU_BWD, dy, in1=pre, out=out)
-def axpby(x, y, a: float, b: float, out=None): return _launch(T_AXPBY, x, in1=y, out=out, f0=a, f1=b)
-def rmsnorm(x, weight, eps: float = 1e-6, out=None): return _launch(T_RMSNORM, x, in1=weight, out=out, f0=eps)
+def _load_quick(kind, x, *rest):
+    global _quick
+    if not x.is_cuda:
+        return None
+    _quick = N.fastcall("elementwise")
+    return _quick(kind, x, *rest)
+
+
+# The ordinary call, plain contiguous tensors on the GPU, as one call into C; None: it is not one, and the general path decides.
+# 4 x 512 bf16, host time of an RMSNorm: 8.3 us through Python and ctypes, 5.8 this way (2.6 the launch, 1.4 the result's allocation).
+_quick = _load_quick
+
+
+def _run(kind: int, x, in1, in2, out, f0, f1) -> torch.Tensor:
+    res = _quick(kind, x, in1, in2, out, f0, f1)
+    if res is None:
+        return _launch(kind, x, in1=in1, in2=in2, out=out, f0=f0, f1=f1)
+    if res.__class__ is int:
+        N.check(res, "maco_elementwise")
+    return res
+
+
+def gelu(x, out=None): return _run(T_GELU, x, None, None, out, 0.0, 0.0)
+def silu(x, out=None): return _run(T_SILU, x, None, None, out, 0.0, 0.0)
+def softmax(x, out=None): return _run(T_SOFTMAX, x, None, None, out, 0.0, 0.0)
+def scale(x, factor: float, out=None): return _run(T_SCALE, x, None, None, out, factor, 0.0)
+def add(a, b, out=None): return _run(T_ADD, a, b, None, out, 0.0, 0.0)
+def silu_gate(gate, up, out=None): return _run(T_SILU_GATE, gate, up, None, out, 0.0, 0.0)
+def gelu_bwd(dy, pre, out=None): return _run(T_GELU_BWD, dy, pre, None, out, 0.0, 0.0)
+def axpby(x, y, a: float, b: float, out=None): return _run(T_AXPBY, x, y, None, out, a, b)
+def rmsnorm(x, weight, eps: float = 1e-6, out=None): return _run(T_RMSNORM, x, weight, None, out, eps, 0.0)
 def layernorm(x, weight, bias, eps: float = 1e-5, out=None):
-    return _launch(T_LAYERNORM, x, in1=weight, in2=bias, out=out, f0=eps)
+    return _run(T_LAYERNORM, x, weight, bias, out, eps, 0.0)
 
 
 def rope(x: torch.Tensor, cos: torch.Tensor, sin: torch.Tensor, out=None) -> torch.Tensor:

@@ -1,0 +1,95 @@
+"""Calls through the C extension (csrc/py/fastcall.c) against the general path in Python: the same results over what it takes, and everything
+else still answered by the general path, errors among it."""
+import pytest
+import torch
+
+from maco_b200 import _build, _native as N, ops
+from maco_b200.ops import attention as A, elementwise as E
+
+
+def test_builds_and_leaves_cpu_tensors_to_the_general_path():
+    if _build.build_fastcall() is None:
+        pytest.skip("no compiler or no Python header")
+    quick = N.fastcall("elementwise")
+    x = torch.ones(2, 8)
+    assert quick(E.T_GELU, x, None, None, None, 0.0, 0.0) is None
+    assert quick(E.T_ADD, [1.0], None, None, None, 0.0, 0.0) is None              # not a tensor
+    with pytest.raises(TypeError):
+        quick(E.T_GELU, x)
+    q, k = torch.ones(1, 4, 128), torch.ones(1, 2, 16, 128)
+    assert N.fastcall("attention")(q, k, k, None, 0.1) is None
+    with pytest.raises(ValueError):
+        ops.gelu(x)
+    with pytest.raises(AttributeError):
+        ops.add([1.0], x)
+
+
+def _general(monkeypatch, module):
+    monkeypatch.setattr(module, "_quick", lambda *a: None)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(1,), (5,), (4, 512), (3, 7, 33), (2, 0, 8), ()])
+@pytest.mark.parametrize("form", ["plain", "out", "strided", "parameter"])
+def test_elementwise_same_as_general(monkeypatch, dtype, shape, form):
+    g = torch.Generator(device="cuda").manual_seed(1)
+    mk = lambda: torch.randn(*shape, device="cuda", generator=g).to(dtype) if shape else torch.randn((), device="cuda", generator=g).to(dtype)
+    x, y = mk(), mk()
+    if form == "strided" and len(shape) > 1:
+        x = torch.cat([x, x], -1)[..., :shape[-1]]
+    if form == "parameter":
+        x = torch.nn.Parameter(x, requires_grad=False)
+    cols = shape[-1] if shape else 1
+    w, b = torch.randn(cols, device="cuda", generator=g).to(dtype), torch.randn(cols, device="cuda", generator=g).to(dtype)
+
+    def all_of():
+        o = (lambda: torch.empty(shape, device="cuda", dtype=dtype)) if form == "out" else (lambda: None)
+        calls = [lambda: ops.gelu(x, out=o()), lambda: ops.silu(x, out=o()), lambda: ops.softmax(x, out=o()), lambda: ops.scale(x, 3, out=o()),
+                 lambda: ops.add(x, y, out=o()), lambda: ops.silu_gate(x, y, out=o()), lambda: ops.gelu_bwd(x, y, out=o()),
+                 lambda: ops.axpby(x, y, 2.0, -1, out=o()), lambda: ops.rmsnorm(x, w, out=o()), lambda: ops.layernorm(x, w, b, out=o())]
+        res = []
+        for c in calls:
+            try:
+                res.append(c())
+            except (IndexError, ValueError, RuntimeError) as e:
+                res.append(type(e))
+        return res
+
+    got = all_of()
+    _general(monkeypatch, E)
+    for a, b_ in zip(got, all_of()):
+        assert (a == b_) if isinstance(b_, type) else (a.shape == b_.shape and a.dtype == b_.dtype and torch.equal(a, b_))
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("form", ["plain", "out", "view", "one_head_view", "scale", "more_batch", "strided_q"])
+def test_attention_same_as_general(monkeypatch, dtype, form):
+    g = torch.Generator(device="cuda").manual_seed(2)
+    B, H, G, S = (3, 1, 4, 300) if form == "one_head_view" else (3, 2, 4, 300)
+    q = torch.randn(B, H * G, 128, device="cuda", generator=g).to(dtype)
+    k = torch.randn(B + (form == "more_batch"), H, S + 77, 128, device="cuda", generator=g).to(dtype)
+    v = torch.randn_like(k)
+    if form in ("view", "one_head_view", "more_batch"):
+        k, v = k[:, :, :S], v[:, :, :S]
+    if form == "strided_q":
+        q = torch.cat([q, q], 1)[:, :H * G]
+    kw = {"scale": 0.05} if form == "scale" else {}
+    run = lambda: ops.attention_decode(q, k, v, out=torch.empty(B, H * G, 128, device="cuda", dtype=dtype) if form == "out" else None, **kw)
+    got = run()
+    _general(monkeypatch, A)
+    assert torch.equal(got, run())
+
+
+@pytest.mark.gpu
+def test_refusals_stay():
+    q = torch.randn(2, 8, 128, device="cuda").bfloat16()
+    k = torch.randn(2, 2, 64, 128, device="cuda").bfloat16()
+    for bad_k, bad_v in ((k, k[:, :, :32]), (k.transpose(1, 2), k.transpose(1, 2)), (k[:1], k[:1])):
+        with pytest.raises(ValueError):
+            ops.attention_decode(q, bad_k, bad_v)
+    with pytest.raises(ValueError):
+        ops.gelu(torch.randn(4, 8, device="cuda"), out=torch.empty(8, 4, device="cuda").t())
+    with pytest.raises(ValueError):
+        ops.gelu(torch.ones(4, 8, device="cuda", dtype=torch.int32))
