@@ -70,7 +70,10 @@ struct AttnStreamParams {
 constexpr int kStreamThreads = 160;
 constexpr int kStreamSmem = 1024 + kAttnStages * kAttnStageBytes + kAttnTcScratchBytes + 128;
 
-MACO_DEVICE long long share_begin(const AttnStreamParams& p, int cta, int n) { return p.total * cta / n; }
+// (32-bit division where the product fits: 2^24 chunks times 148 shares)
+MACO_DEVICE long long share_begin(const AttnStreamParams& p, int cta, int n) {
+  return p.total < (1ll << 24) ? (long long)((uint32_t)p.total * (uint32_t)cta / (uint32_t)n) : p.total * cta / n;
+}
 
 template <int DTT>
 __global__ void __launch_bounds__(kStreamThreads, 1)
@@ -94,7 +97,7 @@ attn_stream_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
   bool ok = true;
   for (long long pos = begin; pos < end && ok;) {
-    const int group = (int)(pos / p.chunks_per_head), c0 = (int)(pos - (long long)group * p.chunks_per_head);
+    const int group = p.total < (1ll << 24) ? (int)((uint32_t)pos / (uint32_t)p.chunks_per_head) : (int)(pos / p.chunks_per_head), c0 = (int)(pos - (long long)group * p.chunks_per_head);
     const int n = (int)min((long long)(p.chunks_per_head - c0), end - pos);
     const int key0 = c0 * 128, rows = min(p.S - key0, n * 128);
     if (warp == 4) {
@@ -127,25 +130,55 @@ attn_stream_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   if (tid == 0 && *abort_word != 0 && p.status != nullptr) st_relaxed_sys_u32(p.status, MACO_STATUS_TIMEOUT);
 }
 
-template <int DTT>
+// ONE_HEAD: a CTA per head. With all G heads of a group in one CTA a thread has registers for two records, and the twelve records of a cache
+// of 1357 keys in 128-key shares were six round trips to L2 in a row (16.4 us for the call, 13.9 with a CTA per head). Where a group has two or three
+// records there is nothing to gain, and G times the CTAs cost (16 x 8 kv heads x 8192 keys 88.2 us, 89.3 with a CTA per head): see launch_stream.
+constexpr int kMergeAhead = 8;
+template <int DTT, bool ONE_HEAD>
 __global__ void __launch_bounds__(128) attn_stream_merge_kernel(const AttnStreamParams p, int n_ctas) {
   asm volatile("griddepcontrol.wait;" ::: "memory");
-  const int group = blockIdx.x, tid = threadIdx.x;
+  const int group = blockIdx.x, g = blockIdx.y, tid = threadIdx.x;
   const long long first = (long long)group * p.chunks_per_head, last = first + p.chunks_per_head - 1;
   // the CTA whose share holds chunk x: floor estimate, then exact (shares differ by at most one chunk)
   auto owner = [&](long long x) {
-    int c = (int)(x * n_ctas / p.total);
+    int c = p.total < (1ll << 24) ? (int)((uint32_t)x * (uint32_t)n_ctas / (uint32_t)p.total) : (int)(x * n_ctas / p.total);
     while (c > 0 && share_begin(p, c, n_ctas) > x) --c;
     while (c + 1 < n_ctas && share_begin(p, c + 1, n_ctas) <= x) ++c;
     return c;
   };
-  const int lo = owner(first), hi = owner(last);
-  if (lo == hi) return;                              // one share held the whole group and wrote its rows
+  const int lo = owner(first), hi = owner(last), n = hi - lo + 1;
+  if (n == 1) return;                                // one share held the whole group and wrote its rows
   const int rec = p.G * kAttnD + 2 * p.G;
-  attn_merge_records<DTT>(reinterpret_cast<uint8_t*>(p.out) + (size_t)group * p.G * kAttnD * 2, p.G, hi - lo + 1, tid, [&](int i) {
-    const int c = lo + i, slot = share_begin(p, c, n_ctas) >= first ? 0 : 1;
-    return (const float*)(p.scratch + ((size_t)c * 2 + slot) * rec);
-  });
+  // a share behind the first one begins inside the group (slot 0); the first one may have begun in front of it (slot 1)
+  const float* r0 = p.scratch + ((size_t)lo * 2 + (share_begin(p, lo, n_ctas) >= first ? 0 : 1)) * rec;
+  const float* rest = p.scratch + (size_t)lo * 2 * rec;
+  if constexpr (!ONE_HEAD) {
+    attn_merge_records<DTT>(reinterpret_cast<uint8_t*>(p.out) + (size_t)group * p.G * kAttnD * 2, p.G, n, tid,
+                            [&](int i) { return i == 0 ? r0 : rest + (size_t)i * 2 * rec; });
+    return;
+  }
+  float M = -INFINITY, L = 0.f, acc = 0.f;
+#pragma unroll 1
+  for (int i0 = 0; i0 < n; i0 += kMergeAhead) {
+    float ms[kMergeAhead], ls[kMergeAhead], os[kMergeAhead];
+#pragma unroll
+    for (int i = 0; i < kMergeAhead; ++i) {
+      const bool have = i0 + i < n;
+      const float* r = i0 + i == 0 ? r0 : rest + (size_t)(i0 + i) * 2 * rec;
+      ms[i] = have ? __ldcg(r + p.G * kAttnD + g) : -INFINITY;
+      ls[i] = have ? __ldcg(r + p.G * kAttnD + p.G + g) : 0.f;
+      os[i] = have ? __ldcg(r + g * kAttnD + tid) : 0.f;
+    }
+#pragma unroll
+    for (int i = 0; i < kMergeAhead; ++i) {
+      const float m = fmaxf(M, ms[i]);
+      const float a = M == -INFINITY ? 0.f : attn_ex2(M - m), b = ms[i] == -INFINITY ? 0.f : attn_ex2(ms[i] - m);
+      L = L * a + ls[i] * b;
+      acc = acc * a + os[i] * b;
+      M = m;
+    }
+  }
+  store1(reinterpret_cast<uint8_t*>(p.out) + (size_t)group * p.G * kAttnD * 2, g * kAttnD + tid, DTT, L > 0.f ? acc / L : 0.f);
 }
 
 template <int DTT>
@@ -161,11 +194,12 @@ int launch_stream(const CUtensorMap& tmK, const CUtensorMap& tmV, const AttnStre
   MACO_CHECK_CUDA(cudaGetLastError());
   if (p.chunks_per_head > 1) {                       // else a group is one chunk, and no share can end inside it
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(p.groups); cfg.blockDim = dim3(128); cfg.stream = stream;
+    const bool one_head = (long long)p.chunks_per_head * grid >= 4 * p.total;       // a group is four shares or more
+    cfg.gridDim = dim3(p.groups, one_head ? p.G : 1); cfg.blockDim = dim3(128); cfg.stream = stream;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization; at[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = at; cfg.numAttrs = 1;
-    MACO_CHECK_CUDA(cudaLaunchKernelEx(&cfg, attn_stream_merge_kernel<DTT>, p, grid));
+    MACO_CHECK_CUDA(cudaLaunchKernelEx(&cfg, one_head ? attn_stream_merge_kernel<DTT, true> : attn_stream_merge_kernel<DTT, false>, p, grid));
   }
   return 0;
 }

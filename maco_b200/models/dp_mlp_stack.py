@@ -77,11 +77,16 @@ class DPMLPStackBackward:
     # ------------------------------------------------------------------ forward (set-up, separate launches)
     def forward(self) -> torch.Tensor:
         cur = self.x
+        # Up to 4 Mi activations the product with the GELU in its epilogue, one launch a layer instead of two. 3 layers, one B200, us, as product and
+        # GELU / in one: 256 x 512 68 / 46, 8192 x 512 56.2 / 55.9, 300 x 4096 127 / 118. Beyond that the launches no longer count and which is faster
+        # goes with the last round of tiles and the power cap: 4096 x 2048 117 / 111, 2304 x 2304 130 / 136, 8192 x 3072 457 / 414, 8192 x 4096 651 / 690.
+        fused = self.tokens * self.hidden <= 1 << 22
         for l in range(self.layers):
-            # two launches: the product with the GELU in its epilogue (gelu_dual) gains 1 % at 2816 x 8192 tokens and loses elsewhere. It / these,
-            # 3 layers, one B200, us: 1024 x 8192 tokens 132 / 100, 2048 x 4096 156 / 132, 3072 x 8192 430 / 428, 4096 x 8192 701 / 665
-            ops.gemm(cur, self.weights[l], out=self.z[l])
-            ops.gelu(self.z[l], out=self.a[l])
+            if fused:
+                ops.gemm(cur, self.weights[l], out=self.z[l], epilogue="gelu_dual", aux=self.a[l])
+            else:
+                ops.gemm(cur, self.weights[l], out=self.z[l])
+                ops.gelu(self.z[l], out=self.a[l])
             cur = self.a[l]
         return cur
 
