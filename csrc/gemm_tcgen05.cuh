@@ -365,7 +365,10 @@ struct EpiBroadcast {
 // stored / loaded to 308 / 404 with this form inlined and the general one behind a call.
 MACO_DEVICE bool epi_is_lean(const GemmEpilogue& e, int n0, int bn) {
   const bool plain = e.mode == MACO_EPI_STORE || e.mode == MACO_EPI_F32_STORE;
-  return e.out_type != MACO_DT_F32 && e.bias == nullptr && n0 + bn <= e.N && (plain || e.mode == MACO_EPI_SWIGLU || e.mode == MACO_EPI_SCATTER_ROWS);
+  if (e.out_type == MACO_DT_F32 || e.bias != nullptr) return false;
+  // (a plain tile may end early, at a whole step of the loop: the few columns of a router)
+  if (n0 + bn > e.N) return plain && (e.N - n0) % 32 == 0;
+  return plain || e.mode == MACO_EPI_SWIGLU || e.mode == MACO_EPI_SCATTER_ROWS;
 }
 template <int SBN>
 MACO_DEVICE bool gemm_epilogue_lean(int bn, const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e, void* out_base, long long row_off,
@@ -390,7 +393,7 @@ MACO_DEVICE bool gemm_epilogue_lean(int bn, const GemmCtrl& c, uint32_t tmem_bas
   const float alpha = e.alpha;
   uint8_t* dst = reinterpret_cast<uint8_t*>(out_base) + (out_row * e.ld_out + (swiglu ? n0 / 2 : n0)) * 2;
   const uint32_t t_row = tmem_base + ((q * 32u) << 16) + acc * SBN;
-  const int cols = swiglu ? bn / 2 : bn;
+  const int cols = swiglu ? bn / 2 : min(bn, e.N - n0);
 #pragma unroll 1
   for (int col = 0; col < cols; col += 32) {
     uint32_t r[32];

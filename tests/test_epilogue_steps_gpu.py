@@ -67,3 +67,17 @@ def test_graph(dtype, M, N):
         graph.execute()
     _close(y.output, z, dtype)
     _close(s.output, y.output.double() + r.double(), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N", [32, 64, 96, 160, 288, 40, 264])       # whole steps of 32 columns, and not
+@pytest.mark.parametrize("M", [129, 640])
+def test_graph_tiles_that_end_early(dtype, N, M):
+    import maco_b200 as maco
+    x, w, _, z = _operands(M, N, 320, dtype, N)
+    graph = maco.TaskGraph()
+    y = graph.linear(x, w)
+    graph.compile()
+    y.output.fill_(7.0)
+    graph.execute()
+    _close(y.output, z, dtype)
