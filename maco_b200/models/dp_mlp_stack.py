@@ -36,8 +36,9 @@ class DPMLPStackBackward:
                  cta_pair: Optional[bool] = None):
         # ``cta_pair``: two-CTA tiles (True) or one-CTA ones (False) whatever the size. None: two-CTA tiles on one GPU where both GEMM kinds
         # have about one 256 x 256 tile per worker or more (two per pair: below that the last wave costs more than the smaller operand
-        # traffic gains). Backward pass, one- / two-CTA, one B200: 4 layers of 4096 x 8192 tokens 1650 / 1535 us, 2 of 3072 x 6144 342 / 319,
-        # 4 of 2304 x 2304 271 / 297, 3 of 1024 x 8192 197 / 213. (More ranks: not measured, one-CTA.)
+        # traffic gains). Backward pass, one- / two-CTA, one B200: 4 layers of 4096 x 8192 tokens 1518 / 1444 us, 2 of 3072 x 6144 309 / 286.
+        # (Below the line two-CTA tiles have since become the faster form down to about 2048 x 1024: 4 layers of 2304 x 2304 235 / 222, 3 of
+        # 1024 x 8192 173 / 171, but 3 of 1536 x 1536 94 / 97; ask for them there.) (More ranks: not measured, one-CTA.)
         if cta_pair is None:
             sms = torch.cuda.get_device_properties(device if device is not None else torch.cuda.current_device()).multi_processor_count \
                 if torch.cuda.is_available() and (device is None or torch.device(device).type == "cuda") else 148
