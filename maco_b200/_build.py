@@ -9,6 +9,7 @@ from __future__ import annotations
 
 import hashlib
 import os
+import shlex
 import shutil
 import subprocess
 import sys
@@ -74,8 +75,9 @@ def build_fastcall() -> "Path | None":
     """The C extension behind the smallest calls (csrc/py/fastcall.c), for this interpreter. None where there is no compiler or no Python
     header: those calls then take their general path."""
     include = sysconfig.get_paths()["include"]
-    cc = os.environ.get("CC") or shutil.which("gcc") or shutil.which("cc")
-    if cc is None or not os.path.exists(os.path.join(include, "Python.h")):
+    # CC may hold arguments, or a launcher in front of the compiler ("gcc -pthread", "ccache gcc")
+    cc = shlex.split(os.environ.get("CC", "")) or [c for c in (shutil.which("gcc") or shutil.which("cc"),) if c]
+    if not cc or not os.path.exists(os.path.join(include, "Python.h")):
         return None
     digest = hashlib.sha256(FASTCALL_SRC.read_bytes() + sys.version.encode()).hexdigest()
     stamp = OBJ_DIR / "fastcall.sha"
@@ -84,9 +86,9 @@ def build_fastcall() -> "Path | None":
     LIB_DIR.mkdir(parents=True, exist_ok=True)
     OBJ_DIR.mkdir(parents=True, exist_ok=True)
     tmp = FASTCALL_PATH.with_suffix(f".{os.getpid()}.tmp")
-    res = subprocess.run([cc, "-O2", "-shared", "-fPIC", "-I", include, str(FASTCALL_SRC), "-o", str(tmp)], capture_output=True, text=True)
+    res = subprocess.run([*cc, "-O2", "-shared", "-fPIC", "-I", include, str(FASTCALL_SRC), "-o", str(tmp)], capture_output=True, text=True)
     if res.returncode != 0:
-        raise RuntimeError(f"{cc} failed for {FASTCALL_SRC.name}:\n{res.stdout}\n{res.stderr}")
+        raise RuntimeError(f"{shlex.join(cc)} failed for {FASTCALL_SRC.name}:\n{res.stdout}\n{res.stderr}")
     os.replace(tmp, FASTCALL_PATH)
     stamp.write_text(digest)
     return FASTCALL_PATH

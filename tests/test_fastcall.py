@@ -24,6 +24,23 @@ def test_builds_and_leaves_cpu_tensors_to_the_general_path():
         ops.add([1.0], x)
 
 
+@pytest.fixture
+def empty_build(monkeypatch, tmp_path):
+    """The extension's build with folders of its own, nothing built yet."""
+    if _build.build_fastcall() is None:
+        pytest.skip("no compiler or no Python header")
+    monkeypatch.setattr(_build, "LIB_DIR", tmp_path)
+    monkeypatch.setattr(_build, "OBJ_DIR", tmp_path)
+    monkeypatch.setattr(_build, "FASTCALL_PATH", tmp_path / _build.FASTCALL_PATH.name)
+    return tmp_path
+
+
+@pytest.mark.parametrize("cc", ["gcc -pthread", "env gcc", "", " "])
+def test_compiler_with_arguments(empty_build, monkeypatch, cc):
+    monkeypatch.setenv("CC", cc)
+    assert _build.build_fastcall() == _build.FASTCALL_PATH and _build.FASTCALL_PATH.exists()
+
+
 def _general(monkeypatch, module):
     monkeypatch.setattr(module, "_quick", lambda *a: None)
 
