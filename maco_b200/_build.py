@@ -14,6 +14,7 @@ import shutil
 import subprocess
 import sys
 import sysconfig
+import warnings
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -73,7 +74,7 @@ def _compile_one(src: Path, verbose: bool) -> Path:
 
 def build_fastcall() -> "Path | None":
     """The C extension behind the smallest calls (csrc/py/fastcall.c), for this interpreter. None where there is no compiler or no Python
-    header: those calls then take their general path."""
+    header, an exception where the compiler fails: those calls then take their general path."""
     include = sysconfig.get_paths()["include"]
     # CC may hold arguments, or a launcher in front of the compiler ("gcc -pthread", "ccache gcc")
     cc = shlex.split(os.environ.get("CC", "")) or [c for c in (shutil.which("gcc") or shutil.which("cc"),) if c]
@@ -112,7 +113,10 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         res = subprocess.run(cmd, capture_output=True, text=True)
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
-    build_fastcall()
+    try:
+        build_fastcall()
+    except (OSError, RuntimeError, ValueError) as exc:       # the calls it is for take their general path
+        warnings.warn(f"the C extension was not built: {exc}")
     return LIB_PATH
 
 

@@ -114,7 +114,7 @@ def _load_fastcall(handle):
         loader = importlib.machinery.ExtensionFileLoader("maco_fastcall", str(_FASTCALL_PATH))
         mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("maco_fastcall", loader))
         loader.exec_module(mod)
-    except (ImportError, OSError, RuntimeError):             # (another interpreter's build, a read-only tree without one)
+    except (ImportError, OSError, RuntimeError, ValueError): # (another interpreter's build, a read-only tree without one)
         return None
     address = lambda fn: ctypes.cast(fn, ctypes.c_void_p).value
     mod.setup(torch.Tensor, torch.nn.Parameter, DTYPE_CODE, torch.empty_like, torch.empty, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream,

@@ -1,5 +1,7 @@
 """Calls through the C extension (csrc/py/fastcall.c) against the general path in Python: the same results over what it takes, and everything
 else still answered by the general path, errors among it."""
+import subprocess
+
 import pytest
 import torch
 
@@ -39,6 +41,21 @@ def empty_build(monkeypatch, tmp_path):
 def test_compiler_with_arguments(empty_build, monkeypatch, cc):
     monkeypatch.setenv("CC", cc)
     assert _build.build_fastcall() == _build.FASTCALL_PATH and _build.FASTCALL_PATH.exists()
+
+
+@pytest.mark.parametrize("cc", ["false", "/nonexistent/cc", "gcc -no-such-option", "gcc 'unbalanced"])
+def test_the_build_survives_without_it(empty_build, monkeypatch, cc):
+    from types import SimpleNamespace
+    done = empty_build / "done.o"
+    done.touch()
+    monkeypatch.setattr(_build, "_compile_one", lambda src, verbose: done)
+    monkeypatch.setattr(_build, "subprocess", SimpleNamespace(run=lambda cmd, **kw: (
+        SimpleNamespace(returncode=0) if cmd[1] == "-shared" else subprocess.run(cmd, **kw))))        # (the link)
+    monkeypatch.setattr(_build, "_nvcc", lambda: "nvcc")
+    monkeypatch.setenv("CC", cc)
+    with pytest.warns(UserWarning, match="not built"):
+        assert _build.build() == _build.LIB_PATH
+    assert not _build.FASTCALL_PATH.exists()
 
 
 def _general(monkeypatch, module):
