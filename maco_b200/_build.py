@@ -25,7 +25,6 @@ LIB_DIR = PKG_DIR / "_lib"
 LIB_PATH = LIB_DIR / "libmaco_b200.so"
 OBJ_DIR = REPO_DIR / "build" / "obj"
 FASTCALL_SRC = CSRC_DIR / "py" / "fastcall.c"
-FASTCALL_PATH = LIB_DIR / "maco_fastcall.so"
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a",
@@ -72,7 +71,14 @@ def _compile_one(src: Path, verbose: bool) -> Path:
     return obj
 
 
-def build_fastcall() -> "Path | None":
+def fastcall_path() -> Path:
+    """Where the C extension of this source and this interpreter lies. Both are part of the name: CPython loads an untagged extension that
+    another minor version built without a word, and runs it with that version's inlined reference counts and tuple layout."""
+    digest = hashlib.sha256(FASTCALL_SRC.read_bytes()).hexdigest()[:12]
+    return LIB_DIR / f"maco_fastcall-{digest}{sysconfig.get_config_var('EXT_SUFFIX')}"
+
+
+def build_fastcall(force: bool = False) -> "Path | None":
     """The C extension behind the smallest calls (csrc/py/fastcall.c), for this interpreter. None where there is no compiler or no Python
     header, an exception where the compiler fails: those calls then take their general path."""
     include = sysconfig.get_paths()["include"]
@@ -80,19 +86,19 @@ def build_fastcall() -> "Path | None":
     cc = shlex.split(os.environ.get("CC", "")) or [c for c in (shutil.which("gcc") or shutil.which("cc"),) if c]
     if not cc or not os.path.exists(os.path.join(include, "Python.h")):
         return None
-    digest = hashlib.sha256(FASTCALL_SRC.read_bytes() + sys.version.encode()).hexdigest()
-    stamp = OBJ_DIR / "fastcall.sha"
-    if FASTCALL_PATH.exists() and stamp.exists() and stamp.read_text() == digest:
-        return FASTCALL_PATH
+    path = fastcall_path()
+    if path.exists() and not force:
+        return path
     LIB_DIR.mkdir(parents=True, exist_ok=True)
-    OBJ_DIR.mkdir(parents=True, exist_ok=True)
-    tmp = FASTCALL_PATH.with_suffix(f".{os.getpid()}.tmp")
+    tmp = path.with_name(f"{path.name}.{os.getpid()}.tmp")
     res = subprocess.run([*cc, "-O2", "-shared", "-fPIC", "-I", include, str(FASTCALL_SRC), "-o", str(tmp)], capture_output=True, text=True)
     if res.returncode != 0:
         raise RuntimeError(f"{shlex.join(cc)} failed for {FASTCALL_SRC.name}:\n{res.stdout}\n{res.stderr}")
-    os.replace(tmp, FASTCALL_PATH)
-    stamp.write_text(digest)
-    return FASTCALL_PATH
+    os.replace(tmp, path)
+    for old in LIB_DIR.glob("maco_fastcall*"):              # of other states of the source; other interpreters keep theirs
+        if old != path and (old.name == "maco_fastcall.so" or old.name.endswith(sysconfig.get_config_var("EXT_SUFFIX"))):
+            old.unlink(missing_ok=True)
+    return path
 
 
 def build(force: bool = False, verbose: bool = False) -> Path:
@@ -114,7 +120,7 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         if res.returncode != 0:
             raise RuntimeError(f"link failed:\n{res.stdout}\n{res.stderr}")
     try:
-        build_fastcall()
+        build_fastcall(force)
     except (OSError, RuntimeError, ValueError) as exc:       # the calls it is for take their general path
         warnings.warn(f"the C extension was not built: {exc}")
     return LIB_PATH

@@ -87,7 +87,6 @@ def lib() -> ctypes.CDLL:
         return _lib
 
 
-_FASTCALL_PATH = _LIB_PATH.parent / "maco_fastcall.so"
 _fastcall = None
 
 
@@ -106,15 +105,15 @@ def fastcall(name: str):
 def _load_fastcall(handle):
     import importlib.machinery
     import importlib.util
+    from . import _build
     try:
-        if not _FASTCALL_PATH.exists():
-            from . import _build
-            if _build.build_fastcall() is None:
-                return None
-        loader = importlib.machinery.ExtensionFileLoader("maco_fastcall", str(_FASTCALL_PATH))
+        path = _build.fastcall_path()                        # (of this source and interpreter, no other)
+        if not path.exists() and _build.build_fastcall() is None:
+            return None
+        loader = importlib.machinery.ExtensionFileLoader("maco_fastcall", str(path))
         mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("maco_fastcall", loader))
         loader.exec_module(mod)
-    except (ImportError, OSError, RuntimeError, ValueError): # (another interpreter's build, a read-only tree without one)
+    except (ImportError, OSError, RuntimeError, ValueError): # (a compiler that fails, a read-only tree without a build)
         return None
     address = lambda fn: ctypes.cast(fn, ctypes.c_void_p).value
     mod.setup(torch.Tensor, torch.nn.Parameter, DTYPE_CODE, torch.empty_like, torch.empty, torch._C._cuda_getDevice, torch._C._cuda_getCurrentRawStream,

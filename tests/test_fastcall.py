@@ -1,6 +1,8 @@
 """Calls through the C extension (csrc/py/fastcall.c) against the general path in Python: the same results over what it takes, and everything
 else still answered by the general path, errors among it."""
+import pathlib
 import subprocess
+import sysconfig
 
 import pytest
 import torch
@@ -32,15 +34,14 @@ def empty_build(monkeypatch, tmp_path):
     if _build.build_fastcall() is None:
         pytest.skip("no compiler or no Python header")
     monkeypatch.setattr(_build, "LIB_DIR", tmp_path)
-    monkeypatch.setattr(_build, "OBJ_DIR", tmp_path)
-    monkeypatch.setattr(_build, "FASTCALL_PATH", tmp_path / _build.FASTCALL_PATH.name)
     return tmp_path
 
 
 @pytest.mark.parametrize("cc", ["gcc -pthread", "env gcc", "", " "])
 def test_compiler_with_arguments(empty_build, monkeypatch, cc):
     monkeypatch.setenv("CC", cc)
-    assert _build.build_fastcall() == _build.FASTCALL_PATH and _build.FASTCALL_PATH.exists()
+    path = _build.build_fastcall()
+    assert path.parent == empty_build and path.exists()
 
 
 @pytest.mark.parametrize("cc", ["false", "/nonexistent/cc", "gcc -no-such-option", "gcc 'unbalanced"])
@@ -55,7 +56,27 @@ def test_the_build_survives_without_it(empty_build, monkeypatch, cc):
     monkeypatch.setenv("CC", cc)
     with pytest.warns(UserWarning, match="not built"):
         assert _build.build() == _build.LIB_PATH
-    assert not _build.FASTCALL_PATH.exists()
+    assert not list(empty_build.glob("maco_fastcall*"))
+
+
+def _loaded_from():
+    mod = N._load_fastcall(N.lib())
+    return mod and pathlib.Path(mod.__file__)
+
+
+def test_only_this_sources_and_interpreters_build_is_loaded(empty_build, monkeypatch):
+    others = [empty_build / n for n in ("maco_fastcall.so", "maco_fastcall-0123456789ab.cpython-37m-x86_64-linux-gnu.so")]
+    for o in others:
+        o.write_bytes(b"another interpreter's")
+    first = _loaded_from()
+    assert first.parent == empty_build and first.name.endswith(sysconfig.get_config_var("EXT_SUFFIX"))
+    assert others[1].exists()
+    # an edited source is another file, built when it is asked for, and what it replaces goes
+    edited = empty_build / "fastcall.c"
+    edited.write_text(_build.FASTCALL_SRC.read_text().replace("elementwise: seven arguments", "elementwise: 7 arguments"))
+    monkeypatch.setattr(_build, "FASTCALL_SRC", edited)
+    second = _loaded_from()
+    assert second != first and second.exists() and not first.exists() and b"elementwise: 7 arguments" in second.read_bytes()
 
 
 def _general(monkeypatch, module):
