@@ -108,7 +108,7 @@ def _load_fastcall(handle):
     from . import _build
     try:
         path = _build.fastcall_path()                        # (of this source and interpreter, no other)
-        if not path.exists() and _build.build_fastcall() is None:
+        if not path.exists() and (os.environ.get("MACO_NO_AUTOBUILD", "0") == "1" or _build.build_fastcall() is None):
             return None
         loader = importlib.machinery.ExtensionFileLoader("maco_fastcall", str(path))
         mod = importlib.util.module_from_spec(importlib.util.spec_from_loader("maco_fastcall", loader))

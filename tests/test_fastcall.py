@@ -79,6 +79,17 @@ def test_only_this_sources_and_interpreters_build_is_loaded(empty_build, monkeyp
     assert second != first and second.exists() and not first.exists() and b"elementwise: 7 arguments" in second.read_bytes()
 
 
+def test_nothing_is_built_where_that_is_switched_off(empty_build, monkeypatch):
+    monkeypatch.setenv("MACO_NO_AUTOBUILD", "1")
+    assert _loaded_from() is None and not list(empty_build.iterdir())
+    monkeypatch.setattr(N, "_fastcall", None)
+    assert N.fastcall("elementwise")(E.T_GELU, None, None, None, None, 0.0, 0.0) is None       # the general path
+    monkeypatch.delenv("MACO_NO_AUTOBUILD")
+    built = _loaded_from()
+    monkeypatch.setenv("MACO_NO_AUTOBUILD", "1")
+    assert _loaded_from() == built                           # what is there is loaded
+
+
 def _general(monkeypatch, module):
     monkeypatch.setattr(module, "_quick", lambda *a: None)
 
