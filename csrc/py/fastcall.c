@@ -56,6 +56,12 @@ static int dtype_code(PyObject* t, int* bad) {           /* -1: not one of the l
   if (!c) { if (PyErr_Occurred()) *bad = 1; return -1; }
   return (int)PyLong_AsLong(c);
 }
+/* 1, or 0 for what float() may still take (a text) or refuse: the general path's to say */
+static int number(PyObject* o, double* v) {
+  *v = PyFloat_AsDouble(o);
+  if (*v == -1.0 && PyErr_Occurred()) { PyErr_Clear(); return 0; }
+  return 1;
+}
 static void* current_stream(int* bad) {
   PyObject* d = PyObject_CallNoArgs(g_device);
   if (!d) { *bad = 1; return NULL; }
@@ -88,9 +94,10 @@ static PyObject* py_elementwise(PyObject* self, PyObject* const* a, Py_ssize_t n
   PyObject* size = PyObject_CallMethodOneArg(x, s_size, g_m1);
   if (!size) { PyErr_Clear(); Py_RETURN_NONE; }         /* (no dimensions) */
   const long long cols = int_of(size, &bad);
-  const double f0 = PyFloat_AsDouble(a[5]), f1 = PyFloat_AsDouble(a[6]);
   const long kind = PyLong_AsLong(a[0]);
   if (bad || PyErr_Occurred()) return NULL;
+  double f0, f1;
+  if (!number(a[5], &f0) || !number(a[6], &f1)) Py_RETURN_NONE;
   PyObject* out = a[4];
   if (out == Py_None) {
     out = PyObject_CallOneArg(g_empty_like, x);
@@ -155,8 +162,8 @@ static PyObject* py_attention(PyObject* self, PyObject* const* a, Py_ssize_t n) 
   if (!kv_strides(sk, tk, &kb, &kh) || !kv_strides(sv, tv, &vb, &vh) || kb != vb || kh != vh) Py_RETURN_NONE;
   const int dt = dtype_code(q, &bad);
   if (bad) return NULL;
-  const double scale = PyFloat_AsDouble(a[4]);
-  if (dt < 0 || PyErr_Occurred()) { if (PyErr_Occurred()) return NULL; Py_RETURN_NONE; }
+  double scale;
+  if (dt < 0 || !number(a[4], &scale)) Py_RETURN_NONE;
   PyObject* dev = PyObject_GetAttr(q, s_device);
   if (!dev) return NULL;
   PyObject* words = PyLong_FromUnsignedLongLong(g_scratch((int)(sq[1] / sk[1])) / 4);

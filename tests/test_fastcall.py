@@ -159,3 +159,15 @@ def test_refusals_stay():
         ops.gelu(torch.randn(4, 8, device="cuda"), out=torch.empty(8, 4, device="cuda").t())
     with pytest.raises(ValueError):
         ops.gelu(torch.ones(4, 8, device="cuda", dtype=torch.int32))
+
+
+@pytest.mark.gpu
+def test_factors_that_only_float_takes():
+    x = torch.randn(4, 8, device="cuda")
+    assert torch.equal(ops.scale(x, "2.5"), ops.scale(x, 2.5))
+    assert torch.equal(ops.softmax(ops.axpby(x, x, torch.tensor(2.0), "-1")), ops.softmax(ops.axpby(x, x, 2.0, -1.0)))
+    for factor, error in (("two", ValueError), (None, TypeError), (torch.ones(2), (RuntimeError, ValueError))):
+        with pytest.raises(error):
+            ops.scale(x, factor)
+    q, k = torch.randn(1, 4, 128, device="cuda").half(), torch.randn(1, 2, 16, 128, device="cuda").half()
+    assert torch.equal(ops.attention_decode(q, k, k, scale="0.1"), ops.attention_decode(q, k, k, scale=0.1))
