@@ -642,8 +642,8 @@ __device__ __noinline__ bool gemm_epilogue_beside_as(int bn, const GemmCtrl& c, 
         reinterpret_cast<uint4*>(dst)[1] = make_uint4(w[4], w[5], w[6], w[7]);
       }
       dst += 32;
+      __syncwarp();                                    // tcgen05.ld takes a converged warp; and every lane has read its row of the block that is filled next
     }
-    __syncwarp();                                      // every lane has read its row of the block that is filled next
     cur = cur + 2048u == mine + kEpiWarpBytes ? mine : cur + 2048u;
     fetch();
   }

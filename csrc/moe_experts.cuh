@@ -177,6 +177,7 @@ __device__ __noinline__ int experts_epilogue(const Program& p, const MacoExpertA
           to[0] = make_uint4(w[0], w[1], w[2], w[3]);
           to[1] = make_uint4(w[4], w[5], w[6], w[7]);
         }
+        __syncwarp();                                                   // (the lanes that stored and the others: tcgen05.ld takes a converged warp)
       }
       if (lines)
         epi_flush_rows<8>(mine, lane, [&](uint32_t r) -> uint8_t* {

@@ -130,3 +130,33 @@ def test_expert_layer_in_both_types_against_its_own_logits(dtype, mode, fused_re
     assert (out.double() - ref).norm() <= 2 * half * ref.norm()
     assert ((out.double() - ref).norm(dim=1) <= 8 * half * ref.norm(dim=1) + half).all()
     assert _native.status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16])
+def test_slabs_around_a_row_block(dtype):
+    """Slabs of a few rows store from registers, of a whole row block through shared memory, warps without rows not at all: no row, one, a
+    warp's 32 less and more one, a row block's 128 less and more one. The router sends token t where it is told to."""
+    from maco_b200 import _native
+    from maco_b200.models.moe_layer import MoEEPLayer
+    counts = [0, 1, 31, 33, 127, 128, 129, 63]
+    E, H, I, T = len(counts), 256, 128, sum(counts)
+    layer = MoEEPLayer(hidden=H, experts=E, top_k=1, inter=I, tokens=T, capacity_factor=4.0, seed=3, dtype=dtype, weight_std=0.05)
+    layer.w_router.copy_(4.0 * torch.eye(E, H, device="cuda"))
+    g = torch.Generator("cuda").manual_seed(5)
+    to = torch.cat([torch.full((n,), e, device="cuda") for e, n in enumerate(counts)])[torch.randperm(T, generator=g, device="cuda")]
+    x = torch.randn(T, H, device="cuda", generator=g)
+    x[:, :E] = torch.nn.functional.one_hot(to, E).float()
+    x = x.to(dtype)
+    rnd = lambda t: t.to(dtype).double()
+    half = 2.0 ** -8 if dtype == torch.bfloat16 else 2.0 ** -11
+    for _ in range(2):
+        out = layer(x)
+        assert layer.cnt.view(-1).tolist() == counts and layer.dropped() == 0
+        for e in range(E):
+            wg, wu, wd = (w.double() for w in layer.expert_weights(e))
+            xe = x[to == e].double()
+            ref = rnd(rnd(torch.nn.functional.silu(xe @ wg.t()) * (xe @ wu.t())) @ wd.t())
+            # rounded alike on both sides but for fp32 sums near a tie, in the activations and in the result (routing weight 1)
+            assert ((out[to == e].double() - ref).norm(dim=1) <= 4 * half * ref.norm(dim=1)).all()
+    assert _native.status() == 0
