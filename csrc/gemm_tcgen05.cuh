@@ -439,8 +439,7 @@ MACO_DEVICE bool gemm_epilogue_lean(int bn, const GemmCtrl& c, uint32_t tmem_bas
 // shared memory every instruction moves whole sectors of a few rows. PIECES 16-byte pieces a row (8 or 4), swizzled by the row: free of
 // bank conflicts in both directions. The block is the calling warp's own. `row_ptr(r)`: where row r of the 32 starts in this column
 // group, null for a row that does not exist.
-constexpr int kEpiRowsBytes = 4096;                    // 32 rows of 128 bytes
-constexpr int kEpiWarpBytes = 6144;                    // ... and of a warp in all: three blocks of 32 rows of 64 bytes (gemm_epilogue_beside)
+constexpr int kEpiWarpBytes = 6144;                    // a warp's: 32 rows of 128 bytes, or three blocks of 32 rows of 64 bytes (gemm_epilogue_beside)
 constexpr int kEpiBlockBytes = 4 * kEpiWarpBytes;
 template <int PIECES>
 MACO_DEVICE uint32_t epi_piece(uint32_t block, uint32_t row, uint32_t piece) {
@@ -551,15 +550,15 @@ MACO_DEVICE bool gemm_epilogue_stepped(int bn, const GemmCtrl& c, uint32_t tmem_
 }
 
 // Tiles with a second tensor beside the result, 16-bit, whole columns, no bias, 16-byte rows: the result times gelu'(aux)
-// (MACO_EPI_GELU_BWD), the result and its GELU (MACO_EPI_GELU_DUAL), the result and its sum with aux (MACO_EPI_RESIDUAL_DUAL). In
-// steps of 16 columns as above; aux comes in by cp.async, whole sectors of eight rows an instruction, up to three groups of 32 columns ahead
+// (MACO_EPI_GELU_BWD), the result and its GELU (MACO_EPI_GELU_DUAL: stand-alone products), the result and its sum with aux
+// (MACO_EPI_RESIDUAL_DUAL: graphs). DUAL: which of the last two a kernel has code for. In steps of 16 columns as above; aux comes in by cp.async, whole sectors of eight rows an instruction, up to three groups of 32 columns ahead
 // without a register held for it. One B200, us, before (32 columns at a time, aux in registers, the operators in one function with 12 local loads per step)
 // / now: linear + add of 8192 x 4096 x 256 180 / 110, 2048 x 4096 x 4096 84 / 66; training stack of four 4096 x 4096 layers 2788 / 2595.
-MACO_DEVICE bool epi_is_dual(const GemmEpilogue& e) { return e.mode == MACO_EPI_GELU_DUAL || e.mode == MACO_EPI_RESIDUAL_DUAL; }
+template <int DUAL>
 MACO_DEVICE bool epi_is_beside(const GemmEpilogue& e, int n0, int bn) {
-  const bool res = e.mode == MACO_EPI_RESIDUAL_DUAL;
+  const bool res = DUAL == MACO_EPI_RESIDUAL_DUAL && e.mode == DUAL;
   const uintptr_t p = reinterpret_cast<uintptr_t>(e.aux) | (uintptr_t)(e.ld_aux * 2) | (res ? reinterpret_cast<uintptr_t>(e.bias) : 0);
-  return (e.mode == MACO_EPI_GELU_BWD || e.mode == MACO_EPI_GELU_DUAL || res) && (res || e.bias == nullptr) && n0 + bn <= e.N &&
+  return (e.mode == MACO_EPI_GELU_BWD || e.mode == DUAL) && (res || e.bias == nullptr) && n0 + bn <= e.N &&
          e.out_type != MACO_DT_F32 && (p & 15) == 0;
 }
 template <int SBN, int MODE>
@@ -659,18 +658,16 @@ __device__ __noinline__ bool gemm_epilogue_beside_as(int bn, const GemmCtrl& c, 
 }
 
 // (a function per operator: together they keep more values than a callee of the persistent kernel has registers for)
-template <int SBN>
+template <int SBN, int DUAL>
 MACO_DEVICE bool gemm_epilogue_beside(int bn, const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e, void* out_base, long long row_off,
                                       int m0, int n0, uint32_t tile_seq, uint64_t budget_ns, uint32_t pair_empty_bar, uint8_t* block) {
   if (e.mode == MACO_EPI_GELU_BWD)
     return gemm_epilogue_beside_as<SBN, MACO_EPI_GELU_BWD>(bn, c, tmem_base, e, out_base, row_off, m0, n0, tile_seq, budget_ns, pair_empty_bar, block);
-  if (e.mode == MACO_EPI_GELU_DUAL)
-    return gemm_epilogue_beside_as<SBN, MACO_EPI_GELU_DUAL>(bn, c, tmem_base, e, out_base, row_off, m0, n0, tile_seq, budget_ns, pair_empty_bar, block);
-  return gemm_epilogue_beside_as<SBN, MACO_EPI_RESIDUAL_DUAL>(bn, c, tmem_base, e, out_base, row_off, m0, n0, tile_seq, budget_ns, pair_empty_bar, block);
+  return gemm_epilogue_beside_as<SBN, DUAL>(bn, c, tmem_base, e, out_base, row_off, m0, n0, tile_seq, budget_ns, pair_empty_bar, block);
 }
 
-// (DUAL: with the two modes that write a second tensor, for tiles of such a product that are ragged or not aligned)
-template <int BN, int SBN, bool DUAL>
+// (DUAL: with this mode that writes a second tensor, or 0, for tiles of such a product that are ragged or not aligned)
+template <int BN, int SBN, int DUAL>
 MACO_DEVICE bool gemm_epilogue_tile(const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e_in,
                                     void* out_base, long long row_off, int m0, int n0,
                                     uint32_t tile_seq, uint64_t budget_ns, const EpiBroadcast* bc = nullptr,
@@ -766,7 +763,7 @@ MACO_DEVICE bool gemm_epilogue_tile(const GemmCtrl& c, uint32_t tmem_base, const
           v[j] = f.x * row_weight; v[j + 1] = f.y * row_weight;
         }
       }
-      if (e.bias != nullptr && e.mode != MACO_EPI_SPLITK_FUSED && !(DUAL && e.mode == MACO_EPI_RESIDUAL_DUAL)) {     // (those keep counters / an output there)
+      if (e.bias != nullptr && e.mode != MACO_EPI_SPLITK_FUSED && !(DUAL == MACO_EPI_RESIDUAL_DUAL && e.mode == DUAL)) {     // (those keep counters / an output there)
 #pragma unroll
         for (int j = 0; j < 32; ++j) if (j < valid) v[j] += epi_bias(e, col0 + j);
       }
@@ -788,14 +785,14 @@ MACO_DEVICE bool gemm_epilogue_tile(const GemmCtrl& c, uint32_t tmem_base, const
 #pragma unroll
           for (int j = 0; j < 32; ++j) v[j] *= gelu_tanh_grad(ax[j]);
         }
-      } else if (DUAL && e.mode == MACO_EPI_RESIDUAL_DUAL) {
+      } else if (DUAL == MACO_EPI_RESIDUAL_DUAL && e.mode == DUAL) {
         uint16_t* sum = reinterpret_cast<uint16_t*>(const_cast<void*>(e.bias)) + out_row * e.ld_out + col0;
         for (int j = 0; j < valid; ++j) {
           const uint32_t z = epi_pack(e.out_type, v[j], 0.f);
           const float f = e.out_type == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&z)).x : unpack_bf16x2(z).x;
           sum[j] = (uint16_t)(epi_pack(e.out_type, f + epi_load_aux(e, row, col0 + j), 0.f) & 0xffffu);
         }
-      } else if (DUAL && e.mode == MACO_EPI_GELU_DUAL) {
+      } else if (DUAL == MACO_EPI_GELU_DUAL && e.mode == DUAL) {
         uint16_t* act = reinterpret_cast<uint16_t*>(const_cast<void*>(e.aux)) + row * e.ld_aux + col0;
 #pragma unroll
         for (int j = 0; j < 32; ++j) {
@@ -1118,12 +1115,12 @@ gemm_tcgen05_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_c
         if (lane == 0) mbar_arrive_cluster(tempty_leader + (seq & 1) * 8);
         continue;
       }
-      if (BESIDE && epi_is_beside(epi, nb * BN, BN))
-        ok = gemm_epilogue_beside<256>(BN, c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns, tempty_leader, block);
+      if (BESIDE && epi_is_beside<MACO_EPI_GELU_DUAL>(epi, nb * BN, BN))
+        ok = gemm_epilogue_beside<256, MACO_EPI_GELU_DUAL>(BN, c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns, tempty_leader, block);
       else if (!BESIDE && epi_is_stepped(epi, nb * BN, BN))
         ok = gemm_epilogue_stepped<256>(BN, c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns, tempty_leader, block);
       else
-        ok = gemm_epilogue_tile<BN, 256, BESIDE>(c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns,
+        ok = gemm_epilogue_tile<BN, 256, BESIDE ? MACO_EPI_GELU_DUAL : 0>(c, tmem_base, epi, epi.out, 0, (mp * 2 + (int)rank) * kBM, nb * BN, seq, budget_ns,
                                                  nullptr, nullptr, tempty_leader);
     }
   }
@@ -1187,12 +1184,12 @@ gemm_tcgen05_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_consta
         mbar_arrive(&c.tmem_empty[seq & 1]);
         continue;
       }
-      if (BESIDE && epi_is_beside(epi, nb * BN, BN))
-        ok = gemm_epilogue_beside<BN>(BN, c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns, 0, block);
+      if (BESIDE && epi_is_beside<MACO_EPI_GELU_DUAL>(epi, nb * BN, BN))
+        ok = gemm_epilogue_beside<BN, MACO_EPI_GELU_DUAL>(BN, c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns, 0, block);
       else if (!BESIDE && epi_is_stepped(epi, nb * BN, BN))
         ok = gemm_epilogue_stepped<BN>(BN, c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns, 0, block);
       else
-        ok = gemm_epilogue_tile<BN, BN, BESIDE>(c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns);
+        ok = gemm_epilogue_tile<BN, BN, BESIDE ? MACO_EPI_GELU_DUAL : 0>(c, tmem_base, epi, epi.out, 0, mb * kBM, nb * BN, seq, budget_ns);
     }
   }
   gemm_cta_teardown<BN>(c, tmem_base, status);

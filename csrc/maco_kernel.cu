@@ -568,8 +568,8 @@ __device__ __noinline__ bool run_topk(const MacoProgram& p, const MacoEltArgs& a
 }
 
 // The epilogue of a tile that is not a lean one (gemm_epilogue_lean), out of line. DUAL: ragged tiles with a second output, apart from the
-// others, whose spills those two modes triple (two-CTA form: 244 / 768 bytes stored / loaded without them, 760 / 1444 with them).
-template <bool DUAL>
+// others, whose spills that mode triples (two-CTA form: 244 / 768 bytes stored / loaded without it, 760 / 1444 with it).
+template <int DUAL>
 __device__ __noinline__ bool run_epilogue(const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e, void* out_base, const MacoGemmArgs& g,
                                           uint32_t seq, uint64_t budget_ns, const EpiBroadcast* bc, uint8_t* stage, uint32_t pair_empty_bar,
                                           int row_limit) {
@@ -694,16 +694,16 @@ __device__ void general_role(const MacoProgram& p, uint32_t w, uint32_t q_base, 
       uint8_t* stage = g.peer != -1 ? scratch_smem : nullptr;  // tiles that leave the GPU go through the bulk engine
       // run-time row count of a counted tile's operand block (rows at or beyond it hold no tokens)
       const int row_limit = (d.flags & MACO_TF_COUNTED) ? (int)ld_relaxed_gpu_u32(g.count_ptr) : 0x7fffffff;
-      if (g.peer == -1 && epi_is_beside(e, g.n0, (int)g.bn))
-        ok = gemm_epilogue_beside<kMkBN>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, pair_empty_bar, scratch_smem);
+      if (g.peer == -1 && epi_is_beside<MACO_EPI_RESIDUAL_DUAL>(e, g.n0, (int)g.bn))
+        ok = gemm_epilogue_beside<kMkBN, MACO_EPI_RESIDUAL_DUAL>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, pair_empty_bar, scratch_smem);
       else if (g.peer == -1 && epi_is_lean(e, g.n0, (int)g.bn))
         ok = gemm_epilogue_lean<kMkBN>((int)g.bn, c, tmem_base, e, out_base, g.row_off, g.m0, g.n0, seq, p.budget_ns, pair_empty_bar, row_limit);
       else if (g.peer == -1 && epi_is_stepped(e, g.n0, (int)g.bn))
         ok = run_epilogue_stepped(c, tmem_base, e, out_base, g, seq, p.budget_ns, pair_empty_bar, scratch_smem);
-      else if (epi_is_dual(e))
-        ok = run_epilogue<true>(c, tmem_base, e, out_base, g, seq, p.budget_ns, bcp, stage, pair_empty_bar, row_limit);
+      else if (e.mode == MACO_EPI_RESIDUAL_DUAL)
+        ok = run_epilogue<MACO_EPI_RESIDUAL_DUAL>(c, tmem_base, e, out_base, g, seq, p.budget_ns, bcp, stage, pair_empty_bar, row_limit);
       else
-        ok = run_epilogue<false>(c, tmem_base, e, out_base, g, seq, p.budget_ns, bcp, stage, pair_empty_bar, row_limit);
+        ok = run_epilogue<0>(c, tmem_base, e, out_base, g, seq, p.budget_ns, bcp, stage, pair_empty_bar, row_limit);
       if (!ok) cur[2] = 1;
       ++seq;
       if (e.mode == MACO_EPI_SPLITK_FUSED) {
