@@ -81,3 +81,41 @@ def test_graph_tiles_that_end_early(dtype, N, M):
     y.output.fill_(7.0)
     graph.execute()
     _close(y.output, z, dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N", [16, 32, 144, 272, 40, 264])           # whole steps of 16 columns, and not
+@pytest.mark.parametrize("M", [1, 129, 640])
+def test_bias_on_tiles_that_end_early(dtype, N, M):
+    import maco_b200 as maco
+    from maco_b200 import ops
+    x, w, g, z = _operands(M, N, 320, dtype, N)
+    bias = torch.randn(N, device="cuda", generator=g)
+    for b in (bias, bias.to(dtype)):
+        _close(ops.gemm(x, w, bias=b), z + b.double(), dtype)
+    graph = maco.TaskGraph()
+    y = graph.linear(x, w, bias=bias.to(dtype))
+    graph.compile()
+    y.output.fill_(7.0)
+    graph.execute()
+    _close(y.output, z + bias.to(dtype).double(), dtype)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N", [264, 520, 1032])
+@pytest.mark.parametrize("act", [None, "gelu", "silu"])
+def test_both_epilogues_of_one_product_agree(dtype, N, act):
+    """The last 8 columns, a tile of their own, go through the general epilogue, the others through the one in steps: equal weight rows, biases
+    and scales of 1 to 100 give equal bits."""
+    import maco_b200 as maco
+    from maco_b200 import ops
+    x, w, g, _ = _operands(300, 8, 320, dtype, N)
+    w, x = w.repeat(N // 8, 1), (x * torch.logspace(0, 2, 300, device="cuda")[:, None]).to(dtype)
+    bias = torch.randn(8, device="cuda", generator=g).to(dtype).repeat(N // 8)
+    graph = maco.TaskGraph()
+    y = graph.linear(x, w, bias=bias, activation=act) if act else graph.linear(x, w, bias=bias)
+    graph.compile()
+    graph.execute()
+    for out in (y.output, ops.gemm(x, w, bias=bias, epilogue=act)):
+        cols = out.view(300, N // 8, 8)
+        assert torch.equal(cols, cols[:, -1:].expand_as(cols))

@@ -94,6 +94,52 @@ def _general(monkeypatch, module):
     monkeypatch.setattr(module, "_quick", lambda *a: None)
 
 
+def _taken(name, args, out=None):
+    """The C call itself: it takes the call, and writes where it is told to."""
+    if _build.build_fastcall() is None:
+        pytest.skip("no compiler or no Python header")
+    res = N.fastcall(name)(*args)
+    assert type(res) is torch.Tensor and (out is None or res is out)
+    return res
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
+@pytest.mark.parametrize("shape", [(1,), (4, 512), (3, 7, 33)])
+def test_ordinary_calls_are_taken(monkeypatch, dtype, shape):
+    x, y = (torch.randn(*shape, device="cuda").to(dtype) for _ in range(2))
+    w, b = (torch.randn(shape[-1], device="cuda").to(dtype) for _ in range(2))
+    calls = [(E.T_GELU, x, None, None, 0.0, 0.0, lambda: ops.gelu(x)), (E.T_SOFTMAX, x, None, None, 0.0, 0.0, lambda: ops.softmax(x)),
+             (E.T_ADD, x, y, None, 0.0, 0.0, lambda: ops.add(x, y)), (E.T_AXPBY, x, y, None, 2, -1.5, lambda: ops.axpby(x, y, 2, -1.5)),
+             (E.T_RMSNORM, x, w, None, 1e-6, 0.0, lambda: ops.rmsnorm(x, w)), (E.T_LAYERNORM, x, w, b, 1e-5, 0.0, lambda: ops.layernorm(x, w, b)),
+             (E.T_GELU, torch.nn.Parameter(x, requires_grad=False), None, None, 0.0, 0.0, lambda: ops.gelu(x))]
+    got = []
+    for kind, a, in1, in2, f0, f1, _ in calls:
+        out = torch.empty(shape, device="cuda", dtype=dtype)
+        _taken("elementwise", (kind, a, in1, in2, out, f0, f1), out)
+        got.append((out, _taken("elementwise", (kind, a, in1, in2, None, f0, f1))))
+    _general(monkeypatch, E)
+    for (out, new), call in zip(got, calls):
+        want = call[-1]()
+        assert torch.equal(out, want) and torch.equal(new, want)
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("form", ["plain", "view", "one_head_view", "scale", "more_batch"])
+def test_ordinary_attention_is_taken(monkeypatch, dtype, form):
+    B, H, G, S = (3, 1, 4, 300) if form == "one_head_view" else (3, 2, 4, 300)
+    q = torch.randn(B, H * G, 128, device="cuda").to(dtype)
+    k, v = (torch.randn(B + (form == "more_batch"), H, S + 77 * (form != "plain"), 128, device="cuda").to(dtype)[:, :, :S] for _ in range(2))
+    scale, out = (0.05 if form == "scale" else 128 ** -0.5), torch.empty_like(q)
+    A._lib()
+    _taken("attention", (q, k, v, out, scale), out)
+    new = _taken("attention", (q, k, v, None, scale))
+    _general(monkeypatch, A)
+    want = ops.attention_decode(q, k, v, scale=scale)
+    assert torch.equal(out, want) and torch.equal(new, want)
+
+
 @pytest.mark.gpu
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16, torch.float32])
 @pytest.mark.parametrize("shape", [(1,), (5,), (4, 512), (3, 7, 33), (2, 0, 8), ()])

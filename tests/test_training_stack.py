@@ -36,3 +36,21 @@ def test_gradients_on_both_kinds_of_tiles(layers, hidden, tokens, cta_pair):
         assert (g - r).abs().max().item() < 3e-2 * r.abs().max().item() + 1e-7
     assert torch.equal(outs[0], outs[1]) and torch.equal(outs[0], outs[2])
     assert _native.status() == 0
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("layers,hidden,tokens", [(2, 256, 128), (3, 768, 384), (2, 2048, 2048), (2, 2048, 2176)])     # 2^22 activations, and more
+def test_forward_in_one_launch_a_layer_or_two(layers, hidden, tokens, dtype):
+    """Pre-activations and activations of both forms of the forward are those of the product and its GELU one behind the other, bit by bit."""
+    from maco_b200 import ops
+    from maco_b200.models.dp_mlp_stack import DPMLPStackBackward
+    m = DPMLPStackBackward(layers=layers, hidden=hidden, tokens=tokens, seed=2, weight_std=0.05, dtype=dtype)
+    for t in m.z + m.a:
+        t.fill_(float("nan"))
+    last, cur = m.forward(), m.x
+    for l in range(layers):
+        z = ops.gemm(cur, m.weights[l])
+        cur = ops.gelu(z)
+        assert torch.equal(m.z[l], z) and torch.equal(m.a[l], cur)
+    assert last is m.a[-1]
