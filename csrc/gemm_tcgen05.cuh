@@ -787,10 +787,13 @@ MACO_DEVICE bool gemm_epilogue_tile(const GemmCtrl& c, uint32_t tmem_base, const
         }
       } else if (DUAL == MACO_EPI_RESIDUAL_DUAL && e.mode == DUAL) {
         uint16_t* sum = reinterpret_cast<uint16_t*>(const_cast<void*>(e.bias)) + out_row * e.ld_out + col0;
-        for (int j = 0; j < valid; ++j) {
+        float ax[32];
+        epi_load_aux32(e, row, col0, valid, ax);
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
           const uint32_t z = epi_pack(e.out_type, v[j], 0.f);
           const float f = e.out_type == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&z)).x : unpack_bf16x2(z).x;
-          sum[j] = (uint16_t)(epi_pack(e.out_type, f + epi_load_aux(e, row, col0 + j), 0.f) & 0xffffu);
+          if (j < valid) sum[j] = (uint16_t)(epi_pack(e.out_type, f + ax[j], 0.f) & 0xffffu);
         }
       } else if (DUAL == MACO_EPI_GELU_DUAL && e.mode == DUAL) {
         uint16_t* act = reinterpret_cast<uint16_t*>(const_cast<void*>(e.aux)) + row * e.ld_aux + col0;

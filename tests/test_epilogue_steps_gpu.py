@@ -119,3 +119,22 @@ def test_both_epilogues_of_one_product_agree(dtype, N, act):
     for out in (y.output, ops.gemm(x, w, bias=bias, epilogue=act)):
         cols = out.view(300, N // 8, 8)
         assert torch.equal(cols, cols[:, -1:].expand_as(cols))
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("N", [8, 200, 264, 640])                    # last column chunks of 8 columns and whole ones
+@pytest.mark.parametrize("pair", [False, True])
+@pytest.mark.parametrize("offset", [0, 1])                           # rows beside the product aligned to 16 bytes, and not
+def test_residual_beside_ragged_tiles(dtype, N, pair, offset):
+    from maco_b200.ops import megakernel as mk
+    M = 300
+    x, w, g, z = _operands(M, N, 320, dtype, N)
+    aux = torch.randn(M, N + 8, device="cuda", generator=g).to(dtype)[:, offset:offset + N]
+    out, both = (torch.full((M + 1, N), 7.0, device="cuda", dtype=dtype) for _ in range(2))
+    b = mk.ProgramBuilder(torch.device("cuda"), cta_pair=pair)
+    b.gemm(x, w, out[:M], epilogue="residual_dual", aux=aux, second=both[:M])
+    b.build().run()
+    torch.cuda.synchronize()
+    _close(out[:M], z, dtype)
+    assert torch.equal(both[:M], (out[:M].float() + aux.float()).to(dtype))      # the sum of two rounded values, rounded once
+    assert (out[M:] == 7).all() and (both[M:] == 7).all()
