@@ -73,9 +73,15 @@ def _compile_one(src: Path, verbose: bool) -> Path:
 
 def fastcall_path() -> Path:
     """Where the C extension of this source and this interpreter lies. Both are part of the name: CPython loads an untagged extension that
-    another minor version built without a word, and runs it with that version's inlined reference counts and tuple layout."""
+    another minor version built without a word, and runs it with that version's inlined reference counts and tuple layout. Where the package
+    lies without its source, the build that came with it."""
+    suffix = sysconfig.get_config_var("EXT_SUFFIX")
+    if not FASTCALL_SRC.exists():
+        came = sorted(LIB_DIR.glob(f"maco_fastcall-*{suffix}"))
+        if len(came) == 1:
+            return came[0]
     digest = hashlib.sha256(FASTCALL_SRC.read_bytes()).hexdigest()[:12]
-    return LIB_DIR / f"maco_fastcall-{digest}{sysconfig.get_config_var('EXT_SUFFIX')}"
+    return LIB_DIR / f"maco_fastcall-{digest}{suffix}"
 
 
 def build_fastcall(force: bool = False) -> "Path | None":

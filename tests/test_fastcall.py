@@ -79,6 +79,15 @@ def test_only_this_sources_and_interpreters_build_is_loaded(empty_build, monkeyp
     assert second != first and second.exists() and not first.exists() and b"elementwise: 7 arguments" in second.read_bytes()
 
 
+def test_the_package_without_its_sources(empty_build, monkeypatch):
+    built = _loaded_from()
+    (empty_build / "maco_fastcall-0123456789ab.cpython-37m-x86_64-linux-gnu.so").write_bytes(b"another interpreter's")
+    monkeypatch.setattr(_build, "FASTCALL_SRC", empty_build / "fastcall.c")
+    assert _loaded_from() == built
+    built.unlink()
+    assert _loaded_from() is None
+
+
 def test_nothing_is_built_where_that_is_switched_off(empty_build, monkeypatch):
     monkeypatch.setenv("MACO_NO_AUTOBUILD", "1")
     assert _loaded_from() is None and not list(empty_build.iterdir())
