@@ -97,7 +97,8 @@ attn_stream_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
   const int tid = threadIdx.x, warp = warp_uniform(tid >> 5);
   bool ok = true;
   for (long long pos = begin; pos < end && ok;) {
-    const int group = p.total < (1ll << 24) ? (int)((uint32_t)pos / (uint32_t)p.chunks_per_head) : (int)(pos / p.chunks_per_head), c0 = (int)(pos - (long long)group * p.chunks_per_head);
+    const int group = p.total < (1ll << 24) ? (int)((uint32_t)pos / (uint32_t)p.chunks_per_head) : (int)(pos / p.chunks_per_head);
+    const int c0 = (int)(pos - (long long)group * p.chunks_per_head);
     const int n = (int)min((long long)(p.chunks_per_head - c0), end - pos);
     const int key0 = c0 * 128, rows = min(p.S - key0, n * 128);
     if (warp == 4) {
@@ -131,7 +132,7 @@ attn_stream_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constan
 }
 
 // ONE_HEAD: a CTA per head. With all G heads of a group in one CTA a thread has registers for two records, and the twelve records of a cache
-// of 1357 keys in 128-key shares were six round trips to L2 in a row (16.4 us for the call, 13.9 with a CTA per head). Where a group has two or three
+// of 1357 keys in 128-key shares were six round trips to L2 in a row (16.2 us for the call, 13.7 with a CTA per head and the call in C). Where a group has two or three
 // records there is nothing to gain, and G times the CTAs cost (16 x 8 kv heads x 8192 keys 88.2 us, 89.3 with a CTA per head): see launch_stream.
 constexpr int kMergeAhead = 8;
 template <int DTT, bool ONE_HEAD>

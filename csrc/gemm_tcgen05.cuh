@@ -468,7 +468,8 @@ MACO_DEVICE void epi_flush_rows(uint32_t block, uint32_t lane, RowFn row_ptr) {
 }
 MACO_DEVICE float2 epi_unpack(int type, uint32_t w) { return type == MACO_DT_F16 ? __half22float2(*reinterpret_cast<const __half2*>(&w)) : unpack_bf16x2(w); }
 
-// Whole columns into this GPU's memory: fp32 rows, and 16-bit ones with a bias, GELU or SiLU. Same arithmetic as gemm_epilogue_tile below,
+// Whole columns into this GPU's memory: fp32 rows, and 16-bit ones with a bias, GELU or SiLU; and plain 16-bit tiles, with or without a bias,
+// that end early at a whole step. Same results as gemm_epilogue_tile below (SiLU by silu_16: other steps, the same 16-bit values),
 // in steps of 16 columns so that nothing lives in local memory: the persistent kernel leaves its L1 28 KB, a spilled value of the
 // column loop is a miss to L2 two times in three, and one warp per scheduler has nothing to cover it with (32 columns at a time,
 // with GELU: 20 local loads per 32 columns). fp32 rows go through `block`; 16-bit rows do not (a short chain per step counts for more there: through
@@ -1048,7 +1049,7 @@ MACO_DEVICE void pair_cta_teardown(const GemmCtrl& c, uint32_t tmem_base, uint32
 constexpr int kPairStages = 6;
 
 // Stand-alone GEMM on two-CTA tiles: grid = 2 x (number of CTA pairs), launched as clusters of two. BESIDE: with the out-of-line epilogue of
-// tiles that have a second tensor. It takes the kernel's parameters by reference, which puts them on the stack (256 bytes) and costs 20
+// tiles that have a second tensor. It takes the kernel's parameters by reference, which puts them on the stack (120 bytes) and costs some
 // registers, so that products without such a tensor have instances of their own. With it / without, one B200, us: 512 x 2048 x 2048 plain
 // 24.2 / 20.5, 4096^3 plain 119 / 112, with GELU 173 / 147, 8192 x 4096 x 4096 plain 201 / 190, with GELU 288 / 242.
 template <int BN, bool A_MN, bool B_MN, bool BESIDE>

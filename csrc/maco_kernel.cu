@@ -568,7 +568,7 @@ __device__ __noinline__ bool run_topk(const MacoProgram& p, const MacoEltArgs& a
 }
 
 // The epilogue of a tile that is not a lean one (gemm_epilogue_lean), out of line. DUAL: ragged tiles with a second output, apart from the
-// others, whose spills that mode triples (two-CTA form: 244 / 768 bytes stored / loaded without it, 760 / 1444 with it).
+// others, whose spills such modes tripled (two-CTA form: 244 / 768 bytes stored / loaded without them, 760 / 1444 with them).
 template <int DUAL>
 __device__ __noinline__ bool run_epilogue(const GemmCtrl& c, uint32_t tmem_base, const GemmEpilogue& e, void* out_base, const MacoGemmArgs& g,
                                           uint32_t seq, uint64_t budget_ns, const EpiBroadcast* bc, uint8_t* stage, uint32_t pair_empty_bar,

@@ -36,9 +36,10 @@ class DPMLPStackBackward:
                  cta_pair: Optional[bool] = None):
         # ``cta_pair``: two-CTA tiles (True) or one-CTA ones (False) whatever the size. None: two-CTA tiles on one GPU where both GEMM kinds
         # have about one 256 x 256 tile per worker or more (two per pair: below that the last wave costs more than the smaller operand
-        # traffic gains). Backward pass, one- / two-CTA, one B200: 4 layers of 4096 x 8192 tokens 1518 / 1444 us, 2 of 3072 x 6144 309 / 286.
-        # (Below the line two-CTA tiles have since become the faster form down to about 2048 x 1024: 4 layers of 2304 x 2304 235 / 222, 3 of
-        # 1024 x 8192 173 / 171, but 3 of 1536 x 1536 94 / 97; ask for them there.) (More ranks: not measured, one-CTA.)
+        # traffic gains). Backward pass, one- / two-CTA, one B200: 4 layers of 4096 x 8192 tokens 1531 / 1420 us, 2 of 3072 x 6144 309 / 288.
+        # (The line is from slower issue loops. Below it two-CTA tiles are now the faster form down to about 2048 x 1024: 4 layers of 2304 x 2304
+        # 235 / 222, 3 of 1024 x 8192 173 / 170, 3 of 2048 x 1024 105 / 101, but 3 of 1536 x 1536 94 / 96 and of 512 x 2048 73 / 75; ask for them
+        # there.) (More ranks: not measured, one-CTA.)
         if cta_pair is None:
             sms = torch.cuda.get_device_properties(device if device is not None else torch.cuda.current_device()).multi_processor_count \
                 if torch.cuda.is_available() and (device is None or torch.device(device).type == "cuda") else 148
@@ -78,9 +79,11 @@ class DPMLPStackBackward:
     # ------------------------------------------------------------------ forward (set-up, separate launches)
     def forward(self) -> torch.Tensor:
         cur = self.x
-        # Up to 4 Mi activations the product with the GELU in its epilogue, one launch a layer instead of two. 3 layers, one B200, us, as product and
-        # GELU / in one: 256 x 512 68 / 46, 8192 x 512 56.2 / 55.9, 300 x 4096 127 / 118. Beyond that the launches no longer count and which is faster
-        # goes with the last round of tiles and the power cap: 4096 x 2048 117 / 111, 2304 x 2304 130 / 136, 8192 x 3072 457 / 414, 8192 x 4096 651 / 690.
+        # Up to 4 Mi activations the product with the GELU in its epilogue, one launch a layer instead of two. 3 layers of tokens x hidden, one B200, us,
+        # as product and GELU / in one: 256 x 512 46 / 37, 1024 x 1024 47 / 38, 8192 x 512 57 / 56, 4096 x 1024 68 / 62, 1024 x 4096 126 / 119, 2048 x
+        # 2048 87 / 81. Beyond that the launches no longer count and which is faster goes with the last round of tiles and the power cap: 4096 x 2048
+        # 118 / 112, 8192 x 3072 465 / 424, 4096 x 4096 371 / 360, but 2304 x 2304 141 / 142, 8192 x 2048 197 / 205; 8192 x 4096 684 / 646 in one run and
+        # 651 / 690 in another.
         fused = self.tokens * self.hidden <= 1 << 22
         for l in range(self.layers):
             if fused:

@@ -347,9 +347,9 @@ def simulate_static_queues(programs: Sequence[Tuple[Sequence[dict], List[List[in
 
 
 def default_task_cost(t: dict) -> float:
-    """Rough duration of a task in microseconds for ``estimate_makespan``, from figures measured on B200 with this
-    kernel: a 128 x 256 x 64 k-block of a GEMM tile 0.45 us (a pair half the same: two CTAs, twice the rows) plus 2 us
-    per tile; a 128-wide k-step of a few-row part (32 KB of weights) 1 us plus 2 us per part; a bulk push 43 us per MB; a staged reduction
+    """Rough duration of a task in microseconds for ``estimate_makespan``, from figures measured on B200: a 128 x 256 x 64
+    k-block of a GEMM tile 0.45 us (a pair half the same: two CTAs, twice the rows; with the issue loops as they are it is 0.20 to 0.26, so that
+    spans of GEMM-bound launches come out long, and the share of everything else short) plus 2 us per tile; a 128-wide k-step of a few-row part (32 KB of weights) 1 us plus 2 us per part; a bulk push 43 us per MB; a staged reduction
     0.06 us per KB of sources; what the builder knows better (``cost_us``: a worker's share of an expert layer, by its tiles under even
     routing); everything else 5 us. Callers with better numbers for their shapes pass their own function."""
     if t.get("cost_us") is not None:
@@ -1607,8 +1607,8 @@ def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None)
     gemm_nodes = [n for n in graph._nodes if n.task_type in (TaskType.LINEAR, TaskType.MATMUL) and n.outputs and n.outputs[0].numel()]
     def _waves(n: TaskNode, pair: bool) -> float:
         """Rounds of tiles times their length, in k-blocks of 128 columns (``ProgramBuilder.gemm`` takes 128-column tiles where 256 leave
-        workers idle). A two-CTA tile of 256 columns takes about 5 % less than two one-CTA ones; one of 128 columns, or with a bias or an
-        activation in its epilogue, about 5 % more."""
+        workers idle). A two-CTA tile of 256 columns is counted 5 % below two one-CTA ones, one of 128 columns, or with a bias or an activation
+        in its epilogue, 5 % above: what they took while a k-block's issue was the longer part (see below)."""
         x2, w = _flat2d(n.inputs[0]), n.inputs[1]
         rows, (cols, k) = x2.shape[0], (w.shape if n.task_type == TaskType.LINEAR else w.shape[::-1])
         bn = 256 if n.attrs.get("activation") == "swiglu" or -(-rows // BM) * -(-cols // 256) >= workers else 128
@@ -1619,11 +1619,12 @@ def lower_graph(graph, mode: Optional[str] = None, trace: Optional[bool] = None)
         return -(-tiles // (workers // 2)) * length * (0.95 if bn == 256 and (n.task_type == TaskType.MATMUL or _plain_linear(n)) else 1.05)
 
     # Two-CTA tiles where they take less time by that count and the products are long: a third less operand traffic per flop.
-    # Two- / one-CTA, one B200, us: MLP blocks of rows x hidden x ffn 1003 x 2048 x 8192 109 / 119, 300 x 4096 x 8192 107 / 118, 640 x 2048 x
-    # 4096 64 / 63, with hidden of 1024 the two halves of a tile wait for each other's epilogue (2048 x 1024 x 2816 76.5 / 73.4);
-    # single products of rows x N x K, all in tiles of 128 columns, 200 x 8192 x 2048 25 / 24, 640 x 4096 x 2048 35 / 33, 2000 x 1024 x 4096 37 / 34
-    # (a K of 8192 at 200 or 300 rows gains 3 % and is not told apart), 1000 x 4096 x 4096 with a bias 73 / 68. Every graph keeps the older
-    # rule too, where tiles of 256 x 256 outputs cover every pair (4000 x 4096 x 4096 104 / 116); few-row nodes keep it on one-CTA tiles.
+    # Two- / one-CTA, one B200, us: MLP blocks of rows x hidden x ffn 1003 x 2048 x 8192 109 / 131, 300 x 4096 x 8192 108 / 132, 640 x 2048 x
+    # 4096 70 / 72, with hidden of 1024 the two halves of a tile wait for each other's epilogue (2048 x 1024 x 2816 68 / 68). Every graph
+    # keeps the older rule too, where tiles of 256 x 256 outputs cover every pair (4000 x 4096 x 4096 102 / 113); few-row nodes keep it on
+    # one-CTA tiles. Single products of rows x N x K in tiles of 128 columns, which the weights leave on one-CTA tiles: as fast with a K of
+    # 2048 (200 x 8192 x 2048 20.7 / 20.8, 640 x 4096 x 2048 28.9 / 29.0), but slower there with a longer one (2000 x 1024 x 4096 26.5 / 28.9, 1000 x
+    # 4096 x 4096 39 / 45 and with a bias 41 / 48, 200 x 8192 x 8192 49 / 59): the weights would have to be set anew for the loops as they are.
     cta_pair = mode == "static" and workers >= 4 and bool(gemm_nodes) and not any(_few_rows(n) for n in gemm_nodes)
     if cta_pair:
         long = all(_flat2d(n.inputs[0]).shape[0] > BM and _flat2d(n.inputs[0]).shape[1] >= 1536 for n in gemm_nodes)
